@@ -1,6 +1,7 @@
 // The C ABI: argument validation, handle lifetime, launch sequencing.
 // No entry point below allocates after shrike_moe_create / shrike_pool_create /
 // shrike_residency_create.
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -123,17 +124,8 @@ bool router_operands_aligned(const shrike_moe_config& c, const shrike_router_ope
 
 namespace {
 
-template <typename P>
-cudaError_t dev_alloc(P** p, size_t bytes) {
-    return cudaMalloc((void**)p, bytes ? bytes : 16);
-}
-
 void free_workspace(Workspace& w) {
-    void* ptrs[] = {w.fused_logits, w.fused_acts, w.fused_epoch, w.yacc, w.xs, w.chunk_inst, w.n_chunk_inst, w.done_counter, w.xsum, w.logits, w.xh, w.acts, w.acts_shared, w.sorted, w.inst, w.n_inst, w.status, w.block_hist,
-                    w.expert_offsets, w.expert_counts, w.slot_of_expert, w.x_dev, w.y_dev,
-                    w.ids_dev, w.w_dev, w.gate_dev, w.slots_dev, w.counts_dev};
-    for (void* p : ptrs)
-        if (p) cudaFree(p);
+    if (w.slab) cudaFree(w.slab);
     free(w.tensor_maps);
     free(w.fused_geom);
     free(w.fused_maps);
@@ -172,6 +164,20 @@ int fill_expert_args(shrike_moe* m, const shrike_pool* pool, const shrike_expert
     return SHRIKE_OK;
 }
 
+
+// The expert projections of a decode call's work lists (phases: 1, 2 or 3 = both). From 9 rows on the streaming kernel
+// takes every shape whose tiles its ring and the tiled copies can hold. The per-tile kernels take the others, and the
+// calls of fewer rows: they lay no operands out ahead of the first tile (layer call, 8 rows of the 256-expert shape:
+// 63.5 us against 66.6; 12 rows: 86.5 against 82.4).
+cudaError_t launch_experts(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, uint32_t T, uint32_t phases, void* y,
+                           void* hidden, bool pdl) {
+    const uint32_t n_shared = m->cfg.has_shared ? (T + 7) / 8 : 0;
+    cudaError_t e = T > 8 ? launch_expert_stream(m, st, a, T, n_shared, phases, false, y, hidden, pdl) : cudaErrorNotSupported;
+    if (e != cudaErrorNotSupported) return e;
+    const uint32_t mi = max_instances(m->cfg, T);
+    if ((phases & 1u) && (e = launch_phase1(m, st, a, mi, pdl)) != cudaSuccess) return e;
+    return (phases & 2u) ? launch_phase2(m, st, a, T, mi, y, hidden, pdl) : cudaSuccess;
+}
 
 // The prefill call with the status word of a streamed batch (moe.metal:36-39, 918-921): when io_status is
 // given and the word is neither READY nor 3, the routed experts are skipped and y is the shared term alone.
@@ -270,7 +276,22 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
     w.max_inst = max_instances(c, c.max_tokens);
     const size_t ab = act_bytes(c.act_dtype), yb = act_bytes(c.y_dtype);
     bool ok = true;
-    auto A = [&](auto** p, size_t bytes) { if (ok && dev_alloc(p, bytes) != cudaSuccess) ok = false; };
+    // one device allocation: the parts take their places first (a handle per layer is made at load time, and thirty
+    // calls of the allocator per handle were most of that)
+    struct Part { void** p; size_t at; };
+    std::vector<Part> slab_parts;
+    size_t slab = 0;
+    auto A = [&](auto** p, size_t bytes) {
+        slab_parts.push_back({(void**)p, slab});
+        slab += (bytes + 255) / 256 * 256;
+    };
+    // words that start at zero
+    A(&w.status, 4);
+    A(&w.n_inst, 4);
+    A(&w.done_counter, 4);
+    A(&w.arrived, 4);
+    A(&w.fused_epoch, 4);
+    const size_t zeroed = slab;
     A(&w.logits, T * c.num_experts * 4);
     A(&w.xh, T * c.d * 2);
     A(&w.xsum, T * (c.d / c.group_size) * 4);
@@ -278,9 +299,9 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
     A(&w.acts_shared, c.has_shared ? T * c.shared_f * 2 : 0);
     A(&w.sorted, T * K * 4);
     A(&w.inst, (size_t)w.max_inst * sizeof(Instance));
-    A(&w.n_inst, 4);
-    A(&w.status, 4);
-    A(&w.done_counter, 4);
+    A(&w.inst_done, (size_t)w.max_inst * 4);
+    A(&w.parts, stream_parts_bytes(c));
+    A(&w.pair_cell, std::min(T, (size_t)SHRIKE_MAX_DECODE_TOKENS) * K * 4);
     A(&w.block_hist, ((T + 127) / 128) * c.num_experts * 4);
     A(&w.expert_offsets, c.num_experts * 4);
     A(&w.expert_counts, c.num_experts * 4);
@@ -288,7 +309,7 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
     A(&w.yacc, T > SHRIKE_MAX_DECODE_TOKENS ? T * c.d * 4 : 0);
     A(&w.chunk_inst, T > SHRIKE_MAX_DECODE_TOKENS ? umma_max_chunk_instances(c, c.max_tokens) * umma_chunk_instance_bytes() : 0);
     A(&w.n_chunk_inst, 8);
-    A(&w.xs, T > SHRIKE_MAX_DECODE_TOKENS ? T * K * c.d * 2 : 0);
+    if (T > SHRIKE_MAX_DECODE_TOKENS) A(&w.xs, T * K * c.d * 2);   // prefill operands
     A(&w.x_dev, T * c.d * ab);
     A(&w.y_dev, T * c.d * yb);
     A(&w.ids_dev, T * K * 4);
@@ -299,34 +320,32 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
     // the one-row layer kernel: sizes of its shared-memory ring, and its hand-over buffers
     int smem_optin = 0;
     cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    m->smem_optin = (uint32_t)smem_optin;
     w.fused_geom = malloc(fused_geom_bytes());
     w.fused_maps = calloc(1, fused_map_cache_bytes());
-    if (w.fused_geom && w.fused_maps && fused_geometry(c, m->sm_count, smem_optin, *(FusedGeom*)w.fused_geom)) {
+    if (!w.fused_maps) ok = false;
+    if (w.fused_geom && fused_geometry(c, m->sm_count, smem_optin, *(FusedGeom*)w.fused_geom)) {
         A((uint8_t**)&w.fused_logits, fused_logits_bytes(c));
         A(&w.fused_acts, fused_acts_bytes(c));
-        A(&w.fused_epoch, 4);
     } else {
         free(w.fused_geom);
-        free(w.fused_maps);
         w.fused_geom = nullptr;
-        w.fused_maps = nullptr;
     }
+    if (ok) ok = cudaMalloc(&w.slab, slab) == cudaSuccess;
     if (!ok) {
         free_workspace(w);
         delete m;
         cudaGetLastError();
         return fail(nullptr, SHRIKE_ENOMEM, "device allocation of the workspace failed");
     }
+    for (const Part& p : slab_parts) *p.p = (uint8_t*)w.slab + p.at;
+    cudaMemset(w.slab, 0, zeroed);
     if (w.fused_geom) {
         // no logit carries the first epoch's tag, no activation has been published
         cudaMemset(w.fused_logits, 0xff, fused_logits_bytes(c));
         cudaMemset(w.fused_acts, 0xff, fused_acts_bytes(c));
-        cudaMemset(w.fused_epoch, 0, 4);
     }
-    if (T <= SHRIKE_MAX_DECODE_TOKENS) {   // decode-only handle: no prefill operands
-        cudaFree(w.xs);
-        w.xs = nullptr;
-    } else {
+    if (T > SHRIKE_MAX_DECODE_TOKENS) {
         w.tensor_maps = aligned_alloc(64, umma_tensor_map_bytes());
         const cudaError_t me = w.tensor_maps ? umma_prepare(m) : cudaErrorMemoryAllocation;
         if (me != cudaSuccess) {
@@ -336,9 +355,6 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
             return fail(nullptr, SHRIKE_EIO, "TMA descriptors of the prefill operands: %s", cudaGetErrorString(me));
         }
     }
-    cudaMemset(w.status, 0, 4);
-    cudaMemset(w.done_counter, 0, 4);
-    cudaMemset(w.n_inst, 0, 4);
     *out = m;
     return SHRIKE_OK;
 }
@@ -587,7 +603,7 @@ int shrike_encode_phase1(shrike_moe* m, void* stream, const shrike_pool* pool,
     int rc = fill_expert_args(m, pool, routed_offsets, shared, nullptr, nullptr, a, false);
     if (rc) return rc;
     if ((rc = check_device(m))) return rc;
-    CU(launch_phase1(m, (cudaStream_t)stream, a, max_instances(m->cfg, query_count), false));
+    CU(launch_experts(m, (cudaStream_t)stream, a, query_count, 1u, nullptr, nullptr, false));
     return SHRIKE_OK;
 }
 
@@ -603,7 +619,7 @@ int shrike_encode_phase2_reduce(shrike_moe* m, void* stream, const shrike_pool* 
     int rc = fill_expert_args(m, pool, routed_offsets, shared, routing_weights, shared_gate, a, true);
     if (rc) return rc;
     if ((rc = check_device(m))) return rc;
-    CU(launch_phase2(m, (cudaStream_t)stream, a, query_count, max_instances(m->cfg, query_count), y, hidden, false));
+    CU(launch_experts(m, (cudaStream_t)stream, a, query_count, 2u, y, hidden, false));
     return SHRIKE_OK;
 }
 
@@ -690,10 +706,8 @@ int shrike_encode_decode_layer(shrike_moe* m, void* stream, const shrike_pool* p
     ExpertArgs a;
     rc = fill_expert_args(m, pool, routed_offsets, shared, wt, gate, a);
     if (rc) return rc;
-    const uint32_t mi = max_instances(m->cfg, query_count);
-    // phase 1 and phase 2 may start before their predecessor has drained
-    CU(launch_phase1(m, (cudaStream_t)stream, a, mi, !m->no_pdl));
-    CU(launch_phase2(m, (cudaStream_t)stream, a, query_count, mi, y, hidden, !m->no_pdl));
+    // the expert kernels may start before their predecessor has drained
+    CU(launch_experts(m, (cudaStream_t)stream, a, query_count, 3u, y, hidden, !m->no_pdl));
     return SHRIKE_OK;
 }
 
@@ -878,7 +892,7 @@ int shrike_ep_create(shrike_moe* home, shrike_moe* routed, uint32_t rank, uint32
     ep->lay = ep_layout(c, world, rows_per_call);
     const size_t T = rows_per_call, K = c.top_k;
     bool ok = true;
-    auto A = [&](auto** p, size_t bytes) { if (ok && dev_alloc(p, bytes) != cudaSuccess) ok = false; };
+    auto A = [&](auto** p, size_t bytes) { if (ok && cudaMalloc((void**)p, bytes ? bytes : 16) != cudaSuccess) ok = false; };
     A(&ep->mine, ep->lay.bytes);
     A(&ep->ids, T * K * 4); A(&ep->w, T * K * 4); A(&ep->gate, T * 4); A(&ep->row_of, T * world * 4);
     A(&ep->send_counts, SHRIKE_EP_MAX_WORLD * 4); A(&ep->miss_slots, T * K * 4);

@@ -57,8 +57,10 @@
 
 #include <algorithm>
 
+#include "block_maps.cuh"
 #include "router_math.cuh"
 #include "select.cuh"
+#include "tile_math.cuh"
 
 namespace shrike {
 
@@ -97,14 +99,6 @@ struct FusedGeom {
     uint32_t rcp_blocks, rcp_upe, rcp_slots, rcp_epp, rcp_bps, rcp_gmax2, rcp_cpe_r;
 };
 
-// Tensor maps of one expert block layout: entries 0..7 the pool's chunks, entry 8 the shared expert's block.
-struct FusedMaps {
-    CUtensorMap w1[SHRIKE_MAX_POOL_CHUNKS + 1];   // gate + up rows: (group bytes, rows, groups, 2, cells)
-    CUtensorMap m1[SHRIKE_MAX_POOL_CHUNKS + 1];   // their scales and biases: (8 rows' worth, rows / 8, scale|bias, 2, cells)
-    CUtensorMap w2[SHRIKE_MAX_POOL_CHUNKS + 1];   // down rows: (group bytes, rows, groups, cells)
-    CUtensorMap m2[SHRIKE_MAX_POOL_CHUNKS + 1];   // their scales and biases: (8 rows' worth, rows / 8, scale|bias, cells)
-};
-
 struct FusedArgs {
     PoolView pool;
     Offsets3 routed, shared;
@@ -140,22 +134,10 @@ struct FusedArgs {
 #endif
     uint32_t rcp_cpc;               // ceil(2^32 / cells_per_chunk): cell / cells_per_chunk = mulhi(cell, rcp_cpc)
     FusedGeom g;
-    FusedMaps maps;
+    BlockMaps maps;
 };
 
 namespace {
-
-template <int BITS, int GROUP>
-struct FQ {
-    static constexpr int kWords = GROUP * BITS / 128;   // u32 per thread, row and group
-    static constexpr int kMmas = GROUP / 16;
-    static constexpr int kBRegs = GROUP / 8;
-    static constexpr uint32_t kGroupBytes = GROUP * BITS / 8;
-    // what the tiles multiply is offset + q: 1024 + q for nibbles in bits 0..3 (and for bytes), 64 + q for
-    // nibbles in bits 4..7 (the fp16 value 64 has its unit in the last place at bit 4): no shift to unpack
-    static constexpr float kOffEven = 1024.0f;
-    static constexpr float kOffOdd = BITS == 4 ? 64.0f : 1024.0f;
-};
 
 // One unit of work of a block, as every warp reads it from the block's table (8 bytes).
 //   bits 0     kind: 0 phase 1 (8 gate + 8 up rows of one instance), 1 phase 2 (16 output rows x a pack)
@@ -316,32 +298,6 @@ struct BlockPlan {
     }
 };
 
-template <int BITS>
-__device__ __forceinline__ void unpack2(const uint32_t* w, int m, uint32_t& lo, uint32_t& hi) {
-    if constexpr (BITS == 4) {
-        const uint32_t v = w[m >> 1] >> ((m & 1) * 8);
-        lo = lop3_and_or(v, 0x000F000Fu, 0x64006400u);   // (1024 + n0, 1024 + n4)
-        hi = lop3_and_or(v, 0x00F000F0u, 0x54005400u);   // (64 + n1, 64 + n5)
-    } else {
-        const uint32_t v = w[m];
-        lo = prmt(v, 0x64646464u, 0x5140u);
-        hi = prmt(v, 0x64646464u, 0x5342u);
-    }
-}
-
-template <int W>
-__device__ __forceinline__ void lds_words(const uint8_t* p, uint32_t (&w)[W]) {
-    if constexpr (W == 1) {
-        w[0] = *(const uint32_t*)p;
-    } else if constexpr (W == 2) {
-        const uint2 v = *(const uint2*)p;
-        w[0] = v.x; w[1] = v.y;
-    } else {
-        const uint4 v = *(const uint4*)p;
-        w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-    }
-}
-
 // CG consecutive 16-bit values starting at an address that is a multiple of min(2 * CG, 4) bytes.
 template <int CG, int META>
 __device__ __forceinline__ void lds_meta(const uint8_t* p, float (&out)[CG]) {
@@ -466,20 +422,6 @@ __device__ __noinline__ float2 group_sums(const uint16_t* row, uint32_t grp) {
 #else
 #define FUSED_TS(slot) do { } while (0)
 #endif
-
-// Tiled TMA loads (no multicast): the box lands densely, innermost dimension first.
-__device__ __forceinline__ void tma_4d(uint32_t dst, const CUtensorMap* map, int32_t c0, int32_t c1, int32_t c2, int32_t c3,
-                                       uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tma_5d(uint32_t dst, const CUtensorMap* map, int32_t c0, int32_t c1, int32_t c2, int32_t c3,
-                                       int32_t c4, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(bar)) : "memory");
-}
 
 // Top-k of the logits in shared memory by the first kSelWarps consumer warps, without serial rounds: (score
 // descending, expert id ascending) is a total order, so the number of experts that beat one is its rank.
@@ -1253,7 +1195,7 @@ bool fused_geometry(const shrike_moe_config& c, int sm_count, int max_smem_optin
 // biases) or the driver refuses a map: the layer call then keeps its three launches.
 static bool make_block_maps(const shrike_moe_config& c, const uint8_t* base, const Offsets3& off, uint32_t F,
                             uint64_t cells, uint64_t cell_stride, CUtensorMap* w1, CUtensorMap* m1, CUtensorMap* w2,
-                            CUtensorMap* m2) {
+                            CUtensorMap* m2, CUtensorMap* l1, CUtensorMap* l2) {
     EncodeFn enc = encode_tiled();
     if (!enc) return false;
     const uint64_t gb = c.group_size * c.weight_bits / 8;
@@ -1273,6 +1215,21 @@ static bool make_block_maps(const shrike_moe_config& c, const uint8_t* base, con
         const cuuint32_t box[5] = {(cuuint32_t)gb, 8, (cuuint32_t)G1, 2, 1};
         if (!ok(enc(w1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, (void*)(base + off.w[0]), dims, strides, box, ones,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)))
+            return false;
+    }
+    {   // the same weights in whole 128-byte pieces, gate and up rows of a piece side by side (a row's last piece may
+        // run into the next row: those bytes are not used, and what follows a matrix is its scales)
+        const cuuint64_t n1 = (rb1 + 127) / 128, n2 = (rb2 + 127) / 128;
+        const cuuint64_t dims1[5] = {128, F, 2, n1, cells}, strides1[4] = {rb1, mat, 128, cs};
+        const cuuint32_t box1[5] = {128, 8, 2, (cuuint32_t)n1, 1};
+        const cuuint64_t dims2[4] = {128, c.d, n2, cells}, strides2[3] = {rb2, 128, cs};
+        const cuuint32_t box2[4] = {128, 16, (cuuint32_t)n2, 1};
+        if (!ok(enc(l1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, (void*)(base + off.w[0]), dims1, strides1, box1, ones,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)) ||
+            !ok(enc(l2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)(base + off.w[2]), dims2, strides2, box2, ones,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)))
             return false;
     }
@@ -1308,16 +1265,16 @@ static bool make_block_maps(const shrike_moe_config& c, const uint8_t* base, con
 
 // The maps of a call's pool and shared block, cached on the handle: they change only when the host changes
 // the pool, the offsets or the shared block.
-struct FusedMapCache {
+struct BlockMapCache {
     PoolView pool;
     Offsets3 routed, shared;
     const uint8_t* shared_block;
     bool valid, usable;
-    FusedMaps maps;
+    BlockMaps maps;
 };
 
-static const FusedMaps* fused_maps_for(const shrike_moe* m, const ExpertArgs& ea) {
-    FusedMapCache* cache = (FusedMapCache*)m->ws.fused_maps;
+const BlockMaps* block_maps_for(const shrike_moe* m, const ExpertArgs& ea) {
+    BlockMapCache* cache = (BlockMapCache*)m->ws.fused_maps;
     if (!cache) return nullptr;
     const bool same = cache->valid && memcmp(&cache->pool, &ea.pool, sizeof(PoolView)) == 0 &&
                       memcmp(&cache->routed, &ea.routed, sizeof(Offsets3)) == 0 &&
@@ -1333,18 +1290,20 @@ static const FusedMaps* fused_maps_for(const shrike_moe* m, const ExpertArgs& ea
         if (!ea.pool.base[ch]) break;
         const uint32_t cells = left < ea.pool.cells_per_chunk ? left : ea.pool.cells_per_chunk;
         ok = make_block_maps(c, ea.pool.base[ch], ea.routed, c.f, cells, ea.pool.stride, &cache->maps.w1[ch],
-                             &cache->maps.m1[ch], &cache->maps.w2[ch], &cache->maps.m2[ch]);
+                             &cache->maps.m1[ch], &cache->maps.w2[ch], &cache->maps.m2[ch], &cache->maps.l1[ch],
+                             &cache->maps.l2[ch]);
         left -= cells;
     }
     if (ok && c.has_shared)
         ok = make_block_maps(c, ea.shared_block, ea.shared, c.shared_f, 1, 16, &cache->maps.w1[SHRIKE_MAX_POOL_CHUNKS],
                              &cache->maps.m1[SHRIKE_MAX_POOL_CHUNKS], &cache->maps.w2[SHRIKE_MAX_POOL_CHUNKS],
-                             &cache->maps.m2[SHRIKE_MAX_POOL_CHUNKS]);
+                             &cache->maps.m2[SHRIKE_MAX_POOL_CHUNKS], &cache->maps.l1[SHRIKE_MAX_POOL_CHUNKS],
+                             &cache->maps.l2[SHRIKE_MAX_POOL_CHUNKS]);
     cache->usable = ok;
     return ok ? &cache->maps : nullptr;
 }
 
-size_t fused_map_cache_bytes() { return sizeof(FusedMapCache); }
+size_t fused_map_cache_bytes() { return sizeof(BlockMapCache); }
 
 size_t fused_geom_bytes() { return sizeof(FusedGeom); }
 // {epoch, logit} words of the experts and the gate row, then the selecting blocks' copies of the instance list
@@ -1402,7 +1361,7 @@ cudaError_t launch_fused_layer(const shrike_moe* m, cudaStream_t st, const Exper
                                const uint32_t* io_status, const void* x, uint32_t* ids, float* weights,
                                uint32_t* slots, float* gate, void* y, void* hidden) {
     const shrike_moe_config& c = m->cfg;
-    const FusedMaps* maps = fused_maps_for(m, ea);
+    const BlockMaps* maps = block_maps_for(m, ea);
     if (!maps) return cudaErrorNotSupported;   // the caller falls back to the three launches
     FusedArgs a;
     memset(&a, 0, sizeof a);

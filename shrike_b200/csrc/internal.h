@@ -68,6 +68,7 @@ struct ExpertArgs {
 };
 
 struct Workspace {
+    void* slab = nullptr;           // the one device allocation that the pointers below lie in
     float* logits = nullptr;        // [max_tokens x num_experts]
     uint16_t* xh = nullptr;
     float* xsum = nullptr;
@@ -78,6 +79,10 @@ struct Workspace {
     uint32_t* n_inst = nullptr;
     uint32_t* status = nullptr;     // device status word
     uint32_t* done_counter = nullptr; // blocks finished, fused route kernel
+    uint32_t* arrived = nullptr;    // blocks past phase 2 of the streaming expert kernel, over all launches
+    uint32_t* inst_done = nullptr;  // its finished gate/up units of every instance; the plan zeroes them
+    float* parts = nullptr;         // its weighted rows per pair and per shared row [<= 64 tokens x (top_k + 1) x d]
+    uint32_t* pair_cell = nullptr;  // decode plan: cell of every pair, or SHRIKE_SLOT_MISS
     uint32_t* block_hist = nullptr; // prefill grouping scratch
     uint32_t* expert_offsets = nullptr;
     uint32_t* expert_counts = nullptr;
@@ -117,6 +122,7 @@ struct shrike_moe {
     uint64_t* residency = nullptr;
     uint32_t residency_layers = 0;
     int sm_count = 148;
+    uint32_t smem_optin = 0;      // most dynamic shared memory of a block
     bool no_pdl = false;          // SHRIKE_NO_PDL was set when the handle was created (diagnostics)
     bool single_stream = false;   // SHRIKE_SINGLE_STREAM was set when the handle was created: nothing else runs on the GPU
                                   // beside this handle's stream, so the one-launch layer need not be a cooperative launch
@@ -171,6 +177,10 @@ cudaError_t launch_phase1(const shrike_moe* m, cudaStream_t st, const ExpertArgs
                           uint32_t max_inst, bool pdl);
 cudaError_t launch_phase2(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, uint32_t T,
                           uint32_t max_inst, void* y, void* hidden, bool pdl);
+// expert_stream.cu
+cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const ExpertArgs& ea, uint32_t T, uint32_t n_shared,
+                                 uint32_t phases, bool accumulate, void* y, void* hidden, bool pdl);
+size_t stream_parts_bytes(const shrike_moe_config& c);
 // synth.cu
 cudaError_t launch_synth_fill(const shrike_moe* m, cudaStream_t st, const PoolView& pool,
                               uint32_t first_cell, uint32_t count, uint64_t seed, uint32_t layer,
