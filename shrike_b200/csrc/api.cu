@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "route_args.cuh"
 
 using namespace shrike;
 
@@ -165,14 +166,13 @@ int fill_expert_args(shrike_moe* m, const shrike_pool* pool, const shrike_expert
 }
 
 
-// The expert projections of a decode call's work lists (phases: 1, 2 or 3 = both). From 9 rows on the streaming kernel
-// takes every shape whose tiles its ring and the tiled copies can hold. The per-tile kernels take the others, and the
-// calls of fewer rows: they lay no operands out ahead of the first tile (layer call, 8 rows of the 256-expert shape:
-// 63.5 us against 66.6; 12 rows: 86.5 against 82.4).
+// The expert projections of a decode call's work lists (phases: 1, 2 or 3 = both). The streaming kernel takes every
+// shape whose tiles its ring and the tiled copies can hold; the per-tile kernels take the others, and single rows, which
+// have nothing to lay out ahead of the first tile.
 cudaError_t launch_experts(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, uint32_t T, uint32_t phases, void* y,
                            void* hidden, bool pdl) {
     const uint32_t n_shared = m->cfg.has_shared ? (T + 7) / 8 : 0;
-    cudaError_t e = T > 8 ? launch_expert_stream(m, st, a, T, n_shared, phases, false, y, hidden, pdl) : cudaErrorNotSupported;
+    cudaError_t e = T > 1 ? launch_expert_stream(m, st, a, T, n_shared, phases, false, y, hidden, pdl) : cudaErrorNotSupported;
     if (e != cudaErrorNotSupported) return e;
     const uint32_t mi = max_instances(m->cfg, T);
     if ((phases & 1u) && (e = launch_phase1(m, st, a, mi, pdl)) != cudaSuccess) return e;
@@ -289,7 +289,7 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
     A(&w.status, 4);
     A(&w.n_inst, 4);
     A(&w.done_counter, 4);
-    A(&w.arrived, 4);
+    A(&w.arrived, 8);
     A(&w.fused_epoch, 4);
     const size_t zeroed = slab;
     A(&w.logits, T * c.num_experts * 4);
@@ -299,7 +299,7 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
     A(&w.acts_shared, c.has_shared ? T * c.shared_f * 2 : 0);
     A(&w.sorted, T * K * 4);
     A(&w.inst, (size_t)w.max_inst * sizeof(Instance));
-    A(&w.inst_done, (size_t)w.max_inst * 4);
+    A(&w.inst_done, stream_done_bytes());
     A(&w.parts, stream_parts_bytes(c));
     A(&w.pair_cell, std::min(T, (size_t)SHRIKE_MAX_DECODE_TOKENS) * K * 4);
     A(&w.block_hist, ((T + 127) / 128) * c.num_experts * 4);
@@ -671,18 +671,6 @@ int shrike_encode_decode_layer(shrike_moe* m, void* stream, const shrike_pool* p
     uint32_t* ids = out_indices ? out_indices : w.ids_dev;
     float* wt = out_weights ? out_weights : w.w_dev;
     float* gate = m->cfg.shared_gated ? w.gate_dev : nullptr;
-    // A few dozen rows on a handle that owns the prefill operands: the expert-grouped tensor-core call reads
-    // every expert once for all its rows, where the 8-row tiles read it once per 8 (gpt-oss shape, 64 rows:
-    // 279 us per layer against 740).
-    if (query_count > 16 && w.xs && umma_supported(m->cfg) && !m->force_warp_mma) {
-        int rcg = shrike_encode_router(m, stream, router, x, query_count, m->cfg.d, ids, wt, gate);
-        if (rcg) return rcg;
-        rcg = shrike_encode_residency_classification(m, stream, ids, residency_table_row, query_count, w.slots_dev,
-                                                     nullptr, nullptr, nullptr);
-        if (rcg) return rcg;
-        return encode_prefill(m, stream, pool, routed_offsets, ids, w.slots_dev, wt, x, query_count, shared, gate,
-                              io_status, y, hidden);
-    }
     if (query_count == 1 && w.fused_geom) {
         // one row: router, selection, lookup, both projections and the combine in ONE launch (fused_layer.cu)
         if (!residency_table_row || !pool) return fail(m, SHRIKE_EINVAL, "decode_layer: null operand");
@@ -699,6 +687,39 @@ int shrike_encode_decode_layer(shrike_moe* m, void* stream, const shrike_pool* p
         if (fe == cudaSuccess) return SHRIKE_OK;
         if (fe != cudaErrorNotSupported) return cuda_fail(m, fe, "launch_fused_layer");
         // a block layout the tiled copies cannot describe: the three launches below
+    }
+    if (query_count > 1) {
+        // some rows: the same in one launch of the streaming kernel (expert_stream.cu). In three launches the last
+        // block of the router ranked every row while the others' SMs idled (8 us of 4 rows' 43, 20 of 16 rows' 92), and
+        // the next launch began 3 us later.
+        if (!residency_table_row || !pool) return fail(m, SHRIKE_EINVAL, "decode_layer: null operand");
+        const uint32_t limit = m->cfg.max_tokens < SHRIKE_MAX_DECODE_TOKENS ? m->cfg.max_tokens : SHRIKE_MAX_DECODE_TOKENS;
+        int rcs = check_router_call(m, router, x, query_count, limit, m->cfg.d, false, nullptr);
+        if (rcs) return rcs;
+        ExpertArgs ea;
+        rcs = fill_expert_args(m, pool, routed_offsets, shared, wt, gate, ea);
+        if (rcs) return rcs;
+        if ((rcs = check_device(m))) return rcs;
+        RouterArgs ra = make_router_args(m, *router, x, query_count, m->cfg.d, ids, wt, gate);
+        ra.table = residency_table_row; ra.pool_cells = pool->view.cells; ra.io_status = io_status;
+        ra.with_shared = m->cfg.has_shared; ra.int4 = m->cfg.weight_bits == 4; ra.group = m->cfg.group_size;
+        ra.slots = w.slots_dev; ra.xh = w.xh; ra.xsum = w.xsum; ra.status = w.status;
+        const cudaError_t se = launch_expert_stream(m, (cudaStream_t)stream, ea, query_count, m->cfg.has_shared ? (query_count + 7) / 8 : 0,
+                                                    3u, false, y, hidden, !m->no_pdl, &ra);
+        if (se == cudaSuccess) return SHRIKE_OK;
+        if (se != cudaErrorNotSupported) return cuda_fail(m, se, "launch_expert_stream");
+    }
+    // A few dozen rows on a handle that owns the prefill operands: the expert-grouped tensor-core call reads
+    // every expert once for all its rows, where the 8-row tiles read it once per 8 (gpt-oss shape, 64 rows:
+    // 279 us per layer against 740).
+    if (query_count > 16 && w.xs && umma_supported(m->cfg) && !m->force_warp_mma) {
+        int rcg = shrike_encode_router(m, stream, router, x, query_count, m->cfg.d, ids, wt, gate);
+        if (rcg) return rcg;
+        rcg = shrike_encode_residency_classification(m, stream, ids, residency_table_row, query_count, w.slots_dev,
+                                                     nullptr, nullptr, nullptr);
+        if (rcg) return rcg;
+        return encode_prefill(m, stream, pool, routed_offsets, ids, w.slots_dev, wt, x, query_count, shared, gate,
+                              io_status, y, hidden);
     }
     int rc = shrike_encode_route_decode(m, stream, router, residency_table_row, pool, x, query_count, m->cfg.d,
                                         io_status, ids, wt, gate, w.slots_dev, nullptr);

@@ -30,6 +30,10 @@
 // per-tile kernels took 82; inside the unit loops 6.5 TB/s, the rest is the start (7 us), the hand-over between the
 // phases (5 us) and the last one (3 us).
 #include "block_maps.cuh"
+#include "plan.cuh"
+#include "route_args.cuh"
+#include "router_math.cuh"
+#include "select.cuh"
 #include "tile_math.cuh"
 
 #include <algorithm>
@@ -41,9 +45,12 @@ namespace {
 
 constexpr uint32_t kWarps = 16, kFinish = 4;         // multiplying and finishing warps
 constexpr uint32_t kThreads = (kWarps + kFinish) * 32;
-constexpr uint32_t kMaxSlots = 32, kMaxSlots2 = 64;
+constexpr uint32_t kMaxSlots = 32, kMaxSlots2 = 48;
 constexpr uint32_t kRedCol = 20;                     // floats per column of a warp's partial sums (16 + padding)
 constexpr uint32_t kRedWarp = 8 * kRedCol;
+// most instances of a call: each expert once, once more per eight pairs, and the shared expert's
+constexpr uint32_t kMaxTable = SHRIKE_MAX_EXPERTS + kPlanMaxPairs / 8 + SHRIKE_MAX_DECODE_TOKENS / 8;
+static_assert(kMaxTable <= 65536 && kThreads >= SHRIKE_MAX_EXPERTS, "work list");
 
 }  // namespace
 
@@ -53,9 +60,21 @@ constexpr uint32_t kRedWarp = 8 * kRedCol;
 struct StreamGeom {
     uint32_t meta_off, ab_off, slot_bytes, n_slots, w1;   // phase 1: scales/biases and additive biases in a slot; warps of a team
     uint32_t ab_off2[2], w_bytes2, m_bytes2, n_slots2, w2;   // phase 2, [0] routed, [1] shared; [slot] weights, then [slot] the rest
-    uint32_t off_red, off_ring, smem_bytes;
+    uint32_t off_red, off_ring, ring_bytes, smem_bytes;
 };
 
+// The call's work list as every block keeps it: instance i is block cell[i] (the first n_shared: the shared expert's) for
+// count[i] rows, the pairs sorted[first[i]] and on (shared: the rows first[i] and on).
+struct StreamTable {
+    uint32_t cell[kMaxTable];
+    uint16_t first[kMaxTable];
+    uint8_t count[kMaxTable];
+    uint16_t sorted[kPlanMaxPairs];
+    float weight[kPlanMaxPairs];                     // a routing launch: the pairs' route weights
+    uint8_t live[SHRIKE_MAX_DECODE_TOKENS];          // bit q: the row's pick q has a cell
+    uint32_t warp_sum[SHRIKE_MAX_EXPERTS / 32];
+    uint32_t misses;
+};
 struct StreamArgs {
     PoolView pool;
     Offsets3 routed, shared;
@@ -69,21 +88,35 @@ struct StreamArgs {
     uint16_t* acts_shared;
     float* yacc;                                     // accumulate: fp32 rows that phase 2 adds into
     float* parts;                                    // [T x top_k routed | T shared][d] weighted rows (decode)
-    const uint32_t* pair_cell;                       // cell of every pair or SHRIKE_SLOT_MISS: which parts exist
+    const uint32_t* sorted;                          // plan of a call that does not route: the pairs by instance
+    const uint32_t* pair_cell;                       // and the cell of every pair or SHRIKE_SLOT_MISS
     const float* route_w;
     const float* shared_gate;
     uint32_t* status;
-    uint32_t* arrived;                               // blocks done with phase 2, over all launches
-    uint32_t* inst_done;                             // both phases: finished units of every instance (zeroed ahead of this launch)
+    unsigned long long* arrived;                     // blocks past a grid barrier, over all launches
+    uint32_t* inst_done;                             // both phases: finished units of every instance
     uint32_t T;
     void* y;
     void* hidden;
     uint32_t phases;                                 // bit 0, bit 1 (the last with phase 3 unless accumulate)
     uint32_t accumulate;
     uint32_t rcp_cpc;                                // ceil(2^32 / cells_per_chunk)
+    uint32_t n_chunks;
+    uint32_t routes;                                 // this launch routes its rows first
+    uint32_t token_groups;                           // of the logits: a block takes one group's rows against its share of the experts
+    RouterArgs r;
     StreamGeom g;
-    BlockMaps maps;
 };
+
+// Scratch of the routing, in front of the ring: the pairs of every expert as a bit mask, the experts' residency words
+// and the cells of those picked.
+struct RouteScratch {
+    uint32_t mask[kPlanMaxPairs / 32][SHRIKE_MAX_EXPERTS];
+    uint64_t word[SHRIKE_MAX_EXPERTS];
+    uint32_t cell[SHRIKE_MAX_EXPERTS];
+};
+// Bytes of the kernel's static shared memory: the table, the barriers and two words.
+constexpr uint32_t kStaticBytes = (sizeof(StreamTable) + 15) / 16 * 16 + (2 * (kMaxSlots + kMaxSlots2) + 1) * 8 + 24;
 
 namespace {
 
@@ -137,6 +170,11 @@ __device__ __forceinline__ uint32_t lds32(uint32_t a) {
 __device__ __forceinline__ uint32_t lds16(uint32_t a) {
     uint16_t v;
     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds8(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
     return v;
 }
 __device__ __forceinline__ void sts32(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
@@ -307,19 +345,19 @@ __device__ __forceinline__ void piece_tiles(uint32_t w, uint32_t sc, uint32_t d_
 __device__ __noinline__ float glu_of(float gate, float up, uint32_t activation) { return glu(gate, up, activation); }
 
 // Everything this block did so far is visible to the blocks that have passed the same counter.
-__device__ __forceinline__ bool grid_sync(uint32_t* counter) {
+__device__ __forceinline__ bool grid_sync(unsigned long long* counter) {
     bool ok = true;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        // the counter only grows: every launch adds the grid's size once
-        const uint32_t goal = (atomicAdd(counter, 1u) / gridDim.x + 1u) * gridDim.x;
+        // the counter only grows (for more launches than there is time for): every barrier adds the grid's size once
+        const unsigned long long goal = (atomicAdd(counter, 1ull) / gridDim.x + 1ull) * gridDim.x;
         ok = false;
 #pragma unroll 1
         for (uint32_t it = 0; it < (1u << 18) && !ok; ++it) {
-            uint32_t v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-            ok = (int32_t)(v - goal) >= 0;
+            unsigned long long v;
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(counter) : "memory");
+            ok = v >= goal;
             if (!ok && it > 8) __nanosleep(it > 1024 ? 256 : 20);
         }
     }
@@ -327,15 +365,268 @@ __device__ __forceinline__ bool grid_sync(uint32_t* counter) {
     return ok;
 }
 
+// Lane sums of two rows against two activation rows (fp32, scaled where the router scales columns), all in shared memory:
+// acc[row][x]. fp32 rows in the order of lane_dot_f32; a lane's chunks past the row's end are left out.
+__device__ __forceinline__ void dots_f32(uint32_t w0, uint32_t w1, uint32_t x0, uint32_t x1, uint32_t chunks, uint32_t lane, float (&acc)[2][2]) {
+#pragma unroll 2
+    for (uint32_t c = lane; c < chunks; c += 32) {
+        uint32_t w[2][4], x[2][4];
+        lds_packed<4>(w0 + c * 16, w[0]);
+        lds_packed<4>(w1 + c * 16, w[1]);
+        lds_packed<4>(x0 + c * 16, x[0]);
+        lds_packed<4>(x1 + c * 16, x[1]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+#pragma unroll
+                for (int u = 0; u < 2; ++u) acc[k][u] = __fmaf_rn(__uint_as_float(w[k][i]), __uint_as_float(x[u][i]), acc[k][u]);
+    }
+}
+// Affine rows (their packed integers and {scale, bias} pairs), in the order of lane_dot_affine.
+__device__ __forceinline__ void dots_affine(uint32_t w0, uint32_t w1, uint32_t sb0, uint32_t sb1, uint32_t x0, uint32_t x1, uint32_t groups,
+                                            uint32_t bits, uint32_t lane, float (&acc)[2][2]) {
+#pragma unroll 2
+    for (uint32_t gi = 0; gi < groups; ++gi) {
+        const uint2 xr[2] = {lds64(x0 + (gi * 32 + lane) * 8), lds64(x1 + (gi * 32 + lane) * 8)};
+        const uint2 sb[2] = {lds64(sb0 + gi * 8), lds64(sb1 + gi * 8)};
+        uint32_t q[2];
+        if (bits == 4) {
+            q[0] = lds8(w0 + gi * 32 + lane); q[1] = lds8(w1 + gi * 32 + lane);
+            q[0] = (q[0] & 0xfu) | (q[0] & 0xf0u) << 4; q[1] = (q[1] & 0xfu) | (q[1] & 0xf0u) << 4;
+        } else {
+            q[0] = lds16(w0 + gi * 64 + lane * 2); q[1] = lds16(w1 + gi * 64 + lane * 2);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const float q0 = (float)(q[k] & 0xffu), q1 = (float)(q[k] >> 8), sc = __uint_as_float(sb[k].x), bi = __uint_as_float(sb[k].y);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float xa = __uint_as_float(xr[u].x), xb = __uint_as_float(xr[u].y);
+                acc[k][u] = __fmaf_rn(sc, __fadd_rn(__fmul_rn(q0, xa), __fmul_rn(q1, xb)), acc[k][u]);
+                acc[k][u] = __fmaf_rn(bi, __fadd_rn(xa, xb), acc[k][u]);
+            }
+        }
+    }
+}
+
+// The call's work list into `tab`: routed here, or read from the plan of an earlier launch. Returns the number of
+// instances. (Inlined: what a call saves of its caller's registers goes through an L1 that the ring leaves 28 KB.)
+__device__ __forceinline__ uint32_t work_list(const StreamArgs& a, uint8_t* dsm, uint8_t* ring, StreamTable& tab, uint64_t* rows_here,
+                                           uint32_t* failed) {
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ring0 = smem_u32(ring), D = a.d;
+    auto give_up = [&]() {
+        report_status(a.status, kStatusWaitTimeout);
+        *failed = 1;
+    };
+    uint32_t n_inst;
+    const uint32_t n_sh = a.n_shared;
+    if (a.routes) {
+        // ================= router, selection, lookup, work list =================
+        // A block has a share of the expert rows (they go to the ring's memory, asked for ahead of the wait) and of the
+        // activation rows; what follows the logits every block does for itself: another hand-over between blocks costs
+        // more than the work (a row's picks 1 us by one warp, the list 1 us).
+        const RouterArgs& r = a.r;
+        const uint32_t rows = r.ne + (r.gate_row ? 1u : 0u), bx = blockIdx.x / a.token_groups, by = blockIdx.x - bx * a.token_groups;
+        const uint32_t nbx = gridDim.x / a.token_groups, e0 = bx < nbx ? rows * bx / nbx : 0u, e1 = bx < nbx ? rows * (bx + 1) / nbx : 0u;
+        const uint32_t t0 = a.T * by / a.token_groups, nt = a.T * (by + 1) / a.token_groups - t0;
+        const uint32_t row_bytes = r.bits ? D * r.bits / 8 : D * 4, n_exp = min(e1, r.ne) - min(e0, r.ne), groups = D / 64;
+        const bool gate_here = r.gate_row && e1 == rows && e1 > e0;
+        const uint32_t gate_at = ring0 + n_exp * row_bytes, sb_at = gate_at + (gate_here ? D * 4 : 0u);
+        if (tid == 0 && e1 > e0) {
+            mbar_expect_tx(rows_here, n_exp * row_bytes + (gate_here ? D * 4 : 0u));
+            if (n_exp) bulk_g2s(ring, (const uint8_t*)r.w + (size_t)e0 * row_bytes, n_exp * row_bytes, rows_here);
+            if (gate_here) bulk_g2s(ring + n_exp * row_bytes, r.gate_row, D * 4, rows_here);
+        }
+        if (r.bits)
+            for (uint32_t j = tid; j < n_exp * groups; j += kThreads) {
+                const float2 v = make_float2(bf16_bits_to_f32(r.scales[(size_t)e0 * groups + j]), bf16_bits_to_f32(r.biases[(size_t)e0 * groups + j]));
+                *(float2*)(ring + (sb_at - ring0) + j * 8) = v;
+            }
+        pdl_wait();
+        pdl_launch_dependents();   // (the next kernel waits for this one to end; its blocks find no room before that)
+        RouteScratch& rs = *(RouteScratch*)dsm;
+        const uint32_t n_pairs = a.T * r.top_k, n_words = (n_pairs + 31) / 32;
+        uint32_t io = 1u;
+        if (r.io_status) io = *r.io_status;
+        if (tid < r.ne) rs.word[tid] = r.table[tid];
+        for (uint32_t j = tid; j < n_words * SHRIKE_MAX_EXPERTS; j += kThreads) (&rs.mask[0][0])[j] = 0;
+        if (blockIdx.x == gridDim.x - 1)
+            for (uint32_t j = tid; j < kMaxTable; j += kThreads) a.inst_done[j] = 0;
+        // The block's activation rows go to shared memory too, as many at a time as there is room for: read where they
+        // are used, every batch of a row costs a round trip to L2 of its own.
+        const bool x32 = r.dt == SHRIKE_DTYPE_FP32;
+        const size_t x_stride = (size_t)r.stride * (x32 ? 4 : 2);
+        const uint32_t x_bytes = D * 4, xs_at = (sb_at + (r.bits ? n_exp * groups * 8 : 0u) + 15u) & ~15u, quads = D / 4;
+        const uint32_t room = ((a.g.ring_bytes - (xs_at - ring0)) / x_bytes) & ~1u;
+        const uint32_t n_f = r.bits ? 0u : n_exp, pairs_a = r.bits ? (n_exp + 1) / 2 : 0u;
+        const uint32_t n_f32 = n_f + (gate_here ? 1u : 0u), f_at = gate_at - n_f * row_bytes;   // (the gate row follows the expert rows)
+        for (uint32_t s0 = 0; s0 < nt; s0 += room) {
+            const uint32_t here = min(room, nt - s0);
+            if (s0) __syncthreads();
+            if (e1 > e0) {
+#pragma unroll 4
+                for (uint32_t j = tid; j < here * quads; j += kThreads) {
+                    const uint32_t row = j / quads, c = j - row * quads;
+                    float x[4];
+                    load_act4((const uint8_t*)r.hidden + (t0 + s0 + row) * x_stride, c, r.dt, x);
+                    if (r.eff_scale) {
+                        const uint2 e = __ldg((const uint2*)r.eff_scale + c);
+                        x[0] = __fmul_rn(x[0], __uint_as_float(e.x << 16)); x[1] = __fmul_rn(x[1], __uint_as_float(e.x & 0xffff0000u));
+                        x[2] = __fmul_rn(x[2], __uint_as_float(e.y << 16)); x[3] = __fmul_rn(x[3], __uint_as_float(e.y & 0xffff0000u));
+                    }
+                    sts128(xs_at + row * x_bytes + c * 16, __float_as_uint(x[0]), __float_as_uint(x[1]), __float_as_uint(x[2]), __float_as_uint(x[3]));
+                }
+            }
+            if (s0 == 0)   // the fp16 operand copy of all rows, by all blocks
+                for (uint32_t j0 = (warp * gridDim.x + blockIdx.x) * 32, items = a.T * (D / 8); j0 < items; j0 += kThreads * gridDim.x)
+                    xprep_item(r.hidden, x_stride, D, r.group, r.dt, r.int4 != 0, j0 + lane, j0 + lane < items, r.xh, r.xsum, r.status);
+            __syncthreads();
+            const uint32_t n_tok2 = (here + 1) / 2, tasks = e1 > e0 ? (pairs_a + (n_f32 + 1) / 2) * n_tok2 : 0u;
+            if (warp < tasks && !wait_slot(smem_u32(rows_here), 0)) give_up();
+            for (uint32_t task = warp; task < tasks; task += kWarps + kFinish) {
+                const uint32_t rp = task / n_tok2, tp = (task - rp * n_tok2) * 2;
+                const uint32_t tp2 = min(tp + 1, here - 1), ta = t0 + s0 + tp, tb = t0 + s0 + tp2;
+                const uint32_t xa = xs_at + tp * x_bytes, xb = xs_at + tp2 * x_bytes;
+                float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+                uint32_t ea, eb;
+                if (rp < pairs_a) {
+                    const uint32_t ja = 2 * rp, jb = min(ja + 1, n_exp - 1);
+                    ea = e0 + ja; eb = e0 + jb;
+                    dots_affine(ring0 + ja * row_bytes, ring0 + jb * row_bytes, sb_at + ja * groups * 8, sb_at + jb * groups * 8, xa, xb, groups, r.bits, lane, acc);
+                } else {
+                    const uint32_t ja = 2 * (rp - pairs_a), jb = min(ja + 1, n_f32 - 1);
+                    ea = e0 + n_exp - n_f + ja; eb = e0 + n_exp - n_f + jb;
+                    dots_f32(f_at + ja * D * 4, f_at + jb * D * 4, xa, xb, quads, lane, acc);
+                }
+                if (r.eff_scale && eb == r.ne) {   // the gate row takes no column scale
+                    const uint32_t w = gate_at;
+                    float ga = 0.f, gb = 0.f;
+#pragma unroll 1
+                    for (uint32_t c = lane; c < quads; c += 32) {
+                        uint32_t wr[4];
+                        float xf[4], xg[4];
+                        lds_packed<4>(w + c * 16, wr);
+                        load_act4((const uint8_t*)r.hidden + ta * x_stride, c, r.dt, xf);
+                        load_act4((const uint8_t*)r.hidden + tb * x_stride, c, r.dt, xg);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) { ga = __fmaf_rn(__uint_as_float(wr[i]), xf[i], ga); gb = __fmaf_rn(__uint_as_float(wr[i]), xg[i], gb); }
+                    }
+                    acc[1][0] = ga; acc[1][1] = gb;
+                    if (ea == r.ne) { acc[0][0] = ga; acc[0][1] = gb; }
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) acc[k >> 1][k & 1] = butterfly_sum(acc[k >> 1][k & 1]);
+                if (lane < 4) {
+                    const float v = lane == 0 ? acc[0][0] : lane == 1 ? acc[0][1] : lane == 2 ? acc[1][0] : acc[1][1];
+                    const uint32_t e = lane >> 1 ? eb : ea, tk = lane & 1 ? tb : ta;
+                    if (e == r.ne) r.gate_out[tk] = sigmoid_det(v);
+                    else r.logits[(size_t)tk * r.ne + e] = v;
+                }
+            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the ring's next writers are copies
+        if (!grid_sync(a.arrived)) give_up();
+        const bool ready = io == 1u || io == 3u;
+        for (uint32_t row = warp; row < a.T; row += kWarps + kFinish) {
+            uint32_t id;
+            float w;
+            select_row<true>(r.logits + (size_t)row * r.ne, r, lane, id, w);
+            const uint32_t p = row * r.top_k + lane, e = min(id, r.ne - 1u);
+            bool live = false;
+            if (lane < r.top_k) {
+                const uint64_t word = rs.word[e];
+                uint32_t slot = (uint32_t)(word & 0xffffffffu);
+                if ((uint32_t)(word >> 32) != 2u) slot = SHRIKE_SLOT_MISS;
+                const bool inside = slot < r.pool_cells;
+                live = inside && ready;
+                tab.weight[p] = w;
+                if (live) {
+                    rs.cell[e] = slot;
+                    atomicOr(&rs.mask[p >> 5][e], 1u << (p & 31u));
+                }
+                if (blockIdx.x == row) {
+                    r.ids[p] = id;
+                    r.weights[p] = w;
+                    if (r.slots) r.slots[p] = slot;
+                    if (slot != SHRIKE_SLOT_MISS && !inside) report_status(a.status, kStatusBadIndex);
+                }
+                if (slot == SHRIKE_SLOT_MISS && blockIdx.x == 0 && r.counts) atomicAdd(&tab.misses, 1u);
+            }
+            const uint32_t bits = __ballot_sync(0xffffffffu, live);
+            if (lane == 0) tab.live[row] = (uint8_t)bits;
+        }
+        __syncthreads();
+        if (tid == 0 && blockIdx.x == 0 && r.counts) {
+            r.counts[0] = n_pairs - tab.misses;
+            r.counts[1] = tab.misses;
+        }
+        uint32_t cnt = 0, incl = 0;   // thread e: pairs of expert e, and {instances, pairs} of the experts up to it
+        if (tid < SHRIKE_MAX_EXPERTS) {
+            for (uint32_t w = 0; w < n_words; ++w) cnt += __popc(rs.mask[w][tid]);
+            incl = ((cnt + 7) / 8) << 16 | cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= (uint32_t)o) incl += v;
+            }
+            if (lane == 31) tab.warp_sum[warp] = incl;
+        }
+        __syncthreads();
+        uint32_t before = 0, total = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < SHRIKE_MAX_EXPERTS / 32; ++w) {
+            const uint32_t v = tab.warp_sum[w];
+            if (w < warp) before += v;
+            total += v;
+        }
+        n_inst = n_sh + (total >> 16);
+        if (cnt) {
+            const uint32_t ni = (cnt + 7) / 8, at = before + incl - (ni << 16 | cnt), i0 = n_sh + (at >> 16), p0 = at & 0xffffu;
+            for (uint32_t c = 0; c < ni; ++c) {
+                tab.cell[i0 + c] = rs.cell[tid];
+                tab.first[i0 + c] = (uint16_t)(p0 + 8 * c);
+                tab.count[i0 + c] = (uint8_t)min(8u, cnt - 8 * c);
+            }
+            uint32_t j = p0;
+            for (uint32_t w = 0; w < n_words; ++w)
+                for (uint32_t m = rs.mask[w][tid]; m; m &= m - 1) tab.sorted[j++] = (uint16_t)(w * 32 + __ffs(m) - 1);
+        }
+    } else {
+        pdl_wait();
+        pdl_launch_dependents();
+        n_inst = min(*a.n_inst, kMaxTable);
+        for (uint32_t j = tid; j < kMaxTable; j += kThreads) {
+            const uint4 h = *(const uint4*)&a.inst[j < n_inst ? j : 0];
+            if (j < n_inst) { tab.cell[j] = h.y; tab.first[j] = (uint16_t)h.z; tab.count[j] = (uint8_t)h.w; }
+        }
+        for (uint32_t j = tid; j < a.T * a.top_k; j += kThreads) tab.sorted[j] = (uint16_t)a.sorted[j];
+        if ((a.phases & 2u) && tid < a.T) {
+            uint32_t live = 0;
+            for (uint32_t q = 0; q < a.top_k; ++q)
+                if (a.pair_cell[tid * a.top_k + q] != SHRIKE_SLOT_MISS) live |= 1u << q;
+            tab.live[tid] = (uint8_t)live;
+        }
+    }
+    if (tid < n_sh) {
+        tab.cell[tid] = 0;
+        tab.first[tid] = (uint16_t)(8 * tid);
+        tab.count[tid] = (uint8_t)min(8u, a.T - 8 * tid);
+    }
+    return n_inst;
+}
+
 }  // namespace
 
 template <int BITS, int GROUP, int META, bool AL>
-__global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid_constant__ StreamArgs a) {
+__global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid_constant__ StreamArgs a, const __grid_constant__ BlockMaps maps) {
     using Q = FQ<BITS, GROUP>;
     constexpr uint32_t GP = 128 / Q::kGroupBytes, H = GROUP / 32;   // groups of a piece; 16-byte operand parts of a group
     extern __shared__ __align__(128) uint8_t dsm_raw[];
     uint8_t* const dsm = dsm_raw + ((1024u - (smem_u32(dsm_raw) & 1023u)) & 1023u);   // the swizzle follows the address
     __shared__ uint64_t full1[kMaxSlots], done1[kMaxSlots], full2[kMaxSlots2], done2[kMaxSlots2];
+    __shared__ uint64_t rows_here;
+    __shared__ StreamTable tab;
     __shared__ uint32_t s_failed;
     const StreamGeom& G = a.g;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -346,16 +637,25 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
 
     if (tid < G.n_slots) { mbar_init(&full1[tid], 1); mbar_init(&done1[tid], G.w1); }
     if (tid < G.n_slots2) { mbar_init(&full2[tid], 1); mbar_init(&done2[tid], G.w2); }
+    if (tid == 0) mbar_init(&rows_here, 1);
     if (tid < kMaxSlots2) fence_mbar_init();
-    if (tid == 0) s_failed = 0;
+    if (tid == 0) { s_failed = 0; tab.misses = 0; }
+    if (warp == 1 && lane < 4 * (SHRIKE_MAX_POOL_CHUNKS + 1)) {   // descriptors on their way before the first copy needs them
+        const uint32_t ch = lane >> 2;
+        const CUtensorMap* m = (lane & 2u) ? ((lane & 1u) ? maps.l1 : maps.m1) : ((lane & 1u) ? maps.l2 : maps.m2);
+        if (ch < a.n_chunks) asm volatile("prefetch.tensormap [%0];" ::"l"(m + ch) : "memory");
+    }
     __syncthreads();
-    pdl_wait();
-    pdl_launch_dependents();   // (the next kernel waits for this one to end; its blocks find no room before that)
-    const uint32_t n_inst = *a.n_inst, n_sh = min(a.n_shared, n_inst);
     auto give_up = [&]() {
         report_status(a.status, kStatusWaitTimeout);
         s_failed = 1;
     };
+    const uint32_t n_inst = work_list(a, dsm, ring, tab, &rows_here, &s_failed);
+    const uint32_t n_sh = min(a.n_shared, n_inst);
+    __syncthreads();
+    const float* const pair_weight = a.routes ? tab.weight : a.route_w;
+    // the row of pairs (shared: of rows) behind column c of instance i
+    auto pair_of = [&](uint32_t i, uint32_t c) -> uint32_t { return i < n_sh ? tab.first[i] + c : tab.sorted[tab.first[i] + c]; };
     // this lane's row g of the eight, and its first byte in the row's piece
     const uint32_t pr = box_row<Q::kWords>(g), w_lane = pr * 128 + ((t * (Q::kWords * 4)) ^ (pr << 4));
     // where its partial sums go, [column][row mod 4]{row r, r + 4, r + 8, r + 12 of the 16}
@@ -391,25 +691,19 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
         };
 
         // ---- one lane asks for one unit ----
-        uint32_t have = 0xffffffffu, mi = 0;
-        int32_t cc = 0;
-        const uint8_t* base = nullptr;
         auto ask = [&](uint32_t slot, uint32_t i, uint32_t k) {
             const bool sh = i < n_sh;
-            if (i != have) {
-                const uint32_t cell = sh ? 0u : a.inst[i].slot, ch = __umulhi(cell, a.rcp_cpc);
-                mi = sh ? SHRIKE_MAX_POOL_CHUNKS : ch;
-                cc = sh ? 0 : (int32_t)(cell - ch * a.pool.cells_per_chunk);
-                base = sh ? a.shared_block : pool_cell_base(a.pool, cell);
-                have = i;
-            }
+            const uint32_t cell = sh ? 0u : tab.cell[i], ch = __umulhi(cell, a.rcp_cpc);
+            const uint32_t mi = sh ? SHRIKE_MAX_POOL_CHUNKS : ch;
+            const int32_t cc = sh ? 0 : (int32_t)(cell - ch * a.pool.cells_per_chunk);
+            const uint8_t* base = sh || !a.expert_bias ? a.shared_block : pool_cell_base(a.pool, cell);
             const Offsets3& off = sh ? a.shared : a.routed;
             if constexpr (P1) {
                 uint64_t* bar = &full1[slot];
                 const uint32_t at = slot * G.slot_bytes;
                 mbar_expect_tx(bar, 2048 * ((D * BITS / 8 + 127) / 128) + 64 * (D / GROUP) + (a.expert_bias ? 32u : 0u));
-                tma_5d(ring0 + at + G.meta_off, &a.maps.m1[mi], 0, (int32_t)k, 0, 0, cc, bar);
-                tma_5d(ring0 + at, &a.maps.l1[mi], 0, (int32_t)(k * 8), 0, 0, cc, bar);
+                tma_5d_once(ring0 + at + G.meta_off, &maps.m1[mi], 0, (int32_t)k, 0, 0, cc, bar, evict_first_policy());
+                tma_5d_once(ring0 + at, &maps.l1[mi], 0, (int32_t)(k * 8), 0, 0, cc, bar, evict_first_policy());
                 if (a.expert_bias) {
                     bulk_g2s(ring + at + G.ab_off, base + off.ab[0] + (size_t)k * 16, 16, bar);
                     bulk_g2s(ring + at + G.ab_off + 16, base + off.ab[1] + (size_t)k * 16, 16, bar);
@@ -418,8 +712,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
                 const uint32_t F = sh ? a.f_shared : a.f, mt = G.n_slots2 * G.w_bytes2 + slot * G.m_bytes2;
                 uint64_t* bar = &full2[slot];
                 mbar_expect_tx(bar, 2048 * ((F * BITS / 8 + 127) / 128) + 64 * (F / GROUP) + (a.expert_bias ? 32u : 0u));
-                tma_4d(ring0 + mt, &a.maps.m2[mi], 0, (int32_t)(k * 2), 0, cc, bar);
-                tma_4d(ring0 + slot * G.w_bytes2, &a.maps.l2[mi], 0, (int32_t)(k * 16), 0, cc, bar);
+                tma_4d_once(ring0 + mt, &maps.m2[mi], 0, (int32_t)(k * 2), 0, cc, bar, evict_first_policy());
+                tma_4d_once(ring0 + slot * G.w_bytes2, &maps.l2[mi], 0, (int32_t)(k * 16), 0, cc, bar, evict_first_policy());
                 if (a.expert_bias) bulk_g2s(ring + mt + G.ab_off2[sh], base + off.ab[2] + (size_t)k * 32, 32, bar);
             }
         };
@@ -432,55 +726,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
             }
             __syncwarp();
         }
-        // ---- the instance of this warp's units ----
-        uint32_t i = 0, k = 0, cur = 0xffffffffu, count = 0, G2 = 0, groups_left = 0, pieces = 0;
-        uint32_t b0 = 0, cq0 = 0, z0 = 0, sB = 0, w_at = 0, s_at = 0, ab_at = 0, d_s = 0, d_z = 0, k0 = 0;
-        uint16_t* dst = nullptr;   // gate/up: where column g's activations go
-        float* out0 = nullptr;     // down: where the rows of column g (W == 1: columns 2t and 2t + 1) go, and their weights
-        float* out1 = nullptr;
-        float wt0 = 0.f, wt1 = 0.f;
         const uint32_t meta0 = ring0 + (P1 ? G.meta_off : G.n_slots2 * G.w_bytes2);
-        auto open_instance = [&](uint32_t buf) {
-            cur = i;
-            const bool sh = i < n_sh;
-            const uint32_t K = P1 ? D : sh ? a.f_shared : a.f, P = (K * BITS / 8 + 127) / 128;
-            G2 = K / GROUP;
-            count = a.inst[i].count;
-            const uint32_t p0 = P * wi / W;
-            pieces = P * (wi + 1) / W - p0;
-            groups_left = G2 - min(G2, p0 * GP);
-            const BufferLayout lay(G2, H, count);
-            const uint32_t col = min(g, count - 1u);
-            sB = count * 64;
-            b0 = buf + col * 64 + t * 16 + p0 * GP * H * sB;
-            cq0 = buf + lay.cq_off + t * 16 + p0 * GP * 64;
-            z0 = buf + lay.z_off + col * 64 + t * 16 + (GP == 2 ? p0 / 2 : p0 * (GP / 4)) * sB;
-            k0 = GP == 2 ? 2 * (p0 & 1) : 0u;
-            w_at = ring0 + w_lane + p0 * 2048;
-            s_at = meta0 + (pr * G2 + p0 * GP) * 2;
-            d_s = P1 ? 32 * G2 : 16 * G2;
-            d_z = P1 ? 16 * G2 : 32 * G2;
-            ab_at = meta0 - (P1 ? G.meta_off : 0u) + (P1 ? G.ab_off : G.ab_off2[sh]) + pr * 2;
-            if constexpr (P1) {
-                const uint32_t pair = a.inst[i].pair[g];
-                const uint32_t F = sh ? a.f_shared : a.f;
-                dst = g < count ? (sh ? a.acts_shared : a.acts) + (size_t)pair * F + (BITS == 4 ? 2 * t : t) : nullptr;
-            } else {
-                auto target = [&](uint32_t c, float*& out, float& w) {
-                    const uint32_t pair = a.inst[i].pair[c];
-                    w = sh ? (a.shared_gate ? a.shared_gate[pair] : 1.0f) : a.route_w[pair];
-                    float* rows = a.accumulate ? a.yacc + (size_t)(sh ? pair : pair / a.top_k) * D
-                                               : a.parts + ((size_t)pair + (sh ? a.T * a.top_k : 0u)) * D;
-                    out = c < count ? rows + (W == 1 ? pr : t) : nullptr;
-                };
-                target(W == 1 ? 2 * t : g, out0, wt0);
-                target(W == 1 ? 2 * t + 1 : g, out1, wt1);
-            }
-        };
-        auto put = [&](float* at, float v) {
-            if (a.accumulate) atomicAdd(at, v);
-            else *at = v;
-        };
 
         uint32_t i0 = 0, i_end = 0;   // the first staged instance, the end of the block's
         if (n) {
@@ -491,15 +737,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
         }
         // (W == 1: the warps finish their units themselves; fewer teams than finishing warps: some have none)
         uint32_t u = finisher && (W == 1 || team >= nT) ? n : team, slot = team, par = 0;
+        uint32_t i = 0, k = 0;        // unit u: instance, unit in it
         if (u < n) find(u, i, k);
-        uint32_t pend = 0;            // units of `cur` whose activations this warp wrote and has not announced
-        auto announce = [&]() {
-            if (P1 && do2 && pend) {
-                __syncwarp();
-                if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(a.inst_done + cur), "r"(pend) : "memory");
-                pend = 0;
-            }
-        };
         bool later = false;
         while (i0 < i_end) {
             // every warp works out for itself which instances fit: lane l has instance i0 + l
@@ -509,7 +748,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
                 uint32_t bytes = 0;
                 if (ii < i_end) {
                     const uint32_t K = P1 ? D : ii < n_sh ? a.f_shared : a.f;
-                    bytes = BufferLayout(K / GROUP, H, a.inst[ii].count).bytes;
+                    bytes = BufferLayout(K / GROUP, H, tab.count[ii]).bytes;
                 }
                 uint32_t end = bytes;
 #pragma unroll
@@ -534,9 +773,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
                         ++ii;
                     }
                     const bool sh = ii < n_sh;
-                    const uint32_t mine = a.inst[ii].pair[g];
-                    cnt = a.inst[ii].count;
-                    const uint32_t p = __shfl_sync(0xffffffffu, mine, 4 * min(g, cnt - 1u) + t);   // past the count: the last row
+                    cnt = tab.count[ii];
+                    const uint32_t p = pair_of(ii, min(g, cnt - 1u));   // past the count: the last row
                     if constexpr (P1) {
                         row = a.xh + (size_t)(sh ? p : p / a.top_k) * D;
                     } else {
@@ -572,105 +810,165 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
                     stage_group<BITS, GROUP>(xb, jb, gb, cb, bb, BufferLayout(gb, H, cb), lane);
                 }
             }
-            if (u < n && i < i1 && i != cur) {   // (its loads run while the others stage)
-                announce();
-                open_instance(dsm0 + __shfl_sync(0xffffffffu, at, i - i0));
-            }
             __syncthreads();
-            for (; u < n && i < i1; u += pace) {
-                if (i != cur) {
-                    announce();
-                    open_instance(dsm0 + __shfl_sync(0xffffffffu, at, i - i0));
-                }
-                const uint32_t bar_at = slot * 8, rb = dsm0 + G.off_red + slot * W * (kRedWarp * 4);
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);   // column g, rows t, t + 4, t + 8, t + 12
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
-                if (!finisher) {
-                    if (!try_slot(full + bar_at, par) && !wait_slot_slow(full + bar_at, par)) give_up();
-                    const uint32_t mo = slot * (P1 ? G.slot_bytes : G.m_bytes2);
-                    if (a.expert_bias && wi == 0) {
-                        acc[0] = acc[1] = bf16_bits_to_f32((uint16_t)lds16(ab_at + mo));
-                        acc[2] = acc[3] = bf16_bits_to_f32((uint16_t)lds16(ab_at + mo + 16));
+            // The units of the staged instances, by what the warp does with them (a copy of the loop each: it holds only
+            // that role's registers): multiplies, finishes, or, in a team of one, both.
+            auto units = [&](auto role) {
+                constexpr bool MUL = decltype(role)::value != 1, FIN = decltype(role)::value != 0, ONE = MUL && FIN;
+                uint32_t cur = 0xffffffffu, count = 0, groups_left = 0, pieces = 0;
+                uint32_t b0 = 0, cq0 = 0, z0 = 0, sB = 0, w_at = 0, s_at = 0, ab_at = 0, d_s = 0, d_z = 0, k0 = 0;
+                uint16_t* dst = nullptr;   // gate/up: where column g's activations go
+                float* out0 = nullptr;     // down: where the rows of column g (ONE: columns 2t and 2t + 1) go, and their weights
+                float* out1 = nullptr;
+                float wt0 = 0.f, wt1 = 0.f;
+                uint32_t pend = 0;         // units of `cur` whose activations this warp wrote and has not announced
+                auto announce = [&]() {
+                    if (P1 && FIN && do2 && pend) {
+                        __syncwarp();
+                        if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(a.inst_done + cur), "r"(pend) : "memory");
+                        pend = 0;
                     }
-                    uint32_t w = w_at + slot * (P1 ? G.slot_bytes : G.w_bytes2), sc = s_at + mo, b = b0, cq = cq0, z = z0, kk = k0, left = groups_left;
-#pragma unroll 1
-                    for (uint32_t p = 0; p < pieces; ++p) {
-                        piece_tiles<BITS, GROUP, META, !AL>(w, sc, d_s, d_z, b, cq, z, sB, min(GP, left), kk, t, acc);
-                        w += 2048;
-                        sc += 2 * GP;
-                        b += GP * H * sB;
-                        cq += GP * 64;
-                        if constexpr (GP == 2) {
-                            kk ^= 2u;
-                            z += kk ? 0u : sB;
-                        } else {
-                            z += GP / 4 * sB;
+                };
+                auto open_instance = [&](uint32_t buf) {
+                    cur = i;
+                    const bool sh = i < n_sh;
+                    count = tab.count[i];
+                    const uint32_t col = min(g, count - 1u);
+                    if constexpr (MUL) {
+                        const uint32_t K = P1 ? D : sh ? a.f_shared : a.f, P = (K * BITS / 8 + 127) / 128, G2 = K / GROUP;
+                        const uint32_t p0 = P * wi / W;
+                        pieces = P * (wi + 1) / W - p0;
+                        groups_left = G2 - min(G2, p0 * GP);
+                        const BufferLayout lay(G2, H, count);
+                        sB = count * 64;
+                        b0 = buf + col * 64 + t * 16 + p0 * GP * H * sB;
+                        cq0 = buf + lay.cq_off + t * 16 + p0 * GP * 64;
+                        z0 = buf + lay.z_off + col * 64 + t * 16 + (GP == 2 ? p0 / 2 : p0 * (GP / 4)) * sB;
+                        k0 = GP == 2 ? 2 * (p0 & 1) : 0u;
+                        w_at = ring0 + w_lane + p0 * 2048;
+                        s_at = meta0 + (pr * G2 + p0 * GP) * 2;
+                        d_s = P1 ? 32 * G2 : 16 * G2;
+                        d_z = P1 ? 16 * G2 : 32 * G2;
+                        ab_at = meta0 - (P1 ? G.meta_off : 0u) + (P1 ? G.ab_off : G.ab_off2[sh]) + pr * 2;
+                    }
+                    if constexpr (FIN && P1) {
+                        const uint32_t pair = pair_of(i, col);
+                        const uint32_t F = sh ? a.f_shared : a.f;
+                        dst = g < count ? (sh ? a.acts_shared : a.acts) + (size_t)pair * F + (BITS == 4 ? 2 * t : t) : nullptr;
+                    } else if constexpr (FIN) {
+                        auto target = [&](uint32_t c, float*& out, float& w) {
+                            const uint32_t pair = pair_of(i, min(c, count - 1u));
+                            w = sh ? (a.shared_gate ? __ldcg(a.shared_gate + pair) : 1.0f) : pair_weight[pair];
+                            float* rows = a.accumulate ? a.yacc + (size_t)(sh ? pair : pair / a.top_k) * D
+                                                       : a.parts + ((size_t)pair + (sh ? a.T * a.top_k : 0u)) * D;
+                            out = c < count ? rows + (ONE ? pr : t) : nullptr;
+                        };
+                        target(ONE ? 2 * t : g, out0, wt0);
+                        if constexpr (ONE) target(2 * t + 1, out1, wt1);
+                    }
+                };
+                auto put = [&](float* at, float v) {
+                    if (a.accumulate) atomicAdd(at, v);
+                    else *at = v;
+                };
+                for (; u < n && i < i1; u += pace) {
+                    if (i != cur) {
+                        announce();
+                        open_instance(dsm0 + __shfl_sync(0xffffffffu, at, i - i0));
+                    }
+                    const uint32_t bar_at = slot * 8, rb = dsm0 + G.off_red + slot * W * (kRedWarp * 4);
+                    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                    if constexpr (MUL) {
+                        if (!try_slot(full + bar_at, par) && !wait_slot_slow(full + bar_at, par)) give_up();
+                        const uint32_t mo = slot * (P1 ? G.slot_bytes : G.m_bytes2);
+                        if (a.expert_bias && wi == 0) {
+                            acc[0] = acc[1] = bf16_bits_to_f32((uint16_t)lds16(ab_at + mo));
+                            acc[2] = acc[3] = bf16_bits_to_f32((uint16_t)lds16(ab_at + mo + 16));
                         }
-                        left -= GP;
-                    }
-                    if (P1 || W > 1) {
-                        const uint32_t at = rb + wi * (kRedWarp * 4) + my_red;
-                        sts32(at, acc[0]);
-                        sts32(at + kRedCol * 4, acc[1]);
-                        sts32(at + 8, acc[2]);
-                        sts32(at + kRedCol * 4 + 8, acc[3]);
-                    }
-                    __syncwarp();
-                    if (W > 1 && lane == 0) arrive(done + bar_at);
-                } else {
-                    if (!try_slot(done + bar_at, par) && !wait_slot_slow(done + bar_at, par)) give_up();
-                }
-                if (finisher || W == 1) {
-                    if (P1 || W > 1) {
-#pragma unroll 4
-                        for (uint32_t w = 0; w < W; ++w) {
-                            const uint4 p = lds128(rb + w * (kRedWarp * 4) + g * (kRedCol * 4) + t * 16);
-                            v.x += __uint_as_float(p.x); v.y += __uint_as_float(p.y); v.z += __uint_as_float(p.z); v.w += __uint_as_float(p.w);
+                        uint32_t w = w_at + slot * (P1 ? G.slot_bytes : G.w_bytes2), sc = s_at + mo, b = b0, cq = cq0, z = z0, kk = k0, left = groups_left;
+#pragma unroll 1
+                        for (uint32_t p = 0; p < pieces; ++p) {
+                            piece_tiles<BITS, GROUP, META, !AL>(w, sc, d_s, d_z, b, cq, z, sB, min(GP, left), kk, t, acc);
+                            w += 2048;
+                            sc += 2 * GP;
+                            b += GP * H * sB;
+                            cq += GP * 64;
+                            if constexpr (GP == 2) {
+                                kk ^= 2u;
+                                z += kk ? 0u : sB;
+                            } else {
+                                z += GP / 4 * sB;
+                            }
+                            left -= GP;
+                        }
+                        if (P1 || !ONE) {
+                            const uint32_t to = rb + wi * (kRedWarp * 4) + my_red;
+                            sts32(to, acc[0]);
+                            sts32(to + kRedCol * 4, acc[1]);
+                            sts32(to + 8, acc[2]);
+                            sts32(to + kRedCol * 4 + 8, acc[3]);
                         }
                         __syncwarp();
+                        if (!FIN && lane == 0) arrive(done + bar_at);
+                    } else {
+                        if (!try_slot(done + bar_at, par) && !wait_slot_slow(done + bar_at, par)) give_up();
                     }
-                    if (lane == 0 && u + n_slots < n) {
-                        uint32_t ri, rk;
-                        find(u + n_slots, ri, rk);
-                        ask(slot, ri, rk);
-                    }
-                    __syncwarp();
-                    if constexpr (P1) {
-                        const uint16_t h0 = act_to_half_bits(glu_of(v.x, v.z, a.activation), a.status);
-                        const uint16_t h1 = act_to_half_bits(glu_of(v.y, v.w, a.activation), a.status);
-                        if (dst) {
-                            if constexpr (BITS == 4) {   // rows t and t + 4 are neighbours in the operand order
-                                *(uint32_t*)(dst + k * 8) = h0 | ((uint32_t)h1 << 16);
-                            } else {
-                                dst[k * 8] = h0;
-                                dst[k * 8 + 4] = h1;
+                    if constexpr (FIN) {
+                        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);   // column g, rows t, t + 4, t + 8, t + 12
+                        if (P1 || !ONE) {
+#pragma unroll 4
+                            for (uint32_t w = 0; w < (ONE ? 1u : W); ++w) {
+                                const uint4 p = lds128(rb + w * (kRedWarp * 4) + g * (kRedCol * 4) + t * 16);
+                                v.x += __uint_as_float(p.x); v.y += __uint_as_float(p.y); v.z += __uint_as_float(p.z); v.w += __uint_as_float(p.w);
                             }
+                            __syncwarp();
                         }
-                        ++pend;
-                    } else if (W == 1) {
-                        if (out0) {
-                            put(out0 + k * 16, wt0 * acc[0]);
-                            put(out0 + k * 16 + 8, wt0 * acc[2]);
+                        if (lane == 0 && u + n_slots < n) {
+                            uint32_t ri, rk;
+                            find(u + n_slots, ri, rk);
+                            ask(slot, ri, rk);
                         }
-                        if (out1) {
-                            put(out1 + k * 16, wt1 * acc[1]);
-                            put(out1 + k * 16 + 8, wt1 * acc[3]);
+                        __syncwarp();
+                        if constexpr (P1) {
+                            const uint16_t h0 = act_to_half_bits(glu_of(v.x, v.z, a.activation), a.status);
+                            const uint16_t h1 = act_to_half_bits(glu_of(v.y, v.w, a.activation), a.status);
+                            if (dst) {
+                                if constexpr (BITS == 4) {   // rows t and t + 4 are neighbours in the operand order
+                                    *(uint32_t*)(dst + k * 8) = h0 | ((uint32_t)h1 << 16);
+                                } else {
+                                    dst[k * 8] = h0;
+                                    dst[k * 8 + 4] = h1;
+                                }
+                            }
+                            ++pend;
+                        } else if constexpr (ONE) {
+                            if (out0) {
+                                put(out0 + k * 16, wt0 * acc[0]);
+                                put(out0 + k * 16 + 8, wt0 * acc[2]);
+                            }
+                            if (out1) {
+                                put(out1 + k * 16, wt1 * acc[1]);
+                                put(out1 + k * 16 + 8, wt1 * acc[3]);
+                            }
+                        } else if (out0) {
+                            float* o = out0 + k * 16;
+                            put(o, wt0 * v.x);
+                            put(o + 4, wt0 * v.y);
+                            put(o + 8, wt0 * v.z);
+                            put(o + 12, wt0 * v.w);
                         }
-                    } else if (out0) {
-                        float* o = out0 + k * 16;
-                        put(o, wt0 * v.x);
-                        put(o + 4, wt0 * v.y);
-                        put(o + 8, wt0 * v.z);
-                        put(o + 12, wt0 * v.w);
                     }
+                    step(i, k);
+                    slot += pace;
+                    if (slot >= n_slots) { slot -= n_slots; par ^= 1u; }
                 }
-                step(i, k);
-                slot += pace;
-                if (slot >= n_slots) { slot -= n_slots; par ^= 1u; }
-            }
+                announce();
+            };
+            if (finisher) units(std::integral_constant<int, 1>());
+            else if (W == 1) units(std::integral_constant<int, 2>());
+            else units(std::integral_constant<int, 0>());
             i0 = i1;
         }
-        announce();
     };
 
     if (do1) phase(std::integral_constant<int, 1>());
@@ -686,17 +984,10 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
     // (warps go round the blocks, so that a small call keeps every SM busy)
     const uint32_t half = D / 2, items = a.T * half, stride = gridDim.x * kThreads;
     uint32_t j = (warp * gridDim.x + blockIdx.x) * 32 + lane;
-    auto live_of = [&](uint32_t tk) {
-        uint32_t live = 0;
-#pragma unroll
-        for (uint32_t q = 0; q < SHRIKE_MAX_TOP_K; ++q)
-            if (q < a.top_k && a.pair_cell[tk * a.top_k + q] != SHRIKE_SLOT_MISS) live |= 1u << q;
-        return live;
-    };
     uint32_t live = 0;
     float h0 = 0.f, h1 = 0.f;
     if (j < items) {
-        live = live_of(j / half);
+        live = tab.live[j / half];
         if (a.hidden) {
             h0 = load_act(a.hidden, (size_t)j * 2, a.act_dtype);
             h1 = load_act(a.hidden, (size_t)j * 2 + 1, a.act_dtype);
@@ -705,7 +996,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
     if (!grid_sync(a.arrived)) give_up();
     for (bool first = true; j < items; j += stride, first = false) {
         const uint32_t tk = j / half, c = j - tk * half;
-        if (!first) live = live_of(tk);
+        if (!first) live = tab.live[tk];
         float2 s = make_float2(0.f, 0.f), p[SHRIKE_MAX_TOP_K];
         if (n_sh) s = __ldcg((const float2*)(a.parts + ((size_t)a.T * a.top_k + tk) * D) + c);
 #pragma unroll
@@ -750,8 +1041,8 @@ bool stream_geometry(const shrike_moe_config& c, uint32_t smem_optin, StreamGeom
         g.ab_off2[sh] = align_up(64 * (F / c.group_size), 128);
         g.m_bytes2 = std::max(g.m_bytes2, g.ab_off2[sh] + (c.expert_bias ? 128u : 0u));
     }
-    const uint32_t least = std::max(buffer(G1), buffer(std::max(G2, Gs))), most_pieces2 = g.w_bytes2 / 2048;
-    const uint32_t budget = smem_optin - 3072 - 1024;   // less the static part, the reserved kilobyte, the ring's alignment
+    const uint32_t least = std::max({buffer(G1), buffer(std::max(G2, Gs)), (uint32_t)sizeof(RouteScratch)}), most_pieces2 = g.w_bytes2 / 2048;
+    const uint32_t budget = smem_optin - kStaticBytes - 1024;   // less the static part and the ring's alignment
     if (least > budget) return false;
     // Teams as small as leaves every team two slots (more warps on a unit mean more partial sums), no smaller than four
     // pieces a warp needs. Slots are a multiple of the teams: a team that runs ahead then cannot take an older round of
@@ -773,16 +1064,17 @@ bool stream_geometry(const shrike_moe_config& c, uint32_t smem_optin, StreamGeom
     const uint32_t ring = std::max(g.n_slots * g.slot_bytes, g.n_slots2 * (g.w_bytes2 + g.m_bytes2));
     const uint32_t red = std::max(g.n_slots * g.w1, g.w2 > 1 ? g.n_slots2 * g.w2 : 0u) * kRedWarp * 4;
     if (ring + red + least > budget) return false;
-    g.off_red = (budget - ring - red) / 128 * 128;
-    g.off_ring = align_up(g.off_red + red, 1024);
-    if (g.off_ring > budget + 1023 - ring) { g.off_red -= 1024; g.off_ring -= 1024; }
+    g.off_ring = (budget - ring) / 1024 * 1024;
+    if (g.off_ring < red + least) return false;
+    g.off_red = (g.off_ring - red) / 128 * 128;
     if (g.off_red < least) return false;
+    g.ring_bytes = ring;
     g.smem_bytes = g.off_ring + ring + 1024;
     return true;
 }
 
 template <int BITS, int GROUP, int META, bool AL>
-cudaError_t launch_stream_t(const shrike_moe* m, cudaStream_t st, StreamArgs& a, bool pdl) {
+cudaError_t launch_stream_t(const shrike_moe* m, cudaStream_t st, const StreamArgs& a, const BlockMaps& maps, bool pdl) {
     auto k = expert_stream_kernel<BITS, GROUP, META, AL>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.g.smem_bytes);
     if (e != cudaSuccess) return e;
@@ -805,16 +1097,16 @@ cudaError_t launch_stream_t(const shrike_moe* m, cudaStream_t st, StreamArgs& a,
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, k, a);
+    return cudaLaunchKernelEx(&cfg, k, a, maps);
 }
 
 template <int BITS, int GROUP, int META>
-cudaError_t launch_stream_m(const shrike_moe* m, cudaStream_t st, StreamArgs& a, bool pdl) {
+cudaError_t launch_stream_m(const shrike_moe* m, cudaStream_t st, const StreamArgs& a, const BlockMaps& maps, bool pdl) {
     // every row whole 128-byte pieces?
     const shrike_moe_config& c = m->cfg;
     const uint32_t gp = 128 / (GROUP * BITS / 8);
     const bool al = c.d / GROUP % gp == 0 && c.f / GROUP % gp == 0 && (!c.has_shared || c.shared_f / GROUP % gp == 0);
-    return al ? launch_stream_t<BITS, GROUP, META, true>(m, st, a, pdl) : launch_stream_t<BITS, GROUP, META, false>(m, st, a, pdl);
+    return al ? launch_stream_t<BITS, GROUP, META, true>(m, st, a, maps, pdl) : launch_stream_t<BITS, GROUP, META, false>(m, st, a, maps, pdl);
 }
 
 }  // namespace
@@ -824,10 +1116,26 @@ size_t stream_parts_bytes(const shrike_moe_config& c) {
     return T * (c.top_k + (c.has_shared ? 1u : 0u)) * c.d * 4;
 }
 
-// phases: 1, 2 or both. accumulate: phase 2 adds into ea.yacc (prefill) instead of writing y and hidden.
-// cudaErrorNotSupported when the shape does not fit: nothing was launched.
+size_t stream_done_bytes() { return kMaxTable * 4; }
+
+// How many groups the call's rows form for the logits: with more rows than two warps' worth a block takes a part of them
+// against more expert rows, since the experts' rows are on the block's chip already and the activations are not. 0 when a
+// block's rows of the router do not fit into the ring.
+static uint32_t stream_token_groups(const shrike_moe_config& c, uint32_t sm_count, uint32_t T, uint32_t ring_bytes) {
+    const uint32_t rows = c.num_experts + (c.shared_gated ? 1u : 0u), bits = c.router_weight_bits;
+    const uint32_t row_bytes = bits ? c.d * bits / 8 + c.d / 64 * 8 : c.d * 4;
+    for (uint32_t n = T <= 16 ? 1 : T <= 32 ? 2 : 4; n; n /= 2) {
+        const uint32_t nbx = sm_count / n, most = (rows + nbx - 1) / nbx;
+        if (nbx && most * row_bytes + c.d * 4 + 16 + 2 * c.d * 4 <= ring_bytes) return n;
+    }
+    return 0;
+}
+
+// phases: 1, 2 or both. accumulate: phase 2 adds into ea.yacc (prefill) instead of writing y and hidden. route (with both
+// phases): the launch routes the rows itself and needs no plan. cudaErrorNotSupported when the shape does not fit: nothing
+// was launched.
 cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const ExpertArgs& ea, uint32_t T, uint32_t n_shared,
-                                 uint32_t phases, bool accumulate, void* y, void* hidden, bool pdl) {
+                                 uint32_t phases, bool accumulate, void* y, void* hidden, bool pdl, const RouterArgs* route) {
     const shrike_moe_config& c = m->cfg;
     const uint64_t cpc = ea.pool.cells_per_chunk ? ea.pool.cells_per_chunk : 1;
     if (cpc < 2 || (uint64_t)ea.pool.cells * cpc >= (1ull << 32)) return cudaErrorNotSupported;
@@ -835,27 +1143,33 @@ cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const Exp
     if (!maps) return cudaErrorNotSupported;
     StreamArgs a;
     memset(&a, 0, sizeof a);
-    a.maps = *maps;
     if (!stream_geometry(c, m->smem_optin, a.g)) return cudaErrorNotSupported;
     a.pool = ea.pool; a.routed = ea.routed; a.shared = ea.shared; a.shared_block = ea.shared_block;
     a.d = c.d; a.f = c.f; a.f_shared = c.has_shared ? c.shared_f : 0; a.top_k = c.top_k;
     a.activation = c.activation; a.expert_bias = c.expert_bias; a.act_dtype = c.act_dtype; a.y_dtype = c.y_dtype;
     a.inst = ea.inst; a.n_inst = ea.n_inst; a.n_shared = n_shared;
     a.xh = ea.xh; a.acts = ea.acts; a.acts_shared = ea.acts_shared; a.yacc = ea.yacc;
-    a.parts = m->ws.parts; a.pair_cell = m->ws.pair_cell;
+    a.parts = m->ws.parts; a.sorted = ea.sorted; a.pair_cell = m->ws.pair_cell;
+    for (a.n_chunks = 0; a.n_chunks < SHRIKE_MAX_POOL_CHUNKS && ea.pool.base[a.n_chunks];) ++a.n_chunks;
+    if (route) {
+        a.routes = 1;
+        a.r = *route;
+        a.token_groups = stream_token_groups(c, m->sm_count, T, a.g.ring_bytes);
+        if (!a.token_groups) return cudaErrorNotSupported;
+    }
     a.route_w = ea.route_w; a.shared_gate = ea.shared_gate; a.status = ea.status; a.arrived = m->ws.arrived; a.inst_done = m->ws.inst_done;
     a.T = T; a.y = y; a.hidden = hidden; a.phases = phases; a.accumulate = accumulate ? 1u : 0u;
     a.rcp_cpc = (uint32_t)(((1ull << 32) + cpc - 1) / cpc);
     const uint32_t bits = c.weight_bits, grp = c.group_size;
     const bool f16 = c.meta_dtype == SHRIKE_DTYPE_FP16;
-    if (bits == 4 && grp == 64 && !f16) return launch_stream_m<4, 64, SHRIKE_DTYPE_BF16>(m, st, a, pdl);
-    if (bits == 4 && grp == 64 && f16) return launch_stream_m<4, 64, SHRIKE_DTYPE_FP16>(m, st, a, pdl);
-    if (bits == 4 && grp == 32 && !f16) return launch_stream_m<4, 32, SHRIKE_DTYPE_BF16>(m, st, a, pdl);
-    if (bits == 4 && grp == 32 && f16) return launch_stream_m<4, 32, SHRIKE_DTYPE_FP16>(m, st, a, pdl);
-    if (bits == 8 && grp == 64 && !f16) return launch_stream_m<8, 64, SHRIKE_DTYPE_BF16>(m, st, a, pdl);
-    if (bits == 8 && grp == 64 && f16) return launch_stream_m<8, 64, SHRIKE_DTYPE_FP16>(m, st, a, pdl);
-    if (bits == 8 && grp == 32 && !f16) return launch_stream_m<8, 32, SHRIKE_DTYPE_BF16>(m, st, a, pdl);
-    if (bits == 8 && grp == 32 && f16) return launch_stream_m<8, 32, SHRIKE_DTYPE_FP16>(m, st, a, pdl);
+    if (bits == 4 && grp == 64 && !f16) return launch_stream_m<4, 64, SHRIKE_DTYPE_BF16>(m, st, a, *maps, pdl);
+    if (bits == 4 && grp == 64 && f16) return launch_stream_m<4, 64, SHRIKE_DTYPE_FP16>(m, st, a, *maps, pdl);
+    if (bits == 4 && grp == 32 && !f16) return launch_stream_m<4, 32, SHRIKE_DTYPE_BF16>(m, st, a, *maps, pdl);
+    if (bits == 4 && grp == 32 && f16) return launch_stream_m<4, 32, SHRIKE_DTYPE_FP16>(m, st, a, *maps, pdl);
+    if (bits == 8 && grp == 64 && !f16) return launch_stream_m<8, 64, SHRIKE_DTYPE_BF16>(m, st, a, *maps, pdl);
+    if (bits == 8 && grp == 64 && f16) return launch_stream_m<8, 64, SHRIKE_DTYPE_FP16>(m, st, a, *maps, pdl);
+    if (bits == 8 && grp == 32 && !f16) return launch_stream_m<8, 32, SHRIKE_DTYPE_BF16>(m, st, a, *maps, pdl);
+    if (bits == 8 && grp == 32 && f16) return launch_stream_m<8, 32, SHRIKE_DTYPE_FP16>(m, st, a, *maps, pdl);
     return cudaErrorInvalidValue;
 }
 

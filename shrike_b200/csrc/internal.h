@@ -79,7 +79,7 @@ struct Workspace {
     uint32_t* n_inst = nullptr;
     uint32_t* status = nullptr;     // device status word
     uint32_t* done_counter = nullptr; // blocks finished, fused route kernel
-    uint32_t* arrived = nullptr;    // blocks past phase 2 of the streaming expert kernel, over all launches
+    unsigned long long* arrived = nullptr;   // grid barriers of the streaming expert kernel: arrivals over all launches
     uint32_t* inst_done = nullptr;  // its finished gate/up units of every instance; the plan zeroes them
     float* parts = nullptr;         // its weighted rows per pair and per shared row [<= 64 tokens x (top_k + 1) x d]
     uint32_t* pair_cell = nullptr;  // decode plan: cell of every pair, or SHRIKE_SLOT_MISS
@@ -178,9 +178,12 @@ cudaError_t launch_phase1(const shrike_moe* m, cudaStream_t st, const ExpertArgs
 cudaError_t launch_phase2(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, uint32_t T,
                           uint32_t max_inst, void* y, void* hidden, bool pdl);
 // expert_stream.cu
+struct RouterArgs;
 cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const ExpertArgs& ea, uint32_t T, uint32_t n_shared,
-                                 uint32_t phases, bool accumulate, void* y, void* hidden, bool pdl);
+                                 uint32_t phases, bool accumulate, void* y, void* hidden, bool pdl,
+                                 const RouterArgs* route = nullptr);
 size_t stream_parts_bytes(const shrike_moe_config& c);
+size_t stream_done_bytes();
 // synth.cu
 cudaError_t launch_synth_fill(const shrike_moe* m, cudaStream_t st, const PoolView& pool,
                               uint32_t first_cell, uint32_t count, uint64_t seed, uint32_t layer,

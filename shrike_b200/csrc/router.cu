@@ -13,6 +13,7 @@
 // 64g+2l+1 of every group g, as the shader does. exp() is a fixed sequence of
 // fp32 operations (exp_det) instead of the library routine for the same reason.
 #include "plan.cuh"
+#include "route_args.cuh"
 #include "router_math.cuh"
 #include "select.cuh"
 
@@ -20,46 +21,6 @@ namespace shrike {
 
 constexpr int kRouterWarps = 8;       // expert rows per block (router_gemv_r4 has four); the block that finishes last
                                       // selects with as many warps
-
-struct RouterArgs {
-    const void* w;                 // fp32 rows, or packed affine rows
-    const uint16_t* scales;        // affine only
-    const uint16_t* biases;        // affine only
-    uint32_t bits;                 // 0 = fp32
-    const float* gate_row;         // shared expert scalar gate row or NULL
-    const uint16_t* eff_scale;
-    const uint16_t* logit_bias;
-    const uint16_t* per_expert_scale;
-    const void* hidden;
-    uint32_t T, stride, dt, ne, d, top_k;
-    uint32_t sigmoid_scores;
-    float scaling;
-    uint32_t round_f16;
-    float* logits;
-    uint32_t* ids;
-    float* weights;
-    float* gate_out;
-    uint32_t tokens_per_block;
-    uint32_t no_tail;              // fused decode: stop after the logits and the operand copy (the expert kernels route)
-    uint32_t row_base;             // first row of this launch (the tiled prefill router leaves only the gate row)
-    // fused decode tail (route_fused_kernel only)
-    const uint64_t* table;
-    uint32_t pool_cells;
-    const uint32_t* io_status;
-    uint32_t with_shared, int4, group;
-    uint32_t* slots;
-    uint32_t* counts;
-    Instance* inst;
-    uint32_t* n_inst;
-    uint32_t* sorted;
-    uint16_t* xh;
-    float* xsum;
-    uint32_t* done_counter;
-    uint32_t* pair_cell;
-    uint32_t* inst_done;
-    uint32_t* status;
-    uint32_t max_inst;
-};
 
 // Logits (and the shared expert's scalar gate as row `ne`) of this warp's row
 // for the block's tokens. `pre` runs between the weight-row prefetch and the
@@ -103,58 +64,6 @@ __device__ __forceinline__ void logits_body(const RouterArgs& a, Pre pre) {
     if (a.d == 2048) logits_rows<16, false>(a, pre);
     else if (a.d == 2304) logits_rows<18, false>(a, pre);
     else logits_rows<kRouterMaxChunks, true>(a, pre);
-}
-
-// Top-k of one row by one warp. The (score desc, expert asc) order is total,
-// so K rounds of a warp arg-max give exactly the list the reference's
-// insertion scan builds (moe.metal:436-456). Lane r returns the r-th pick.
-// CG: read the logits past L1 (they were written by other blocks of this launch).
-template <bool CG>
-__device__ __forceinline__ void select_row(const float* lg, const RouterArgs& a, uint32_t lane,
-                                           uint32_t& out_id, float& out_w) {
-    const uint32_t ne = a.ne, top_k = a.top_k;
-    // order-preserving integer keys (0 = not a candidate): one warp-wide max and one warp-wide min per pick
-    uint32_t key[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) key[i] = selection_key<CG>(lg, a, lane + 32 * i);
-    float my_score = 0.f;
-    uint32_t my_id = 0;
-    for (uint32_t r = 0; r < top_k; ++r) {
-        uint32_t bestk = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) bestk = max(bestk, key[i]);
-        const uint32_t wmax = __reduce_max_sync(0xffffffffu, bestk);
-        uint32_t cand = 0xffffffffu;
-#pragma unroll
-        for (int i = 7; i >= 0; --i) cand = (key[i] == wmax && wmax != 0u) ? lane + 32u * i : cand;
-        const uint32_t win = __reduce_min_sync(0xffffffffu, cand);  // ties: the lower expert id
-        if (win != 0xffffffffu && (win & 31u) == lane) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) key[i] = (win >> 5) == (uint32_t)i ? 0u : key[i];
-        }
-        if (lane == r) {
-            my_score = score_of_key(wmax);
-            my_id = win == 0xffffffffu ? 0u : win;
-        }
-    }
-    // weights (moe.metal:458-490), sums in rank order
-    float val;
-    if (a.sigmoid_scores) {
-        val = lane < top_k ? sigmoid_det(CG ? __ldcg(lg + my_id) : lg[my_id]) : 0.f;
-    } else {
-        const float mx = __shfl_sync(0xffffffffu, my_score, 0);
-        val = lane < top_k ? exp_det(__fsub_rn(my_score, mx)) : 0.f;
-    }
-    float sum = 0.f;
-    for (uint32_t r = 0; r < top_k; ++r) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, val, r));
-    float w;
-    if (a.sigmoid_scores) w = __fmul_rn(val, __fdiv_rn(a.scaling, __fadd_rn(sum, 1e-20f)));
-    else w = __fdiv_rn(val, sum);
-    const float pes = a.per_expert_scale ? bf16_bits_to_f32(a.per_expert_scale[my_id]) : 1.0f;
-    w = __fmul_rn(w, pes);
-    if (a.round_f16) w = __half2float(__float2half_rn(w));
-    out_id = my_id;
-    out_w = w;
 }
 
 // grid (ceil((ne + has_gate)/4), token blocks)
@@ -653,9 +562,8 @@ __global__ void __launch_bounds__(1024) classify_kernel(const uint32_t* __restri
     }
 }
 
-static RouterArgs make_router_args(const shrike_moe* m, const shrike_router_operands& ops, const void* hidden,
-                                   uint32_t T, uint32_t stride, uint32_t* ids, float* weights,
-                                   float* shared_gate) {
+RouterArgs make_router_args(const shrike_moe* m, const shrike_router_operands& ops, const void* hidden, uint32_t T,
+                            uint32_t stride, uint32_t* ids, float* weights, float* shared_gate) {
     const shrike_moe_config& c = m->cfg;
     RouterArgs a = {};
     a.w = ops.weights; a.scales = ops.scales; a.biases = ops.biases; a.bits = c.router_weight_bits;

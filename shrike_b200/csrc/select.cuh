@@ -97,6 +97,72 @@ __device__ __forceinline__ float selection_weight(const float* lg, const A& a, u
     return w;
 }
 
+// Top-k of one row by one warp. The (score desc, expert asc) order is total,
+// so K rounds of a warp arg-max give exactly the list the reference's
+// insertion scan builds (moe.metal:436-456). Lane r returns the r-th pick.
+// CG: read the logits past L1 (they were written by other blocks of this launch).
+template <bool CG, class A>
+__device__ __forceinline__ void select_row(const float* lg, const A& a, uint32_t lane,
+                                           uint32_t& out_id, float& out_w) {
+    const uint32_t ne = a.ne, top_k = a.top_k;
+    // order-preserving integer keys (0 = not a candidate): one warp-wide max and one warp-wide min per pick
+    uint32_t key[8];
+    {
+        // all logits (and biases) are requested before the first is used
+        float raw[8];
+        uint16_t lb[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t e = lane + 32 * i;
+            raw[i] = e < ne ? (CG ? __ldcg(lg + e) : lg[e]) : 0.f;
+            lb[i] = a.logit_bias && e < ne ? a.logit_bias[e] : (uint16_t)0;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float score = a.sigmoid_scores ? sigmoid_det(raw[i]) : raw[i];
+            key[i] = lane + 32 * i < ne ? key_of_score(__fadd_rn(score, bf16_bits_to_f32(lb[i]))) : 0u;
+        }
+    }
+    float my_score = 0.f;
+    uint32_t my_id = 0;
+    for (uint32_t r = 0; r < top_k; ++r) {
+        uint32_t bestk = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) bestk = max(bestk, key[i]);
+        const uint32_t wmax = __reduce_max_sync(0xffffffffu, bestk);
+        uint32_t cand = 0xffffffffu;
+#pragma unroll
+        for (int i = 7; i >= 0; --i) cand = (key[i] == wmax && wmax != 0u) ? lane + 32u * i : cand;
+        const uint32_t win = __reduce_min_sync(0xffffffffu, cand);  // ties: the lower expert id
+        if (win != 0xffffffffu && (win & 31u) == lane) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) key[i] = (win >> 5) == (uint32_t)i ? 0u : key[i];
+        }
+        if (lane == r) {
+            my_score = score_of_key(wmax);
+            my_id = win == 0xffffffffu ? 0u : win;
+        }
+    }
+    // weights (moe.metal:458-490), sums in rank order
+    float val;
+    if (a.sigmoid_scores) {
+        val = lane < top_k ? sigmoid_det(CG ? __ldcg(lg + my_id) : lg[my_id]) : 0.f;
+    } else {
+        const float mx = __shfl_sync(0xffffffffu, my_score, 0);
+        val = lane < top_k ? exp_det(__fsub_rn(my_score, mx)) : 0.f;
+    }
+    float sum = 0.f;
+    for (uint32_t r = 0; r < top_k; ++r) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, val, r));
+    float w;
+    if (a.sigmoid_scores) w = __fmul_rn(val, __fdiv_rn(a.scaling, __fadd_rn(sum, 1e-20f)));
+    else w = __fdiv_rn(val, sum);
+    const float pes = a.per_expert_scale ? bf16_bits_to_f32(a.per_expert_scale[my_id]) : 1.0f;
+    w = __fmul_rn(w, pes);
+    if (a.round_f16) w = __half2float(__float2half_rn(w));
+    out_id = my_id;
+    out_w = w;
+}
+
 struct alignas(16) SelectSmem {
     uint32_t keys[SHRIKE_MAX_EXPERTS];   // read back 16 bytes at a time
     uint32_t cand_key[32], cand_id[32];
