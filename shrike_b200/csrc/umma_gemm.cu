@@ -106,6 +106,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
+// One lane of the converged warp, the same one every time.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -248,7 +254,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, c
     const uint32_t G = kdim / GROUP;
     // scale rows that are whole 16-byte units come by TMA; others (G % 8 != 0) are read by the converters
     const bool sc_tma = (G & 7u) == 0;
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t N = (in.count + 15u) & ~15u;           // MMA N: rows padded to 16
     uint32_t ncols = 32;                                   // TMEM columns of one accumulator
     while (ncols < N) ncols <<= 1;
@@ -451,32 +457,41 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, c
                 if (++st == a_stages) { st = 0; ++a_round; }
             }
         }
-    } else if (warp == kConvWarps && lane == 0) {
+    } else if (warp == kConvWarps) {
         // ---------------- MMA issue ----------------
-        const uint32_t idesc = umma_idesc(N);
-        uint32_t sa = 0, a_round = 0;
-        for (uint32_t kb = 0; kb < KB; ++kb) {
-            const uint32_t sb = kb % kBStages;
-            if (!pipe_wait(&a_full[sa], a_round & 1) || !pipe_wait(&b_full[sb], (kb / kBStages) & 1)) {
+        // The whole warp walks the loop on warp-uniform values and one elected lane issues: a branch on the lane number
+        // made every descriptor a per-thread value, and eight instructions took 550 to 750 cycles to issue.
+        const uint32_t idesc = __shfl_sync(0xffffffffu, umma_idesc(N), 0), acc0 = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const uint32_t acc1 = acc0 + __shfl_sync(0xffffffffu, ncols, 0), stages = __shfl_sync(0xffffffffu, a_stages, 0);
+        const uint32_t a_smem = __shfl_sync(0xffffffffu, smem_base + off_a, 0), b_smem = __shfl_sync(0xffffffffu, smem_base, 0);
+        const uint32_t b_step = __shfl_sync(0xffffffffu, b_stage, 0), n_kb = __shfl_sync(0xffffffffu, KB, 0);
+        uint32_t sa = 0, a_round = 0, sb = 0, b_round = 0;
+        for (uint32_t kb = 0; kb < n_kb; ++kb) {
+            if (!pipe_wait(&b_full[sb], b_round & 1) || !pipe_wait(&a_full[sa], a_round & 1)) {
                 give_up();
                 break;
             }
+            __syncwarp();
             tc_fence_after();
-            const uint32_t a_addr = smem_base + off_a + sa * kAStageBytes;
-            const uint64_t da0 = umma_smem_desc(a_addr), da1 = umma_smem_desc(a_addr + kTileBytes);
-            const uint64_t db = umma_smem_desc(smem_base + sb * b_stage);
-            // 4 x K16 per 64-wide block: 32 bytes further along the row. The two tiles alternate: consecutive
-            // instructions then add into different accumulators.
+            if (elect_one()) {
+                const uint64_t da0 = umma_smem_desc(a_smem + sa * kAStageBytes), da1 = umma_smem_desc(a_smem + sa * kAStageBytes + kTileBytes);
+                const uint64_t db = umma_smem_desc(b_smem + sb * b_step);
+                // 4 x K16 per 64-wide block: 32 bytes further along the row. The two tiles alternate: consecutive
+                // instructions then add into different accumulators.
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) {
-                umma_f16(tmem_base, da0 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-                umma_f16(tmem_base + ncols, da1 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                for (uint32_t k = 0; k < 4; ++k) {
+                    umma_f16(acc0, da0 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                    umma_f16(acc1, da1 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                }
+                umma_commit(&a_empty[sa]);
+                umma_commit(&b_empty[sb]);
             }
-            umma_commit(&a_empty[sa]);
-            umma_commit(&b_empty[sb]);
-            if (++sa == a_stages) { sa = 0; ++a_round; }
+            __syncwarp();
+            if (++sa == stages) { sa = 0; ++a_round; }
+            if (++sb == kBStages) { sb = 0; ++b_round; }
         }
-        umma_commit(accum);
+        if (elect_one()) umma_commit(accum);
+        __syncwarp();
     } else if (warp == kConvWarps + 1 && lane == 0) {
         // ---------------- activation tiles ----------------
         // One or two boxes per K block: these tiles are most of what a block pulls out of L2, and a short instance
