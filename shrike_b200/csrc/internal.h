@@ -89,7 +89,7 @@ struct Workspace {
     uint32_t* slot_of_expert = nullptr;
     float* yacc = nullptr;          // prefill: fp32 output accumulator [max_tokens x d]
     void* chunk_inst = nullptr;     // prefill: instances of up to 256 rows (tensor-core path)
-    uint32_t* n_chunk_inst = nullptr; // [0] instances, [1] sorted rows
+    uint32_t* n_chunk_inst = nullptr; // [0] instances, [1] sorted rows, [2], [3] tiles handed out per phase
     uint16_t* xs = nullptr;         // prefill: fp16 activation rows in expert-sorted order [max_tokens x top_k x d]
     void* tensor_maps = nullptr;    // host: the TMA descriptors of xs, acts, xh, acts_shared
     // one-row decode layer in one launch (fused_layer.cu)

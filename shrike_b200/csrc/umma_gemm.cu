@@ -37,8 +37,7 @@
 // Every wait is bounded; a wait that gives up sets the status word and the
 // block falls through to the TMEM release.
 #include <cuda.h>
-// -DSHRIKE_TRACE: every block records entry / set-up / accumulators-ready / exit timestamps
-// in the handle's trace buffer (shrike_debug_set_trace, debug builds only); compiled out of the shipped library.
+#include <algorithm>
 
 #include "internal.h"
 
@@ -59,8 +58,8 @@ constexpr uint32_t kOffA = kBStages * kBTileBytes;
 constexpr uint32_t kOffPk = kOffA + kAStages * kAStageBytes;
 constexpr uint32_t kOffSc = kOffPk + kPkSlots * kPkSlotBytes;
 constexpr uint32_t kOffBar = kOffSc + 2 * kScHalfBytes;
-constexpr uint32_t kNumBars = 2 * kMaxAStages + 2 * kBStages + 2 * kPkSlots + 3;
-constexpr uint32_t kUmmaSmemBytes = kOffBar + kNumBars * 8 + 2 * kUmmaMaxN * 4 + 16 + 1024 /*alignment slack*/;
+constexpr uint32_t kNumBars = 2 * kMaxAStages + 2 * kBStages + 2 * kPkSlots + 3 + 5;
+constexpr uint32_t kUmmaSmemBytes = kOffBar + kNumBars * 8 + 4 * kUmmaMaxN * 4 + 16 + 1024 /*alignment slack*/;
 
 struct WeightMaps {       // TMA descriptors of the two 128-row tiles of a block
     CUtensorMap w[2];     // packed weights   [cells][rows][row bytes]
@@ -94,17 +93,6 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint6
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 // One lane of the converged warp, the same one every time.
 __device__ __forceinline__ bool elect_one() {
@@ -161,11 +149,10 @@ __device__ __forceinline__ uint32_t half2_dup(float v) {
     return h | (h << 16);
 }
 
-__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
+__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
         : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
@@ -220,15 +207,38 @@ __device__ __forceinline__ uint16_t pick16(const uint32_t (&v)[4], uint32_t idx)
     return (uint16_t)((idx & 1u) ? (w >> 16) : (w & 0xffffu));
 }
 
-struct ChunkInstance {  // up to 256 rows that share one expert block
+struct alignas(16) ChunkInstance {  // up to 256 rows that share one expert block
     uint32_t kind, slot, first, count;
 };
 
-// grid (row tiles, max chunk instances); block 608.
+// The instance's rows as one or two boxes of 16 << i rows (the largest that fits, then the smallest that holds the
+// rest), and the layout of the activation and weight stages. An instance with few rows needs narrow activation tiles and
+// gets more weight stages instead: what paces such a tile is the round trip converters -> tensor core -> converters.
+struct TileShape {
+    uint32_t N, n1, b1, n2, b2, b_stage, off_a, a_stages;
+    __device__ explicit TileShape(uint32_t count) {
+        N = (count + 15u) & ~15u;           // MMA N: rows padded to 16
+        n1 = 16; b1 = 0;
+        while ((n1 << 1) <= N && b1 + 1 < (uint32_t)kActBoxes) { n1 <<= 1; ++b1; }
+        n2 = 0; b2 = 0;
+        if (N > n1) {
+            n2 = 16;
+            while (n2 < N - n1) { n2 <<= 1; ++b2; }
+        }
+        // three layouts: 64, 128 or 256 activation rows a stage
+        b_stage = N <= 64 ? 64u * 128u : N <= 128 ? 128u * 128u : 256u * 128u;
+        off_a = kBStages * b_stage;
+        a_stages = min(kMaxAStages, (kOffPk - off_a) / kAStageBytes);
+    }
+};
+
+// A persistent block per SM; tiles (instance, 128 or 256 weight rows) come from a counter, in list order. The copy
+// threads run ahead into the next tile while the converters finish this one: as one block per tile, set-up, the first
+// copies' way and the launch gap cost 4 us of every tile's 8 (512 x 16 columns) to 37 (2048 x 256).
 template <int BITS, int GROUP, int META, int PHASE>
 __global__ void __launch_bounds__(kUmmaThreads, 1)
-umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, const uint32_t* __restrict__ n_inst,
-                   const __grid_constant__ UmmaMaps maps) {
+umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, uint32_t* __restrict__ n_inst,
+                   const uint32_t row_tiles, const __grid_constant__ UmmaMaps maps) {
     constexpr uint32_t kRowBlockBytes = 64 * BITS / 8;  // packed bytes of one row per K block (32 or 64)
     constexpr uint32_t kWordsPerBlock = kRowBlockBytes / 4;
     constexpr uint32_t kGroupsPerBlock = 64 / GROUP;    // 1 (g64) or 2 (g32)
@@ -236,44 +246,8 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, c
     constexpr uint32_t kKbPerSc = 8 / kGroupsPerBlock;  // K blocks per scale copy (8 or 4)
     constexpr float kZero = BITS == 4 ? 8.0f : 128.0f;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-#ifdef SHRIKE_TRACE
-    const uint64_t t_entry = globaltimer_ns();
-#endif
-    const uint32_t ii = blockIdx.y;
-    if (ii >= *n_inst) return;
-    const ChunkInstance in = inst[ii];
-    const bool shared = in.kind == 1;
-    const uint32_t F = shared ? a.f_shared : a.f;
-    const uint32_t kdim = PHASE == 0 ? a.d : F;
-    const uint32_t out_rows = PHASE == 0 ? F : a.d;       // rows of the weight matrix
-    const uint32_t r0 = blockIdx.x * (PHASE == 0 ? 128u : 256u);
-    if (r0 >= out_rows) return;
-    const Offsets3& off = shared ? a.shared : a.routed;
-    const uint8_t* base = shared ? a.shared_block : pool_cell_base(a.pool, in.slot);
-    const uint32_t KB = kdim / 64;
-    const uint32_t G = kdim / GROUP;
-    // scale rows that are whole 16-byte units come by TMA; others (G % 8 != 0) are read by the converters
-    const bool sc_tma = (G & 7u) == 0;
     const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    const uint32_t N = (in.count + 15u) & ~15u;           // MMA N: rows padded to 16
-    uint32_t ncols = 32;                                   // TMEM columns of one accumulator
-    while (ncols < N) ncols <<= 1;
-    // The activation tiles and the converted weight tiles share one region of shared memory: an instance with
-    // few rows needs narrow activation tiles and gets more weight stages instead. What paces such a block is the
-    // round trip converters -> tensor core -> converters (barrier, issue, commit, barrier: about half a
-    // microsecond against a few hundred nanoseconds of arithmetic), so it wants more tiles in flight.
-    // the instance's rows as one or two boxes of 16 << i rows: the largest that fits, then the smallest that
-    // holds the rest
-    uint32_t n1 = 16, b1 = 0;
-    while ((n1 << 1) <= N && b1 + 1 < (uint32_t)kActBoxes) { n1 <<= 1; ++b1; }
-    uint32_t n2 = 0, b2 = 0;
-    if (N > n1) {
-        n2 = 16;
-        while (n2 < N - n1) { n2 <<= 1; ++b2; }
-    }
-    const uint32_t b_stage = (((n1 + n2) * 128u + 2047u) / 2048u) * 2048u;   // bytes of one activation stage
-    const uint32_t off_a = kBStages * b_stage;
-    const uint32_t a_stages = min(kMaxAStages, (kOffPk - off_a) / kAStageBytes);
+    const uint32_t n_tiles = n_inst[0] * row_tiles;
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -286,10 +260,14 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, c
     uint64_t* pk_empty = pk_full + kPkSlots;       // converters -> weight copy
     uint64_t* sc_full = pk_empty + kPkSlots;
     uint64_t* sc_empty = sc_full + 1;
-    uint64_t* accum = sc_empty + 1;
-    uint32_t* rowid = (uint32_t*)(bars + kNumBars);   // token of column n
-    float* roww = (float*)(rowid + kUmmaMaxN);        // route weight (routed) or gate (shared) of column n
-    uint32_t* tmem_slot = (uint32_t*)(roww + kUmmaMaxN);
+    uint64_t* accum = sc_empty + 1;                // all of a tile's MMAs are done
+    uint64_t* next_full = accum + 1;               // [2] weight copy -> everyone: the next tile's number
+    uint64_t* next_empty = next_full + 2;
+    uint64_t* conv = next_empty + 2;               // the converter warps among themselves (a named barrier has no bounded wait)
+    uint32_t* rowid = (uint32_t*)(bars + kNumBars);                 // [2][column] token of a column, tiles in turn
+    float* roww = (float*)(rowid + 2 * kUmmaMaxN);                  // [2][column] route weight (routed) or gate (shared)
+    uint32_t* next_tile = (uint32_t*)(roww + 2 * kUmmaMaxN);        // [2]
+    uint32_t* tmem_slot = next_tile + 2;
     __shared__ uint32_t s_failed;
 
     if (tid == 0) {
@@ -299,81 +277,67 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, c
         mbar_init(sc_full, 1);
         mbar_init(sc_empty, kConvWarps);
         mbar_init(accum, 1);
+        mbar_init(conv, kConvWarps);
+        for (uint32_t s = 0; s < 2; ++s) { mbar_init(&next_full[s], 1); mbar_init(&next_empty[s], kConvWarps + 2); }
         fence_mbar_init();
         s_failed = 0;
     }
-    // the descriptors this block's copy threads will use: fetched while the barriers are set up
-    if (warp == kConvWarps + 1 && lane < 2) {
-        const CUtensorMap* mb = shared ? maps.act_shared : maps.act_routed;
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&mb[lane == 0 ? b1 : b2]) : "memory");
-    }
-    if (warp == kConvWarps + 2 && lane < 6) {
-        const WeightMaps* wm = shared ? &maps.shared : &maps.routed[in.slot / a.pool.cells_per_chunk];
-        const CUtensorMap* mp = lane < 2 ? &wm->w[lane] : lane < 4 ? &wm->s[lane - 2] : &wm->b[lane - 4];
-        asm volatile("prefetch.tensormap [%0];" ::"l"(mp) : "memory");
-    }
-    if (warp == kConvWarps) tmem_alloc(smem_u32(tmem_slot), 2 * ncols);
+    // two accumulators of up to 256 columns: all of TMEM (a block per SM)
+    if (warp == kConvWarps) tmem_alloc(smem_u32(tmem_slot), 2 * kUmmaMaxN);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-#ifdef SHRIKE_TRACE
-    uint64_t* const tr = a.trace ? a.trace + 8 * ((size_t)(PHASE * 4096 + blockIdx.y) * 8 + blockIdx.x) : nullptr;
-    if (tr && tid == 0) { tr[0] = t_entry; tr[1] = globaltimer_ns(); tr[7] = ((uint64_t)N << 32) | KB; }
-#endif
     auto give_up = [&]() {
         report_status(a.status, kStatusWaitTimeout);
-        s_failed = 1;
+        *(volatile uint32_t*)&s_failed = 1;
+    };
+    auto failed = [&]() { return *(volatile uint32_t*)&s_failed != 0; };
+    // Every barrier's use is counted in one bit per stage, kept by each role for itself: full barriers are waited for
+    // with the bit, empty ones with its complement (the first use of a stage finds it empty).
+    // The tile after `turn` others; n_tiles and above: none.
+    auto take_tile = [&](uint32_t turn) -> uint32_t {
+        const uint32_t s = turn & 1;
+        if (!__all_sync(0xffffffffu, pipe_wait(&next_full[s], (turn >> 1) & 1))) { give_up(); return 0xffffffffu; }
+        const uint32_t t = *(volatile uint32_t*)&next_tile[s];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&next_empty[s]);
+        return __shfl_sync(0xffffffffu, t, 0);
+    };
+    struct Work {
+        ChunkInstance in;
+        bool shared;
+        uint32_t F, KB, out_rows, r0;
+    };
+    auto open_tile = [&](uint32_t t, Work& w) {   // false: no such rows (a narrower shared or routed expert)
+        const uint32_t ii = t / row_tiles;
+        const uint4 v = __ldg((const uint4*)(inst + ii));
+        w.in.kind = v.x; w.in.slot = v.y; w.in.first = v.z; w.in.count = v.w;
+        w.shared = w.in.kind == 1;
+        w.F = w.shared ? a.f_shared : a.f;
+        w.KB = (PHASE == 0 ? a.d : w.F) / 64;
+        w.out_rows = PHASE == 0 ? w.F : a.d;       // rows of the weight matrix
+        w.r0 = (t - ii * row_tiles) * (PHASE == 0 ? 128u : 256u);
+        return w.r0 < w.out_rows;
     };
 
     if (warp < kConvWarps) {
-        // ---------------- converters ----------------
-        // the tokens and route weights of the columns: the epilogue reads them, long after these loads
-        if (PHASE == 1) {
-            for (uint32_t n = tid; n < kUmmaMaxN; n += kConverters) {
-                const uint32_t src = n < in.count ? n : 0;
-                if (shared) {
-                    rowid[n] = in.first + src;
-                    roww[n] = a.shared_gate ? a.shared_gate[in.first + src] : 1.0f;
-                } else {
-                    const uint32_t pair = a.sorted[in.first + src];
-                    rowid[n] = pair / a.top_k;
-                    roww[n] = a.route_w[pair];
-                }
-            }
-        }
+        // ---------------- converters, then the tile's epilogue ----------------
+        uint32_t a_use = 0, pk_use = 0, sc_use = 0, slot = 0, acc_use = 0, conv_use = 0, odd = 0;
+        auto converters_meet = [&]() {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(conv);
+            const bool ok = pipe_wait(conv, conv_use);
+            conv_use ^= 1;
+            if (!ok) give_up();
+            return ok;
+        };
         // Two threads per weight row: thread `half` converts 32 of the K block's 64 weights.
         const uint32_t tile = tid >> 8, r = (tid >> 1) & 127, half = tid & 1;
         constexpr uint32_t kWordsPerThread = kWordsPerBlock / 2;   // 4 (int4) or 8 (int8)
         const uint32_t pk_row = kOffPk + tile * (kPkSlotBytes / 2) + r * 64, pk_xor = (r >> 1) & 3;
-        uint32_t sreg[4] = {0, 0, 0, 0}, breg[4] = {0, 0, 0, 0};
-        uint32_t snext[4] = {0, 0, 0, 0}, bnext[4] = {0, 0, 0, 0};
-        const uint32_t mrow = r0 + (PHASE == 0 ? r : tile * 128 + r);
-        const int mat = PHASE == 0 ? (int)tile : 2;
-        const uint16_t* srow = (const uint16_t*)(base + off.s[mat]) + (size_t)mrow * G;
-        const uint16_t* brow = (const uint16_t*)(base + off.b[mat]) + (size_t)mrow * G;
-        // groups 8*blk .. 8*blk+7 of this thread's row, straight from global memory (rows past the matrix
-        // and groups past the row read as zero: the converted weights are then zero)
-        auto fetch_scales = [&](uint32_t blk) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint32_t gi = blk * 8 + 2 * i;
-                uint32_t sv = 0, bv = 0;
-                if (mrow < out_rows && gi < G) {
-                    sv = __ldg(srow + gi);
-                    bv = __ldg(brow + gi);
-                    if (gi + 1 < G) {
-                        sv |= (uint32_t)__ldg(srow + gi + 1) << 16;
-                        bv |= (uint32_t)__ldg(brow + gi + 1) << 16;
-                    }
-                }
-                snext[i] = sv;
-                bnext[i] = bv;
-            }
-        };
-        if (!sc_tma) fetch_scales(0);
         // What does not change along K: this thread's chunk positions in a packed slot and in the converted
-        // tile (both swizzled by the row), and the tile rows of the two stages.
+        // tile (both swizzled by the row).
         uint32_t pk_off[kKbPerPk * (kWordsPerThread / 4)];
 #pragma unroll
         for (uint32_t sub = 0; sub < kKbPerPk; ++sub)
@@ -384,228 +348,346 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, c
                 pk_off[sub * (kWordsPerThread / 4) + q] = pk_row + ((c ^ pk_xor) << 4);
             }
         constexpr uint32_t kStores = BITS == 4 ? kWordsPerThread : kWordsPerThread / 2;   // 16-byte chunks written
-        uint32_t a_off[kStores];
+        uint32_t a_pos[kStores];
 #pragma unroll
         for (uint32_t i = 0; i < kStores; ++i)   // A row r: 8 chunks of 8 fp16; chunk c lives at position c ^ (r & 7)
-            a_off[i] = off_a + tile * kTileBytes + r * 128 + (((half * kStores + i) ^ (r & 7)) << 4);
-        // A scale block (8 groups of the row) at a time, its K blocks unrolled: the position in the packed slot
-        // and the group of a K block are then constants of the instruction stream.
-        uint32_t st = 0, a_round = 0;   // the stage of the next K block and how often the stages have gone round
-        for (uint32_t kb0 = 0; kb0 < KB; kb0 += kKbPerSc) {
-            if (*(volatile uint32_t*)&s_failed) break;
-            if (sc_tma) {
-                if (!pipe_wait(sc_full, (kb0 / kKbPerSc) & 1)) { give_up(); break; }
-                const uint4 sv = *(const uint4*)(smem + kOffSc + tile * (kScHalfBytes / 2) + r * 16);
-                const uint4 bv = *(const uint4*)(smem + kOffSc + kScHalfBytes + tile * (kScHalfBytes / 2) + r * 16);
-                sreg[0] = sv.x; sreg[1] = sv.y; sreg[2] = sv.z; sreg[3] = sv.w;
-                breg[0] = bv.x; breg[1] = bv.y; breg[2] = bv.z; breg[3] = bv.w;
-                // the values are in registers: the copy thread may fetch the next block's
-                __syncwarp();
-                if (lane == 0) mbar_arrive(sc_empty);
-            } else {
-                // this block's 8 groups were fetched one block ago; fetch the next block's now
-#pragma unroll
-                for (int i = 0; i < 4; ++i) { sreg[i] = snext[i]; breg[i] = bnext[i]; }
-                fetch_scales(kb0 / kKbPerSc + 1);
+            a_pos[i] = tile * kTileBytes + r * 128 + (((half * kStores + i) ^ (r & 7)) << 4);
+
+        for (uint32_t turn = 0;; ++turn) {
+            const uint32_t t = take_tile(turn);
+            if (t >= n_tiles || failed()) break;
+            Work wk;
+            if (!open_tile(t, wk)) continue;
+            const ChunkInstance& in = wk.in;
+            const bool shared = wk.shared;
+            const uint32_t F = wk.F, KB = wk.KB, out_rows = wk.out_rows, r0 = wk.r0, G = KB * 64 / GROUP;
+            const TileShape ts(in.count);
+            const Offsets3& off = shared ? a.shared : a.routed;
+            const uint8_t* base = shared ? a.shared_block : pool_cell_base(a.pool, in.slot);
+            // scale rows that are whole 16-byte units come by TMA; others (G % 8 != 0) are read by the converters
+            const bool sc_tma = (G & 7u) == 0;
+            uint32_t* const ids = rowid + odd * kUmmaMaxN;
+            float* const wts = roww + odd * kUmmaMaxN;
+            odd ^= 1;
+            // the tokens and route weights of the columns: the epilogue reads them, long after these loads
+            if (PHASE == 1 && tid < kUmmaMaxN) {
+                const uint32_t src = tid < in.count ? tid : 0;
+                if (shared) {
+                    ids[tid] = in.first + src;
+                    wts[tid] = a.shared_gate ? a.shared_gate[in.first + src] : 1.0f;
+                } else {
+                    const uint32_t pair = a.sorted[in.first + src];
+                    ids[tid] = pair / a.top_k;
+                    wts[tid] = a.route_w[pair];
+                }
             }
-            uint32_t slot_base = 0, slot = 0;
+            uint32_t sreg[4] = {0, 0, 0, 0}, breg[4] = {0, 0, 0, 0};
+            uint32_t snext[4] = {0, 0, 0, 0}, bnext[4] = {0, 0, 0, 0};
+            const uint32_t mrow = r0 + (PHASE == 0 ? r : tile * 128 + r);
+            const int mat = PHASE == 0 ? (int)tile : 2;
+            const uint16_t* srow = (const uint16_t*)(base + off.s[mat]) + (size_t)mrow * G;
+            const uint16_t* brow = (const uint16_t*)(base + off.b[mat]) + (size_t)mrow * G;
+            // groups 8*blk .. 8*blk+7 of this thread's row, straight from global memory (rows past the matrix
+            // and groups past the row read as zero: the converted weights are then zero)
+            auto fetch_scales = [&](uint32_t blk) {
 #pragma unroll
-            for (uint32_t j = 0; j < kKbPerSc; ++j) {
-                const uint32_t kb = kb0 + j;
-                if (kb >= KB) break;
-                constexpr uint32_t kSubMask = kKbPerPk - 1;
-                const uint32_t sub = j & kSubMask;         // K block within its packed slot
-                if (sub == 0) {
-                    const uint32_t u = kb / kKbPerPk;
-                    slot = u % kPkSlots;
-                    slot_base = slot * kPkSlotBytes;
-                    if (!pipe_wait(&pk_full[slot], (u / kPkSlots) & 1)) { give_up(); break; }
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t gi = blk * 8 + 2 * i;
+                    uint32_t sv = 0, bv = 0;
+                    if (mrow < out_rows && gi < G) {
+                        sv = __ldg(srow + gi);
+                        bv = __ldg(brow + gi);
+                        if (gi + 1 < G) {
+                            sv |= (uint32_t)__ldg(srow + gi + 1) << 16;
+                            bv |= (uint32_t)__ldg(brow + gi + 1) << 16;
+                        }
+                    }
+                    snext[i] = sv;
+                    bnext[i] = bv;
                 }
-                uint32_t pk[kWordsPerThread];
+            };
+            if (!sc_tma) fetch_scales(0);
+            // A scale block (8 groups of the row) at a time, its K blocks unrolled: the position in the packed slot
+            // and the group of a K block are then constants of the instruction stream.
+            uint32_t st = 0;
+            for (uint32_t kb0 = 0; kb0 < KB; kb0 += kKbPerSc) {
+                if (failed()) break;
+                if (sc_tma) {
+                    if (!pipe_wait(sc_full, sc_use)) { give_up(); break; }
+                    sc_use ^= 1;
+                    const uint4 sv = *(const uint4*)(smem + kOffSc + tile * (kScHalfBytes / 2) + r * 16);
+                    const uint4 bv = *(const uint4*)(smem + kOffSc + kScHalfBytes + tile * (kScHalfBytes / 2) + r * 16);
+                    sreg[0] = sv.x; sreg[1] = sv.y; sreg[2] = sv.z; sreg[3] = sv.w;
+                    breg[0] = bv.x; breg[1] = bv.y; breg[2] = bv.z; breg[3] = bv.w;
+                    // the values are in registers: the copy thread may fetch the next block's
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(sc_empty);
+                } else {
+                    // this block's 8 groups were fetched one block ago; fetch the next block's now
 #pragma unroll
-                for (uint32_t q = 0; q < kWordsPerThread / 4; ++q) {
-                    const uint4 v = *(const uint4*)(smem + slot_base + pk_off[sub * (kWordsPerThread / 4) + q]);
-                    pk[4 * q] = v.x; pk[4 * q + 1] = v.y; pk[4 * q + 2] = v.z; pk[4 * q + 3] = v.w;
+                    for (int i = 0; i < 4; ++i) { sreg[i] = snext[i]; breg[i] = bnext[i]; }
+                    fetch_scales(kb0 / kKbPerSc + 1);
                 }
-                // a thread's half of a 64-wide block lies inside one group of 32 or 64
-                const uint32_t gsel = j * kGroupsPerBlock + (GROUP == 64 ? 0u : half);
-                const float sc = meta_to_f32<META>(pick16(sreg, gsel));
-                const float zf = fmaf(kZero, sc, meta_to_f32<META>(pick16(breg, gsel)));
-                const uint32_t s2 = half2_dup(sc), z2 = half2_dup(zf);
-                if (a_round && !pipe_wait(&a_empty[st], (a_round - 1) & 1)) { give_up(); break; }
-                uint8_t* a_stage = smem + st * kAStageBytes;
 #pragma unroll
-                for (uint32_t i = 0; i < kWordsPerThread; ++i) {
-                    uint32_t o[4];
-                    dequant_word<BITS>(pk[i], s2, z2, o);
-                    if constexpr (BITS == 4) {
-                        *(uint4*)(a_stage + a_off[i]) = make_uint4(o[0], o[1], o[2], o[3]);
-                    } else {
-                        // two words make one 16-byte chunk
-                        *((uint2*)(a_stage + a_off[i >> 1]) + (i & 1)) = make_uint2(o[0], o[1]);
+                for (uint32_t j = 0; j < kKbPerSc; ++j) {
+                    const uint32_t kb = kb0 + j;
+                    if (kb >= KB) break;
+                    constexpr uint32_t kSubMask = kKbPerPk - 1;
+                    const uint32_t sub = j & kSubMask;         // K block within its packed slot
+                    if (sub == 0 && !pipe_wait(&pk_full[slot], (pk_use >> slot) & 1)) { give_up(); break; }
+                    uint32_t pk[kWordsPerThread];
+#pragma unroll
+                    for (uint32_t q = 0; q < kWordsPerThread / 4; ++q) {
+                        const uint4 v = *(const uint4*)(smem + slot * kPkSlotBytes + pk_off[sub * (kWordsPerThread / 4) + q]);
+                        pk[4 * q] = v.x; pk[4 * q + 1] = v.y; pk[4 * q + 2] = v.z; pk[4 * q + 3] = v.w;
+                    }
+                    // a thread's half of a 64-wide block lies inside one group of 32 or 64
+                    const uint32_t gsel = j * kGroupsPerBlock + (GROUP == 64 ? 0u : half);
+                    const float sc = meta_to_f32<META>(pick16(sreg, gsel));
+                    const float zf = fmaf(kZero, sc, meta_to_f32<META>(pick16(breg, gsel)));
+                    const uint32_t s2 = half2_dup(sc), z2 = half2_dup(zf);
+                    if (!pipe_wait(&a_empty[st], ((a_use >> st) & 1) ^ 1)) { give_up(); break; }
+                    a_use ^= 1u << st;
+                    uint8_t* a_stage = smem + ts.off_a + st * kAStageBytes;
+#pragma unroll
+                    for (uint32_t i = 0; i < kWordsPerThread; ++i) {
+                        uint32_t o[4];
+                        dequant_word<BITS>(pk[i], s2, z2, o);
+                        if constexpr (BITS == 4) {
+                            *(uint4*)(a_stage + a_pos[i]) = make_uint4(o[0], o[1], o[2], o[3]);
+                        } else {
+                            // two words make one 16-byte chunk
+                            *((uint2*)(a_stage + a_pos[i >> 1]) + (i & 1)) = make_uint2(o[0], o[1]);
+                        }
+                    }
+                    fence_async_smem();
+                    __syncwarp();
+                    const bool slot_done = sub == kSubMask || kb + 1 == KB;
+                    if (lane == 0) {
+                        // one arrival per warp: 512 arrivals on one barrier word would serialise every K block
+                        mbar_arrive(&a_full[st]);
+                        // The ring slots are handed back only here: by now the values read from them have been
+                        // consumed, so the reads are complete before the copy thread may overwrite the slot.
+                        if (slot_done) mbar_arrive(&pk_empty[slot]);
+                    }
+                    if (slot_done) {
+                        pk_use ^= 1u << slot;
+                        if (++slot == kPkSlots) slot = 0;
+                    }
+                    if (++st == ts.a_stages) st = 0;
+                }
+            }
+            // ---------------- epilogue (warp w: TMEM lanes 32*(w & 3) .. +31, every fourth 16-column group) ----------------
+            bool ok = pipe_wait(accum, acc_use);
+            acc_use ^= 1;
+            if (!ok) give_up();
+            if (failed()) break;
+            tc_fence_after();
+            // the columns' tokens and weights were written by other converter threads at the start of the tile
+            if (PHASE == 1 && !converters_meet()) break;
+            // (eight columns at a time and loops that are not unrolled further: the code runs once per tile, and fetching
+            // it takes longer than what unrolling saves)
+            const uint32_t q = warp & 3, h = warp >> 2, N = ts.N;
+            const uint32_t trow = q * 32 + lane;                       // row inside each 128-row tile
+            const uint32_t taddr = tmem_base + ((q * 32) << 16);
+            constexpr uint32_t kColStep = 8 * (kConvWarps / 4);
+            if (PHASE == 0) {
+                const uint32_t f = r0 + trow;
+                float gab = 0.f, uab = 0.f;
+                if (a.expert_bias && f < F) {
+                    gab = bf16_bits_to_f32(((const uint16_t*)(base + off.ab[0]))[f]);
+                    uab = bf16_bits_to_f32(((const uint16_t*)(base + off.ab[1]))[f]);
+                }
+                uint16_t* const dst = (shared ? a.acts_shared : a.acts) + (size_t)in.first * F + perm_index(f, BITS == 4);
+                auto columns = [&](auto glu_of) {
+                    bool over = false;
+#pragma unroll 1
+                    for (uint32_t c0 = h * 8; c0 < N; c0 += kColStep) {
+                        uint32_t g[8], u[8];
+                        tmem_ld8_issue(taddr + c0, g);
+                        tmem_ld8_issue(taddr + kUmmaMaxN + c0, u);
+                        tmem_ld_wait();
+                        uint16_t* p = dst + (size_t)c0 * F;
+                        const uint32_t live = f < F ? min(8u, in.count > c0 ? in.count - c0 : 0u) : 0u;   // rows of this group
+#pragma unroll
+                        for (int j = 0; j < 8; j += 2) {
+                            float v[2];
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                v[e] = glu_of(__uint_as_float(g[j + e]) + gab, __uint_as_float(u[j + e]) + uab);
+                                if (fabsf(v[e]) > kHalfMax) {   // false for NaN, which passes through
+                                    over |= (uint32_t)(j + e) < live;
+                                    v[e] = copysignf(kHalfMax, v[e]);
+                                }
+                            }
+                            const __half2 hv = __floats2half2_rn(v[0], v[1]);
+                            if ((uint32_t)j < live) *p = __half_as_ushort(__low2half(hv));
+                            p += F;
+                            if ((uint32_t)j + 1 < live) *p = __half_as_ushort(__high2half(hv));
+                            p += F;
+                        }
+                    }
+                    if (over) report_status(a.status, kStatusOperandRange);
+                };
+                if (a.activation == SHRIKE_ACT_CLAMPED_SWIGLU) columns([](float x, float y) { return glu_epilogue(x, y, SHRIKE_ACT_CLAMPED_SWIGLU); });
+                else if (a.activation == SHRIKE_ACT_GELU_TANH) columns([](float x, float y) { return glu_epilogue(x, y, SHRIKE_ACT_GELU_TANH); });
+                else columns([](float x, float y) { return glu_epilogue(x, y, SHRIKE_ACT_SILU); });
+            } else {
+                const uint32_t d0 = r0 + trow, d1 = d0 + 128;
+                float ab0 = 0.f, ab1 = 0.f;
+                if (a.expert_bias) {
+                    const uint16_t* dab = (const uint16_t*)(base + off.ab[2]);
+                    if (d0 < a.d) ab0 = bf16_bits_to_f32(dab[d0]);
+                    if (d1 < a.d) ab1 = bf16_bits_to_f32(dab[d1]);
+                }
+                const bool ok0 = d0 < a.d, ok1 = d1 < a.d;
+#pragma unroll 1
+                for (uint32_t c0 = h * 8; c0 < N; c0 += kColStep) {
+                    uint32_t v0[8], v1[8];
+                    tmem_ld8_issue(taddr + c0, v0);
+                    tmem_ld8_issue(taddr + kUmmaMaxN + c0, v1);
+                    tmem_ld_wait();
+                    const uint32_t live = min(8u, in.count > c0 ? in.count - c0 : 0u);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        if ((uint32_t)j < live) {
+                            // lanes hold consecutive output rows: one 128-byte reduction per warp and column
+                            float* o = a.yacc + (size_t)ids[c0 + j] * a.d + d0;
+                            const float w = wts[c0 + j];
+                            if (ok0) atomicAdd(o, w * (__uint_as_float(v0[j]) + ab0));
+                            if (ok1) atomicAdd(o + 128, w * (__uint_as_float(v1[j]) + ab1));
+                        }
                     }
                 }
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) {
-                    // one arrival per warp: 512 arrivals on one barrier word would serialise every K block
-                    mbar_arrive(&a_full[st]);
-                    // The ring slots are handed back only here: by now the values read from them have been
-                    // consumed, so the reads are complete before the copy thread may overwrite the slot.
-                    if (sub == kSubMask || kb + 1 == KB) mbar_arrive(&pk_empty[slot]);
-                }
-                if (++st == a_stages) { st = 0; ++a_round; }
             }
+            tc_fence_before();   // these reads of the accumulators come before the next tile's instructions
         }
     } else if (warp == kConvWarps) {
         // ---------------- MMA issue ----------------
-        // The whole warp walks the loop on warp-uniform values and one elected lane issues: a branch on the lane number
-        // made every descriptor a per-thread value, and eight instructions took 550 to 750 cycles to issue.
-        const uint32_t idesc = __shfl_sync(0xffffffffu, umma_idesc(N), 0), acc0 = __shfl_sync(0xffffffffu, tmem_base, 0);
-        const uint32_t acc1 = acc0 + __shfl_sync(0xffffffffu, ncols, 0), stages = __shfl_sync(0xffffffffu, a_stages, 0);
-        const uint32_t a_smem = __shfl_sync(0xffffffffu, smem_base + off_a, 0), b_smem = __shfl_sync(0xffffffffu, smem_base, 0);
-        const uint32_t b_step = __shfl_sync(0xffffffffu, b_stage, 0), n_kb = __shfl_sync(0xffffffffu, KB, 0);
-        uint32_t sa = 0, a_round = 0, sb = 0, b_round = 0;
-        for (uint32_t kb = 0; kb < n_kb; ++kb) {
-            if (!pipe_wait(&b_full[sb], b_round & 1) || !pipe_wait(&a_full[sa], a_round & 1)) {
-                give_up();
-                break;
-            }
-            __syncwarp();
-            tc_fence_after();
-            if (elect_one()) {
-                const uint64_t da0 = umma_smem_desc(a_smem + sa * kAStageBytes), da1 = umma_smem_desc(a_smem + sa * kAStageBytes + kTileBytes);
-                const uint64_t db = umma_smem_desc(b_smem + sb * b_step);
-                // 4 x K16 per 64-wide block: 32 bytes further along the row. The two tiles alternate: consecutive
-                // instructions then add into different accumulators.
-#pragma unroll
-                for (uint32_t k = 0; k < 4; ++k) {
-                    umma_f16(acc0, da0 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-                    umma_f16(acc1, da1 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+        // The whole warp walks the loop on warp-uniform values and one elected lane issues: behind a branch on the lane
+        // number every descriptor was a per-thread value, and all tiles ran at 0.7 us per K block (0.5 now at 16 columns).
+        uint32_t a_use = 0, b_use = 0;
+        for (uint32_t turn = 0;; ++turn) {
+            const uint32_t t = take_tile(turn);
+            if (t >= n_tiles || failed()) break;
+            Work wk;
+            if (!open_tile(t, wk)) continue;
+            const TileShape ts(wk.in.count);
+            const uint32_t idesc = __shfl_sync(0xffffffffu, umma_idesc(ts.N), 0), acc0 = __shfl_sync(0xffffffffu, tmem_base, 0);
+            const uint32_t acc1 = acc0 + kUmmaMaxN, stages = __shfl_sync(0xffffffffu, ts.a_stages, 0);
+            const uint32_t b_smem = __shfl_sync(0xffffffffu, smem_base, 0), a_smem = b_smem + __shfl_sync(0xffffffffu, ts.off_a, 0);
+            const uint32_t b_step = __shfl_sync(0xffffffffu, ts.b_stage, 0), n_kb = __shfl_sync(0xffffffffu, wk.KB, 0);
+            uint32_t sa = 0, sb = 0;
+            for (uint32_t kb = 0; kb < n_kb; ++kb) {
+                // (the first stage of converted weights also says that the last tile's accumulators have been read)
+                const bool got = pipe_wait(&b_full[sb], (b_use >> sb) & 1) && pipe_wait(&a_full[sa], (a_use >> sa) & 1);
+                if (!__all_sync(0xffffffffu, got)) {
+                    give_up();
+                    break;
                 }
-                umma_commit(&a_empty[sa]);
-                umma_commit(&b_empty[sb]);
+                a_use ^= 1u << sa;
+                b_use ^= 1u << sb;
+                __syncwarp();
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint64_t da0 = umma_smem_desc(a_smem + sa * kAStageBytes), da1 = umma_smem_desc(a_smem + sa * kAStageBytes + kTileBytes);
+                    const uint64_t db = umma_smem_desc(b_smem + sb * b_step);
+                    // 4 x K16 per 64-wide block: 32 bytes further along the row. The two tiles alternate: consecutive
+                    // instructions then add into different accumulators.
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k) {
+                        umma_f16(acc0, da0 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                        umma_f16(acc1, da1 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                    }
+                    umma_commit(&a_empty[sa]);
+                    umma_commit(&b_empty[sb]);
+                }
+                __syncwarp();
+                if (++sa == stages) sa = 0;
+                if (++sb == kBStages) sb = 0;
             }
+            if (elect_one()) umma_commit(accum);
             __syncwarp();
-            if (++sa == stages) { sa = 0; ++a_round; }
-            if (++sb == kBStages) { sb = 0; ++b_round; }
         }
-        if (elect_one()) umma_commit(accum);
-        __syncwarp();
-    } else if (warp == kConvWarps + 1 && lane == 0) {
+    } else if (warp == kConvWarps + 1) {
         // ---------------- activation tiles ----------------
         // One or two boxes per K block: these tiles are most of what a block pulls out of L2, and a short instance
         // does not pay for 256 rows, nor one of 80 rows for 128.
-        const CUtensorMap* maps_b = shared ? maps.act_shared : maps.act_routed;
-        const uint32_t b_bytes = (n1 + n2) * 128u;
-        for (uint32_t kb = 0; kb < KB; ++kb) {
-            if (*(volatile uint32_t*)&s_failed) break;
-            const uint32_t sb = kb % kBStages;
-            if (kb >= kBStages && !pipe_wait(&b_empty[sb], ((kb / kBStages) - 1) & 1)) { give_up(); break; }
-            mbar_expect_tx(&b_full[sb], b_bytes);
-            tma_load_2d(smem_base + sb * b_stage, &maps_b[b1], (int32_t)(kb * 64), (int32_t)in.first, &b_full[sb]);
-            if (n2)
-                tma_load_2d(smem_base + sb * b_stage + n1 * 128u, &maps_b[b2], (int32_t)(kb * 64),
-                            (int32_t)(in.first + n1), &b_full[sb]);
-        }
-    } else if (warp == kConvWarps + 2 && lane == 0) {
-        // ---------------- packed weights, scales, biases ----------------
-        const WeightMaps* wm = shared ? &maps.shared : &maps.routed[in.slot / a.pool.cells_per_chunk];
-        const int32_t cell = shared ? 0 : (int32_t)(in.slot % a.pool.cells_per_chunk);
-        const int32_t y0 = (int32_t)r0, y1 = (int32_t)(PHASE == 0 ? r0 : r0 + 128);
-        for (uint32_t kb = 0; kb < KB; ++kb) {
-            if (*(volatile uint32_t*)&s_failed) break;
-            if (sc_tma && kb % kKbPerSc == 0) {
-                const uint32_t blk = kb / kKbPerSc;
-                if (blk > 0 && !pipe_wait(sc_empty, (blk - 1) & 1)) { give_up(); break; }
-                mbar_expect_tx(sc_full, 2 * kScHalfBytes);
-                const uint32_t dst = smem_base + kOffSc;
-                tma_load_3d(dst, &wm->s[0], (int32_t)(blk * 8), y0, cell, sc_full);
-                tma_load_3d(dst + kScHalfBytes / 2, &wm->s[1], (int32_t)(blk * 8), y1, cell, sc_full);
-                tma_load_3d(dst + kScHalfBytes, &wm->b[0], (int32_t)(blk * 8), y0, cell, sc_full);
-                tma_load_3d(dst + kScHalfBytes + kScHalfBytes / 2, &wm->b[1], (int32_t)(blk * 8), y1, cell, sc_full);
+        uint32_t b_use = 0, acc_use = 0, last_stage = 0;
+        for (uint32_t turn = 0;; ++turn) {
+            const uint32_t t = take_tile(turn);
+            if (t >= n_tiles || failed()) break;
+            Work wk;
+            if (!open_tile(t, wk)) continue;
+            const TileShape ts(wk.in.count);
+            if (last_stage) {
+                // another layout: its stages lie across the last one's, so the last tile's instructions have to be done
+                if (ts.b_stage != last_stage && !pipe_wait(accum, acc_use)) { give_up(); break; }
+                acc_use ^= 1;
             }
-            if (kb % kKbPerPk == 0) {
-                const uint32_t u = kb / kKbPerPk, slot = u % kPkSlots;
-                if (u >= kPkSlots && !pipe_wait(&pk_empty[slot], ((u / kPkSlots) - 1) & 1)) { give_up(); break; }
-                mbar_expect_tx(&pk_full[slot], kPkSlotBytes);
-                const uint32_t dst = smem_base + kOffPk + slot * kPkSlotBytes;
-                tma_load_3d(dst, &wm->w[0], (int32_t)(u * 64), y0, cell, &pk_full[slot]);
-                tma_load_3d(dst + kPkSlotBytes / 2, &wm->w[1], (int32_t)(u * 64), y1, cell, &pk_full[slot]);
-            }
-        }
-    }
-
-    // ---------------- epilogue (warp w: TMEM lanes 32*(w & 3) .. +31, every fourth 16-column group) ----------------
-    if (warp < kConvWarps) {
-        bool ok = pipe_wait(accum, 0);
-        if (!ok) report_status(a.status, kStatusWaitTimeout);
-        if (*(volatile uint32_t*)&s_failed) ok = false;
-        tc_fence_after();
-        // the columns' tokens and weights were written by other converter threads at the start of the block
-        if (PHASE == 1) asm volatile("bar.sync 1, %0;" ::"n"(kConverters) : "memory");
-#ifdef SHRIKE_TRACE
-        if (tr && tid == 0) tr[5] = globaltimer_ns();
-#endif
-        const uint32_t q = warp & 3, h = warp >> 2;
-        const uint32_t trow = q * 32 + lane;                       // row inside each 128-row tile
-        const uint32_t taddr = tmem_base + ((q * 32) << 16);
-        constexpr uint32_t kColStep = 16 * (kConvWarps / 4);
-        if (PHASE == 0) {
-            const uint32_t f = r0 + trow;
-            const bool f_ok = f < F && ok;
-            float gab = 0.f, uab = 0.f;
-            if (a.expert_bias && f < F) {
-                gab = bf16_bits_to_f32(((const uint16_t*)(base + off.ab[0]))[f]);
-                uab = bf16_bits_to_f32(((const uint16_t*)(base + off.ab[1]))[f]);
-            }
-            uint16_t* dst = (shared ? a.acts_shared : a.acts) + (size_t)in.first * F + perm_index(f, BITS == 4);
-            for (uint32_t c0 = h * 16; c0 < N; c0 += kColStep) {
-                uint32_t g[16], u[16];
-                tmem_ld16_issue(taddr + c0, g);
-                tmem_ld16_issue(taddr + ncols + c0, u);
-                tmem_ld_wait();
-                uint16_t* p = dst + (size_t)c0 * F;
-                const uint32_t live = f_ok ? min(16u, in.count > c0 ? in.count - c0 : 0u) : 0u;   // rows of this group
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float v = glu_epilogue(__uint_as_float(g[j]) + gab, __uint_as_float(u[j]) + uab, a.activation);
-                    if ((uint32_t)j < live) *p = act_to_half_bits(v, a.status);
-                    p += F;
+            last_stage = ts.b_stage;
+            const CUtensorMap* maps_b = wk.shared ? maps.act_shared : maps.act_routed;
+            if (lane == 0) {
+                const uint32_t b_bytes = (ts.n1 + ts.n2) * 128u;
+                uint32_t sb = 0;
+                for (uint32_t kb = 0; kb < wk.KB; ++kb) {
+                    if (failed()) break;
+                    if (!pipe_wait(&b_empty[sb], ((b_use >> sb) & 1) ^ 1)) { give_up(); break; }
+                    b_use ^= 1u << sb;
+                    mbar_expect_tx(&b_full[sb], b_bytes);
+                    tma_load_2d(smem_base + sb * ts.b_stage, &maps_b[ts.b1], (int32_t)(kb * 64), (int32_t)wk.in.first, &b_full[sb]);
+                    if (ts.n2)
+                        tma_load_2d(smem_base + sb * ts.b_stage + ts.n1 * 128u, &maps_b[ts.b2], (int32_t)(kb * 64),
+                                    (int32_t)(wk.in.first + ts.n1), &b_full[sb]);
+                    if (++sb == kBStages) sb = 0;
                 }
             }
-        } else {
-            const uint32_t d0 = r0 + trow, d1 = d0 + 128;
-            float ab0 = 0.f, ab1 = 0.f;
-            if (a.expert_bias) {
-                const uint16_t* dab = (const uint16_t*)(base + off.ab[2]);
-                if (d0 < a.d) ab0 = bf16_bits_to_f32(dab[d0]);
-                if (d1 < a.d) ab1 = bf16_bits_to_f32(dab[d1]);
-            }
-            const bool ok0 = ok && d0 < a.d, ok1 = ok && d1 < a.d;
-            for (uint32_t c0 = h * 16; c0 < N; c0 += kColStep) {
-                uint32_t v0[16], v1[16];
-                tmem_ld16_issue(taddr + c0, v0);
-                tmem_ld16_issue(taddr + ncols + c0, v1);
-                tmem_ld_wait();
-                const uint32_t live = min(16u, in.count > c0 ? in.count - c0 : 0u);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    if ((uint32_t)j < live) {
-                        // lanes hold consecutive output rows: one 128-byte reduction per warp and column
-                        float* o = a.yacc + (size_t)rowid[c0 + j] * a.d + d0;
-                        const float w = roww[c0 + j];
-                        if (ok0) atomicAdd(o, w * (__uint_as_float(v0[j]) + ab0));
-                        if (ok1) atomicAdd(o + 128, w * (__uint_as_float(v1[j]) + ab1));
-                    }
+            __syncwarp();
+        }
+    } else if (lane == 0) {
+        // ---------------- tile numbers; packed weights, scales, biases ----------------
+        uint32_t pk_use = 0, sc_use = 0, slot = 0;
+        for (uint32_t turn = 0;; ++turn) {
+            const uint32_t s = turn & 1;
+            const uint32_t t = turn == 0 ? blockIdx.x : gridDim.x + atomicAdd(n_inst + 2 + PHASE, 1u);
+            if (!pipe_wait(&next_empty[s], ((turn >> 1) & 1) ^ 1)) { give_up(); break; }
+            *(volatile uint32_t*)&next_tile[s] = t;
+            mbar_arrive(&next_full[s]);
+            if (t >= n_tiles || failed()) break;
+            Work wk;
+            if (!open_tile(t, wk)) continue;
+            const ChunkInstance& in = wk.in;
+            const WeightMaps* wm = wk.shared ? &maps.shared : &maps.routed[in.slot / a.pool.cells_per_chunk];
+            const int32_t cell = wk.shared ? 0 : (int32_t)(in.slot % a.pool.cells_per_chunk);
+            const int32_t y0 = (int32_t)wk.r0, y1 = (int32_t)(PHASE == 0 ? wk.r0 : wk.r0 + 128);
+            const bool sc_tma = (wk.KB * 64 / GROUP & 7u) == 0;
+            for (uint32_t kb = 0; kb < wk.KB; ++kb) {
+                if (failed()) break;
+                if (sc_tma && kb % kKbPerSc == 0) {
+                    const int32_t g0 = (int32_t)(kb / kKbPerSc * 8);
+                    if (!pipe_wait(sc_empty, sc_use ^ 1)) { give_up(); break; }
+                    sc_use ^= 1;
+                    mbar_expect_tx(sc_full, 2 * kScHalfBytes);
+                    const uint32_t dst = smem_base + kOffSc;
+                    tma_load_3d(dst, &wm->s[0], g0, y0, cell, sc_full);
+                    tma_load_3d(dst + kScHalfBytes / 2, &wm->s[1], g0, y1, cell, sc_full);
+                    tma_load_3d(dst + kScHalfBytes, &wm->b[0], g0, y0, cell, sc_full);
+                    tma_load_3d(dst + kScHalfBytes + kScHalfBytes / 2, &wm->b[1], g0, y1, cell, sc_full);
+                }
+                if (kb % kKbPerPk == 0) {
+                    const int32_t x = (int32_t)(kb / kKbPerPk * 64);
+                    if (!pipe_wait(&pk_empty[slot], ((pk_use >> slot) & 1) ^ 1)) { give_up(); break; }
+                    pk_use ^= 1u << slot;
+                    mbar_expect_tx(&pk_full[slot], kPkSlotBytes);
+                    const uint32_t dst = smem_base + kOffPk + slot * kPkSlotBytes;
+                    tma_load_3d(dst, &wm->w[0], x, y0, cell, &pk_full[slot]);
+                    tma_load_3d(dst + kPkSlotBytes / 2, &wm->w[1], x, y1, cell, &pk_full[slot]);
+                    if (++slot == kPkSlots) slot = 0;
                 }
             }
         }
     }
-#ifdef SHRIKE_TRACE
-    if (tr && tid == 0) tr[6] = globaltimer_ns();
-#endif
-    if (*(volatile uint32_t*)&s_failed && lane == 0 && warp > kConvWarps) {
+    if (failed() && lane == 0 && warp > kConvWarps) {
         // a copy of this block may still be in flight: give it a bounded time to land
         for (int i = 0; i < 200; ++i) __nanosleep(1000);
     }
@@ -613,7 +695,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, c
     __syncthreads();
     if (warp == kConvWarps) {
         __syncwarp();
-        tmem_dealloc(tmem_base, 2 * ncols);
+        tmem_dealloc(tmem_base, 2 * kUmmaMaxN);
     }
 }
 
@@ -624,8 +706,23 @@ chunk_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __r
                        const uint32_t* __restrict__ slot_of_expert, uint32_t ne, uint32_t T, uint32_t with_shared,
                        uint32_t pool_cells, ChunkInstance* __restrict__ inst, uint32_t* __restrict__ n_inst,
                        uint32_t* status) {
-    __shared__ uint32_t warp_sums[8], warp_rows[8];
-    const uint32_t e = threadIdx.x;
+    __shared__ uint32_t warp_sums[8], warp_rows[8], by_size[256];
+    __shared__ __align__(16) uint32_t key[256];
+    // Experts with the most rows first: a tile of 256 rows takes twice the time of one of 16, and a list that ends on long
+    // ones leaves SMs idle (4096 rows: the last ended a tenth after the median SM).
+    key[threadIdx.x] = (threadIdx.x < ne ? counts[threadIdx.x] << 8 : 0u) | (255u - threadIdx.x);
+    __syncthreads();
+    {
+        const uint32_t mine = key[threadIdx.x];
+        uint32_t rank = 0;
+        for (uint32_t j = 0; j < 256; j += 4) {
+            const uint4 v = *(const uint4*)&key[j];
+            rank += (v.x > mine) + (v.y > mine) + (v.z > mine) + (v.w > mine);
+        }
+        by_size[rank] = threadIdx.x;
+    }
+    __syncthreads();
+    const uint32_t e = by_size[threadIdx.x];
     uint32_t n = 0, slot = SHRIKE_SLOT_MISS, c = 0;
     if (e < ne && counts[e] > 0) {
         c = counts[e];
@@ -670,6 +767,7 @@ chunk_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __r
     if (threadIdx.x == 0) {
         n_inst[0] = total + n_shared;
         n_inst[1] = total_rows;
+        n_inst[2] = n_inst[3] = 0;   // tiles handed out, per phase
     }
 }
 
@@ -773,7 +871,7 @@ cudaError_t umma_prepare(shrike_moe* m) {
 
 template <int BITS, int GROUP, int META>
 static cudaError_t launch_umma_t(cudaStream_t st, const ExpertArgs& a, const ChunkInstance* inst,
-                                 const uint32_t* n_inst, uint32_t max_inst, const UmmaMaps& m0, const UmmaMaps& m1) {
+                                 uint32_t* n_inst, uint32_t max_inst, uint32_t sm_count, const UmmaMaps& m0, const UmmaMaps& m1) {
     auto k0 = umma_expert_kernel<BITS, GROUP, META, 0>;
     auto k1 = umma_expert_kernel<BITS, GROUP, META, 1>;
     cudaError_t e = cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUmmaSmemBytes);
@@ -781,10 +879,11 @@ static cudaError_t launch_umma_t(cudaStream_t st, const ExpertArgs& a, const Chu
     e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUmmaSmemBytes);
     if (e != cudaSuccess) return e;
     const uint32_t fmax = a.f_shared > a.f ? a.f_shared : a.f;
-    k0<<<dim3((fmax + 127) / 128, max_inst), kUmmaThreads, kUmmaSmemBytes, st>>>(a, inst, n_inst, m0);
+    const uint32_t t0 = (fmax + 127) / 128, t1 = (a.d + 255) / 256;
+    k0<<<std::min(sm_count, max_inst * t0), kUmmaThreads, kUmmaSmemBytes, st>>>(a, inst, n_inst, t0, m0);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k1<<<dim3((a.d + 255) / 256, max_inst), kUmmaThreads, kUmmaSmemBytes, st>>>(a, inst, n_inst, m1);
+    k1<<<std::min(sm_count, max_inst * t1), kUmmaThreads, kUmmaSmemBytes, st>>>(a, inst, n_inst, t1, m1);
     return cudaGetLastError();
 }
 
@@ -844,7 +943,7 @@ cudaError_t launch_umma_prefill(const shrike_moe* m, cudaStream_t st, const Expe
     const uint32_t bits = c.weight_bits, grp = c.group_size;
     const bool f16 = c.meta_dtype == SHRIKE_DTYPE_FP16;
 #define SHRIKE_UMMA(B, G, M) \
-    return launch_umma_t<B, G, M>(st, a, inst, ws.n_chunk_inst, max_inst, maps[0], maps[1])
+    return launch_umma_t<B, G, M>(st, a, inst, ws.n_chunk_inst, max_inst, (uint32_t)m->sm_count, maps[0], maps[1])
     if (bits == 4 && grp == 64 && !f16) SHRIKE_UMMA(4, 64, SHRIKE_DTYPE_BF16);
     if (bits == 4 && grp == 64 && f16) SHRIKE_UMMA(4, 64, SHRIKE_DTYPE_FP16);
     if (bits == 4 && grp == 32 && !f16) SHRIKE_UMMA(4, 32, SHRIKE_DTYPE_BF16);

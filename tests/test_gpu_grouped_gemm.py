@@ -1,0 +1,35 @@
+"""The expert-grouped GEMM with more tiles than SMs, against the oracle: instances on both sides of every stage layout
+(1, 16, 64, 65, 128, 129 and 256 rows and one more than 256) follow one another on an SM, shared and routed experts have
+different numbers of row tiles, and the last ones are partial."""
+import numpy as np
+import pytest
+import torch
+
+from shrike_b200 import capi
+from gpu_harness import Layer, inputs, rel_l2, small_config, to_act_tensor
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kw", [
+    dict(d=1088, f=192, shared_f=448),
+    dict(d=1024, f=320, shared_f=64, weight_bits=8, group_size=32, meta_dtype=capi.DTYPE_FP16),
+    dict(d=960, f=448, shared_f=192, weight_bits=4, group_size=32, expert_bias=1, activation=capi.ACT_CLAMPED_SWIGLU),
+], ids=lambda kw: "-".join(f"{k}{v}" for k, v in kw.items()))
+def test_tiles_of_every_layout(cuda_device, kw):
+    sizes = [257, 256, 129, 128, 65, 64, 17, 16] + [1] * 40
+    cfg = small_config(num_experts=64, top_k=1, max_tokens=1024, shared_gated=False, **kw)
+    layer = Layer(cfg)
+    ids = np.concatenate([np.full(n, e, np.uint32) for e, n in enumerate(sizes)])
+    ids = np.random.default_rng(3).permutation(ids)[:, None]
+    x = inputs(len(ids), kw["d"], seed=5)
+    w = np.random.default_rng(4).uniform(0.2, 1.0, ids.shape).astype(np.float32)
+    x_dev = to_act_tensor(x, cfg.act_dtype, layer.device)
+    ids_dev = torch.from_numpy(ids.view(np.int32)).to(layer.device)
+    slots, _ = layer.classify(ids_dev)
+    y = torch.empty(x_dev.shape, dtype=cfg.torch_y_dtype, device=layer.device)
+    layer.moe.encode_prefill(layer.pool, layer.offsets, ids_dev, slots, torch.from_numpy(w).to(layer.device), x_dev, y, None,
+                             layer.shared, None)
+    layer.moe.status()
+    assert rel_l2(y.cpu().numpy(), layer.oracle_forward(x, ids, w)) <= 1e-3
+    layer.close()
