@@ -248,6 +248,9 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t n_tiles = n_inst[0] * row_tiles;
+    // Scale rows that are whole 16-byte units come by TMA; others (groups % 8 != 0) are read by the converters. One way for
+    // all instances: both use the same memory, which the copy thread would fill a tile ahead.
+    const bool sc_tma = PHASE == 0 ? (a.d / GROUP & 7u) == 0 : ((a.f / GROUP | a.f_shared / GROUP) & 7u) == 0;
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -364,8 +367,6 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             const TileShape ts(in.count);
             const Offsets3& off = shared ? a.shared : a.routed;
             const uint8_t* base = shared ? a.shared_block : pool_cell_base(a.pool, in.slot);
-            // scale rows that are whole 16-byte units come by TMA; others (G % 8 != 0) are read by the converters
-            const bool sc_tma = (G & 7u) == 0;
             uint32_t* const ids = rowid + odd * kUmmaMaxN;
             float* const wts = roww + odd * kUmmaMaxN;
             odd ^= 1;
@@ -387,9 +388,25 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             const int mat = PHASE == 0 ? (int)tile : 2;
             const uint16_t* srow = (const uint16_t*)(base + off.s[mat]) + (size_t)mrow * G;
             const uint16_t* brow = (const uint16_t*)(base + off.b[mat]) + (size_t)mrow * G;
-            // groups 8*blk .. 8*blk+7 of this thread's row, straight from global memory (rows past the matrix
-            // and groups past the row read as zero: the converted weights are then zero)
+            // Groups 8*blk .. 8*blk+7 straight from global memory (rows past the matrix and groups past the row read as
+            // zero: the converted weights are then zero). An even number of groups: the warp's sixteen rows in 32-bit
+            // words, four lanes a row, put into the rows' places in shared memory when they are needed; read by each
+            // row's two threads in 16-bit pieces they kept L1 busy for 1.3 us per K block of 90-group rows.
+            const bool words = (G & 1u) == 0;
+            const uint32_t my_rows = r0 + (PHASE == 0 ? 0u : tile * 128u) + ((warp * 16) & 127u) + (lane >> 2);
             auto fetch_scales = [&](uint32_t blk) {
+                if (words) {
+                    const uint32_t gi = blk * 8 + 2 * (lane & 3);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const uint32_t row = my_rows + 8 * i;
+                        const bool there = row < out_rows && gi < G;
+                        const size_t at = (size_t)row * G + gi;
+                        snext[i] = there ? __ldg((const uint32_t*)((const uint16_t*)(base + off.s[mat]) + at)) : 0u;
+                        bnext[i] = there ? __ldg((const uint32_t*)((const uint16_t*)(base + off.b[mat]) + at)) : 0u;
+                    }
+                    return;
+                }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const uint32_t gi = blk * 8 + 2 * i;
@@ -424,8 +441,22 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                     if (lane == 0) mbar_arrive(sc_empty);
                 } else {
                     // this block's 8 groups were fetched one block ago; fetch the next block's now
+                    if (words) {
+                        uint8_t* const to = smem + kOffSc + (warp * 16 + (lane >> 2)) * 16 + (lane & 3) * 4;
+                        __syncwarp();   // the last block's have been read
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) { sreg[i] = snext[i]; breg[i] = bnext[i]; }
+                        for (int i = 0; i < 2; ++i) {
+                            *(uint32_t*)(to + i * 128) = snext[i];
+                            *(uint32_t*)(to + kScHalfBytes + i * 128) = bnext[i];
+                        }
+                        __syncwarp();
+                        const uint4 sv = *(const uint4*)(smem + kOffSc + (tid >> 1) * 16), bv = *(const uint4*)(smem + kOffSc + kScHalfBytes + (tid >> 1) * 16);
+                        sreg[0] = sv.x; sreg[1] = sv.y; sreg[2] = sv.z; sreg[3] = sv.w;
+                        breg[0] = bv.x; breg[1] = bv.y; breg[2] = bv.z; breg[3] = bv.w;
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) { sreg[i] = snext[i]; breg[i] = bnext[i]; }
+                    }
                     fetch_scales(kb0 / kKbPerSc + 1);
                 }
 #pragma unroll
@@ -660,7 +691,6 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             const WeightMaps* wm = wk.shared ? &maps.shared : &maps.routed[in.slot / a.pool.cells_per_chunk];
             const int32_t cell = wk.shared ? 0 : (int32_t)(in.slot % a.pool.cells_per_chunk);
             const int32_t y0 = (int32_t)wk.r0, y1 = (int32_t)(PHASE == 0 ? wk.r0 : wk.r0 + 128);
-            const bool sc_tma = (wk.KB * 64 / GROUP & 7u) == 0;
             for (uint32_t kb = 0; kb < wk.KB; ++kb) {
                 if (failed()) break;
                 if (sc_tma && kb % kKbPerSc == 0) {
