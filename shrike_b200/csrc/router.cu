@@ -91,6 +91,39 @@ __device__ __forceinline__ void cp_async_16_zfill(uint32_t smem_addr, const void
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr), "l"(gptr), "r"(n) : "memory");
 }
 
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+    return v;
+}
+
+// The lane sums of a warp's tile, [token][row], meet in the xor 16..1 order of butterfly_sum, each lane keeping half of the
+// values at every step (124 exchanges instead of 640; an addition does not care which side it is on). Lane l ends with
+// values 4l .. 4l + 3: rows 4 (l & 1) and on of token l / 2.
+__device__ __forceinline__ void store_tile(const RouterArgs& a, float (&v)[kTileWarpTokens * kTileWarpRows], uint32_t e, uint32_t tok, uint32_t lane) {
+    static_assert(kTileWarpTokens * kTileWarpRows == 128 && kTileWarpRows == 8, "four values a lane");
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) {
+        const bool up = (lane & m) != 0;
+#pragma unroll
+        for (int i = 0; i < 4 * m; ++i) {
+            const float keep = up ? v[i + 4 * m] : v[i], send = up ? v[i] : v[i + 4 * m];
+            v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, m));
+        }
+    }
+    tok += lane >> 1;
+    e += (lane & 1) * 4;
+    if (tok >= a.T) return;
+    float* const dst = a.logits + (size_t)tok * a.ne + e;
+    if (e + 4 <= a.ne && (a.ne & 3u) == 0) {
+        *(float4*)dst = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i)
+            if (e + i < a.ne) dst[i] = v[i];
+    }
+}
+
 __global__ void __launch_bounds__(256, 1) router_logits_tiled_kernel(const RouterArgs a) {
     extern __shared__ __align__(16) float tile_smem[];
     float* const w_s = tile_smem;                                           // [2][32][256]
@@ -209,33 +242,12 @@ __global__ void __launch_bounds__(256, 1) router_logits_tiled_kernel(const Route
         __syncthreads();
     }
 
-    // butterfly, then lane 2t + (r / 4) stores the four logits (r & ~3 .. +3) of token t
-    float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
+    float sums[kTileWarpTokens * kTileWarpRows];
 #pragma unroll
     for (int t = 0; t < kTileWarpTokens; ++t)
 #pragma unroll
-        for (int r = 0; r < kTileWarpRows; ++r) {
-            const float v = butterfly_sum(acc[r][t]);
-            if (lane == (uint32_t)(2 * t + r / 4)) {
-                if ((r & 3) == 0) out.x = v;
-                else if ((r & 3) == 1) out.y = v;
-                else if ((r & 3) == 2) out.z = v;
-                else out.w = v;
-            }
-        }
-    const uint32_t tok = t0 + tg * kTileWarpTokens + (lane >> 1);
-    const uint32_t e = e0 + rg * kTileWarpRows + (lane & 1) * 4;
-    if (tok < a.T) {
-        float* const dst = a.logits + (size_t)tok * a.ne + e;
-        if (e + 4 <= a.ne && (a.ne & 3u) == 0) {
-            *(float4*)dst = out;
-        } else {
-            if (e + 0 < a.ne) dst[0] = out.x;
-            if (e + 1 < a.ne) dst[1] = out.y;
-            if (e + 2 < a.ne) dst[2] = out.z;
-            if (e + 3 < a.ne) dst[3] = out.w;
-        }
-    }
+        for (int r = 0; r < kTileWarpRows; ++r) sums[t * kTileWarpRows + r] = acc[r][t];
+    store_tile(a, sums, e0 + rg * kTileWarpRows, t0 + tg * kTileWarpTokens, lane);
 }
 
 // The same tile for 16-bit activations without a per-column scale (the common case): both operands go to
@@ -276,11 +288,12 @@ __global__ void __launch_bounds__(256, 1) router_logits_tiled16_kernel(const Rou
         cp_async_commit();
     };
 
-    float acc[kTileWarpRows][kTileWarpTokens];
+    // [row][token pair]: one packed instruction does a fused multiply-add for each of two tokens, each rounded as ever
+    uint64_t acc[kTileWarpRows][kTileWarpTokens / 2];
 #pragma unroll
     for (int r = 0; r < kTileWarpRows; ++r)
 #pragma unroll
-        for (int t = 0; t < kTileWarpTokens; ++t) acc[r][t] = 0.f;
+        for (int t = 0; t < kTileWarpTokens / 2; ++t) acc[r][t] = 0;
 
     fetch(0, 0);
     if (stages > 1) fetch(1, 1);
@@ -295,73 +308,58 @@ __global__ void __launch_bounds__(256, 1) router_logits_tiled16_kernel(const Rou
         const uint2* const xb = (const uint2*)(tile16_smem + (size_t)buf * kTile16Buf + kTile16WBytes) + tg * kTileWarpTokens * (kTileStage / 4);
 #pragma unroll
         for (int ii = 0; ii < kTileStage / 128; ++ii) {
-            float4 wv[kTileWarpRows];
+            uint64_t wv[kTileWarpRows][4];
 #pragma unroll
-            for (int r = 0; r < kTileWarpRows; ++r) wv[r] = wb[r * (kTileStage / 4) + ii * 32 + lane];
+            for (int r = 0; r < kTileWarpRows; ++r) {
+                const float4 v = wb[r * (kTileStage / 4) + ii * 32 + lane];
+                wv[r][0] = pack2(v.x, v.x); wv[r][1] = pack2(v.y, v.y); wv[r][2] = pack2(v.z, v.z); wv[r][3] = pack2(v.w, v.w);
+            }
 #pragma unroll
-            for (int t = 0; t < kTileWarpTokens; ++t) {
-                const uint2 q = xb[t * (kTileStage / 4) + ii * 32 + lane];
-                float4 xv;
-                if (FP16)
-                    xv = make_float4(f16_bits_to_f32(q.x & 0xffff), f16_bits_to_f32(q.x >> 16), f16_bits_to_f32(q.y & 0xffff),
-                                     f16_bits_to_f32(q.y >> 16));
-                else
-                    xv = make_float4(__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xffff0000u), __uint_as_float(q.y << 16),
-                                     __uint_as_float(q.y & 0xffff0000u));
+            for (int t = 0; t < kTileWarpTokens / 2; ++t) {
+                float x[2][4];
 #pragma unroll
-                for (int r = 0; r < kTileWarpRows; ++r) {
-                    float v = acc[r][t];
-                    v = __fmaf_rn(wv[r].x, xv.x, v);
-                    v = __fmaf_rn(wv[r].y, xv.y, v);
-                    v = __fmaf_rn(wv[r].z, xv.z, v);
-                    v = __fmaf_rn(wv[r].w, xv.w, v);
-                    acc[r][t] = v;
+                for (int u = 0; u < 2; ++u) {
+                    const uint2 q = xb[(2 * t + u) * (kTileStage / 4) + ii * 32 + lane];
+                    if (FP16) {
+                        x[u][0] = f16_bits_to_f32(q.x & 0xffff); x[u][1] = f16_bits_to_f32(q.x >> 16);
+                        x[u][2] = f16_bits_to_f32(q.y & 0xffff); x[u][3] = f16_bits_to_f32(q.y >> 16);
+                    } else {
+                        x[u][0] = __uint_as_float(q.x << 16); x[u][1] = __uint_as_float(q.x & 0xffff0000u);
+                        x[u][2] = __uint_as_float(q.y << 16); x[u][3] = __uint_as_float(q.y & 0xffff0000u);
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const uint64_t xv = pack2(x[0][c], x[1][c]);
+#pragma unroll
+                    for (int r = 0; r < kTileWarpRows; ++r)
+                        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[r][t]) : "l"(wv[r][c]), "l"(xv));
                 }
             }
         }
     }
 
-    // butterfly, then lane 2t + (r / 4) stores the four logits (r & ~3 .. +3) of token t
-    float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
+    float sums[kTileWarpTokens * kTileWarpRows];
 #pragma unroll
-    for (int t = 0; t < kTileWarpTokens; ++t)
+    for (int t = 0; t < kTileWarpTokens / 2; ++t)
 #pragma unroll
-        for (int r = 0; r < kTileWarpRows; ++r) {
-            const float v = butterfly_sum(acc[r][t]);
-            if (lane == (uint32_t)(2 * t + r / 4)) {
-                if ((r & 3) == 0) out.x = v;
-                else if ((r & 3) == 1) out.y = v;
-                else if ((r & 3) == 2) out.z = v;
-                else out.w = v;
-            }
-        }
-    const uint32_t tok = t0 + tg * kTileWarpTokens + (lane >> 1);
-    const uint32_t e = e0 + rg * kTileWarpRows + (lane & 1) * 4;
-    if (tok < a.T) {
-        float* const dst = a.logits + (size_t)tok * a.ne + e;
-        if (e + 4 <= a.ne && (a.ne & 3u) == 0) {
-            *(float4*)dst = out;
-        } else {
-            if (e + 0 < a.ne) dst[0] = out.x;
-            if (e + 1 < a.ne) dst[1] = out.y;
-            if (e + 2 < a.ne) dst[2] = out.z;
-            if (e + 3 < a.ne) dst[3] = out.w;
-        }
-    }
+        for (int r = 0; r < kTileWarpRows; ++r)
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(sums[2 * t * kTileWarpRows + r]), "=f"(sums[(2 * t + 1) * kTileWarpRows + r]) : "l"(acc[r][t]));
+    store_tile(a, sums, e0 + rg * kTileWarpRows, t0 + tg * kTileWarpTokens, lane);
 }
 
 // The shared expert's scalar gate for many rows (the tiled router covers the expert rows only): one
 // warp per row of activations at a time, the gate row held in registers, the same lane order, fused
-// multiply-adds and butterfly as everywhere else. grid ceil(T / 32), block 256: a warp takes 4 rows.
+// multiply-adds and butterfly as everywhere else. A warp's rows follow one another at an L2 round trip each: a row per
+// warp while the blocks fit the SMs once (333 rows: 8.3 -> 3.5 us), four beyond, where fetching the gate row again costs
+// more (4096 rows: 9 us against 11).
 __global__ void __launch_bounds__(256) router_gate_rows_kernel(const RouterArgs a) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t chunks = a.d / 4;
     const size_t esz = a.dt == SHRIKE_DTYPE_FP32 ? 4 : 2;
     float4 wr[kRouterMaxChunks];
     load_row_f32<kRouterMaxChunks, true>(a.gate_row, chunks, lane, wr);
-    for (uint32_t j = 0; j < 4; ++j) {
-        const uint32_t tk = blockIdx.x * 32 + warp * 4 + j;
-        if (tk >= a.T) break;
+    for (uint32_t tk = blockIdx.x * 8 + warp; tk < a.T; tk += gridDim.x * 8) {
         const void* xrow = (const uint8_t*)a.hidden + (size_t)tk * a.stride * esz;
         const float acc = butterfly_sum(lane_dot_f32<kRouterMaxChunks, true>(wr, chunks, lane, xrow, a.dt, nullptr));
         if (lane == 0) a.gate_out[tk] = sigmoid_det(acc);
@@ -614,7 +612,7 @@ cudaError_t launch_router(const shrike_moe* m, cudaStream_t st, const shrike_rou
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         if (a.gate_row) {
-            router_gate_rows_kernel<<<(T + 31) / 32, 256, 0, st>>>(a);
+            router_gate_rows_kernel<<<T <= 8u * (uint32_t)m->sm_count ? (T + 7) / 8 : (T + 31) / 32, 256, 0, st>>>(a);
             e = cudaGetLastError();
             if (e != cudaSuccess) return e;
         }
