@@ -309,6 +309,7 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
     A(&w.yacc, T > SHRIKE_MAX_DECODE_TOKENS ? T * c.d * 4 : 0);
     A(&w.chunk_inst, T > SHRIKE_MAX_DECODE_TOKENS ? umma_max_chunk_instances(c, c.max_tokens) * umma_chunk_instance_bytes() : 0);
     A(&w.n_chunk_inst, 16);
+    if (T > SHRIKE_MAX_DECODE_TOKENS) A(&w.pos_of_pair, T * K * 4);
     if (T > SHRIKE_MAX_DECODE_TOKENS) A(&w.xs, T * K * c.d * 2);   // prefill operands
     A(&w.x_dev, T * c.d * ab);
     A(&w.y_dev, T * c.d * yb);

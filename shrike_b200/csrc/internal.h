@@ -89,7 +89,8 @@ struct Workspace {
     uint32_t* slot_of_expert = nullptr;
     float* yacc = nullptr;          // prefill: fp32 output accumulator [max_tokens x d]
     void* chunk_inst = nullptr;     // prefill: instances of up to 256 rows (tensor-core path)
-    uint32_t* n_chunk_inst = nullptr; // [0] instances, [1] sorted rows, [2], [3] tiles handed out per phase
+    uint32_t* n_chunk_inst = nullptr; // [0] instances, [1], [2] tiles handed out per phase
+    uint32_t* pos_of_pair = nullptr; // prefill: place of every pair in the expert-sorted order, or 0xffffffff
     uint16_t* xs = nullptr;         // prefill: fp16 activation rows in expert-sorted order [max_tokens x top_k x d]
     void* tensor_maps = nullptr;    // host: the TMA descriptors of xs, acts, xh, acts_shared
     // one-row decode layer in one launch (fused_layer.cu)
@@ -171,7 +172,8 @@ cudaError_t launch_decode_plan(const shrike_moe* m, cudaStream_t st, const uint3
                                bool with_shared, uint32_t pool_cells);
 cudaError_t launch_group_pairs(const shrike_moe* m, cudaStream_t st, const uint32_t* ids,
                                const float* weights, uint32_t T, uint32_t* sorted_pairs,
-                               uint32_t* offsets, uint32_t* counts);
+                               uint32_t* offsets, uint32_t* counts, const uint32_t* slots = nullptr,
+                               const uint32_t* io_status = nullptr);
 // decode.cu
 cudaError_t launch_phase1(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a,
                           uint32_t max_inst, bool pdl);

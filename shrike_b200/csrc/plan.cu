@@ -89,20 +89,29 @@ cudaError_t launch_decode_plan(const shrike_moe* m, cudaStream_t st, const uint3
 constexpr uint32_t kGroupTokens = 128;  // rows per block
 
 // Step 1: per block, a bitmap of the rows that chose each expert; writes the
-// per-(block, expert) counts.
+// per-(block, expert) counts and, given the pairs' cells, the cell of every expert that has a pair (a streamed batch
+// whose status word is not READY, moe_io_ready, moe.metal:36-39, leaves every expert without one).
 __global__ void __launch_bounds__(256)
 group_hist_kernel(const uint32_t* __restrict__ ids, uint32_t T, uint32_t top_k, uint32_t ne,
-                  uint32_t* __restrict__ block_hist, uint32_t* status) {
+                  uint32_t* __restrict__ block_hist, uint32_t* status, const uint32_t* __restrict__ slots,
+                  const uint32_t* __restrict__ io_status, uint32_t* __restrict__ slot_of_expert) {
     __shared__ uint32_t bits[SHRIKE_MAX_EXPERTS][kGroupTokens / 32];
     const uint32_t t0 = blockIdx.x * kGroupTokens;
     for (uint32_t i = threadIdx.x; i < SHRIKE_MAX_EXPERTS * (kGroupTokens / 32); i += blockDim.x)
         (&bits[0][0])[i] = 0;
+    bool ready = true;
+    if (io_status) {
+        const uint32_t s = *io_status;
+        ready = s == 1u || s == 3u;
+    }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < kGroupTokens * top_k; i += blockDim.x) {
         const uint32_t tl = i / top_k, t = t0 + tl;
         if (t < T) {
-            const uint32_t e = ids[(size_t)t * top_k + (i - tl * top_k)];
+            const size_t p = (size_t)t * top_k + (i - tl * top_k);
+            const uint32_t e = ids[p];
             if (e < ne) {
+                if (slots) slot_of_expert[e] = ready ? slots[p] : SHRIKE_SLOT_MISS;
                 // a row that names one expert twice (no top-k router does) is counted once and reported
                 const uint32_t bit = 1u << (tl & 31);
                 if (atomicOr(&bits[e][tl >> 5], bit) & bit) report_status(status, kStatusBadIndex);
@@ -151,7 +160,8 @@ group_scan_kernel(uint32_t* __restrict__ block_hist, uint32_t n_blocks, uint32_t
 __global__ void __launch_bounds__(256)
 group_place_kernel(const uint32_t* __restrict__ ids, const float* __restrict__ weights, uint32_t T,
                    uint32_t top_k, uint32_t ne, const uint32_t* __restrict__ block_base,
-                   uint32_t* __restrict__ sorted_pairs, uint32_t* __restrict__ sorted_ids) {
+                   uint32_t* __restrict__ sorted_pairs, uint32_t* __restrict__ sorted_ids,
+                   const uint32_t* __restrict__ slots, uint32_t* __restrict__ pos_of_pair) {
     __shared__ uint32_t bits[SHRIKE_MAX_EXPERTS][kGroupTokens / 32];
     const uint32_t t0 = blockIdx.x * kGroupTokens;
     for (uint32_t i = threadIdx.x; i < SHRIKE_MAX_EXPERTS * (kGroupTokens / 32); i += blockDim.x)
@@ -169,7 +179,10 @@ group_place_kernel(const uint32_t* __restrict__ ids, const float* __restrict__ w
         const uint32_t tl = i / top_k, t = t0 + tl, r = i - tl * top_k;
         if (t >= T) continue;
         const uint32_t e = ids[(size_t)t * top_k + r];
-        if (e >= ne) continue;
+        if (e >= ne) {
+            if (pos_of_pair) pos_of_pair[(size_t)t * top_k + r] = 0xffffffffu;
+            continue;
+        }
         uint32_t before = 0;
         const uint32_t word = tl >> 5;
         for (uint32_t w = 0; w < word; ++w) before += __popc(bits[e][w]);
@@ -183,12 +196,14 @@ group_place_kernel(const uint32_t* __restrict__ ids, const float* __restrict__ w
             ((uint4*)sorted_pairs)[pos] = p;
         }
         if (sorted_ids) sorted_ids[pos] = t * top_k + r;
+        // (no row is needed where the expert has no cell)
+        if (pos_of_pair) pos_of_pair[(size_t)t * top_k + r] = slots[(size_t)t * top_k + r] == SHRIKE_SLOT_MISS ? 0xffffffffu : pos;
     }
 }
 
 cudaError_t launch_group_pairs(const shrike_moe* m, cudaStream_t st, const uint32_t* ids,
                                const float* weights, uint32_t T, uint32_t* sorted_pairs,
-                               uint32_t* offsets, uint32_t* counts) {
+                               uint32_t* offsets, uint32_t* counts, const uint32_t* slots, const uint32_t* io_status) {
     const uint32_t nb = (T + kGroupTokens - 1) / kGroupTokens;
     const uint32_t ne = m->cfg.num_experts, k = m->cfg.top_k;
     if (nb == 0) {
@@ -196,10 +211,11 @@ cudaError_t launch_group_pairs(const shrike_moe* m, cudaStream_t st, const uint3
         if (e != cudaSuccess) return e;
         return cudaMemsetAsync(offsets, 0xff, ne * 4, st);
     }
-    group_hist_kernel<<<nb, 256, 0, st>>>(ids, T, k, ne, m->ws.block_hist, m->ws.status);
+    group_hist_kernel<<<nb, 256, 0, st>>>(ids, T, k, ne, m->ws.block_hist, m->ws.status, slots, io_status,
+                                          m->ws.slot_of_expert);
     group_scan_kernel<<<1, 256, 0, st>>>(m->ws.block_hist, nb, ne, offsets, counts);
     group_place_kernel<<<nb, 256, 0, st>>>(ids, weights, T, k, ne, m->ws.block_hist, sorted_pairs,
-                                           m->ws.sorted);
+                                           m->ws.sorted, slots, slots ? m->ws.pos_of_pair : nullptr);
     return cudaGetLastError();
 }
 

@@ -61,34 +61,28 @@ prefill_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* _
     if (threadIdx.x == 0) *n_inst = total + n_shared;
 }
 
-// x -> fp16 operand layout and per-group sums, all rows.
+// x -> fp16 operand layout and per-group sums, all rows; given the pairs' places, also into the expert-sorted rows that the
+// grouped GEMM copies its tiles from. (Bound by the sorted rows' bytes, top_k times x's: as a kernel of its own that read
+// them back, the gather took 28 us of a 4096-row call beside 11 here.)
 __global__ void __launch_bounds__(256)
 prefill_xprep_kernel(const void* __restrict__ x, uint32_t T, uint32_t d, uint32_t group, uint32_t act_dtype,
                      uint32_t int4, uint16_t* __restrict__ xh, float* __restrict__ xsum, uint32_t* status,
-                     const uint32_t* __restrict__ row_map, const uint32_t* __restrict__ n_rows_dev) {
+                     const uint32_t* __restrict__ row_map, const uint32_t* __restrict__ n_rows_dev,
+                     const uint32_t* __restrict__ pos_of_pair, uint32_t top_k, uint16_t* __restrict__ xs) {
     const uint32_t items = T * (d / 8);
     const size_t row_bytes = (size_t)d * (act_dtype == SHRIKE_DTYPE_FP32 ? 4 : 2);
     const uint32_t n_rows = n_rows_dev ? *n_rows_dev : T;
-    for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < items; i0 += gridDim.x * blockDim.x)
-        xprep_item(x, row_bytes, d, group, act_dtype, int4 != 0, i0 + threadIdx.x, i0 + threadIdx.x < items, xh,
-                   xsum, status, row_map, n_rows);
-}
-
-// slot_of_expert[e] = the cell every pair of expert e resolved to.
-// A streamed batch whose status word is not READY (moe_io_ready, moe.metal:36-39) leaves every expert
-// without a cell: only the shared term remains.
-__global__ void __launch_bounds__(256)
-prefill_slot_of_expert_kernel(const uint32_t* __restrict__ ids, const uint32_t* __restrict__ slots,
-                              uint32_t n_pairs, uint32_t ne, const uint32_t* __restrict__ io_status,
-                              uint32_t* __restrict__ slot_of_expert) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (io_status) {
-        const uint32_t s = *io_status;
-        if (s != 1u && s != 3u) return;
-    }
-    if (i < n_pairs) {
-        const uint32_t e = ids[i];
-        if (e < ne) slot_of_expert[e] = slots[i];
+    for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < items; i0 += gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + threadIdx.x;
+        xprep_item(x, row_bytes, d, group, act_dtype, int4 != 0, i, i < items, xh, xsum, status, row_map, n_rows);
+        const uint32_t row = i / (d / 8);
+        if (!pos_of_pair || i >= items || row >= n_rows) continue;
+        const uint4 v = *(const uint4*)(xh + (size_t)i * 8);   // this thread's own
+        const uint32_t col = (i - row * (d / 8)) * 8;
+        for (uint32_t r = 0; r < top_k; ++r) {
+            const uint32_t pos = pos_of_pair[(size_t)row * top_k + r];
+            if (pos != 0xffffffffu) *(uint4*)(xs + (size_t)pos * d + col) = v;
+        }
     }
 }
 
@@ -112,15 +106,10 @@ cudaError_t launch_prefill_plan(const shrike_moe* m, cudaStream_t st, const uint
                                 const uint32_t* row_map, const uint32_t* n_rows, float* accumulator) {
     const shrike_moe_config& c = m->cfg;
     const Workspace& ws = m->ws;
-    cudaError_t e = cudaMemsetAsync(ws.slot_of_expert, 0xff, c.num_experts * 4, st);
-    if (e != cudaSuccess) return e;
     // the rows the down epilogue adds into: the workspace's, or the caller's fp32 output itself
-    e = cudaMemsetAsync(accumulator ? accumulator : ws.yacc, 0, (size_t)T * c.d * 4, st);
+    cudaError_t e = cudaMemsetAsync(accumulator ? accumulator : ws.yacc, 0, (size_t)T * c.d * 4, st);
     if (e != cudaSuccess) return e;
-    const uint32_t n_pairs = T * c.top_k;
-    prefill_slot_of_expert_kernel<<<(n_pairs + 255) / 256, 256, 0, st>>>(ids, slots, n_pairs, c.num_experts,
-                                                                         io_status, ws.slot_of_expert);
-    e = launch_group_pairs(m, st, ids, nullptr, T, nullptr, ws.expert_offsets, ws.expert_counts);
+    e = launch_group_pairs(m, st, ids, nullptr, T, nullptr, ws.expert_offsets, ws.expert_counts, slots, io_status);
     if (e != cudaSuccess) return e;
     if (warp_mma_instances)   // the tensor-core path builds its own 256-row instances
         prefill_instances_kernel<<<1, 256, 0, st>>>(ws.expert_offsets, ws.expert_counts, ws.slot_of_expert,
@@ -128,7 +117,8 @@ cudaError_t launch_prefill_plan(const shrike_moe* m, cudaStream_t st, const uint
                                                     ws.inst, ws.n_inst, ws.status);
     const uint32_t items = T * (c.d / 8);
     prefill_xprep_kernel<<<min(2048u, (items + 255) / 256), 256, 0, st>>>(
-        x, T, c.d, c.group_size, c.act_dtype, c.weight_bits == 4 ? 1u : 0u, ws.xh, ws.xsum, ws.status, row_map, n_rows);
+        x, T, c.d, c.group_size, c.act_dtype, c.weight_bits == 4 ? 1u : 0u, ws.xh, ws.xsum, ws.status, row_map, n_rows,
+        warp_mma_instances ? nullptr : ws.pos_of_pair, c.top_k, ws.xs);
     return cudaGetLastError();
 }
 

@@ -680,7 +680,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         uint32_t pk_use = 0, sc_use = 0, slot = 0;
         for (uint32_t turn = 0;; ++turn) {
             const uint32_t s = turn & 1;
-            const uint32_t t = turn == 0 ? blockIdx.x : gridDim.x + atomicAdd(n_inst + 2 + PHASE, 1u);
+            const uint32_t t = turn == 0 ? blockIdx.x : gridDim.x + atomicAdd(n_inst + 1 + PHASE, 1u);
             if (!pipe_wait(&next_empty[s], ((turn >> 1) & 1) ^ 1)) { give_up(); break; }
             *(volatile uint32_t*)&next_tile[s] = t;
             mbar_arrive(&next_full[s]);
@@ -730,13 +730,13 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
 }
 
 // One thread per expert: ceil(count/256) chunk instances each, then the shared expert's.
-// n_inst[0] = instances, n_inst[1] = sorted rows in total.
+// n_inst[0] = instances, [1], [2]: tiles handed out in phase 0, 1.
 __global__ void __launch_bounds__(256)
 chunk_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ counts,
                        const uint32_t* __restrict__ slot_of_expert, uint32_t ne, uint32_t T, uint32_t with_shared,
                        uint32_t pool_cells, ChunkInstance* __restrict__ inst, uint32_t* __restrict__ n_inst,
                        uint32_t* status) {
-    __shared__ uint32_t warp_sums[8], warp_rows[8], by_size[256];
+    __shared__ uint32_t warp_sums[8], by_size[256];
     __shared__ __align__(16) uint32_t key[256];
     // Experts with the most rows first: a tile of 256 rows takes twice the time of one of 16, and a list that ends on long
     // ones leaves SMs idle (4096 rows: the last ended a tenth after the median SM).
@@ -764,21 +764,18 @@ chunk_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __r
         if (slot != SHRIKE_SLOT_MISS) n = (c + kUmmaMaxN - 1) / kUmmaMaxN;
     }
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t inc = n, rows = c;
+    uint32_t inc = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= (uint32_t)o) inc += v;
-        rows += __shfl_xor_sync(0xffffffffu, rows, o);
     }
     if (lane == 31) warp_sums[warp] = inc;
-    if (lane == 0) warp_rows[warp] = rows;
     __syncthreads();
-    uint32_t base = 0, total = 0, total_rows = 0;
+    uint32_t base = 0, total = 0;
     for (uint32_t w = 0; w < 8; ++w) {
         if (w < warp) base += warp_sums[w];
         total += warp_sums[w];
-        total_rows += warp_rows[w];
     }
     // The shared expert's instances come first in the list: they are full (256 rows), and the blocks of the
     // list's end are the last to start -- a launch that ends on its longest blocks ends late.
@@ -796,21 +793,8 @@ chunk_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __r
     }
     if (threadIdx.x == 0) {
         n_inst[0] = total + n_shared;
-        n_inst[1] = total_rows;
-        n_inst[2] = n_inst[3] = 0;   // tiles handed out, per phase
+        n_inst[1] = n_inst[2] = 0;   // tiles handed out, per phase
     }
-}
-
-// The activation rows in expert-sorted order: xs[pos] = xh[token of sorted pair pos].
-// grid (pairs); one block copies one row.
-__global__ void __launch_bounds__(128)
-gather_sorted_rows_kernel(const uint16_t* __restrict__ xh, const uint32_t* __restrict__ sorted,
-                          const uint32_t* __restrict__ n_inst, uint32_t top_k, uint32_t d, uint16_t* __restrict__ xs) {
-    const uint32_t pos = blockIdx.x;
-    if (pos >= n_inst[1]) return;
-    const uint4* src = (const uint4*)(xh + (size_t)(sorted[pos] / top_k) * d);
-    uint4* dst = (uint4*)(xs + (size_t)pos * d);
-    for (uint32_t i = threadIdx.x; i < d / 8; i += blockDim.x) dst[i] = __ldg(src + i);
 }
 
 // ---- tensor maps -------------------------------------------------------------------
@@ -966,9 +950,6 @@ cudaError_t launch_umma_prefill(const shrike_moe* m, cudaStream_t st, const Expe
     chunk_instances_kernel<<<1, 256, 0, st>>>(ws.expert_offsets, ws.expert_counts, ws.slot_of_expert, c.num_experts, T,
                                               c.has_shared, pool_cells, inst, ws.n_chunk_inst, ws.status);
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    gather_sorted_rows_kernel<<<T * c.top_k, 128, 0, st>>>(ws.xh, ws.sorted, ws.n_chunk_inst, c.top_k, c.d, ws.xs);
-    e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const uint32_t bits = c.weight_bits, grp = c.group_size;
     const bool f16 = c.meta_dtype == SHRIKE_DTYPE_FP16;
