@@ -3,7 +3,7 @@
 // mpp_prefill_affine_grouped_f16, tensorops.metal:145-248, and of
 // encodeGroupedExpertGEMMs, PrefillGroupedRoutedMoE.swift:925-1035).
 //
-// One block = 256 weight rows of one expert against up to 256 of the rows routed
+// One tile = 256 weight rows of one expert against up to 256 of the rows routed
 // to it ("swap-AB": the weights are the M operand -- two 128-row tiles, each
 // with its own TMEM accumulator -- and the activation rows the N operand, so an
 // expert with few rows still fills the MMA's M dimension). A 256 x 256 block
@@ -21,10 +21,11 @@
 //   warps 0-15 converters: two threads per weight row; per 64-wide K block
 //              they turn the packed nibbles/bytes into fp16 (q - Z) * scale +
 //              (bias + Z*scale) -- the reference's half(fma(q, scale, bias)),
-//              tensorops.metal:106 -- and writes them, 16 bytes at a time, into
-//              the K-major 128-byte-swizzled tile the MMA reads. After the K
-//              loop the same warps run the epilogue.
-//   warp 16    one thread issues tcgen05.mma (M 128, N = rows, K 16, fp16 in,
+//              tensorops.metal:106 -- and write them to TMEM (instances of up
+//              to 128 rows) or, 16 bytes at a time, into the K-major
+//              128-byte-swizzled tile in shared memory that the MMA reads.
+//              After the K loop the same warps run the epilogue.
+//   warp 16    one elected thread issues tcgen05.mma (M 128, N = rows, K 16, fp16 in,
 //              fp32 accumulate in TMEM) for both tiles and commits to the
 //              mbarriers that free the converted tile and the activation tile.
 //
@@ -33,6 +34,10 @@
 // PHASE 1: tiles = 256 consecutive down rows; epilogue (+ additive bias) x route
 //          weight -> red.global.add into the token's fp32 accumulator row (the
 //          weighted reduce, with no per-(row, rank) partial rows in between).
+//
+// What bounds it (256 experts of 2048 x 512): a K block takes 0.43 us at 16 rows, the converters' chain of waits, loads,
+// arithmetic and stores, and 0.74 us at 256, where shared memory's bandwidth (the instructions' operands, the copies' and
+// converters' stores) holds the tensor cores at 70 %.
 //
 // Every wait is bounded; a wait that gives up sets the status word and the
 // block falls through to the TMEM release.
@@ -89,6 +94,20 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint6
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+// The same with A in TMEM: row = lane, two fp16 a column.
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+          "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
@@ -215,7 +234,8 @@ struct alignas(16) ChunkInstance {  // up to 256 rows that share one expert bloc
 // rest), and the layout of the activation and weight stages. An instance with few rows needs narrow activation tiles and
 // gets more weight stages instead: what paces such a tile is the round trip converters -> tensor core -> converters.
 struct TileShape {
-    uint32_t N, n1, b1, n2, b2, b_stage, off_a, a_stages;
+    uint32_t N, n1, b1, n2, b2, b_stage, off_a, a_stages, acc_step;
+    bool in_tmem;   // converted weights: stages of 64 TMEM columns from column 256 on
     __device__ explicit TileShape(uint32_t count) {
         N = (count + 15u) & ~15u;           // MMA N: rows padded to 16
         n1 = 16; b1 = 0;
@@ -228,7 +248,12 @@ struct TileShape {
         // three layouts: 64, 128 or 256 activation rows a stage
         b_stage = N <= 64 ? 64u * 128u : N <= 128 ? 128u * 128u : 256u * 128u;
         off_a = kBStages * b_stage;
-        a_stages = min(kMaxAStages, (kOffPk - off_a) / kAStageBytes);
+        // Up to 128 rows the accumulators leave TMEM room for the converted weights. From shared memory the tensor core
+        // needs 85 cycles to fetch the weights of an instruction, whatever its N; and the converters' stores and their
+        // fence fall away.
+        in_tmem = N <= 128;
+        acc_step = in_tmem ? 128u : kUmmaMaxN;
+        a_stages = in_tmem ? kMaxAStages : (kOffPk - off_a) / kAStageBytes;
     }
 };
 
@@ -335,8 +360,10 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             if (!ok) give_up();
             return ok;
         };
-        // Two threads per weight row: thread `half` converts 32 of the K block's 64 weights.
-        const uint32_t tile = tid >> 8, r = (tid >> 1) & 127, half = tid & 1;
+        // Two threads per weight row: thread `half` converts 32 of the K block's 64 weights. A lane is a row: the TMEM lanes
+        // that a warp reaches.
+        const uint32_t tile = (warp >> 2) & 1, r = (warp & 3) * 32 + lane, half = warp >> 3;
+        const uint32_t a_tmem = tmem_base + 256u + (((warp & 3) * 32) << 16) + tile * 32 + half * 16;
         constexpr uint32_t kWordsPerThread = kWordsPerBlock / 2;   // 4 (int4) or 8 (int8)
         const uint32_t pk_row = kOffPk + tile * (kPkSlotBytes / 2) + r * 64, pk_xor = (r >> 1) & 3;
         // What does not change along K: this thread's chunk positions in a packed slot and in the converted
@@ -350,12 +377,12 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                 const uint32_t c = sub * (kRowBlockBytes / 16) + half * (kWordsPerThread / 4) + q;
                 pk_off[sub * (kWordsPerThread / 4) + q] = pk_row + ((c ^ pk_xor) << 4);
             }
-        constexpr uint32_t kStores = BITS == 4 ? kWordsPerThread : kWordsPerThread / 2;   // 16-byte chunks written
-        uint32_t a_pos[kStores];
+        uint32_t a_pos[4];
 #pragma unroll
-        for (uint32_t i = 0; i < kStores; ++i)   // A row r: 8 chunks of 8 fp16; chunk c lives at position c ^ (r & 7)
-            a_pos[i] = tile * kTileBytes + r * 128 + (((half * kStores + i) ^ (r & 7)) << 4);
+        for (uint32_t i = 0; i < 4; ++i)   // A row r: 8 chunks of 8 fp16; chunk c lives at position c ^ (r & 7)
+            a_pos[i] = tile * kTileBytes + r * 128 + (((half * 4 + i) ^ (r & 7)) << 4);
 
+        bool wide = false;   // the last tile's accumulators took all of TMEM
         for (uint32_t turn = 0;; ++turn) {
             const uint32_t t = take_tile(turn);
             if (t >= n_tiles || failed()) break;
@@ -389,16 +416,16 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             const uint16_t* srow = (const uint16_t*)(base + off.s[mat]) + (size_t)mrow * G;
             const uint16_t* brow = (const uint16_t*)(base + off.b[mat]) + (size_t)mrow * G;
             // Groups 8*blk .. 8*blk+7 straight from global memory (rows past the matrix and groups past the row read as
-            // zero: the converted weights are then zero). An even number of groups: the warp's sixteen rows in 32-bit
-            // words, four lanes a row, put into the rows' places in shared memory when they are needed; read by each
-            // row's two threads in 16-bit pieces they kept L1 busy for 1.3 us per K block of 90-group rows.
+            // zero: the converted weights are then zero). An even number of groups: the warp's 32 rows in 32-bit words, four
+            // lanes a row, handed to the rows' lanes when they are needed; read by each row's threads in 16-bit pieces
+            // they kept L1 busy for 1.3 us per K block of 90-group rows.
             const bool words = (G & 1u) == 0;
-            const uint32_t my_rows = r0 + (PHASE == 0 ? 0u : tile * 128u) + ((warp * 16) & 127u) + (lane >> 2);
+            const uint32_t my_rows = r0 + (PHASE == 0 ? 0u : tile * 128u) + (warp & 3) * 32 + (lane >> 2);
             auto fetch_scales = [&](uint32_t blk) {
                 if (words) {
                     const uint32_t gi = blk * 8 + 2 * (lane & 3);
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) {
+                    for (int i = 0; i < 4; ++i) {
                         const uint32_t row = my_rows + 8 * i;
                         const bool there = row < out_rows && gi < G;
                         const size_t at = (size_t)row * G + gi;
@@ -426,6 +453,9 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             if (!sc_tma) fetch_scales(0);
             // A scale block (8 groups of the row) at a time, its K blocks unrolled: the position in the packed slot
             // and the group of a K block are then constants of the instruction stream.
+            // (a warp may write the stages while others still read the columns that they take of the last accumulators)
+            if (wide && ts.in_tmem && !converters_meet()) break;
+            wide = !ts.in_tmem;
             uint32_t st = 0;
             for (uint32_t kb0 = 0; kb0 < KB; kb0 += kKbPerSc) {
                 if (failed()) break;
@@ -442,17 +472,31 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                 } else {
                     // this block's 8 groups were fetched one block ago; fetch the next block's now
                     if (words) {
-                        uint8_t* const to = smem + kOffSc + (warp * 16 + (lane >> 2)) * 16 + (lane & 3) * 4;
                         __syncwarp();   // the last block's have been read
+                        if constexpr (GROUP == 32) {
+                            // through the scales' memory: a thread's half has the even or the odd groups, so the two warps
+                            // of a row write 16 bits of every word each
+                            uint8_t* const to = smem + kOffSc + (tile * 128 + (warp & 3) * 32 + (lane >> 2)) * 16 + (lane & 3) * 4 + half * 2;
 #pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            *(uint32_t*)(to + i * 128) = snext[i];
-                            *(uint32_t*)(to + kScHalfBytes + i * 128) = bnext[i];
+                            for (int i = 0; i < 4; ++i) {
+                                *(uint16_t*)(to + i * 128) = (uint16_t)(half ? snext[i] >> 16 : snext[i]);
+                                *(uint16_t*)(to + kScHalfBytes + i * 128) = (uint16_t)(half ? bnext[i] >> 16 : bnext[i]);
+                            }
+                            __syncwarp();
+                            const uint4 sv = *(const uint4*)(smem + kOffSc + (tile * 128 + r) * 16), bv = *(const uint4*)(smem + kOffSc + kScHalfBytes + (tile * 128 + r) * 16);
+                            sreg[0] = sv.x; sreg[1] = sv.y; sreg[2] = sv.z; sreg[3] = sv.w;
+                            breg[0] = bv.x; breg[1] = bv.y; breg[2] = bv.z; breg[3] = bv.w;
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {   // lane 4 (row mod 8) + word of load row / 8
+#pragma unroll
+                                for (int w = 0; w < 4; ++w) {
+                                    const uint32_t sv = __shfl_sync(0xffffffffu, snext[i], 4 * (lane & 7) + w);
+                                    const uint32_t bv = __shfl_sync(0xffffffffu, bnext[i], 4 * (lane & 7) + w);
+                                    if ((lane >> 3) == (uint32_t)i) { sreg[w] = sv; breg[w] = bv; }
+                                }
+                            }
                         }
-                        __syncwarp();
-                        const uint4 sv = *(const uint4*)(smem + kOffSc + (tid >> 1) * 16), bv = *(const uint4*)(smem + kOffSc + kScHalfBytes + (tid >> 1) * 16);
-                        sreg[0] = sv.x; sreg[1] = sv.y; sreg[2] = sv.z; sreg[3] = sv.w;
-                        breg[0] = bv.x; breg[1] = bv.y; breg[2] = bv.z; breg[3] = bv.w;
                     } else {
 #pragma unroll
                         for (int i = 0; i < 4; ++i) { sreg[i] = snext[i]; breg[i] = bnext[i]; }
@@ -479,19 +523,26 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                     const uint32_t s2 = half2_dup(sc), z2 = half2_dup(zf);
                     if (!pipe_wait(&a_empty[st], ((a_use >> st) & 1) ^ 1)) { give_up(); break; }
                     a_use ^= 1u << st;
-                    uint8_t* a_stage = smem + ts.off_a + st * kAStageBytes;
+                    uint32_t o[16];   // 32 weights
 #pragma unroll
                     for (uint32_t i = 0; i < kWordsPerThread; ++i) {
-                        uint32_t o[4];
-                        dequant_word<BITS>(pk[i], s2, z2, o);
-                        if constexpr (BITS == 4) {
-                            *(uint4*)(a_stage + a_pos[i]) = make_uint4(o[0], o[1], o[2], o[3]);
-                        } else {
-                            // two words make one 16-byte chunk
-                            *((uint2*)(a_stage + a_pos[i >> 1]) + (i & 1)) = make_uint2(o[0], o[1]);
-                        }
+                        uint32_t w4[4];
+                        dequant_word<BITS>(pk[i], s2, z2, w4);
+#pragma unroll
+                        for (uint32_t e = 0; e < 16 / kWordsPerThread; ++e) o[i * (16 / kWordsPerThread) + e] = w4[e];
                     }
-                    fence_async_smem();
+                    if (ts.in_tmem) {
+                        __syncwarp();
+                        tc_fence_after();   // the stage's last readers are done
+                        tmem_st16(a_tmem + st * 64, o);
+                        tc_fence_before();
+                    } else {
+                        uint8_t* a_stage = smem + ts.off_a + st * kAStageBytes;
+#pragma unroll
+                        for (uint32_t i = 0; i < 4; ++i)
+                            *(uint4*)(a_stage + a_pos[i]) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+                        fence_async_smem();
+                    }
                     __syncwarp();
                     const bool slot_done = sub == kSubMask || kb + 1 == KB;
                     if (lane == 0) {
@@ -536,7 +587,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                     for (uint32_t c0 = h * 8; c0 < N; c0 += kColStep) {
                         uint32_t g[8], u[8];
                         tmem_ld8_issue(taddr + c0, g);
-                        tmem_ld8_issue(taddr + kUmmaMaxN + c0, u);
+                        tmem_ld8_issue(taddr + ts.acc_step + c0, u);
                         tmem_ld_wait();
                         uint16_t* p = dst + (size_t)c0 * F;
                         const uint32_t live = f < F ? min(8u, in.count > c0 ? in.count - c0 : 0u) : 0u;   // rows of this group
@@ -576,7 +627,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                 for (uint32_t c0 = h * 8; c0 < N; c0 += kColStep) {
                     uint32_t v0[8], v1[8];
                     tmem_ld8_issue(taddr + c0, v0);
-                    tmem_ld8_issue(taddr + kUmmaMaxN + c0, v1);
+                    tmem_ld8_issue(taddr + ts.acc_step + c0, v1);
                     tmem_ld_wait();
                     const uint32_t live = min(8u, in.count > c0 ? in.count - c0 : 0u);
 #pragma unroll
@@ -605,9 +656,10 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             if (!open_tile(t, wk)) continue;
             const TileShape ts(wk.in.count);
             const uint32_t idesc = __shfl_sync(0xffffffffu, umma_idesc(ts.N), 0), acc0 = __shfl_sync(0xffffffffu, tmem_base, 0);
-            const uint32_t acc1 = acc0 + kUmmaMaxN, stages = __shfl_sync(0xffffffffu, ts.a_stages, 0);
+            const uint32_t acc1 = acc0 + __shfl_sync(0xffffffffu, ts.acc_step, 0), stages = __shfl_sync(0xffffffffu, ts.a_stages, 0);
             const uint32_t b_smem = __shfl_sync(0xffffffffu, smem_base, 0), a_smem = b_smem + __shfl_sync(0xffffffffu, ts.off_a, 0);
             const uint32_t b_step = __shfl_sync(0xffffffffu, ts.b_stage, 0), n_kb = __shfl_sync(0xffffffffu, wk.KB, 0);
+            const bool in_tmem = __shfl_sync(0xffffffffu, (uint32_t)ts.in_tmem, 0) != 0;
             uint32_t sa = 0, sb = 0;
             for (uint32_t kb = 0; kb < n_kb; ++kb) {
                 // (the first stage of converted weights also says that the last tile's accumulators have been read)
@@ -621,14 +673,23 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                 __syncwarp();
                 tc_fence_after();
                 if (elect_one()) {
-                    const uint64_t da0 = umma_smem_desc(a_smem + sa * kAStageBytes), da1 = umma_smem_desc(a_smem + sa * kAStageBytes + kTileBytes);
                     const uint64_t db = umma_smem_desc(b_smem + sb * b_step);
-                    // 4 x K16 per 64-wide block: 32 bytes further along the row. The two tiles alternate: consecutive
-                    // instructions then add into different accumulators.
+                    if (in_tmem) {
+                        const uint32_t ta = acc0 + 256u + sa * 64;   // 16 of K are eight columns
 #pragma unroll
-                    for (uint32_t k = 0; k < 4; ++k) {
-                        umma_f16(acc0, da0 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-                        umma_f16(acc1, da1 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                        for (uint32_t k = 0; k < 4; ++k) {
+                            umma_f16_ts(acc0, ta + 8 * k, db + 2 * k, idesc, (kb | k) != 0);
+                            umma_f16_ts(acc1, ta + 32 + 8 * k, db + 2 * k, idesc, (kb | k) != 0);
+                        }
+                    } else {
+                        const uint64_t da0 = umma_smem_desc(a_smem + sa * kAStageBytes), da1 = umma_smem_desc(a_smem + sa * kAStageBytes + kTileBytes);
+                        // 4 x K16 per 64-wide block: 32 bytes further along the row. The two tiles alternate: consecutive
+                        // instructions then add into different accumulators.
+#pragma unroll
+                        for (uint32_t k = 0; k < 4; ++k) {
+                            umma_f16(acc0, da0 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                            umma_f16(acc1, da1 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                        }
                     }
                     umma_commit(&a_empty[sa]);
                     umma_commit(&b_empty[sb]);
