@@ -166,13 +166,19 @@ int fill_expert_args(shrike_moe* m, const shrike_pool* pool, const shrike_expert
 }
 
 
+// Whether the streaming kernel is the faster one for a decode call. A single row has nothing to lay out ahead of the first
+// tile; two rows of small experts are about even (256 experts of 2048 x 512: 29.3 us a layer with the per-tile kernels,
+// 29.7 with it; three rows 34.8 and 33.9; experts of 7 MB at two rows 46.9 and 44.4).
+bool stream_pays(const shrike_moe_config& c, uint32_t T) {
+    return T > 2 || (T == 2 && (uint64_t)3 * c.d * c.f * c.weight_bits / 8 >= (4u << 20));
+}
+
 // The expert projections of a decode call's work lists (phases: 1, 2 or 3 = both). The streaming kernel takes every
-// shape whose tiles its ring and the tiled copies can hold; the per-tile kernels take the others, and single rows, which
-// have nothing to lay out ahead of the first tile.
+// shape whose tiles its ring and the tiled copies can hold; the per-tile kernels take the others.
 cudaError_t launch_experts(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, uint32_t T, uint32_t phases, void* y,
                            void* hidden, bool pdl) {
     const uint32_t n_shared = m->cfg.has_shared ? (T + 7) / 8 : 0;
-    cudaError_t e = T > 1 ? launch_expert_stream(m, st, a, T, n_shared, phases, false, y, hidden, pdl) : cudaErrorNotSupported;
+    cudaError_t e = stream_pays(m->cfg, T) ? launch_expert_stream(m, st, a, T, n_shared, phases, false, y, hidden, pdl) : cudaErrorNotSupported;
     if (e != cudaErrorNotSupported) return e;
     const uint32_t mi = max_instances(m->cfg, T);
     if ((phases & 1u) && (e = launch_phase1(m, st, a, mi, pdl)) != cudaSuccess) return e;
@@ -689,7 +695,7 @@ int shrike_encode_decode_layer(shrike_moe* m, void* stream, const shrike_pool* p
         if (fe != cudaErrorNotSupported) return cuda_fail(m, fe, "launch_fused_layer");
         // a block layout the tiled copies cannot describe: the three launches below
     }
-    if (query_count > 1) {
+    if (stream_pays(m->cfg, query_count)) {
         // some rows: the same in one launch of the streaming kernel (expert_stream.cu). In three launches the last
         // block of the router ranked every row while the others' SMs idled (8 us of 4 rows' 43, 20 of 16 rows' 92), and
         // the next launch began 3 us later.
