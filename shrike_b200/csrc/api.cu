@@ -126,7 +126,7 @@ bool router_operands_aligned(const shrike_moe_config& c, const shrike_router_ope
 namespace {
 
 void free_workspace(Workspace& w) {
-    if (w.slab) cudaFree(w.slab);
+    for (void* p : w.blocks) cudaFree(p);
     free(w.tensor_maps);
     free(w.fused_geom);
     free(w.fused_maps);
@@ -282,14 +282,20 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
     w.max_inst = max_instances(c, c.max_tokens);
     const size_t ab = act_bytes(c.act_dtype), yb = act_bytes(c.y_dtype);
     bool ok = true;
-    // one device allocation: the parts take their places first (a handle per layer is made at load time, and thirty
-    // calls of the allocator per handle were most of that)
+    // The small parts share a device allocation, the others have one each: requests below a megabyte share the driver's
+    // 2 MB mappings, and a mapping (0.3 ms) is what making a handle costs.
     struct Part { void** p; size_t at; };
-    std::vector<Part> slab_parts;
-    size_t slab = 0;
+    std::vector<Part> small_parts;
+    size_t small_bytes = 0;
     auto A = [&](auto** p, size_t bytes) {
-        slab_parts.push_back({(void**)p, slab});
-        slab += (bytes + 255) / 256 * 256;
+        if (bytes < (64u << 10)) {
+            small_parts.push_back({(void**)p, small_bytes});
+            small_bytes += (bytes + 255) / 256 * 256;
+            return;
+        }
+        void* at = nullptr;
+        if (ok && cudaMalloc(&at, bytes) != cudaSuccess) ok = false;
+        if (ok) { w.blocks.push_back(at); *(void**)p = at; }
     };
     // words that start at zero
     A(&w.status, 4);
@@ -297,7 +303,7 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
     A(&w.done_counter, 4);
     A(&w.arrived, 8);
     A(&w.fused_epoch, 4);
-    const size_t zeroed = slab;
+    const size_t zeroed = small_bytes;
     A(&w.logits, T * c.num_experts * 4);
     A(&w.xh, T * c.d * 2);
     A(&w.xsum, T * (c.d / c.group_size) * 4);
@@ -338,15 +344,17 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
         free(w.fused_geom);
         w.fused_geom = nullptr;
     }
-    if (ok) ok = cudaMalloc(&w.slab, slab) == cudaSuccess;
+    void* small = nullptr;
+    if (ok) ok = cudaMalloc(&small, small_bytes) == cudaSuccess;
+    if (ok) w.blocks.push_back(small);
     if (!ok) {
         free_workspace(w);
         delete m;
         cudaGetLastError();
         return fail(nullptr, SHRIKE_ENOMEM, "device allocation of the workspace failed");
     }
-    for (const Part& p : slab_parts) *p.p = (uint8_t*)w.slab + p.at;
-    cudaMemset(w.slab, 0, zeroed);
+    for (const Part& p : small_parts) *p.p = (uint8_t*)small + p.at;
+    cudaMemset(small, 0, zeroed);
     if (w.fused_geom) {
         // no logit carries the first epoch's tag, no activation has been published
         cudaMemset(w.fused_logits, 0xff, fused_logits_bytes(c));

@@ -1,6 +1,7 @@
 // Internals of the opaque handles and the launch entry points the C ABI calls.
 #pragma once
 
+#include <vector>
 #include <string>
 
 #include "common.cuh"
@@ -68,7 +69,7 @@ struct ExpertArgs {
 };
 
 struct Workspace {
-    void* slab = nullptr;           // the one device allocation that the pointers below lie in
+    std::vector<void*> blocks;      // the device allocations that the pointers below lie in
     float* logits = nullptr;        // [max_tokens x num_experts]
     uint16_t* xh = nullptr;
     float* xsum = nullptr;
