@@ -949,6 +949,7 @@ int shrike_ep_create(shrike_moe* home, shrike_moe* routed, uint32_t rank, uint32
     cudaMemset(ep->miss_slots, 0xff, T * K * 4);
     ep->peer[rank] = ep->mine;
     ep->connected = world == 1;
+    home->beside_others = routed->beside_others = true;
     *out = ep;
     return SHRIKE_OK;
 }

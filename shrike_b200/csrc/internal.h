@@ -1,6 +1,7 @@
 // Internals of the opaque handles and the launch entry points the C ABI calls.
 #pragma once
 
+#include <utility>
 #include <vector>
 #include <string>
 
@@ -126,6 +127,8 @@ struct shrike_moe {
     int sm_count = 148;
     uint32_t smem_optin = 0;      // most dynamic shared memory of a block
     bool no_pdl = false;          // SHRIKE_NO_PDL was set when the handle was created (diagnostics)
+    bool beside_others = false;   // one of an expert-parallel layer's handles: another stream's kernels run beside this one's,
+                                  // and blocks that wait on an SM for their predecessor would keep them off it
     bool single_stream = false;   // SHRIKE_SINGLE_STREAM was set when the handle was created: nothing else runs on the GPU
                                   // beside this handle's stream, so the one-launch layer need not be a cooperative launch
     bool force_warp_mma = false;  // SHRIKE_PREFILL_PATH=mma was set when the handle was created (test switch)
@@ -180,6 +183,22 @@ cudaError_t launch_phase1(const shrike_moe* m, cudaStream_t st, const ExpertArgs
                           uint32_t max_inst, bool pdl);
 cudaError_t launch_phase2(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, uint32_t T,
                           uint32_t max_inst, void* y, void* hidden, bool pdl);
+// Launch of a kernel that waits for its predecessor itself (pdl_wait before it reads what that one writes): it is set up
+// while the predecessor ends. The kernels of a prefill call are short beside the gaps between launches.
+template <class... P, class... A>
+cudaError_t launch_after(const shrike_moe* m, cudaStream_t st, void (*k)(P...), dim3 grid, unsigned block, size_t smem, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = m->no_pdl || m->beside_others ? 0 : 1;
+    return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
 // expert_stream.cu
 struct RouterArgs;
 cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const ExpertArgs& ea, uint32_t T, uint32_t n_shared,

@@ -95,6 +95,8 @@ __global__ void __launch_bounds__(256)
 group_hist_kernel(const uint32_t* __restrict__ ids, uint32_t T, uint32_t top_k, uint32_t ne,
                   uint32_t* __restrict__ block_hist, uint32_t* status, const uint32_t* __restrict__ slots,
                   const uint32_t* __restrict__ io_status, uint32_t* __restrict__ slot_of_expert) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ uint32_t bits[SHRIKE_MAX_EXPERTS][kGroupTokens / 32];
     const uint32_t t0 = blockIdx.x * kGroupTokens;
     for (uint32_t i = threadIdx.x; i < SHRIKE_MAX_EXPERTS * (kGroupTokens / 32); i += blockDim.x)
@@ -136,6 +138,8 @@ group_hist_kernel(const uint32_t* __restrict__ ids, uint32_t T, uint32_t top_k, 
 __global__ void __launch_bounds__(256)
 group_scan_kernel(uint32_t* __restrict__ block_hist, uint32_t n_blocks, uint32_t ne,
                   uint32_t* __restrict__ offsets, uint32_t* __restrict__ counts) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ uint32_t warp_sums[8];
     const uint32_t e = threadIdx.x;
     uint32_t total = 0;
@@ -162,6 +166,8 @@ group_place_kernel(const uint32_t* __restrict__ ids, const float* __restrict__ w
                    uint32_t top_k, uint32_t ne, const uint32_t* __restrict__ block_base,
                    uint32_t* __restrict__ sorted_pairs, uint32_t* __restrict__ sorted_ids,
                    const uint32_t* __restrict__ slots, uint32_t* __restrict__ pos_of_pair) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ uint32_t bits[SHRIKE_MAX_EXPERTS][kGroupTokens / 32];
     const uint32_t t0 = blockIdx.x * kGroupTokens;
     for (uint32_t i = threadIdx.x; i < SHRIKE_MAX_EXPERTS * (kGroupTokens / 32); i += blockDim.x)
@@ -213,10 +219,10 @@ cudaError_t launch_group_pairs(const shrike_moe* m, cudaStream_t st, const uint3
     }
     group_hist_kernel<<<nb, 256, 0, st>>>(ids, T, k, ne, m->ws.block_hist, m->ws.status, slots, io_status,
                                           m->ws.slot_of_expert);
-    group_scan_kernel<<<1, 256, 0, st>>>(m->ws.block_hist, nb, ne, offsets, counts);
-    group_place_kernel<<<nb, 256, 0, st>>>(ids, weights, T, k, ne, m->ws.block_hist, sorted_pairs,
-                                           m->ws.sorted, slots, slots ? m->ws.pos_of_pair : nullptr);
-    return cudaGetLastError();
+    cudaError_t e = launch_after(m, st, group_scan_kernel, dim3(1), 256, 0, m->ws.block_hist, nb, ne, offsets, counts);
+    if (e != cudaSuccess) return e;
+    return launch_after(m, st, group_place_kernel, dim3(nb), 256, 0, ids, weights, T, k, ne, m->ws.block_hist, sorted_pairs,
+                        m->ws.sorted, slots, slots ? m->ws.pos_of_pair : nullptr);
 }
 
 }  // namespace shrike

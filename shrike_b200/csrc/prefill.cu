@@ -69,6 +69,8 @@ prefill_xprep_kernel(const void* __restrict__ x, uint32_t T, uint32_t d, uint32_
                      uint32_t int4, uint16_t* __restrict__ xh, float* __restrict__ xsum, uint32_t* status,
                      const uint32_t* __restrict__ row_map, const uint32_t* __restrict__ n_rows_dev,
                      const uint32_t* __restrict__ pos_of_pair, uint32_t top_k, uint16_t* __restrict__ xs) {
+    pdl_wait();
+    pdl_launch_dependents();
     const uint32_t items = T * (d / 8);
     const size_t row_bytes = (size_t)d * (act_dtype == SHRIKE_DTYPE_FP32 ? 4 : 2);
     const uint32_t n_rows = n_rows_dev ? *n_rows_dev : T;
@@ -90,6 +92,8 @@ prefill_xprep_kernel(const void* __restrict__ x, uint32_t T, uint32_t d, uint32_
 __global__ void __launch_bounds__(256)
 prefill_combine_kernel(const float* __restrict__ yacc, uint32_t n, uint32_t act_dtype, uint32_t y_dtype,
                        void* __restrict__ y, void* __restrict__ hidden) {
+    pdl_wait();
+    pdl_launch_dependents();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float acc = yacc[i];
@@ -116,17 +120,15 @@ cudaError_t launch_prefill_plan(const shrike_moe* m, cudaStream_t st, const uint
                                                     c.num_experts, T, with_shared ? 1u : 0u, pool_cells, ws.sorted,
                                                     ws.inst, ws.n_inst, ws.status);
     const uint32_t items = T * (c.d / 8);
-    prefill_xprep_kernel<<<min(2048u, (items + 255) / 256), 256, 0, st>>>(
-        x, T, c.d, c.group_size, c.act_dtype, c.weight_bits == 4 ? 1u : 0u, ws.xh, ws.xsum, ws.status, row_map, n_rows,
-        warp_mma_instances ? nullptr : ws.pos_of_pair, c.top_k, ws.xs);
-    return cudaGetLastError();
+    return launch_after(m, st, prefill_xprep_kernel, dim3(min(2048u, (items + 255) / 256)), 256, 0, x, T, c.d, c.group_size, c.act_dtype,
+                        c.weight_bits == 4 ? 1u : 0u, ws.xh, ws.xsum, ws.status, row_map, n_rows,
+                        (const uint32_t*)(warp_mma_instances ? nullptr : ws.pos_of_pair), c.top_k, ws.xs);
 }
 
 cudaError_t launch_prefill_combine(const shrike_moe* m, cudaStream_t st, uint32_t T, void* y, void* hidden) {
     const shrike_moe_config& c = m->cfg;
     const uint32_t n = T * c.d;
-    prefill_combine_kernel<<<(n + 255) / 256, 256, 0, st>>>(m->ws.yacc, n, c.act_dtype, c.y_dtype, y, hidden);
-    return cudaGetLastError();
+    return launch_after(m, st, prefill_combine_kernel, dim3((n + 255) / 256), 256, 0, m->ws.yacc, n, c.act_dtype, c.y_dtype, y, hidden);
 }
 
 }  // namespace shrike

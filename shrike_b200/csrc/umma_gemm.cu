@@ -272,7 +272,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
     constexpr float kZero = BITS == 4 ? 8.0f : 128.0f;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    const uint32_t n_tiles = n_inst[0] * row_tiles;
+    pdl_launch_dependents();
     // Scale rows that are whole 16-byte units come by TMA; others (groups % 8 != 0) are read by the converters. One way for
     // all instances: both use the same memory, which the copy thread would fill a tile ahead.
     const bool sc_tma = PHASE == 0 ? (a.d / GROUP & 7u) == 0 : ((a.f / GROUP | a.f_shared / GROUP) & 7u) == 0;
@@ -316,6 +316,8 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();   // all of the above runs while the last kernel ends
+    const uint32_t n_tiles = n_inst[0] * row_tiles;
     auto give_up = [&]() {
         report_status(a.status, kStatusWaitTimeout);
         *(volatile uint32_t*)&s_failed = 1;
@@ -797,6 +799,8 @@ chunk_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __r
                        const uint32_t* __restrict__ slot_of_expert, uint32_t ne, uint32_t T, uint32_t with_shared,
                        uint32_t pool_cells, ChunkInstance* __restrict__ inst, uint32_t* __restrict__ n_inst,
                        uint32_t* status) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ uint32_t warp_sums[8], by_size[256];
     __shared__ __align__(16) uint32_t key[256];
     // Experts with the most rows first: a tile of 256 rows takes twice the time of one of 16, and a list that ends on long
@@ -945,8 +949,8 @@ cudaError_t umma_prepare(shrike_moe* m) {
 }
 
 template <int BITS, int GROUP, int META>
-static cudaError_t launch_umma_t(cudaStream_t st, const ExpertArgs& a, const ChunkInstance* inst,
-                                 uint32_t* n_inst, uint32_t max_inst, uint32_t sm_count, const UmmaMaps& m0, const UmmaMaps& m1) {
+static cudaError_t launch_umma_t(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, const ChunkInstance* inst,
+                                 uint32_t* n_inst, uint32_t max_inst, const UmmaMaps& m0, const UmmaMaps& m1) {
     auto k0 = umma_expert_kernel<BITS, GROUP, META, 0>;
     auto k1 = umma_expert_kernel<BITS, GROUP, META, 1>;
     cudaError_t e = cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUmmaSmemBytes);
@@ -954,12 +958,11 @@ static cudaError_t launch_umma_t(cudaStream_t st, const ExpertArgs& a, const Chu
     e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUmmaSmemBytes);
     if (e != cudaSuccess) return e;
     const uint32_t fmax = a.f_shared > a.f ? a.f_shared : a.f;
+    const uint32_t sm_count = (uint32_t)m->sm_count;
     const uint32_t t0 = (fmax + 127) / 128, t1 = (a.d + 255) / 256;
-    k0<<<std::min(sm_count, max_inst * t0), kUmmaThreads, kUmmaSmemBytes, st>>>(a, inst, n_inst, t0, m0);
-    e = cudaGetLastError();
+    e = launch_after(m, st, k0, dim3(std::min(sm_count, max_inst * t0)), kUmmaThreads, kUmmaSmemBytes, a, inst, n_inst, t0, m0);
     if (e != cudaSuccess) return e;
-    k1<<<std::min(sm_count, max_inst * t1), kUmmaThreads, kUmmaSmemBytes, st>>>(a, inst, n_inst, t1, m1);
-    return cudaGetLastError();
+    return launch_after(m, st, k1, dim3(std::min(sm_count, max_inst * t1)), kUmmaThreads, kUmmaSmemBytes, a, inst, n_inst, t1, m1);
 }
 
 uint32_t umma_max_chunk_instances(const shrike_moe_config& c, uint32_t T) {
@@ -1008,14 +1011,13 @@ cudaError_t launch_umma_prefill(const shrike_moe* m, cudaStream_t st, const Expe
     }
     ChunkInstance* inst = (ChunkInstance*)ws.chunk_inst;
     const uint32_t max_inst = umma_max_chunk_instances(c, T);
-    chunk_instances_kernel<<<1, 256, 0, st>>>(ws.expert_offsets, ws.expert_counts, ws.slot_of_expert, c.num_experts, T,
-                                              c.has_shared, pool_cells, inst, ws.n_chunk_inst, ws.status);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_after(m, st, chunk_instances_kernel, dim3(1), 256, 0, ws.expert_offsets, ws.expert_counts, ws.slot_of_expert,
+                                 c.num_experts, T, (uint32_t)c.has_shared, pool_cells, inst, ws.n_chunk_inst, ws.status);
     if (e != cudaSuccess) return e;
     const uint32_t bits = c.weight_bits, grp = c.group_size;
     const bool f16 = c.meta_dtype == SHRIKE_DTYPE_FP16;
 #define SHRIKE_UMMA(B, G, M) \
-    return launch_umma_t<B, G, M>(st, a, inst, ws.n_chunk_inst, max_inst, (uint32_t)m->sm_count, maps[0], maps[1])
+    return launch_umma_t<B, G, M>(m, st, a, inst, ws.n_chunk_inst, max_inst, maps[0], maps[1])
     if (bits == 4 && grp == 64 && !f16) SHRIKE_UMMA(4, 64, SHRIKE_DTYPE_BF16);
     if (bits == 4 && grp == 64 && f16) SHRIKE_UMMA(4, 64, SHRIKE_DTYPE_FP16);
     if (bits == 4 && grp == 32 && !f16) SHRIKE_UMMA(4, 32, SHRIKE_DTYPE_BF16);
