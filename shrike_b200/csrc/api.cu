@@ -178,7 +178,7 @@ bool stream_pays(const shrike_moe_config& c, uint32_t T) {
 cudaError_t launch_experts(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, uint32_t T, uint32_t phases, void* y,
                            void* hidden, bool pdl) {
     const uint32_t n_shared = m->cfg.has_shared ? (T + 7) / 8 : 0;
-    cudaError_t e = stream_pays(m->cfg, T) ? launch_expert_stream(m, st, a, T, n_shared, phases, false, y, hidden, pdl) : cudaErrorNotSupported;
+    cudaError_t e = stream_pays(m->cfg, T) ? launch_expert_stream(m, st, a, T, n_shared, phases, y, hidden, pdl) : cudaErrorNotSupported;
     if (e != cudaErrorNotSupported) return e;
     const uint32_t mi = max_instances(m->cfg, T);
     if ((phases & 1u) && (e = launch_phase1(m, st, a, mi, pdl)) != cudaSuccess) return e;
@@ -720,7 +720,7 @@ int shrike_encode_decode_layer(shrike_moe* m, void* stream, const shrike_pool* p
         ra.with_shared = m->cfg.has_shared; ra.int4 = m->cfg.weight_bits == 4; ra.group = m->cfg.group_size;
         ra.slots = w.slots_dev; ra.xh = w.xh; ra.xsum = w.xsum; ra.status = w.status;
         const cudaError_t se = launch_expert_stream(m, (cudaStream_t)stream, ea, query_count, m->cfg.has_shared ? (query_count + 7) / 8 : 0,
-                                                    3u, false, y, hidden, !m->no_pdl, &ra);
+                                                    3u, y, hidden, !m->no_pdl, &ra);
         if (se == cudaSuccess) return SHRIKE_OK;
         if (se != cudaErrorNotSupported) return cuda_fail(m, se, "launch_expert_stream");
     }

@@ -1,5 +1,5 @@
-// Expert projections of a few rows per expert at memory speed: gate/up + GLU and down for instances of up to 8
-// rows that share an expert block (decode calls of 2 to 64 rows, and the experts with few rows of a prefill).
+// A decode layer of 2 to 64 rows, or its expert projections alone: router and work list, gate/up + GLU and down at memory
+// speed for instances of up to 8 rows that share an expert block.
 //
 //   phase 1: acts[pair, f] = GLU(gate[f,:].x + b, up[f,:].x + b)
 //            (moe_phase1_gate_up_act_spec_u16load, moe.metal:950-998; shared
@@ -21,14 +21,13 @@
 //     team's next slot. A finishing warp waits for the partial sums, adds them up in warp order, asks for the unit
 //     that comes n_slots later and finishes the rows (done by the multiplying warps in turn, the activation function's
 //     long chain held up every unit of the team);
-//   * the parts of a row are added up in the order of its picks: results do not depend on timing. The experts of a
-//     prefill add straight into fp32 rows instead.
+//   * the parts of a row are added up in the order of its picks: results do not depend on timing.
 // All phases run in one launch when the call has them: a block asks for its first phase-2 units before it waits for
 // the other blocks' activations.
 //
-// Measured (256 experts of 2048 x 512, top 8, int4, 16 rows: 181 MB of expert blocks): both projections 56 us where the
-// per-tile kernels took 82; inside the unit loops 6.5 TB/s, the rest is the start (7 us), the hand-over between the
-// phases (5 us) and the last one (3 us).
+// Measured (256 experts of 2048 x 512, top 8, int4, 16 rows: 181 MB of expert blocks): the whole layer 69 us where router,
+// gate/up and down launches took 103; inside the unit loops 6.5 TB/s, the rest is the routing (16 us), the hand-over between
+// the projections (5 us) and the row sums (3 us). 60 rows 127 us where the prefill path took 348.
 #include "block_maps.cuh"
 #include "plan.cuh"
 #include "route_args.cuh"
@@ -86,7 +85,6 @@ struct StreamArgs {
     const uint16_t* xh;
     uint16_t* acts;
     uint16_t* acts_shared;
-    float* yacc;                                     // accumulate: fp32 rows that phase 2 adds into
     float* parts;                                    // [T x top_k routed | T shared][d] weighted rows (decode)
     const uint32_t* sorted;                          // plan of a call that does not route: the pairs by instance
     const uint32_t* pair_cell;                       // and the cell of every pair or SHRIKE_SLOT_MISS
@@ -98,8 +96,7 @@ struct StreamArgs {
     uint32_t T;
     void* y;
     void* hidden;
-    uint32_t phases;                                 // bit 0, bit 1 (the last with phase 3 unless accumulate)
-    uint32_t accumulate;
+    uint32_t phases;                                 // bit 0, bit 1 (with phase 3)
     uint32_t rcp_cpc;                                // ceil(2^32 / cells_per_chunk)
     uint32_t n_chunks;
     uint32_t routes;                                 // this launch routes its rows first
@@ -859,17 +856,12 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
                         auto target = [&](uint32_t c, float*& out, float& w) {
                             const uint32_t pair = pair_of(i, min(c, count - 1u));
                             w = sh ? (a.shared_gate ? __ldcg(a.shared_gate + pair) : 1.0f) : pair_weight[pair];
-                            float* rows = a.accumulate ? a.yacc + (size_t)(sh ? pair : pair / a.top_k) * D
-                                                       : a.parts + ((size_t)pair + (sh ? a.T * a.top_k : 0u)) * D;
+                            float* rows = a.parts + ((size_t)pair + (sh ? a.T * a.top_k : 0u)) * D;
                             out = c < count ? rows + (ONE ? pr : t) : nullptr;
                         };
                         target(ONE ? 2 * t : g, out0, wt0);
                         if constexpr (ONE) target(2 * t + 1, out1, wt1);
                     }
-                };
-                auto put = [&](float* at, float v) {
-                    if (a.accumulate) atomicAdd(at, v);
-                    else *at = v;
                 };
                 for (; u < n && i < i1; u += pace) {
                     if (i != cur) {
@@ -943,19 +935,19 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
                             ++pend;
                         } else if constexpr (ONE) {
                             if (out0) {
-                                put(out0 + k * 16, wt0 * acc[0]);
-                                put(out0 + k * 16 + 8, wt0 * acc[2]);
+                                *(out0 + k * 16) = wt0 * acc[0];
+                                *(out0 + k * 16 + 8) = wt0 * acc[2];
                             }
                             if (out1) {
-                                put(out1 + k * 16, wt1 * acc[1]);
-                                put(out1 + k * 16 + 8, wt1 * acc[3]);
+                                *(out1 + k * 16) = wt1 * acc[1];
+                                *(out1 + k * 16 + 8) = wt1 * acc[3];
                             }
                         } else if (out0) {
                             float* o = out0 + k * 16;
-                            put(o, wt0 * v.x);
-                            put(o + 4, wt0 * v.y);
-                            put(o + 8, wt0 * v.z);
-                            put(o + 12, wt0 * v.w);
+                            *o = wt0 * v.x;
+                            *(o + 4) = wt0 * v.y;
+                            *(o + 8) = wt0 * v.z;
+                            *(o + 12) = wt0 * v.w;
                         }
                     }
                     step(i, k);
@@ -978,7 +970,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
         // a copy of this block may still be in flight: give it a bounded time to land
         for (int i = 0; i < 200; ++i) __nanosleep(1000);
     }
-    if (!do2 || a.accumulate) return;
+    if (!do2) return;
     // ================= y = the rows' parts; hidden += y =================
     // one output element pair per thread over all blocks; what does not depend on the parts is read ahead of the wait
     // (warps go round the blocks, so that a small call keeps every SM busy)
@@ -1085,7 +1077,7 @@ cudaError_t launch_stream_t(const shrike_moe* m, cudaStream_t st, const StreamAr
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     unsigned n = 0;
-    if (a.phases == 3u || ((a.phases & 2u) && !a.accumulate)) {   // the blocks wait for each other between the phases
+    if (a.phases & 2u) {   // the blocks wait for each other
         attr[n].id = cudaLaunchAttributeCooperative;
         attr[n].val.cooperative = 1;
         ++n;
@@ -1131,11 +1123,11 @@ static uint32_t stream_token_groups(const shrike_moe_config& c, uint32_t sm_coun
     return 0;
 }
 
-// phases: 1, 2 or both. accumulate: phase 2 adds into ea.yacc (prefill) instead of writing y and hidden. route (with both
+// phases: 1, 2 or both. route (with both
 // phases): the launch routes the rows itself and needs no plan. cudaErrorNotSupported when the shape does not fit: nothing
 // was launched.
 cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const ExpertArgs& ea, uint32_t T, uint32_t n_shared,
-                                 uint32_t phases, bool accumulate, void* y, void* hidden, bool pdl, const RouterArgs* route) {
+                                 uint32_t phases, void* y, void* hidden, bool pdl, const RouterArgs* route) {
     const shrike_moe_config& c = m->cfg;
     const uint64_t cpc = ea.pool.cells_per_chunk ? ea.pool.cells_per_chunk : 1;
     if (cpc < 2 || (uint64_t)ea.pool.cells * cpc >= (1ull << 32)) return cudaErrorNotSupported;
@@ -1148,7 +1140,7 @@ cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const Exp
     a.d = c.d; a.f = c.f; a.f_shared = c.has_shared ? c.shared_f : 0; a.top_k = c.top_k;
     a.activation = c.activation; a.expert_bias = c.expert_bias; a.act_dtype = c.act_dtype; a.y_dtype = c.y_dtype;
     a.inst = ea.inst; a.n_inst = ea.n_inst; a.n_shared = n_shared;
-    a.xh = ea.xh; a.acts = ea.acts; a.acts_shared = ea.acts_shared; a.yacc = ea.yacc;
+    a.xh = ea.xh; a.acts = ea.acts; a.acts_shared = ea.acts_shared;
     a.parts = m->ws.parts; a.sorted = ea.sorted; a.pair_cell = m->ws.pair_cell;
     for (a.n_chunks = 0; a.n_chunks < SHRIKE_MAX_POOL_CHUNKS && ea.pool.base[a.n_chunks];) ++a.n_chunks;
     if (route) {
@@ -1158,7 +1150,7 @@ cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const Exp
         if (!a.token_groups) return cudaErrorNotSupported;
     }
     a.route_w = ea.route_w; a.shared_gate = ea.shared_gate; a.status = ea.status; a.arrived = m->ws.arrived; a.inst_done = m->ws.inst_done;
-    a.T = T; a.y = y; a.hidden = hidden; a.phases = phases; a.accumulate = accumulate ? 1u : 0u;
+    a.T = T; a.y = y; a.hidden = hidden; a.phases = phases;
     a.rcp_cpc = (uint32_t)(((1ull << 32) + cpc - 1) / cpc);
     const uint32_t bits = c.weight_bits, grp = c.group_size;
     const bool f16 = c.meta_dtype == SHRIKE_DTYPE_FP16;

@@ -165,8 +165,7 @@ cudaError_t launch_router(const shrike_moe* m, cudaStream_t st, const shrike_rou
 cudaError_t launch_route_fused(const shrike_moe* m, cudaStream_t st, const shrike_router_operands& ops,
                                const void* hidden, uint32_t T, uint32_t stride, const uint64_t* table,
                                uint32_t pool_cells, const uint32_t* io_status, uint32_t* ids, float* weights,
-                               float* shared_gate, uint32_t* slots, uint32_t* counts, bool pdl,
-                               bool no_tail = false);
+                               float* shared_gate, uint32_t* slots, uint32_t* counts, bool pdl);
 cudaError_t launch_classify(const shrike_moe* m, cudaStream_t st, const uint32_t* ids,
                             const uint64_t* table, uint32_t T, uint32_t* slots, uint32_t* counts,
                             uint32_t* miss_pos, uint32_t* miss_exp);
@@ -202,7 +201,7 @@ cudaError_t launch_after(const shrike_moe* m, cudaStream_t st, void (*k)(P...), 
 // expert_stream.cu
 struct RouterArgs;
 cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const ExpertArgs& ea, uint32_t T, uint32_t n_shared,
-                                 uint32_t phases, bool accumulate, void* y, void* hidden, bool pdl,
+                                 uint32_t phases, void* y, void* hidden, bool pdl,
                                  const RouterArgs* route = nullptr);
 size_t stream_parts_bytes(const shrike_moe_config& c);
 size_t stream_done_bytes();

@@ -407,7 +407,6 @@ __global__ void __launch_bounds__(kRouterWarps * 32) route_fused_kernel(const Ro
                        a.xh, a.xsum, a.status);
     }
 
-    if (a.no_tail) return;
     __threadfence();
     __syncthreads();
     if (tid == 0) {
@@ -633,9 +632,8 @@ cudaError_t launch_router(const shrike_moe* m, cudaStream_t st, const shrike_rou
 cudaError_t launch_route_fused(const shrike_moe* m, cudaStream_t st, const shrike_router_operands& ops,
                                const void* hidden, uint32_t T, uint32_t stride, const uint64_t* table,
                                uint32_t pool_cells, const uint32_t* io_status, uint32_t* ids, float* weights,
-                               float* shared_gate, uint32_t* slots, uint32_t* counts, bool pdl, bool no_tail) {
+                               float* shared_gate, uint32_t* slots, uint32_t* counts, bool pdl) {
     RouterArgs a = make_router_args(m, ops, hidden, T, stride, ids, weights, shared_gate);
-    a.no_tail = no_tail ? 1u : 0u;
     a.table = table; a.pool_cells = pool_cells; a.io_status = io_status;
     a.with_shared = m->cfg.has_shared; a.int4 = m->cfg.weight_bits == 4; a.group = m->cfg.group_size;
     a.xsum = m->ws.xsum;
