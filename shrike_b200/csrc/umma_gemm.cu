@@ -707,17 +707,21 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         // ---------------- activation tiles ----------------
         // One or two boxes per K block: these tiles are most of what a block pulls out of L2, and a short instance
         // does not pay for 256 rows, nor one of 80 rows for 128.
-        uint32_t b_use = 0, acc_use = 0, last_stage = 0;
+        uint32_t b_use = 0, last_stage = 0;
         for (uint32_t turn = 0;; ++turn) {
             const uint32_t t = take_tile(turn);
             if (t >= n_tiles || failed()) break;
             Work wk;
             if (!open_tile(t, wk)) continue;
             const TileShape ts(wk.in.count);
-            if (last_stage) {
-                // another layout: its stages lie across the last one's, so the last tile's instructions have to be done
-                if (ts.b_stage != last_stage && !pipe_wait(accum, acc_use)) { give_up(); break; }
-                acc_use ^= 1;
+            // Another layout: its stages lie across the last one's, so every old stage's last use has to be done. (The stages
+            // themselves are waited for, not the tile: a tile of two K blocks leaves the third stage to the tile before it,
+            // so the tile barrier could still be two phases behind, where its one parity bit reads as passed.)
+            if (last_stage && ts.b_stage != last_stage) {
+                bool done = true;
+                if (lane == 0)
+                    for (uint32_t s = 0; s < kBStages; ++s) done = done && pipe_wait(&b_empty[s], ((b_use >> s) & 1) ^ 1);
+                if (!__all_sync(0xffffffffu, done)) { give_up(); break; }
             }
             last_stage = ts.b_stage;
             const CUtensorMap* maps_b = wk.shared ? maps.act_shared : maps.act_routed;

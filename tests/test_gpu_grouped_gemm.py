@@ -1,6 +1,7 @@
 """The expert-grouped GEMM with more tiles than SMs, against the oracle: instances on both sides of every stage layout
 (1, 16, 64, 65, 128, 129 and 256 rows and one more than 256) follow one another on an SM, shared and routed experts have
-different numbers of row tiles, and the last ones are partial."""
+different numbers of row tiles, and the last ones are partial. Tiles of two K blocks, which use two of the three activation stages,
+between longer ones and another layout."""
 import numpy as np
 import pytest
 import torch
@@ -17,8 +18,21 @@ pytestmark = pytest.mark.gpu
     dict(d=960, f=448, shared_f=192, weight_bits=4, group_size=32, expert_bias=1, activation=capi.ACT_CLAMPED_SWIGLU),
 ], ids=lambda kw: "-".join(f"{k}{v}" for k, v in kw.items()))
 def test_tiles_of_every_layout(cuda_device, kw):
-    sizes = [257, 256, 129, 128, 65, 64, 17, 16] + [1] * 40
-    cfg = small_config(num_experts=64, top_k=1, max_tokens=1024, shared_gated=False, **kw)
+    run_sizes([257, 256, 129, 128, 65, 64, 17, 16] + [1] * 40, kw)
+
+
+@pytest.mark.parametrize("kw", [
+    dict(d=2048, f=128, shared_f=384),
+    dict(d=2048, f=128, shared_f=192, weight_bits=8, group_size=32),
+], ids=lambda kw: "-".join(f"{k}{v}" for k, v in kw.items()))
+def test_a_short_tile_before_another_layout(cuda_device, kw):
+    """The shared expert's last instance has 24 rows and three or six K blocks in the down projection, the routed experts two:
+    on many SMs a remainder of one row follows it, which leaves the third stage to it, and then a tile of 256 rows."""
+    run_sizes([257] * 24, kw, sample=24)
+
+
+def run_sizes(sizes, kw, sample=None):
+    cfg = small_config(num_experts=64, top_k=1, max_tokens=max(1024, sum(sizes)), shared_gated=False, **kw)
     layer = Layer(cfg)
     ids = np.concatenate([np.full(n, e, np.uint32) for e, n in enumerate(sizes)])
     ids = np.random.default_rng(3).permutation(ids)[:, None]
@@ -31,5 +45,11 @@ def test_tiles_of_every_layout(cuda_device, kw):
     layer.moe.encode_prefill(layer.pool, layer.offsets, ids_dev, slots, torch.from_numpy(w).to(layer.device), x_dev, y, None,
                              layer.shared, None)
     layer.moe.status()
-    assert rel_l2(y.cpu().numpy(), layer.oracle_forward(x, ids, w)) <= 1e-3
+    # all rows, or every expert's last one (the remainders) and a few others
+    rows = np.arange(len(ids)) if sample is None else np.unique(np.concatenate(
+        [[np.flatnonzero(ids[:, 0] == e)[-1] for e in range(len(sizes))], np.random.default_rng(6).choice(len(ids), sample)]))
+    want = layer.oracle_forward(x, ids, w, rows=rows)
+    got = y.cpu().numpy()[rows]
+    assert rel_l2(got, want) <= 1e-3
+    assert max(rel_l2(g, v) for g, v in zip(got, want)) <= 2e-3
     layer.close()
