@@ -413,7 +413,8 @@ int shrike_encode_router_static(const shrike_moe_config* config, void* stream,
 
 /* End-to-end convenience for hosts that keep activations in host memory:
  * copies x_host in, runs router -> classification -> decode/prefill for one
- * layer, copies y (and hidden) back, and synchronises. */
+ * layer, copies y, ids and weights back, and synchronises. x_host holds
+ * query_count x d elements of act_dtype, y_host as many of y_dtype. */
 int shrike_moe_layer_forward_host(shrike_moe* moe, void* stream, const shrike_pool* pool,
                                   const shrike_expert_offsets* routed_offsets,
                                   const uint64_t* residency_table_row,

@@ -823,8 +823,8 @@ int shrike_moe_layer_forward_host(shrike_moe* m, void* stream, const shrike_pool
     if (query_count > c.max_tokens) return fail(m, SHRIKE_ERANGE, "query_count exceeds max_tokens");
     cudaStream_t st = (cudaStream_t)stream;
     Workspace& w = m->ws;
-    const size_t bytes = (size_t)query_count * c.d * act_bytes(c.act_dtype);
-    CU(cudaMemcpyAsync(w.x_dev, x_host, bytes, cudaMemcpyHostToDevice, st));
+    const size_t elements = (size_t)query_count * c.d;
+    CU(cudaMemcpyAsync(w.x_dev, x_host, elements * act_bytes(c.act_dtype), cudaMemcpyHostToDevice, st));
     float* gate = c.shared_gated ? w.gate_dev : nullptr;
     int rc;
     if (query_count <= SHRIKE_MAX_DECODE_TOKENS) {
@@ -840,7 +840,7 @@ int shrike_moe_layer_forward_host(shrike_moe* m, void* stream, const shrike_pool
                                        query_count, shared, gate, w.y_dev, nullptr);
     }
     if (rc) return rc;
-    CU(cudaMemcpyAsync(y_host, w.y_dev, bytes, cudaMemcpyDeviceToHost, st));
+    CU(cudaMemcpyAsync(y_host, w.y_dev, elements * act_bytes(c.y_dtype), cudaMemcpyDeviceToHost, st));
     if (ids_host) CU(cudaMemcpyAsync(ids_host, w.ids_dev, (size_t)query_count * c.top_k * 4, cudaMemcpyDeviceToHost, st));
     if (weights_host) CU(cudaMemcpyAsync(weights_host, w.w_dev, (size_t)query_count * c.top_k * 4, cudaMemcpyDeviceToHost, st));
     return shrike_moe_status(m, stream);

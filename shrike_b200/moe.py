@@ -275,10 +275,12 @@ class MoE:
                            router: RouterOperands, x_host: torch.Tensor, y_host: torch.Tensor,
                            shared: Optional[capi.SharedExpert] = None, ids_host: Optional[torch.Tensor] = None,
                            weights_host: Optional[torch.Tensor] = None) -> None:
-        """One layer with host activations in and out (copies inside the call)."""
+        """One layer with host activations in and out (copies inside the call): x in the activation dtype, y in the y dtype."""
         for t in (x_host, y_host, ids_host, weights_host):
             if t is not None and (t.is_cuda or not t.is_contiguous()):
                 raise ValueError("host operands must be contiguous CPU tensors")
+        if y_host.nbytes < x_host.shape[0] * self.config.d * self.config.torch_y_dtype.itemsize:
+            raise ValueError("y_host is smaller than the rows in the y dtype")
         ops = router.to_c()
         self._check(self._lib.shrike_moe_layer_forward_host(
             self._h, _stream(), pool._h, C.byref(routed_offsets), self.residency_row(layer), C.byref(ops),

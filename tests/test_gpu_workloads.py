@@ -146,6 +146,28 @@ def test_layer_forward_host_round_trip(cuda_device):
     layer.close()
 
 
+@pytest.mark.parametrize("T", [5, 70])
+@pytest.mark.parametrize("act,out", [(capi.DTYPE_BF16, capi.DTYPE_FP32), (capi.DTYPE_FP32, capi.DTYPE_BF16)])
+def test_layer_forward_host_when_y_has_another_size(cuda_device, act, out, T):
+    """y comes back whole, and no more than y, when its elements are wider or narrower than the activations'. All rows
+    of the handle, so that the device buffers have nothing to spare."""
+    import torch
+    cfg = fx.qwen_config(max_tokens=T, act_dtype=act, y_dtype=out, d=512, f=256, shared_f=256, num_experts=64)
+    layer = Layer(cfg, seed=107, device_fill=True)
+    x = inputs(T, cfg.d, seed=4)
+    x_host = torch.from_numpy(x).to(cfg.torch_act_dtype)
+    spare = torch.full((2 * T, cfg.d), -77.0, dtype=cfg.torch_y_dtype)
+    layer.moe.layer_forward_host(layer.pool, layer.offsets, 0, layer.router_ops, x_host, spare[:T], layer.shared)
+    assert (spare[T:] == -77.0).all()
+    ids, w, _ = layer.oracle_route(x)
+    # bf16 rows: half a unit in the last place of each element beside the oracle's tolerance
+    tol = TOL + (2.0 ** -9 if out == capi.DTYPE_BF16 else 0.0)
+    assert rel_l2(spare[:T].float().numpy(), layer.oracle_forward(x, ids, w)) <= tol
+    with pytest.raises(ValueError):
+        layer.moe.layer_forward_host(layer.pool, layer.offsets, 0, layer.router_ops, x_host, spare[:T, :64].contiguous(), layer.shared)
+    layer.close()
+
+
 @pytest.mark.parametrize("T", [1, 3])
 def test_decode_stack_host_entry_point_equals_the_layer_calls(cuda_device, T):
     """shrike_decode_stack_forward_host (host rows in, every layer, host rows out) against the same layers called
