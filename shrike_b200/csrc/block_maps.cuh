@@ -9,18 +9,24 @@
 
 namespace shrike {
 
+// The one-row kernel's.
 struct BlockMaps {
     CUtensorMap w1[SHRIKE_MAX_POOL_CHUNKS + 1];   // gate + up rows: (group bytes, rows, groups, 2, cells)
     CUtensorMap m1[SHRIKE_MAX_POOL_CHUNKS + 1];   // their scales and biases: (8 rows' worth, rows / 8, scale|bias, 2, cells)
     CUtensorMap w2[SHRIKE_MAX_POOL_CHUNKS + 1];   // down rows: (group bytes, rows, groups, cells)
     CUtensorMap m2[SHRIKE_MAX_POOL_CHUNKS + 1];   // their scales and biases: (8 rows' worth, rows / 8, scale|bias, cells)
-    // the same weights in 128-byte pieces of a row (128-byte swizzle): (128 bytes, rows[, 2], pieces, cells)
-    CUtensorMap l1[SHRIKE_MAX_POOL_CHUNKS + 1], l2[SHRIKE_MAX_POOL_CHUNKS + 1];
+};
+// The streaming kernel's: the same weights in 128-byte pieces of a row (128-byte swizzle), (128 bytes, rows[, 2], pieces, cells),
+// and the same scales and biases.
+struct PieceMaps {
+    CUtensorMap l1[SHRIKE_MAX_POOL_CHUNKS + 1], m1[SHRIKE_MAX_POOL_CHUNKS + 1];
+    CUtensorMap l2[SHRIKE_MAX_POOL_CHUNKS + 1], m2[SHRIKE_MAX_POOL_CHUNKS + 1];
 };
 
 // The maps of a call's pool and shared block, cached on the handle; NULL when the layout is not one that they can
-// describe (fused_layer.cu).
+// describe (fused_layer.cu). Either may be there without the other.
 const BlockMaps* block_maps_for(const shrike_moe* m, const ExpertArgs& ea);
+const PieceMaps* piece_maps_for(const shrike_moe* m, const ExpertArgs& ea);
 
 // Tiled TMA loads (no multicast): the box lands densely, innermost dimension first.
 __device__ __forceinline__ void tma_4d(uint32_t dst, const CUtensorMap* map, int32_t c0, int32_t c1, int32_t c2, int32_t c3,

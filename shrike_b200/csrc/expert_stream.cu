@@ -616,7 +616,7 @@ __device__ __forceinline__ uint32_t work_list(const StreamArgs& a, uint8_t* dsm,
 }  // namespace
 
 template <int BITS, int GROUP, int META, bool AL>
-__global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid_constant__ StreamArgs a, const __grid_constant__ BlockMaps maps) {
+__global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid_constant__ StreamArgs a, const __grid_constant__ PieceMaps maps) {
     using Q = FQ<BITS, GROUP>;
     constexpr uint32_t GP = 128 / Q::kGroupBytes, H = GROUP / 32;   // groups of a piece; 16-byte operand parts of a group
     extern __shared__ __align__(128) uint8_t dsm_raw[];
@@ -1066,7 +1066,7 @@ bool stream_geometry(const shrike_moe_config& c, uint32_t smem_optin, StreamGeom
 }
 
 template <int BITS, int GROUP, int META, bool AL>
-cudaError_t launch_stream_t(const shrike_moe* m, cudaStream_t st, const StreamArgs& a, const BlockMaps& maps, bool pdl) {
+cudaError_t launch_stream_t(const shrike_moe* m, cudaStream_t st, const StreamArgs& a, const PieceMaps& maps, bool pdl) {
     auto k = expert_stream_kernel<BITS, GROUP, META, AL>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.g.smem_bytes);
     if (e != cudaSuccess) return e;
@@ -1093,7 +1093,7 @@ cudaError_t launch_stream_t(const shrike_moe* m, cudaStream_t st, const StreamAr
 }
 
 template <int BITS, int GROUP, int META>
-cudaError_t launch_stream_m(const shrike_moe* m, cudaStream_t st, const StreamArgs& a, const BlockMaps& maps, bool pdl) {
+cudaError_t launch_stream_m(const shrike_moe* m, cudaStream_t st, const StreamArgs& a, const PieceMaps& maps, bool pdl) {
     // every row whole 128-byte pieces?
     const shrike_moe_config& c = m->cfg;
     const uint32_t gp = 128 / (GROUP * BITS / 8);
@@ -1131,7 +1131,7 @@ cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const Exp
     const shrike_moe_config& c = m->cfg;
     const uint64_t cpc = ea.pool.cells_per_chunk ? ea.pool.cells_per_chunk : 1;
     if (cpc < 2 || (uint64_t)ea.pool.cells * cpc >= (1ull << 32)) return cudaErrorNotSupported;
-    const BlockMaps* maps = block_maps_for(m, ea);
+    const PieceMaps* maps = piece_maps_for(m, ea);
     if (!maps) return cudaErrorNotSupported;
     StreamArgs a;
     memset(&a, 0, sizeof a);

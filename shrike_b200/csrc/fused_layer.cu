@@ -1190,117 +1190,120 @@ bool fused_geometry(const shrike_moe_config& c, int sm_count, int max_smem_optin
 
 // ---- tensor maps of an expert-block layout -------------------------------------------------------------
 
-// The four maps of one chunk of `cells` blocks at `base` (cells 1: the shared expert's block). False when the
-// layout is not the regular one (gate and up sub-tensors the same distance apart for weights, scales and
-// biases) or the driver refuses a map: the layer call then keeps its three launches.
-static bool make_block_maps(const shrike_moe_config& c, const uint8_t* base, const Offsets3& off, uint32_t F,
-                            uint64_t cells, uint64_t cell_stride, CUtensorMap* w1, CUtensorMap* m1, CUtensorMap* w2,
-                            CUtensorMap* m2, CUtensorMap* l1, CUtensorMap* l2) {
+// One chunk of `cells` blocks at `base` (cells 1: the shared expert's block) and the sizes its maps are made of.
+struct BlockLayout {
+    const uint8_t* base;
+    const Offsets3& off;
+    uint64_t d, F, cells, cs;          // cs: from cell to cell
+    uint64_t gb, rb1, G1, rb2, G2;     // bytes of a group; bytes and groups of a gate/up row, of a down row
+    uint64_t mat, kind1, kind2;        // gate to up; scales to biases
+    BlockLayout(const shrike_moe_config& c, const uint8_t* base, const Offsets3& off, uint32_t F, uint64_t cells, uint64_t cell_stride)
+        : base(base), off(off), d(c.d), F(F), cells(cells), cs(std::max<uint64_t>(cell_stride, 16)), gb(c.group_size * c.weight_bits / 8),
+          rb1((uint64_t)c.d * c.weight_bits / 8), G1(c.d / c.group_size), rb2((uint64_t)F * c.weight_bits / 8), G2(F / c.group_size),
+          mat((uint64_t)off.w[1] - off.w[0]), kind1((uint64_t)off.b[0] - off.s[0]), kind2((uint64_t)off.b[2] - off.s[2]) {}
+    // gate and up sub-tensors the same distance apart for weights, scales and biases, all of it in 16-byte units
+    bool regular() const {
+        return off.w[1] > off.w[0] && off.s[1] - off.s[0] == mat && off.b[1] - off.s[1] == kind1 && off.b[0] > off.s[0] && off.b[2] > off.s[2] &&
+               mat % 16 == 0 && kind1 % 16 == 0 && kind2 % 16 == 0 && cs % 16 == 0 && ((uintptr_t)base & 15) == 0;
+    }
+};
+
+static bool make_map(CUtensorMap* map, CUtensorMapDataType type, uint32_t rank, const uint8_t* at, const cuuint64_t* dims, const cuuint64_t* strides,
+                     const cuuint32_t* box, CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promotion) {
     EncodeFn enc = encode_tiled();
-    if (!enc) return false;
-    const uint64_t gb = c.group_size * c.weight_bits / 8;
-    const uint64_t rb1 = (uint64_t)c.d * c.weight_bits / 8, G1 = c.d / c.group_size;
-    const uint64_t rb2 = (uint64_t)F * c.weight_bits / 8, G2 = F / c.group_size;
-    const uint64_t mat = (uint64_t)off.w[1] - off.w[0], kind1 = (uint64_t)off.b[0] - off.s[0];
-    if (off.w[1] <= off.w[0] || off.s[1] - off.s[0] != mat || off.b[1] - off.s[1] != kind1 || off.b[0] <= off.s[0] ||
-        off.b[2] <= off.s[2])
-        return false;
-    if (mat % 16 || kind1 % 16 || (off.b[2] - off.s[2]) % 16 || cell_stride % 16 || ((uintptr_t)base & 15)) return false;
-    const uint64_t cs = cells > 1 ? cell_stride : std::max<uint64_t>(cell_stride, 16);
     const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
-    auto ok = [](CUresult r) { return r == CUDA_SUCCESS; };
-    {   // gate + up weights: (group bytes, F rows, G1 groups, 2, cells); a box = 8 rows of both
-        const cuuint64_t dims[5] = {gb, F, G1, 2, cells};
-        const cuuint64_t strides[4] = {rb1, gb, mat, cs};
-        const cuuint32_t box[5] = {(cuuint32_t)gb, 8, (cuuint32_t)G1, 2, 1};
-        if (!ok(enc(w1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, (void*)(base + off.w[0]), dims, strides, box, ones,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)))
-            return false;
-    }
-    {   // the same weights in whole 128-byte pieces, gate and up rows of a piece side by side (a row's last piece may
-        // run into the next row: those bytes are not used, and what follows a matrix is its scales)
-        const cuuint64_t n1 = (rb1 + 127) / 128, n2 = (rb2 + 127) / 128;
-        const cuuint64_t dims1[5] = {128, F, 2, n1, cells}, strides1[4] = {rb1, mat, 128, cs};
-        const cuuint32_t box1[5] = {128, 8, 2, (cuuint32_t)n1, 1};
-        const cuuint64_t dims2[4] = {128, c.d, n2, cells}, strides2[3] = {rb2, 128, cs};
-        const cuuint32_t box2[4] = {128, 16, (cuuint32_t)n2, 1};
-        if (!ok(enc(l1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, (void*)(base + off.w[0]), dims1, strides1, box1, ones,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)) ||
-            !ok(enc(l2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)(base + off.w[2]), dims2, strides2, box2, ones,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)))
-            return false;
-    }
-    {   // their scales and biases, 8 rows (16*G1 bytes) at a time in 8-byte units: (2*G1, F/8, scale|bias, 2, cells)
-        const cuuint64_t dims[5] = {2 * G1, F / 8, 2, 2, cells};
-        const cuuint64_t strides[4] = {16 * G1, kind1, mat, cs};
-        const cuuint32_t box[5] = {(cuuint32_t)(2 * G1), 1, 2, 2, 1};
-        if (!ok(enc(m1, CU_TENSOR_MAP_DATA_TYPE_UINT64, 5, (void*)(base + off.s[0]), dims, strides, box, ones,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)))
-            return false;
-    }
-    {   // down weights: (group bytes, D rows, G2 groups, cells); a box = 16 rows
-        const cuuint64_t dims[4] = {gb, c.d, G2, cells};
-        const cuuint64_t strides[3] = {rb2, gb, cs};
-        const cuuint32_t box[4] = {(cuuint32_t)gb, 16, (cuuint32_t)G2, 1};
-        if (!ok(enc(w2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)(base + off.w[2]), dims, strides, box, ones,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)))
-            return false;
-    }
-    {   // their scales and biases, 8 rows at a time: (2*G2, D/8, scale|bias, cells); a box = 16 rows of both
-        const cuuint64_t dims[4] = {2 * G2, c.d / 8, 2, cells};
-        const cuuint64_t strides[3] = {16 * G2, (uint64_t)off.b[2] - off.s[2], cs};
-        const cuuint32_t box[4] = {(cuuint32_t)(2 * G2), 2, 2, 1};
-        if (!ok(enc(m2, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, (void*)(base + off.s[2]), dims, strides, box, ones,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)))
-            return false;
-    }
-    return true;
+    return enc && enc(map, type, rank, (void*)at, dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promotion,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Weights by groups: gate + up (group bytes, F rows, G1 groups, 2, cells), a box = 8 rows of both; down (group bytes, D rows,
+// G2 groups, cells), a box = 16 rows.
+static bool make_group_maps(const BlockLayout& b, CUtensorMap* w1, CUtensorMap* w2) {
+    const cuuint64_t dims1[5] = {b.gb, b.F, b.G1, 2, b.cells}, strides1[4] = {b.rb1, b.gb, b.mat, b.cs};
+    const cuuint32_t box1[5] = {(cuuint32_t)b.gb, 8, (cuuint32_t)b.G1, 2, 1};
+    const cuuint64_t dims2[4] = {b.gb, b.d, b.G2, b.cells}, strides2[3] = {b.rb2, b.gb, b.cs};
+    const cuuint32_t box2[4] = {(cuuint32_t)b.gb, 16, (cuuint32_t)b.G2, 1};
+    return make_map(w1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, b.base + b.off.w[0], dims1, strides1, box1, CU_TENSOR_MAP_SWIZZLE_NONE,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
+           make_map(w2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, b.base + b.off.w[2], dims2, strides2, box2, CU_TENSOR_MAP_SWIZZLE_NONE,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+}
+
+// The same weights in whole 128-byte pieces, gate and up rows of a piece side by side (a row's last piece may run into the
+// next row: those bytes are not used, and what follows a matrix is its scales).
+static bool make_piece_maps(const BlockLayout& b, CUtensorMap* l1, CUtensorMap* l2) {
+    const cuuint64_t n1 = (b.rb1 + 127) / 128, n2 = (b.rb2 + 127) / 128;
+    const cuuint64_t dims1[5] = {128, b.F, 2, n1, b.cells}, strides1[4] = {b.rb1, b.mat, 128, b.cs};
+    const cuuint32_t box1[5] = {128, 8, 2, (cuuint32_t)n1, 1};
+    const cuuint64_t dims2[4] = {128, b.d, n2, b.cells}, strides2[3] = {b.rb2, 128, b.cs};
+    const cuuint32_t box2[4] = {128, 16, (cuuint32_t)n2, 1};
+    return make_map(l1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, b.base + b.off.w[0], dims1, strides1, box1, CU_TENSOR_MAP_SWIZZLE_128B,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B) &&
+           make_map(l2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, b.base + b.off.w[2], dims2, strides2, box2, CU_TENSOR_MAP_SWIZZLE_128B,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+}
+
+// Scales and biases, 8 rows (16 * groups bytes) at a time in 8-byte units: gate + up (2 * G1, F / 8, scale|bias, 2, cells), a box =
+// 8 rows of both; down (2 * G2, D / 8, scale|bias, cells), a box = 16 rows.
+static bool make_meta_maps(const BlockLayout& b, CUtensorMap* m1, CUtensorMap* m2) {
+    const cuuint64_t dims1[5] = {2 * b.G1, b.F / 8, 2, 2, b.cells}, strides1[4] = {16 * b.G1, b.kind1, b.mat, b.cs};
+    const cuuint32_t box1[5] = {(cuuint32_t)(2 * b.G1), 1, 2, 2, 1};
+    const cuuint64_t dims2[4] = {2 * b.G2, b.d / 8, 2, b.cells}, strides2[3] = {16 * b.G2, b.kind2, b.cs};
+    const cuuint32_t box2[4] = {(cuuint32_t)(2 * b.G2), 2, 2, 1};
+    return make_map(m1, CU_TENSOR_MAP_DATA_TYPE_UINT64, 5, b.base + b.off.s[0], dims1, strides1, box1, CU_TENSOR_MAP_SWIZZLE_NONE,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
+           make_map(m2, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, b.base + b.off.s[2], dims2, strides2, box2, CU_TENSOR_MAP_SWIZZLE_NONE,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
 }
 
 // The maps of a call's pool and shared block, cached on the handle: they change only when the host changes
-// the pool, the offsets or the shared block.
+// the pool, the offsets or the shared block. What one kernel's maps cannot describe takes only that kernel's path away.
 struct BlockMapCache {
     PoolView pool;
     Offsets3 routed, shared;
     const uint8_t* shared_block;
-    bool valid, usable;
-    BlockMaps maps;
+    bool valid, blocks_usable, pieces_usable;
+    BlockMaps blocks;
+    PieceMaps pieces;
 };
 
-const BlockMaps* block_maps_for(const shrike_moe* m, const ExpertArgs& ea) {
+static const BlockMapCache* map_cache(const shrike_moe* m, const ExpertArgs& ea) {
     BlockMapCache* cache = (BlockMapCache*)m->ws.fused_maps;
     if (!cache) return nullptr;
     const bool same = cache->valid && memcmp(&cache->pool, &ea.pool, sizeof(PoolView)) == 0 &&
                       memcmp(&cache->routed, &ea.routed, sizeof(Offsets3)) == 0 &&
                       memcmp(&cache->shared, &ea.shared, sizeof(Offsets3)) == 0 && cache->shared_block == ea.shared_block;
-    if (same) return cache->usable ? &cache->maps : nullptr;
+    if (same) return cache;
     const shrike_moe_config& c = m->cfg;
     memset(cache, 0, sizeof *cache);   // padding bytes included: the comparison above is bytewise
     cache->pool = ea.pool; cache->routed = ea.routed; cache->shared = ea.shared; cache->shared_block = ea.shared_block;
-    cache->valid = true;
-    bool ok = true;
+    cache->valid = cache->blocks_usable = cache->pieces_usable = true;
+    auto make = [&](uint32_t i, const BlockLayout& b) {
+        const bool meta = b.regular() && make_meta_maps(b, &cache->blocks.m1[i], &cache->blocks.m2[i]);
+        cache->pieces.m1[i] = cache->blocks.m1[i];
+        cache->pieces.m2[i] = cache->blocks.m2[i];
+        cache->blocks_usable = cache->blocks_usable && meta && make_group_maps(b, &cache->blocks.w1[i], &cache->blocks.w2[i]);
+        cache->pieces_usable = cache->pieces_usable && meta && make_piece_maps(b, &cache->pieces.l1[i], &cache->pieces.l2[i]);
+    };
     uint32_t left = ea.pool.cells;
-    for (uint32_t ch = 0; ch < SHRIKE_MAX_POOL_CHUNKS && ok && left; ++ch) {
+    for (uint32_t ch = 0; ch < SHRIKE_MAX_POOL_CHUNKS && left; ++ch) {
         if (!ea.pool.base[ch]) break;
         const uint32_t cells = left < ea.pool.cells_per_chunk ? left : ea.pool.cells_per_chunk;
-        ok = make_block_maps(c, ea.pool.base[ch], ea.routed, c.f, cells, ea.pool.stride, &cache->maps.w1[ch],
-                             &cache->maps.m1[ch], &cache->maps.w2[ch], &cache->maps.m2[ch], &cache->maps.l1[ch],
-                             &cache->maps.l2[ch]);
+        make(ch, BlockLayout(c, ea.pool.base[ch], ea.routed, c.f, cells, ea.pool.stride));
         left -= cells;
     }
-    if (ok && c.has_shared)
-        ok = make_block_maps(c, ea.shared_block, ea.shared, c.shared_f, 1, 16, &cache->maps.w1[SHRIKE_MAX_POOL_CHUNKS],
-                             &cache->maps.m1[SHRIKE_MAX_POOL_CHUNKS], &cache->maps.w2[SHRIKE_MAX_POOL_CHUNKS],
-                             &cache->maps.m2[SHRIKE_MAX_POOL_CHUNKS], &cache->maps.l1[SHRIKE_MAX_POOL_CHUNKS],
-                             &cache->maps.l2[SHRIKE_MAX_POOL_CHUNKS]);
-    cache->usable = ok;
-    return ok ? &cache->maps : nullptr;
+    if (c.has_shared) make(SHRIKE_MAX_POOL_CHUNKS, BlockLayout(c, ea.shared_block, ea.shared, c.shared_f, 1, 16));
+    return cache;
+}
+
+const BlockMaps* block_maps_for(const shrike_moe* m, const ExpertArgs& ea) {
+    const BlockMapCache* cache = map_cache(m, ea);
+    return cache && cache->blocks_usable ? &cache->blocks : nullptr;
+}
+
+const PieceMaps* piece_maps_for(const shrike_moe* m, const ExpertArgs& ea) {
+    const BlockMapCache* cache = map_cache(m, ea);
+    return cache && cache->pieces_usable ? &cache->pieces : nullptr;
 }
 
 size_t fused_map_cache_bytes() { return sizeof(BlockMapCache); }
