@@ -1197,10 +1197,16 @@ struct BlockLayout {
     uint64_t d, F, cells, cs;          // cs: from cell to cell
     uint64_t gb, rb1, G1, rb2, G2;     // bytes of a group; bytes and groups of a gate/up row, of a down row
     uint64_t mat, kind1, kind2;        // gate to up; scales to biases
+    uint64_t end;                      // bytes from one block's start that belong to it: a cell, or up to the last sub-tensor's end
     BlockLayout(const shrike_moe_config& c, const uint8_t* base, const Offsets3& off, uint32_t F, uint64_t cells, uint64_t cell_stride)
         : base(base), off(off), d(c.d), F(F), cells(cells), cs(std::max<uint64_t>(cell_stride, 16)), gb(c.group_size * c.weight_bits / 8),
           rb1((uint64_t)c.d * c.weight_bits / 8), G1(c.d / c.group_size), rb2((uint64_t)F * c.weight_bits / 8), G2(F / c.group_size),
-          mat((uint64_t)off.w[1] - off.w[0]), kind1((uint64_t)off.b[0] - off.s[0]), kind2((uint64_t)off.b[2] - off.s[2]) {}
+          mat((uint64_t)off.w[1] - off.w[0]), kind1((uint64_t)off.b[0] - off.s[0]), kind2((uint64_t)off.b[2] - off.s[2]), end(cell_stride) {
+        for (int p = 0; p < 3; ++p) {
+            const uint64_t rows = p < 2 ? F : d, meta = rows * (p < 2 ? G1 : G2) * 2;
+            end = std::max({end, off.w[p] + rows * (p < 2 ? rb1 : rb2), off.s[p] + meta, off.b[p] + meta});
+        }
+    }
     // gate and up sub-tensors the same distance apart for weights, scales and biases, all of it in 16-byte units
     bool regular() const {
         return off.w[1] > off.w[0] && off.s[1] - off.s[0] == mat && off.b[1] - off.s[1] == kind1 && off.b[0] > off.s[0] && off.b[2] > off.s[2] &&
@@ -1229,10 +1235,11 @@ static bool make_group_maps(const BlockLayout& b, CUtensorMap* w1, CUtensorMap* 
                     CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
 }
 
-// The same weights in whole 128-byte pieces, gate and up rows of a piece side by side (a row's last piece may run into the
-// next row: those bytes are not used, and what follows a matrix is its scales).
+// The same weights in whole 128-byte pieces, gate and up rows of a piece side by side. A row's last piece may run into what
+// follows the row: those bytes are not used, but they are read, so a block whose weights come last is refused.
 static bool make_piece_maps(const BlockLayout& b, CUtensorMap* l1, CUtensorMap* l2) {
     const cuuint64_t n1 = (b.rb1 + 127) / 128, n2 = (b.rb2 + 127) / 128;
+    if (b.off.w[1] + (b.F - 1) * b.rb1 + n1 * 128 > b.end || b.off.w[2] + (b.d - 1) * b.rb2 + n2 * 128 > b.end) return false;
     const cuuint64_t dims1[5] = {128, b.F, 2, n1, b.cells}, strides1[4] = {b.rb1, b.mat, 128, b.cs};
     const cuuint32_t box1[5] = {128, 8, 2, (cuuint32_t)n1, 1};
     const cuuint64_t dims2[4] = {128, b.d, n2, b.cells}, strides2[3] = {b.rb2, 128, b.cs};

@@ -1,7 +1,9 @@
 """The streaming expert kernel at the edges of its tiling, against the oracle: rows of weights that end inside a
 128-byte piece, group counts that leave a quad of groups open, shared and routed experts of different widths, one to
 eight rows per instance, and the shapes it leaves to the per-tile kernels (an odd number of groups)."""
+import numpy as np
 import pytest
+import torch
 
 from shrike_b200 import capi
 from gpu_harness import Layer, inputs, small_config
@@ -23,4 +25,39 @@ pytestmark = pytest.mark.gpu
 def test_stream_edges(cuda_device, kw, T):
     layer = Layer(small_config(**kw))
     check_layer(layer, inputs(T, kw["d"], seed=T), fused=True)
+    layer.close()
+
+
+def weights_last(cfg, off: capi.ExpertOffsets, block: np.ndarray, f: int):
+    """The block with every matrix's weights behind its scales and biases, and its offsets."""
+    out, moved, at = np.empty_like(block), capi.ExpertOffsets(), 0
+    for name, rows, cols in (("gate", f, cfg.d), ("up", f, cfg.d), ("down", cfg.d, f)):
+        meta = rows * (cols // cfg.group_size) * 2
+        for part, size in (("s", meta), ("b", meta), ("w", rows * cols * cfg.weight_bits // 8)):
+            old = getattr(off, f"{name}_{part}")
+            out[at:at + size] = block[old:old + size]
+            setattr(moved, f"{name}_{part}", at)
+            at += size
+    assert at == block.nbytes
+    return out, moved
+
+
+def test_blocks_that_end_with_weights(cuda_device):
+    """Rows of 192 bytes are one and a half pieces: a copy of the last row's second piece would leave the block (248,832
+    bytes, a whole cell). The streaming kernel leaves such blocks to the per-tile kernels; the one-row kernel reads whole groups
+    and keeps them, with the same sums as ever."""
+    cfg = small_config(d=384, f=384, shared_f=384)
+    layer = Layer(cfg)
+    assert layer.block_bytes == layer.pool.cell_stride
+    x = inputs(1, cfg.d, seed=2)
+    usual = layer.forward(x, fused=True)[0]
+    for e in range(cfg.num_experts):
+        block, moved = weights_last(cfg, layer.offsets, layer.block(e), cfg.f)
+        layer.pool.upload(layer.first_cell + e, block)
+    shared, moved_shared = weights_last(cfg, layer.shared.offsets, layer.shared_block_host, cfg.shared_f)
+    layer.offsets, layer._shared_dev = moved, torch.from_numpy(shared).to(layer.device)
+    layer.shared = capi.SharedExpert(layer._shared_dev.data_ptr(), moved_shared)
+    assert (layer.forward(x, fused=True)[0] == usual).all()
+    for T in (3, 17):
+        check_layer(layer, inputs(T, cfg.d, seed=T), fused=True)
     layer.close()
