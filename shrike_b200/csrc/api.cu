@@ -949,7 +949,6 @@ int shrike_ep_create(shrike_moe* home, shrike_moe* routed, uint32_t rank, uint32
     cudaMemset(ep->miss_slots, 0xff, T * K * 4);
     ep->peer[rank] = ep->mine;
     ep->connected = world == 1;
-    home->beside_others = routed->beside_others = true;
     *out = ep;
     return SHRIKE_OK;
 }
@@ -1028,6 +1027,12 @@ int shrike_ep_forward(shrike_ep* ep, void* stream, const shrike_pool* local_pool
     cudaStream_t st = (cudaStream_t)stream;
     int rc;
     if ((rc = check_device(m))) return rc;
+    // the call's two streams run beside each other; outside of it the handles launch as any other
+    struct Beside {
+        shrike_moe *a, *b;
+        Beside(shrike_moe* a, shrike_moe* b) : a(a), b(b) { a->beside_others = b->beside_others = true; }
+        ~Beside() { a->beside_others = b->beside_others = false; }
+    } beside(m, r);
     const uint32_t epoch = ++ep->epoch;
     const uint32_t T = query_count;
     float* gate = c.shared_gated ? ep->gate : nullptr;

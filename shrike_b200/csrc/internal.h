@@ -127,8 +127,8 @@ struct shrike_moe {
     int sm_count = 148;
     uint32_t smem_optin = 0;      // most dynamic shared memory of a block
     bool no_pdl = false;          // SHRIKE_NO_PDL was set when the handle was created (diagnostics)
-    bool beside_others = false;   // one of an expert-parallel layer's handles: another stream's kernels run beside this one's,
-                                  // and blocks that wait on an SM for their predecessor would keep them off it
+    bool beside_others = false;   // inside an expert-parallel forward: kernels of its other stream run beside this handle's, and
+                                  // blocks that wait on an SM for their predecessor would keep them off it
     bool single_stream = false;   // SHRIKE_SINGLE_STREAM was set when the handle was created: nothing else runs on the GPU
                                   // beside this handle's stream, so the one-launch layer need not be a cooperative launch
     bool force_warp_mma = false;  // SHRIKE_PREFILL_PATH=mma was set when the handle was created (test switch)

@@ -120,6 +120,54 @@ def test_single_rank_expert_parallel_layer(cuda_device, tmp_path, T, exchange):
         assert counts[2] == 0
 
 
+def _edges(call):
+    """(all, programmatic) edges of the graph that the call's launches make on a stream of their own."""
+    import ctypes as C
+    rt = C.CDLL("libcudart.so.12")
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    graph, n = C.c_void_p(), C.c_size_t()
+    with torch.cuda.stream(stream):
+        assert rt.cudaStreamBeginCapture(C.c_void_p(stream.cuda_stream), 1) == 0   # 1: this thread's calls
+        try:
+            call()
+        finally:
+            assert rt.cudaStreamEndCapture(C.c_void_p(stream.cuda_stream), C.byref(graph)) == 0
+    assert rt.cudaGraphGetEdges_v2(graph, None, None, None, C.byref(n)) == 0
+    ends, data = (C.c_void_p * n.value), (C.c_uint8 * 8 * n.value)()
+    assert rt.cudaGraphGetEdges_v2(graph, ends(), ends(), data, C.byref(n)) == 0
+    assert rt.cudaGraphDestroy(graph) == 0
+    return n.value, sum(e[2] == 1 for e in data)   # cudaGraphEdgeData.type, cudaGraphDependencyTypeProgrammatic
+
+
+def test_handles_launch_as_before_once_a_forward_is_over(cuda_device):
+    """An expert-parallel forward launches its kernels without overlap of successive ones; the handles' own prefill
+    calls have it before the layer is made, after a forward, and after the layer has gone."""
+    from shrike_b200.moe import RouterOperands
+    cfg, T = _config(), 96
+    layer = _build_layer(cfg, 0, 1, T, 3, "peer")
+    x_np, router = _problem(T, cfg)
+    ops = RouterOperands(weights=torch.from_numpy(router).cuda())
+    x = torch.from_numpy(x_np).cuda()
+    y = torch.empty_like(x)
+    ids, w = torch.zeros((T, cfg.top_k), dtype=torch.int32, device="cuda"), torch.zeros((T, cfg.top_k), device="cuda")
+    layer.home.encode_router(ops, x, ids, w)
+    slots = torch.full_like(ids, -1)
+
+    def prefill():
+        layer.home.encode_prefill(layer.pool, layer.offsets, ids, slots, w, x, y, None, layer.shared)
+
+    prefill()
+    before = _edges(prefill)
+    layer.forward(ops, x, y)
+    layer.status()
+    assert before[1] > 0 and _edges(prefill) == before
+    layer._lib.shrike_ep_destroy(layer._ep)
+    layer._ep = None
+    assert _edges(prefill) == before
+    layer.close()
+
+
 def test_cuda_dispatch_matches_the_protocol(cuda_device):
     import ep_reference as R
     T, seed = 96, 22
