@@ -268,15 +268,18 @@ int shrike_encode_route_decode(shrike_moe* moe, void* stream, const shrike_route
                                uint32_t* out_indices, float* out_weights, float* out_shared_gate,
                                uint32_t* out_resolved_slots, uint32_t* out_counts);
 
-/* One decode layer in three launches chained with programmatic dependent
- * launch (route -> phase 1 -> phase 2; each starts its weight fetch while its
- * predecessor drains): what encodeDecodeTailStage's router + classification
- * (RealForwardRunner.swift:2834) and encodeSpeculativeRouted
- * (RealForwardRunner.swift:5520-5572) encode for one routed layer.
- * out_indices / out_weights may be NULL. With more than 16 rows, no io_status
- * and a handle created for prefill (max_tokens > 64) the call runs the router,
- * the classification and the expert-grouped tensor-core path instead: the same
- * result within the parity tolerance, every expert read once for all its rows. */
+/* One decode layer (route -> phase 1 -> phase 2): what encodeDecodeTailStage's
+ * router + classification (RealForwardRunner.swift:2834) and
+ * encodeSpeculativeRouted (RealForwardRunner.swift:5520-5572) encode for one
+ * routed layer. out_indices / out_weights may be NULL.
+ * One launch for one row and for 2 to 64 rows. Three launches chained with
+ * programmatic dependent launch where the one-launch kernels do not take the
+ * shape (an odd number of weight groups in a row, a pool of single-cell chunks,
+ * one row too wide for the ring) and for two rows of experts under 4 MB; of
+ * those, calls of more than 48 rows on a handle created for prefill
+ * (max_tokens > 64) run the router, the classification and the expert-grouped
+ * tensor-core path. Results agree within the parity tolerance on every path;
+ * picks and route weights are the same bits. */
 int shrike_encode_decode_layer(shrike_moe* moe, void* stream, const shrike_pool* pool,
                                const shrike_expert_offsets* routed_offsets,
                                const uint64_t* residency_table_row,

@@ -168,7 +168,12 @@ int fill_expert_args(shrike_moe* m, const shrike_pool* pool, const shrike_expert
 
 // Whether the streaming kernel is the faster one for a decode call. A single row has nothing to lay out ahead of the first
 // tile; two rows of small experts are about even (256 experts of 2048 x 512: 29.3 us a layer with the per-tile kernels,
-// 29.7 with it; three rows 34.8 and 33.9; experts of 7 MB at two rows 46.9 and 44.4).
+// 29.7 with it; three rows 34.8 and 33.9; experts of 7 MB at two rows 46.9 and 44.4). Up to 64 rows it also stays ahead of the
+// expert-grouped GEMM, which reads an expert once for all its rows but starts in a dozen launches (us a layer, streaming and
+// grouped, uniform picks; 256 experts of 2048 x 512 int4 | 32 of 2880 x 2880 int4 | 256 of 2304 x 1024 int8):
+//    4 rows  36, 67 |  92, 170 |  62, 123        32 rows   96, 199 | 190, 292 | 186, 322
+//   16 rows  67, 142 | 171, 288 | 130, 234       64 rows  129, 254 | 260, 294 | 251, 413
+// With picks by Zipf(1.1), 64 rows: 85, 124 | 257, 254 | 188, 290.
 bool stream_pays(const shrike_moe_config& c, uint32_t T) {
     return T > 2 || (T == 2 && (uint64_t)3 * c.d * c.f * c.weight_bits / 8 >= (4u << 20));
 }
@@ -724,10 +729,14 @@ int shrike_encode_decode_layer(shrike_moe* m, void* stream, const shrike_pool* p
         if (se == cudaSuccess) return SHRIKE_OK;
         if (se != cudaErrorNotSupported) return cuda_fail(m, se, "launch_expert_stream");
     }
-    // A few dozen rows on a handle that owns the prefill operands: the expert-grouped tensor-core call reads
-    // every expert once for all its rows, where the 8-row tiles read it once per 8 (gpt-oss shape, 64 rows:
-    // 279 us per layer against 740).
-    if (query_count > 16 && w.xs && umma_supported(m->cfg) && !m->force_warp_mma) {
+    // Shapes that the streaming kernel does not take, with many rows, on a handle that owns the prefill operands: the
+    // expert-grouped GEMM reads every expert once for all its rows, where the 8-row tiles read it once per 8. The dozen
+    // launches around it pay from about 50 rows on (us a layer, tiles and grouped, odd numbers of groups, picks uniform or by Zipf(1.1);
+    // 256 experts of 2048 x 576 int4 | 256 of 2304 x 1088 int8 | 32 of 2880 x 2880 int4 in groups of 64):
+    //   17 rows  120, 167 | 191, 256 | 240, 378     Zipf   62, 91 | 150, 221 | 161, 268
+    //   48 rows  226, 266 | 351, 414 | 302, 384     Zipf  124, 119 | 260, 290 | 301, 324
+    //   64 rows  263, 297 | 410, 459 | 374, 386     Zipf  157, 130 | 311, 301 | 368, 321
+    if (query_count > 48 && w.xs && umma_supported(m->cfg) && !m->force_warp_mma) {
         int rcg = shrike_encode_router(m, stream, router, x, query_count, m->cfg.d, ids, wt, gate);
         if (rcg) return rcg;
         rcg = shrike_encode_residency_classification(m, stream, ids, residency_table_row, query_count, w.slots_dev,

@@ -242,7 +242,7 @@ class MoE:
                             hidden: Optional[torch.Tensor] = None, shared: Optional[capi.SharedExpert] = None,
                             out_indices: Optional[torch.Tensor] = None, out_weights: Optional[torch.Tensor] = None,
                             io_status: Optional[torch.Tensor] = None, query_count: Optional[int] = None) -> None:
-        """One decode layer (route -> phase 1 -> phase 2) as three dependent launches."""
+        """One decode layer (route -> phase 1 -> phase 2): one launch for every shape that the one-launch kernels take."""
         q = x.shape[0] if query_count is None else query_count
         ops = router.to_c()
         self._check(self._lib.shrike_encode_decode_layer(

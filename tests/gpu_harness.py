@@ -118,7 +118,7 @@ class Layer:
     def forward(self, x: np.ndarray, prefill: bool | None = None, hidden: np.ndarray | None = None,
                 io_status: int | None = None, fused: bool = False):
         """router -> classification -> decode/prefill. Returns (y fp32, ids, weights, hidden_out).
-        fused=True takes the one-call decode layer (three dependent launches) instead."""
+        fused=True takes the one-call decode layer instead."""
         cfg = self.cfg
         x_dev = to_act_tensor(x, cfg.act_dtype, self.device)
         T = x_dev.shape[0]

@@ -472,15 +472,17 @@ def test_fused_layer_ties_misses_and_unready_batches(cuda_device, T):
     layer.close()
 
 
-@pytest.mark.parametrize("T", [17, 40, 64])
-def test_decode_layer_call_on_a_prefill_handle_with_dozens_of_rows(cuda_device, T):
-    """More than 16 rows on a handle that owns the prefill operands: the one-call layer runs the router, the
-    classification and the expert-grouped tensor-core path. Same ids and weights, outputs inside the tolerance,
+@pytest.mark.parametrize("T", [17, 40, 48, 49, 64])
+@pytest.mark.parametrize("d,f", [(256, 128), (320, 192)])
+def test_decode_layer_call_on_a_prefill_handle_with_dozens_of_rows(cuda_device, d, f, T):
+    """More than 16 rows on a handle that owns the prefill operands: with even numbers of groups the one-call layer is
+    the streaming kernel; with odd ones (5 and 3) the route kernel and the per-tile kernels up to 48 rows, from 49 on the router,
+    the classification and the expert-grouped tensor-core path. Same ids and weights, outputs inside the tolerance,
     the residual updated in place."""
-    cfg = small_config(d=256, f=128, shared_f=128, max_tokens=128)
+    cfg = small_config(d=d, f=f, shared_f=f, max_tokens=128)
     layer = Layer(cfg)
-    x = inputs(T, 256, seed=70 + T)
-    h0 = inputs(T, 256, seed=71 + T)
+    x = inputs(T, d, seed=70 + T)
+    h0 = inputs(T, d, seed=71 + T)
     y, ids, w, h = layer.forward(x, hidden=h0, fused=True)
     ids_ref, w_ref, _ = layer.oracle_route(x)
     assert (ids == ids_ref).all() and (w == w_ref).all()

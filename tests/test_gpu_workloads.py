@@ -118,12 +118,13 @@ def test_qwen_prefill_full_chunk_4096_rows(cuda_device):
 
 
 def test_gpt_oss_64_rows_on_the_expert_grouped_path(cuda_device):
-    """gpt-oss shape, g32, 64 rows on a handle that owns the prefill operands (max_tokens = 128): the layer
-    call takes the tcgen05 path with scale rows of 90 groups (not whole 16-byte units: read by the converter
-    threads) at D = F = 2880."""
+    """gpt-oss shape, g32, 64 rows on a handle that owns the prefill operands (max_tokens = 128): the prefill call takes
+    the tcgen05 path with scale rows of 90 groups (not whole 16-byte units: read by the converter warps) at
+    D = F = 2880; the layer call takes the streaming kernel."""
     cfg = fx.gpt_oss_config(max_tokens=128, group_size=32)
     layer = Layer(cfg, seed=108, device_fill=True)
-    err, gap = run(layer, inputs(64, cfg.d, seed=43), fused=True)
+    run(layer, inputs(64, cfg.d, seed=43), fused=True)
+    err, gap = run(layer, inputs(64, cfg.d, seed=43), prefill=True)
     print(f"gpt-oss g32 64 rows, grouped path: rel L2 {err:.2e}, min top-k gap {gap:.2e}")
     layer.close()
 
