@@ -178,16 +178,20 @@ bool stream_pays(const shrike_moe_config& c, uint32_t T) {
     return T > 2 || (T == 2 && (uint64_t)3 * c.d * c.f * c.weight_bits / 8 >= (4u << 20));
 }
 
-// The expert projections of a decode call's work lists (phases: 1, 2 or 3 = both). The streaming kernel takes every
-// shape whose tiles its ring and the tiled copies can hold; the per-tile kernels take the others.
+// The expert projections of a decode call's work lists (phases: 1, 2 or 3 = both, a launch each). The streaming kernel takes
+// every shape whose tiles its ring and the tiled copies can hold; the per-tile kernels take the others.
 cudaError_t launch_experts(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, uint32_t T, uint32_t phases, void* y,
                            void* hidden, bool pdl) {
     const uint32_t n_shared = m->cfg.has_shared ? (T + 7) / 8 : 0;
-    cudaError_t e = stream_pays(m->cfg, T) ? launch_expert_stream(m, st, a, T, n_shared, phases, y, hidden, pdl) : cudaErrorNotSupported;
-    if (e != cudaErrorNotSupported) return e;
     const uint32_t mi = max_instances(m->cfg, T);
-    if ((phases & 1u) && (e = launch_phase1(m, st, a, mi, pdl)) != cudaSuccess) return e;
-    return (phases & 2u) ? launch_phase2(m, st, a, T, mi, y, hidden, pdl) : cudaSuccess;
+    for (uint32_t phase = 1; phase <= 2; ++phase) {
+        if (!(phases & phase)) continue;
+        cudaError_t e = stream_pays(m->cfg, T) ? launch_expert_stream(m, st, a, T, n_shared, y, hidden, pdl, phase) : cudaErrorNotSupported;
+        if (e == cudaErrorNotSupported)
+            e = phase == 1 ? launch_phase1(m, st, a, mi, pdl) : launch_phase2(m, st, a, T, mi, y, hidden, pdl);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 // The prefill call with the status word of a streamed batch (moe.metal:36-39, 918-921): when io_status is
@@ -725,7 +729,7 @@ int shrike_encode_decode_layer(shrike_moe* m, void* stream, const shrike_pool* p
         ra.with_shared = m->cfg.has_shared; ra.int4 = m->cfg.weight_bits == 4; ra.group = m->cfg.group_size;
         ra.slots = w.slots_dev; ra.xh = w.xh; ra.xsum = w.xsum; ra.status = w.status;
         const cudaError_t se = launch_expert_stream(m, (cudaStream_t)stream, ea, query_count, m->cfg.has_shared ? (query_count + 7) / 8 : 0,
-                                                    3u, y, hidden, !m->no_pdl, &ra);
+                                                    y, hidden, !m->no_pdl, 3u, &ra);
         if (se == cudaSuccess) return SHRIKE_OK;
         if (se != cudaErrorNotSupported) return cuda_fail(m, se, "launch_expert_stream");
     }

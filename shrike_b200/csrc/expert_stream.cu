@@ -72,7 +72,6 @@ struct StreamTable {
     float weight[kPlanMaxPairs];                     // a routing launch: the pairs' route weights
     uint8_t live[SHRIKE_MAX_DECODE_TOKENS];          // bit q: the row's pick q has a cell
     uint32_t warp_sum[SHRIKE_MAX_EXPERTS / 32];
-    uint32_t misses;
 };
 struct StreamArgs {
     PoolView pool;
@@ -92,14 +91,13 @@ struct StreamArgs {
     const float* shared_gate;
     uint32_t* status;
     unsigned long long* arrived;                     // blocks past a grid barrier, over all launches
-    uint32_t* inst_done;                             // both phases: finished units of every instance
+    uint32_t* inst_done;                             // both phases: finished gate/up units of every instance
     uint32_t T;
     void* y;
     void* hidden;
-    uint32_t phases;                                 // bit 0, bit 1 (with phase 3)
+    uint32_t phases;                                 // bit 0, bit 1 (with phase 3); both: this launch routes its rows first
     uint32_t rcp_cpc;                                // ceil(2^32 / cells_per_chunk)
     uint32_t n_chunks;
-    uint32_t routes;                                 // this launch routes its rows first
     uint32_t token_groups;                           // of the logits: a block takes one group's rows against its share of the experts
     RouterArgs r;
     StreamGeom g;
@@ -418,7 +416,7 @@ __device__ __forceinline__ uint32_t work_list(const StreamArgs& a, uint8_t* dsm,
     };
     uint32_t n_inst;
     const uint32_t n_sh = a.n_shared;
-    if (a.routes) {
+    if (a.phases == 3u) {
         // ================= router, selection, lookup, work list =================
         // A block has a share of the expert rows (they go to the ring's memory, asked for ahead of the wait) and of the
         // activation rows; what follows the logits every block does for itself: another hand-over between blocks costs
@@ -548,16 +546,11 @@ __device__ __forceinline__ uint32_t work_list(const StreamArgs& a, uint8_t* dsm,
                     if (r.slots) r.slots[p] = slot;
                     if (slot != SHRIKE_SLOT_MISS && !inside) report_status(a.status, kStatusBadIndex);
                 }
-                if (slot == SHRIKE_SLOT_MISS && blockIdx.x == 0 && r.counts) atomicAdd(&tab.misses, 1u);
             }
             const uint32_t bits = __ballot_sync(0xffffffffu, live);
             if (lane == 0) tab.live[row] = (uint8_t)bits;
         }
         __syncthreads();
-        if (tid == 0 && blockIdx.x == 0 && r.counts) {
-            r.counts[0] = n_pairs - tab.misses;
-            r.counts[1] = tab.misses;
-        }
         uint32_t cnt = 0, incl = 0;   // thread e: pairs of expert e, and {instances, pairs} of the experts up to it
         if (tid < SHRIKE_MAX_EXPERTS) {
             for (uint32_t w = 0; w < n_words; ++w) cnt += __popc(rs.mask[w][tid]);
@@ -636,7 +629,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
     if (tid < G.n_slots2) { mbar_init(&full2[tid], 1); mbar_init(&done2[tid], G.w2); }
     if (tid == 0) mbar_init(&rows_here, 1);
     if (tid < kMaxSlots2) fence_mbar_init();
-    if (tid == 0) { s_failed = 0; tab.misses = 0; }
+    if (tid == 0) s_failed = 0;
     if (warp == 1 && lane < 4 * (SHRIKE_MAX_POOL_CHUNKS + 1)) {   // descriptors on their way before the first copy needs them
         const uint32_t ch = lane >> 2;
         const CUtensorMap* m = (lane & 2u) ? ((lane & 1u) ? maps.l1 : maps.m1) : ((lane & 1u) ? maps.l2 : maps.m2);
@@ -650,7 +643,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
     const uint32_t n_inst = work_list(a, dsm, ring, tab, &rows_here, &s_failed);
     const uint32_t n_sh = min(a.n_shared, n_inst);
     __syncthreads();
-    const float* const pair_weight = a.routes ? tab.weight : a.route_w;
+    const float* const pair_weight = a.phases == 3u ? tab.weight : a.route_w;
     // the row of pairs (shared: of rows) behind column c of instance i
     auto pair_of = [&](uint32_t i, uint32_t c) -> uint32_t { return i < n_sh ? tab.first[i] + c : tab.sorted[tab.first[i] + c]; };
     // this lane's row g of the eight, and its first byte in the row's piece
@@ -1123,11 +1116,10 @@ static uint32_t stream_token_groups(const shrike_moe_config& c, uint32_t sm_coun
     return 0;
 }
 
-// phases: 1, 2 or both. route (with both
-// phases): the launch routes the rows itself and needs no plan. cudaErrorNotSupported when the shape does not fit: nothing
-// was launched.
+// phases: 1 or 2, by the plan of an earlier launch, or both, with `route`: the launch then routes the rows itself.
+// cudaErrorNotSupported when the shape does not fit: nothing was launched.
 cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const ExpertArgs& ea, uint32_t T, uint32_t n_shared,
-                                 uint32_t phases, void* y, void* hidden, bool pdl, const RouterArgs* route) {
+                                 void* y, void* hidden, bool pdl, uint32_t phases, const RouterArgs* route) {
     const shrike_moe_config& c = m->cfg;
     const uint64_t cpc = ea.pool.cells_per_chunk ? ea.pool.cells_per_chunk : 1;
     if (cpc < 2 || (uint64_t)ea.pool.cells * cpc >= (1ull << 32)) return cudaErrorNotSupported;
@@ -1144,7 +1136,6 @@ cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const Exp
     a.parts = m->ws.parts; a.sorted = ea.sorted; a.pair_cell = m->ws.pair_cell;
     for (a.n_chunks = 0; a.n_chunks < SHRIKE_MAX_POOL_CHUNKS && ea.pool.base[a.n_chunks];) ++a.n_chunks;
     if (route) {
-        a.routes = 1;
         a.r = *route;
         a.token_groups = stream_token_groups(c, m->sm_count, T, a.g.ring_bytes);
         if (!a.token_groups) return cudaErrorNotSupported;

@@ -82,7 +82,7 @@ struct Workspace {
     uint32_t* status = nullptr;     // device status word
     uint32_t* done_counter = nullptr; // blocks finished, fused route kernel
     unsigned long long* arrived = nullptr;   // grid barriers of the streaming expert kernel: arrivals over all launches
-    uint32_t* inst_done = nullptr;  // its finished gate/up units of every instance; the plan zeroes them
+    uint32_t* inst_done = nullptr;  // a layer launch's finished gate/up units of every instance; it zeroes them itself
     float* parts = nullptr;         // its weighted rows per pair and per shared row [<= 64 tokens x (top_k + 1) x d]
     uint32_t* pair_cell = nullptr;  // decode plan: cell of every pair, or SHRIKE_SLOT_MISS
     uint32_t* block_hist = nullptr; // prefill grouping scratch
@@ -201,8 +201,7 @@ cudaError_t launch_after(const shrike_moe* m, cudaStream_t st, void (*k)(P...), 
 // expert_stream.cu
 struct RouterArgs;
 cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const ExpertArgs& ea, uint32_t T, uint32_t n_shared,
-                                 uint32_t phases, void* y, void* hidden, bool pdl,
-                                 const RouterArgs* route = nullptr);
+                                 void* y, void* hidden, bool pdl, uint32_t phases, const RouterArgs* route = nullptr);
 size_t stream_parts_bytes(const shrike_moe_config& c);
 size_t stream_done_bytes();
 // synth.cu

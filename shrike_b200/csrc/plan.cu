@@ -42,7 +42,7 @@ decode_plan_kernel(const uint32_t* __restrict__ slots, uint32_t T, uint32_t top_
                    Instance* __restrict__ inst, uint32_t* __restrict__ n_inst,
                    uint32_t* __restrict__ sorted, const void* __restrict__ x, uint32_t act_dtype,
                    uint32_t d, uint32_t int4, uint32_t group, uint16_t* __restrict__ xh,
-                   float* __restrict__ xsum, uint32_t* status, uint32_t max_inst, uint32_t* __restrict__ pair_cell, uint32_t* __restrict__ inst_done) {
+                   float* __restrict__ xsum, uint32_t* status, uint32_t max_inst, uint32_t* __restrict__ pair_cell) {
     __shared__ PlanSmem sm;
     const uint32_t tid = threadIdx.x;
     const uint32_t n_pairs = T * top_k;
@@ -64,7 +64,7 @@ decode_plan_kernel(const uint32_t* __restrict__ slots, uint32_t T, uint32_t top_
         pair_cell[p] = s;
     }
     __syncthreads();
-    plan_body(sm, n_pairs, T, with_shared, inst, n_inst, sorted, max_inst, status, inst_done);
+    plan_body(sm, n_pairs, T, with_shared, inst, n_inst, sorted, max_inst, status);
 
     // fp16 operand copy of the activation rows and their per-group sums
     const uint32_t items = T * (d / 8);
@@ -80,7 +80,7 @@ cudaError_t launch_decode_plan(const shrike_moe* m, cudaStream_t st, const uint3
         slots, T, m->cfg.top_k, io_status, with_shared ? 1u : 0u, pool_cells,
         m->ws.inst, m->ws.n_inst, m->ws.sorted, x, m->cfg.act_dtype, m->cfg.d,
         m->cfg.weight_bits == 4 ? 1u : 0u, m->cfg.group_size, m->ws.xh, m->ws.xsum, m->ws.status, max_instances(m->cfg, T),
-        m->ws.pair_cell, m->ws.inst_done);
+        m->ws.pair_cell);
     return cudaGetLastError();
 }
 

@@ -24,8 +24,7 @@ struct PlanSmem {
 // distinct cells than the layer has experts -- are dropped and reported through the status word.
 __device__ __forceinline__ void plan_body(PlanSmem& sm, uint32_t n_pairs, uint32_t T, uint32_t with_shared,
                                           Instance* __restrict__ inst, uint32_t* __restrict__ n_inst,
-                                          uint32_t* __restrict__ sorted, uint32_t max_inst, uint32_t* status,
-                                          uint32_t* __restrict__ inst_done) {
+                                          uint32_t* __restrict__ sorted, uint32_t max_inst, uint32_t* status) {
     const uint32_t tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) sm.n_valid = 0;
     __syncthreads();
@@ -92,7 +91,6 @@ __device__ __forceinline__ void plan_body(PlanSmem& sm, uint32_t n_pairs, uint32
         if (n_routed + n_shared > max_inst) report_status(status, kStatusBadIndex);
         *n_inst = min(n_routed + n_shared, max_inst);
     }
-    for (uint32_t j = tid; j < min(n_routed + n_shared, max_inst); j += bd) inst_done[j] = 0;
 }
 
 }  // namespace shrike

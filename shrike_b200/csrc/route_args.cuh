@@ -39,7 +39,6 @@ struct RouterArgs {
     float* xsum;
     uint32_t* done_counter;
     uint32_t* pair_cell;
-    uint32_t* inst_done;
     uint32_t* status;
     uint32_t max_inst;
 };

@@ -495,7 +495,6 @@ __global__ void __launch_bounds__(kRouterWarps * 32) route_fused_kernel(const Ro
                 a.inst[rank + (a.with_shared ? 1u : 0u)] = in;
                 a.sorted[rank] = lane;
             }
-            if (lane < n_routed + (a.with_shared ? 1u : 0u)) a.inst_done[lane] = 0;
             if (lane == 0) {
                 if (a.with_shared) {
                     Instance in;
@@ -507,7 +506,7 @@ __global__ void __launch_bounds__(kRouterWarps * 32) route_fused_kernel(const Ro
             }
         }
     }
-    if (!fast) plan_body(sm, n_pairs, a.T, a.with_shared, a.inst, a.n_inst, a.sorted, a.max_inst, a.status, a.inst_done);
+    if (!fast) plan_body(sm, n_pairs, a.T, a.with_shared, a.inst, a.n_inst, a.sorted, a.max_inst, a.status);
 }
 
 // moe_classify_residency_body for T rows. The miss lists keep router order: block b takes pairs
@@ -638,7 +637,7 @@ cudaError_t launch_route_fused(const shrike_moe* m, cudaStream_t st, const shrik
     a.with_shared = m->cfg.has_shared; a.int4 = m->cfg.weight_bits == 4; a.group = m->cfg.group_size;
     a.xsum = m->ws.xsum;
     a.slots = slots; a.counts = counts; a.inst = m->ws.inst; a.n_inst = m->ws.n_inst; a.sorted = m->ws.sorted;
-    a.xh = m->ws.xh; a.done_counter = m->ws.done_counter; a.pair_cell = m->ws.pair_cell; a.inst_done = m->ws.inst_done; a.status = m->ws.status; a.max_inst = max_instances(m->cfg, T);
+    a.xh = m->ws.xh; a.done_counter = m->ws.done_counter; a.pair_cell = m->ws.pair_cell; a.status = m->ws.status; a.max_inst = max_instances(m->cfg, T);
     const uint32_t rows = a.ne + (a.gate_row ? 1u : 0u);
     cudaLaunchConfig_t cfg = {};
     // several rows: up to four blocks share an expert row's tokens (65 blocks would leave half of the SMs idle)
