@@ -94,6 +94,13 @@ int check_device(shrike_moe* m) {
 
 bool aligned_to(const void* p, uintptr_t a) { return ((uintptr_t)p & (a - 1)) == 0; }
 
+// cudaMemset, finished when it returns: it runs on the legacy stream, which a caller's non-blocking stream does not wait for,
+// and a call on such a stream may come next.
+cudaError_t set_now(void* p, int value, size_t bytes) {
+    const cudaError_t e = cudaMemset(p, value, bytes);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 // Makes `device` current for the scope and puts the caller's device back afterwards.
 struct DeviceGuard {
     int prev = -1;
@@ -363,11 +370,17 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
         return fail(nullptr, SHRIKE_ENOMEM, "device allocation of the workspace failed");
     }
     for (const Part& p : small_parts) *p.p = (uint8_t*)small + p.at;
-    cudaMemset(small, 0, zeroed);
+    cudaError_t se = cudaSuccess;
     if (w.fused_geom) {
         // no logit carries the first epoch's tag, no activation has been published
-        cudaMemset(w.fused_logits, 0xff, fused_logits_bytes(c));
-        cudaMemset(w.fused_acts, 0xff, fused_acts_bytes(c));
+        se = cudaMemset(w.fused_logits, 0xff, fused_logits_bytes(c));
+        if (se == cudaSuccess) se = cudaMemset(w.fused_acts, 0xff, fused_acts_bytes(c));
+    }
+    if (se == cudaSuccess) se = set_now(small, 0, zeroed);
+    if (se != cudaSuccess) {
+        free_workspace(w);
+        delete m;
+        return cuda_fail(nullptr, se, "clearing the workspace");
     }
     if (T > SHRIKE_MAX_DECODE_TOKENS) {
         w.tensor_maps = aligned_alloc(64, umma_tensor_map_bytes());
@@ -397,7 +410,7 @@ int shrike_moe_status(shrike_moe* m, void* stream) {
     uint32_t st = 0;
     CU(cudaMemcpy(&st, m->ws.status, 4, cudaMemcpyDeviceToHost));
     if (st != kStatusOk) {
-        cudaMemset(m->ws.status, 0, 4);
+        CU(set_now(m->ws.status, 0, 4));
         if (st == kStatusWaitTimeout) return fail(m, SHRIKE_ETIMEDOUT, "a device-side wait gave up");
         if (st == kStatusOperandRange)
             return fail(m, SHRIKE_ERANGE, "an activation beyond the fp16 operand range (|x| > 65504) was clamped");
@@ -513,7 +526,7 @@ int shrike_residency_create(shrike_moe* m, uint32_t layers, uint64_t** table_out
     cudaError_t e = cudaMalloc((void**)&m->residency, n * 8);
     if (e != cudaSuccess) { cudaGetLastError(); return fail(m, SHRIKE_ENOMEM, "residency table: %s", cudaGetErrorString(e)); }
     // every entry: state 0 (absent)
-    CU(cudaMemset(m->residency, 0, n * 8));
+    CU(set_now(m->residency, 0, n * 8));
     m->residency_layers = layers;
     if (table_out) *table_out = m->residency;
     return SHRIKE_OK;
@@ -958,8 +971,12 @@ int shrike_ep_create(shrike_moe* home, shrike_moe* routed, uint32_t rank, uint32
         return fail(m, SHRIKE_ENOMEM, "ep: allocation of the exchange buffers failed");
     }
     // no arrival word carries the first epoch's tag; the shared-only call of the home rows sees every pick miss
-    cudaMemset(ep->mine, 0, ep->lay.bytes);
-    cudaMemset(ep->miss_slots, 0xff, T * K * 4);
+    cudaError_t se = cudaMemset(ep->mine, 0, ep->lay.bytes);
+    if (se == cudaSuccess) se = set_now(ep->miss_slots, 0xff, T * K * 4);
+    if (se != cudaSuccess) {
+        ep_free(ep);
+        return cuda_fail(m, se, "ep: clearing the exchange buffers");
+    }
     ep->peer[rank] = ep->mine;
     ep->connected = world == 1;
     *out = ep;

@@ -168,6 +168,33 @@ def test_handles_launch_as_before_once_a_forward_is_over(cuda_device):
     layer.close()
 
 
+def test_what_creation_clears_is_clear_when_it_returns(cuda_device):
+    """Handles, residency tables and exchange buffers are cleared on the legacy stream, which a caller's non-blocking
+    stream does not wait for: every create call waits itself, behind whatever that stream still has to do (20 ms here)."""
+    import ctypes as C
+    from shrike_b200 import capi
+    from shrike_b200.ep import ExpertParallelLayer
+    from shrike_b200.moe import MoE
+    cfg = _config()
+    legacy = torch.cuda.default_stream()
+    layer = ExpertParallelLayer(cfg, 0, 1, 0, 96)
+    lib, made = capi.load(), C.c_void_p()
+
+    def after(create):
+        torch.cuda._sleep(40_000_000)
+        assert not legacy.query()
+        create()
+        assert legacy.query()
+
+    moes = []
+    after(lambda: moes.append(MoE(cfg)))
+    after(lambda: moes[0].create_residency(1))
+    after(lambda: layer.home._check(lib.shrike_ep_create(layer.home._h, layer.routed._h, 0, 1, 96, C.byref(made))))
+    lib.shrike_ep_destroy(made)
+    moes[0].close()
+    layer.close()
+
+
 def test_cuda_dispatch_matches_the_protocol(cuda_device):
     import ep_reference as R
     T, seed = 96, 22
