@@ -7,7 +7,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <new>
-#include <vector>
 
 #include "internal.h"
 #include "route_args.cuh"
@@ -16,15 +15,19 @@ using namespace shrike;
 
 namespace {
 
-thread_local std::string g_create_error;
+thread_local char g_create_error[kErrorText];
 
 int fail(shrike_moe* m, int code, const char* fmt, ...) {
-    char buf[512];
     va_list ap;
     va_start(ap, fmt);
-    vsnprintf(buf, sizeof buf, fmt, ap);
+    vsnprintf(m ? m->err : g_create_error, kErrorText, fmt, ap);
     va_end(ap);
-    if (m) m->err = buf; else g_create_error = buf;
+    return code;
+}
+
+// A failure on one handle, reported on another.
+int pass_on(shrike_moe* to, const shrike_moe* from, int code) {
+    if (to != from) memcpy(to->err, from->err, kErrorText);
     return code;
 }
 
@@ -38,7 +41,7 @@ int cuda_fail(shrike_moe* m, cudaError_t e, const char* what) {
         if (e_ != cudaSuccess) return cuda_fail(m, e_, #call);    \
     } while (0)
 
-bool valid_config(const shrike_moe_config& c, std::string& why) {
+bool valid_config(const shrike_moe_config& c, const char*& why) {
     auto bad = [&](const char* s) { why = s; return false; };
     if (c.d == 0 || c.d % 64 != 0 || c.d > 2944) return bad("d must be a multiple of 64, at most 2944");
     if (c.f == 0 || c.f % 64 != 0) return bad("f must be a multiple of 64");
@@ -133,7 +136,7 @@ bool router_operands_aligned(const shrike_moe_config& c, const shrike_router_ope
 namespace {
 
 void free_workspace(Workspace& w) {
-    for (void* p : w.blocks) cudaFree(p);
+    for (uint32_t i = 0; i < w.n_blocks; ++i) cudaFree(w.blocks[i]);
     free(w.tensor_maps);
     free(w.fused_geom);
     free(w.fused_maps);
@@ -250,14 +253,14 @@ size_t act_bytes(uint32_t dt) { return dt == SHRIKE_DTYPE_FP32 ? 4 : 2; }
 extern "C" {
 
 const char* shrike_last_error(const shrike_moe* moe) {
-    return moe ? moe->err.c_str() : g_create_error.c_str();
+    return moe ? moe->err : g_create_error;
 }
 
 int shrike_expert_offsets_make(const shrike_moe_config* config, int shared, shrike_expert_offsets* out,
                                uint64_t* block_bytes) {
-    std::string why;
+    const char* why = nullptr;
     if (!config || !out) return fail(nullptr, SHRIKE_EINVAL, "null argument");
-    if (!valid_config(*config, why)) return fail(nullptr, SHRIKE_EINVAL, "%s", why.c_str());
+    if (!valid_config(*config, why)) return fail(nullptr, SHRIKE_EINVAL, "%s", why);
     if (shared && !config->has_shared) return fail(nullptr, SHRIKE_EINVAL, "config has no shared expert");
     uint64_t bytes;
     make_offsets(*config, shared != 0, *out, bytes);
@@ -268,8 +271,8 @@ int shrike_expert_offsets_make(const shrike_moe_config* config, int shared, shri
 int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** out) {
     if (!config || !out) return fail(nullptr, SHRIKE_EINVAL, "null argument");
     *out = nullptr;
-    std::string why;
-    if (!valid_config(*config, why)) return fail(nullptr, SHRIKE_EINVAL, "%s", why.c_str());
+    const char* why = nullptr;
+    if (!valid_config(*config, why)) return fail(nullptr, SHRIKE_EINVAL, "%s", why);
     int count = 0;
     cudaError_t e = cudaGetDeviceCount(&count);
     if (e != cudaSuccess || count == 0)
@@ -300,18 +303,22 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
     bool ok = true;
     // The small parts share a device allocation, the others have one each: requests below a megabyte share the driver's
     // 2 MB mappings, and a mapping (0.3 ms) is what making a handle costs.
-    struct Part { void** p; size_t at; };
-    std::vector<Part> small_parts;
+    struct Part { void** p; size_t at; } small_parts[kWorkspaceParts];
+    uint32_t n_small = 0;
     size_t small_bytes = 0;
     auto A = [&](auto** p, size_t bytes) {
+        if (!ok || n_small + w.n_blocks + 1 >= kWorkspaceParts) {
+            ok = false;
+            return;
+        }
         if (bytes < (64u << 10)) {
-            small_parts.push_back({(void**)p, small_bytes});
+            small_parts[n_small++] = {(void**)p, small_bytes};
             small_bytes += (bytes + 255) / 256 * 256;
             return;
         }
         void* at = nullptr;
-        if (ok && cudaMalloc(&at, bytes) != cudaSuccess) ok = false;
-        if (ok) { w.blocks.push_back(at); *(void**)p = at; }
+        if (cudaMalloc(&at, bytes) != cudaSuccess) ok = false;
+        else { w.blocks[w.n_blocks++] = at; *(void**)p = at; }
     };
     // words that start at zero
     A(&w.status, 4);
@@ -362,14 +369,14 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
     }
     void* small = nullptr;
     if (ok) ok = cudaMalloc(&small, small_bytes) == cudaSuccess;
-    if (ok) w.blocks.push_back(small);
+    if (ok) w.blocks[w.n_blocks++] = small;
     if (!ok) {
         free_workspace(w);
         delete m;
         cudaGetLastError();
         return fail(nullptr, SHRIKE_ENOMEM, "device allocation of the workspace failed");
     }
-    for (const Part& p : small_parts) *p.p = (uint8_t*)small + p.at;
+    for (uint32_t i = 0; i < n_small; ++i) *small_parts[i].p = (uint8_t*)small + small_parts[i].at;
     cudaError_t se = cudaSuccess;
     if (w.fused_geom) {
         // no logit carries the first epoch's tag, no activation has been published
@@ -1091,7 +1098,7 @@ int shrike_ep_forward(shrike_ep* ep, void* stream, const shrike_pool* local_pool
     {   // local experts on the received rows (read in place through the row map), accumulated per row
         ExpertArgs a;
         rc = fill_expert_args(r, local_pool, routed_offsets, nullptr, ep->c_w, nullptr, a);
-        if (rc) { m->err = r->err; return rc; }
+        if (rc) return pass_on(m, r, rc);
         const bool warp_mma = r->force_warp_mma || !umma_supported(r->cfg);
         CU(launch_prefill_plan(r, st, ep->c_ids, ep->c_slots, ep->mine + ep->lay.off_recv_x, ep->t_max, false,
                                local_pool->view.cells, warp_mma, nullptr, ep->row_map, ep->n_rows));
@@ -1117,8 +1124,7 @@ int shrike_ep_status(shrike_ep* ep, void* stream) {
     int rc = shrike_moe_status(ep->home, stream);
     const int rc2 = shrike_moe_status(ep->routed, stream);
     if (!rc && rc2) {
-        ep->home->err = ep->routed->err;
-        rc = rc2;
+        rc = pass_on(ep->home, ep->routed, rc2);
     }
     return rc;
 }
@@ -1150,9 +1156,11 @@ int shrike_ep_last_counts(shrike_ep* ep, uint32_t* sent_per_rank, uint32_t* rows
 }
 
 struct shrike_decode_stack {
-    std::vector<shrike_stack_layer> layers;
-    uint32_t max_rows;
+    shrike_stack_layer* layers = nullptr;
+    uint32_t layer_count = 0;
+    uint32_t max_rows = 0;
     void* stream_dev = nullptr;   // [(layers + 1) x max_rows x d]
+    ~shrike_decode_stack() { delete[] layers; }
 };
 
 int shrike_decode_stack_create(const shrike_stack_layer* layers, uint32_t layer_count, uint32_t max_rows,
@@ -1174,7 +1182,13 @@ int shrike_decode_stack_create(const shrike_stack_layer* layers, uint32_t layer_
     DeviceGuard guard(m->device);
     shrike_decode_stack* s = new (std::nothrow) shrike_decode_stack();
     if (!s) return fail(m, SHRIKE_ENOMEM, "host allocation failed");
-    s->layers.assign(layers, layers + layer_count);
+    s->layers = new (std::nothrow) shrike_stack_layer[layer_count];
+    if (!s->layers) {
+        delete s;
+        return fail(m, SHRIKE_ENOMEM, "host allocation failed");
+    }
+    std::copy(layers, layers + layer_count, s->layers);
+    s->layer_count = layer_count;
     s->max_rows = max_rows;
     const size_t bytes = (size_t)(layer_count + 1) * max_rows * c.d * act_bytes(c.act_dtype);
     if (cudaMalloc(&s->stream_dev, bytes) != cudaSuccess) {
@@ -1202,7 +1216,7 @@ int shrike_decode_stack_forward_host(shrike_decode_stack* stack, void* stream, c
     if (query_count > stack->max_rows) return fail(m, SHRIKE_ERANGE, "decode_stack: query_count exceeds max_rows");
     const shrike_moe_config& c = m->cfg;
     cudaStream_t st = (cudaStream_t)stream;
-    const uint32_t L = (uint32_t)stack->layers.size();
+    const uint32_t L = stack->layer_count;
     const size_t block = (size_t)query_count * c.d * act_bytes(c.act_dtype);
     uint8_t* dev = (uint8_t*)stack->stream_dev;
     CU(cudaMemcpyAsync(dev, rows_host, (size_t)(L + 1) * block, cudaMemcpyHostToDevice, st));
@@ -1211,10 +1225,7 @@ int shrike_decode_stack_forward_host(shrike_decode_stack* stack, void* stream, c
         const int rc = shrike_encode_decode_layer(ly.moe, stream, ly.pool, ly.routed_offsets, ly.residency_table_row,
                                                   ly.router, ly.shared, dev + (size_t)l * block, query_count, nullptr, nullptr,
                                                   nullptr, ly.moe->ws.y_dev, dev + (size_t)(l + 1) * block);
-        if (rc) {
-            if (ly.moe != m) m->err = ly.moe->err;
-            return rc;
-        }
+        if (rc) return pass_on(m, ly.moe, rc);
     }
     CU(cudaMemcpyAsync(out_host, dev + (size_t)L * block, block, cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));

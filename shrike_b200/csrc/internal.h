@@ -2,8 +2,6 @@
 #pragma once
 
 #include <utility>
-#include <vector>
-#include <string>
 
 #include "common.cuh"
 
@@ -69,8 +67,12 @@ struct ExpertArgs {
 #endif
 };
 
+constexpr uint32_t kErrorText = 512;
+constexpr uint32_t kWorkspaceParts = 64;   // more than the pointers of a workspace
+
 struct Workspace {
-    std::vector<void*> blocks;      // the device allocations that the pointers below lie in
+    void* blocks[kWorkspaceParts] = {};   // the device allocations that the pointers below lie in
+    uint32_t n_blocks = 0;
     float* logits = nullptr;        // [max_tokens x num_experts]
     uint16_t* xh = nullptr;
     float* xsum = nullptr;
@@ -120,7 +122,7 @@ struct shrike_pool {
 struct shrike_moe {
     shrike_moe_config cfg;
     int device;
-    std::string err;
+    char err[shrike::kErrorText] = "";   // text of the last failure
     shrike::Workspace ws;
     uint64_t* residency = nullptr;
     uint32_t residency_layers = 0;
