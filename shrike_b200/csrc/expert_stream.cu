@@ -1101,10 +1101,12 @@ size_t stream_done_bytes() { return kMaxTable * 4; }
 
 // How many groups the call's rows form for the logits: with more rows than two warps' worth a block takes a part of them
 // against more expert rows, since the experts' rows are on the block's chip already and the activations are not. 0 when a
-// block's rows of the router do not fit into the ring.
+// block's rows of the router do not fit into the ring, or there is no block for every row (block t writes row t's picks): both
+// only on a part of a GPU.
 static uint32_t stream_token_groups(const shrike_moe_config& c, uint32_t sm_count, uint32_t T, uint32_t ring_bytes) {
     const uint32_t rows = c.num_experts + (c.shared_gated ? 1u : 0u), bits = c.router_weight_bits;
     const uint32_t row_bytes = bits ? c.d * bits / 8 + c.d / 64 * 8 : c.d * 4;
+    if (T > sm_count) return 0;
     for (uint32_t n = T <= 16 ? 1 : T <= 32 ? 2 : 4; n; n /= 2) {
         const uint32_t nbx = sm_count / n, most = (rows + nbx - 1) / nbx;
         if (nbx && most * row_bytes + c.d * 4 + 16 + 2 * c.d * 4 <= ring_bytes) return n;
