@@ -25,9 +25,10 @@
 // All phases run in one launch when the call has them: a block asks for its first phase-2 units before it waits for
 // the other blocks' activations.
 //
-// Measured (256 experts of 2048 x 512, top 8, int4, 16 rows: 181 MB of expert blocks): the whole layer 69 us where router,
-// gate/up and down launches took 103; inside the unit loops 6.5 TB/s, the rest is the routing (16 us), the hand-over between
-// the projections (5 us) and the row sums (3 us). 60 rows 127 us where the prefill path took 348.
+// Measured (256 experts of 2048 x 512, top 8, int4, 16 rows: 181 MB of expert blocks): the whole layer 67 us where router,
+// gate/up and down launches took 101; gate/up reads 121 MB in 19 us (6.3 TB/s), down 60 MB in 11 (5.3 TB/s), the rest is the
+// routing (16 us), the first units' way (6 us), the hand-over between the projections (5 us) and the row sums (7 us). DRAM reads are the
+// algorithmic bytes (184 MB). 64 rows 129 us where the prefill path takes 254.
 #include "block_maps.cuh"
 #include "plan.cuh"
 #include "route_args.cuh"

@@ -1338,7 +1338,8 @@ static cudaError_t launch_fused_tp(const shrike_moe* m, cudaStream_t st, const F
     unsigned n = 0;
     // The blocks wait on each other's results, so all of them must be resident together. A cooperative launch
     // guarantees it, whatever else runs on the GPU: it is the default. It also keeps every block from starting
-    // until the previous kernel has left, prologue and launch latency exposed (0.5 us per layer). A host that
+    // until the previous kernel has left, prologue and launch latency exposed (launched call by call: 16.6 to 17.5 us a layer
+    // against 14.7, the 32-expert shape 39.1 against 36.5; in a replayed graph 14.3 both). A host that
     // runs one stream on the GPU does not need the guarantee -- the grid is one block per SM and a block needs
     // most of an SM, so the blocks are together as soon as the stream's previous kernel has ended -- and says so
     // with SHRIKE_SINGLE_STREAM at handle creation. (Two such layers on two streams without the guarantee could

@@ -16,8 +16,9 @@
 //              of every row per copy) into shared-memory rings. Whole-line TMA
 //              requests keep the packed experts streaming at HBM speed where
 //              per-thread 32-byte loads ran out of outstanding requests.
-//   warp 17    one thread copies the activation tiles: a 64 x 256 box of the
-//              expert-sorted fp16 rows per K block, 128-byte swizzle.
+//   warp 17    one thread copies the activation tiles: one or two boxes of 64 x
+//              16 to 256 of the expert-sorted fp16 rows per K block, 128-byte
+//              swizzle.
 //   warps 0-15 converters: two threads per weight row; per 64-wide K block
 //              they turn the packed nibbles/bytes into fp16 (q - Z) * scale +
 //              (bias + Z*scale) -- the reference's half(fma(q, scale, bias)),
@@ -36,8 +37,8 @@
 //          weighted reduce, with no per-(row, rank) partial rows in between).
 //
 // What bounds it (256 experts of 2048 x 512): a K block takes 0.43 us at 16 rows, the converters' chain of waits, loads,
-// arithmetic and stores, and 0.74 us at 256, where shared memory's bandwidth (the instructions' operands, the copies' and
-// converters' stores) holds the tensor cores at 70 %.
+// arithmetic and stores, and 0.74 to 0.76 us at 256 rows. That is 8.39 MFLOP on each of 148 SMs: 1.63 to 1.68 PFLOP/s, as fast as
+// the measured burst rate of a library GEMM (1.67). What is left of full tiles lies outside the K loop: 9 of a down tile's 14 us.
 //
 // Every wait is bounded; a wait that gives up sets the status word and the
 // block falls through to the TMEM release.
@@ -937,7 +938,7 @@ cudaError_t umma_prepare(shrike_moe* m) {
     const shrike_moe_config& c = m->cfg;
     Workspace& ws = m->ws;
     if (!ws.xs || !umma_supported(c)) return cudaSuccess;
-    // maps[operand][box]: operands xs, acts, xh, acts_shared; boxes of 32, 64, 128, 256 rows
+    // maps[operand][box]: operands xs, acts, xh, acts_shared; boxes of 16, 32, 64, 128, 256 rows
     CUtensorMap* am = (CUtensorMap*)ws.tensor_maps;
     const uint64_t pairs = (uint64_t)c.max_tokens * c.top_k;
     bool ok = true;
