@@ -6,8 +6,8 @@ import pytest
 import torch
 
 from shrike_b200 import capi
-from gpu_harness import Layer, inputs, small_config
-from test_gpu_parity import check_layer
+from gpu_harness import Layer, inputs, rel_l2, small_config, to_act_tensor
+from test_gpu_parity import TOL, check_layer
 
 pytestmark = pytest.mark.gpu
 
@@ -23,9 +23,31 @@ pytestmark = pytest.mark.gpu
     dict(d=192, f=320, shared_f=64, group_size=32, weight_bits=8, expert_bias=1, activation=capi.ACT_GELU_TANH),
 ], ids=lambda kw: "-".join(f"{k}{v}" for k, v in kw.items()))
 def test_stream_edges(cuda_device, kw, T):
+    """The layer call, and the projections as calls of their own behind the plan and behind the route kernel."""
     layer = Layer(small_config(**kw))
-    check_layer(layer, inputs(T, kw["d"], seed=T), fused=True)
+    x = inputs(T, kw["d"], seed=T)
+    check_layer(layer, x, fused=True)
+    check_layer(layer, x)
+    y, ids, w, hidden = by_separate_calls(layer, x)
+    ids_ref, w_ref, _ = layer.oracle_route(x)
+    assert (ids == ids_ref).all() and (w == w_ref).all()
+    assert rel_l2(y, layer.oracle_forward(x, ids_ref, w_ref)) <= TOL
+    assert np.abs(hidden - (x + y)).max() <= 1e-5 * np.abs(x).max()
     layer.close()
+
+
+def by_separate_calls(layer: Layer, x: np.ndarray):
+    cfg, T = layer.cfg, len(x)
+    x_dev = to_act_tensor(x, cfg.act_dtype, layer.device)
+    y, hidden = torch.empty_like(x_dev), x_dev.clone()
+    ids = torch.empty((T, cfg.top_k), dtype=torch.int32, device=layer.device)
+    w = torch.empty((T, cfg.top_k), dtype=torch.float32, device=layer.device)
+    gate = torch.empty(T, device=layer.device) if cfg.shared_gated else None
+    layer.moe.encode_route_decode(layer.router_ops, layer.layer, layer.pool, x_dev, ids, w, gate)
+    layer.moe.encode_phase1(layer.pool, layer.offsets, T, layer.shared)
+    layer.moe.encode_phase2_reduce(layer.pool, layer.offsets, w, y, T, hidden, layer.shared, gate)
+    layer.moe.status()
+    return y.cpu().numpy(), ids.cpu().numpy().astype(np.uint32), w.cpu().numpy(), hidden.cpu().numpy()
 
 
 def weights_last(cfg, off: capi.ExpertOffsets, block: np.ndarray, f: int):

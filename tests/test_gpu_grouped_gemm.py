@@ -51,5 +51,6 @@ def run_sizes(sizes, kw, sample=None):
     want = layer.oracle_forward(x, ids, w, rows=rows)
     got = y.cpu().numpy()[rows]
     assert rel_l2(got, want) <= 1e-3
-    assert max(rel_l2(g, v) for g, v in zip(got, want)) <= 2e-3
+    # a single row: scale, offset and value of a weight and the activation are rounded to fp16, 2^-11 each
+    assert max(rel_l2(g, v) for g, v in zip(got, want)) <= 4 * 2.0 ** -11
     layer.close()
