@@ -10,25 +10,24 @@
 // reads each activation byte once per 256 weight rows and dequantises each
 // weight once per 256 activation rows.
 //
-//   warp 18    one thread streams the packed weights (64 bytes of every row
-//              per copy: a 3-D TMA box of 128 rows of one matrix of one pool
-//              cell, 64-byte swizzle) and the group scales / biases (16 bytes
+//   warp 19    one thread takes tiles, streams the packed weights (64 or, for narrow tiles, 128
+//              bytes of every row per copy: a 3-D TMA box of 128 rows of one matrix of one pool
+//              cell, swizzled) and the group scales / biases (16 or 32 bytes
 //              of every row per copy) into shared-memory rings. Whole-line TMA
 //              requests keep the packed experts streaming at HBM speed where
 //              per-thread 32-byte loads ran out of outstanding requests.
-//   warp 17    one thread copies the activation tiles: one or two boxes of 64 x
+//   warp 18    one thread copies the activation tiles: one or two boxes of 64 x
 //              16 to 256 of the expert-sorted fp16 rows per K block, 128-byte
 //              swizzle.
-//   warps 0-15 converters: two threads per weight row; per 64-wide K block
-//              they turn the packed nibbles/bytes into fp16 (q - Z) * scale +
-//              (bias + Z*scale) -- the reference's half(fma(q, scale, bias)),
-//              tensorops.metal:106 -- and write them to TMEM (instances of up
-//              to 128 rows) or, 16 bytes at a time, into the K-major
-//              128-byte-swizzled tile in shared memory that the MMA reads.
-//              After the K loop the same warps run the epilogue.
-//   warp 16    one elected thread issues tcgen05.mma (M 128, N = rows, K 16, fp16 in,
-//              fp32 accumulate in TMEM) for both tiles and commits to the
+//   warps 0-15 converters: they turn the packed nibbles/bytes of a 64-wide K block into fp16
+//              (q - Z) * scale + (bias + Z*scale) -- the reference's half(fma(q, scale, bias)),
+//              tensorops.metal:106 -- and write them to TMEM (narrow tiles) or, 16 bytes at a
+//              time, into the K-major 128-byte-swizzled tile in shared memory that the MMA reads.
+//              After the K loop of a tile of more than 64 rows the same warps run the epilogue.
+//   warps 16, 17  one elected thread of each issues tcgen05.mma (M 128, N = rows, K 16, fp16 in,
+//              fp32 accumulate in TMEM) for one of the two tiles and commits to the
 //              mbarriers that free the converted tile and the activation tile.
+//   warps 20-23   epilogues of tiles of up to 64 rows, while the next tile is converted.
 //
 // PHASE 0: tile 0 = 128 gate rows, tile 1 = the matching 128 up rows; epilogue
 //          GLU -> fp16 activations in operand layout, one row per sorted pair.
@@ -36,14 +35,16 @@
 //          weight -> red.global.add into the token's fp32 accumulator row (the
 //          weighted reduce, with no per-(row, rank) partial rows in between).
 //
-// What bounds it (256 experts of 2048 x 512): a K block takes 0.43 us at 16 rows, the converters' chain of waits, loads,
-// arithmetic and stores, and 0.74 to 0.76 us at 256 rows. That is 8.39 MFLOP on each of 148 SMs: 1.63 to 1.68 PFLOP/s, as fast as
-// the measured burst rate of a library GEMM (1.67). What is left of full tiles lies outside the K loop: 9 of a down tile's 14 us.
+// What bounds it (256 experts of 2048 x 512, int4): at 256 rows a K block takes 0.74 to 0.76 us. That is 8.39 MFLOP on each of 148
+// SMs: 1.63 to 1.68 PFLOP/s, as fast as the measured burst rate of a library GEMM (1.67). What is left of full tiles lies outside
+// the K loop: 9 of a down tile's 14 us. With few rows the issue slots of the converters (70 % taken at 10 rows an expert; fp16
+// arithmetic and logic run at half the rate there); 10 rows an expert take 93 us for gate/up and 62 for down, 2.9 TB/s.
 //
 // Every wait is bounded; a wait that gives up sets the status word and the
 // block falls through to the TMEM release.
 #include <cuda.h>
 #include <algorithm>
+#include <type_traits>
 
 #include "internal.h"
 
@@ -53,24 +54,39 @@ constexpr uint32_t kUmmaMaxN = 256;
 constexpr int kActBoxes = 5;
 constexpr uint32_t kConverters = 512;                  // two threads per weight row
 constexpr uint32_t kConvWarps = kConverters / 32;
-constexpr uint32_t kUmmaThreads = kConverters + 96;    // + MMA warp, activation-copy warp, weight-copy warp
-constexpr uint32_t kAStages = 2, kMaxAStages = 4, kBStages = 3, kPkSlots = 3;   // kAStages: at the widest activation tile
+constexpr uint32_t kEpiWarps = 4;
+constexpr uint32_t kUmmaThreads = kConverters + 128 + kEpiWarps * 32;   // + two MMA warps, activation-copy warp, weight-copy warp, epilogue warps
+constexpr uint32_t kSmallN = 64;                       // rows up to which TMEM holds two pairs of accumulators
+constexpr uint32_t kConvRegs = 96, kOtherRegs = 48;    // of the 80 that 768 threads are launched with
+static_assert(kConverters * kConvRegs + (kUmmaThreads - kConverters) * kOtherRegs <= kUmmaThreads * 80, "registers of a block");
 constexpr uint32_t kTileBytes = 128 * 128;             // 128 rows x 64 fp16, one swizzle-128B K block
-constexpr uint32_t kAStageBytes = 2 * kTileBytes;      // both weight tiles
-constexpr uint32_t kBTileBytes = kUmmaMaxN * 128;      // 256 rows x 64 fp16
-constexpr uint32_t kPkSlotBytes = 256 * 64;            // 64 packed bytes of 256 rows
-constexpr uint32_t kScHalfBytes = 256 * 16;            // 8 scales (or biases) of 256 rows
-constexpr uint32_t kOffA = kBStages * kBTileBytes;
-constexpr uint32_t kOffPk = kOffA + kAStages * kAStageBytes;
-constexpr uint32_t kOffSc = kOffPk + kPkSlots * kPkSlotBytes;
-constexpr uint32_t kOffBar = kOffSc + 2 * kScHalfBytes;
-constexpr uint32_t kNumBars = 2 * kMaxAStages + 2 * kBStages + 2 * kPkSlots + 3 + 5;
-constexpr uint32_t kUmmaSmemBytes = kOffBar + kNumBars * 8 + 4 * kUmmaMaxN * 4 + 16 + 1024 /*alignment slack*/;
+constexpr uint32_t kTiles = 4;                         // tiles that the copies may be ahead
+// Shared memory of wide tiles (more than 128 rows):
+//   [activations 3 x 32 KB][converted weights 2 x 32 KB][packed weights 3 x 16 KB][scales 8 KB]
+constexpr uint32_t kWideB = 3, kWideA = 2, kWidePk = 3;
+constexpr uint32_t kWideBBytes = kUmmaMaxN * 128, kWideABytes = 2 * kTileBytes;
+constexpr uint32_t kWidePkBytes = 256 * 64;            // 64 packed bytes of 256 rows
+constexpr uint32_t kWideScBytes = 2 * 256 * 16;        // 8 scales and biases of 256 rows
+constexpr uint32_t kWideOffA = kWideB * kWideBBytes, kWideOffPk = kWideOffA + kWideA * kWideABytes;
+constexpr uint32_t kWideOffSc = kWideOffPk + kWidePk * kWidePkBytes;
+// and of narrow ones, whose converted weights go to TMEM: [activations 5 x 16 KB][packed weights 3 x 32 KB][scales 2 x 16 KB]
+constexpr uint32_t kNarrowN = 128, kNarrowA = 2, kNarrowB = 5, kNarrowPk = 3, kNarrowSc = 2;
+constexpr uint32_t kNarrowBBytes = kNarrowN * 128;     // a K block of 128 rows, two of 64 or four of 32
+constexpr uint32_t kNarrowPkBytes = 256 * 128;         // 128 packed bytes of 256 rows
+constexpr uint32_t kNarrowScBytes = 2 * 256 * 32;      // 16 scales and biases of 256 rows
+constexpr uint32_t kNarrowOffPk = kNarrowB * kNarrowBBytes, kNarrowOffSc = kNarrowOffPk + kNarrowPk * kNarrowPkBytes;
+constexpr uint32_t kOffBar = kWideOffSc + kWideScBytes;
+static_assert(kNarrowOffSc + kNarrowSc * kNarrowScBytes <= kWideOffSc, "the converters' own scales lie beside the narrow tiles' ring");
+constexpr uint32_t kNumBars = 2 * (kWideB + kWideA + kWidePk + 1) + 1 + 2 * (kNarrowA + kNarrowB + kNarrowPk + kNarrowSc) + 2 + 3 * kTiles + 2;
+constexpr uint32_t kOffTiles = (kOffBar + kNumBars * 8 + 15) / 16 * 16;
+constexpr uint32_t kUmmaSmemBytes = kOffTiles + kTiles * 16 + 4 * kUmmaMaxN * 4 + 4 * kSmallN * 4 + 16 + 1024 /*alignment slack*/;
+static_assert(kUmmaSmemBytes + 64 <= 227 * 1024, "shared memory of a block");
 
 struct WeightMaps {       // TMA descriptors of the two 128-row tiles of a block
     CUtensorMap w[2];     // packed weights   [cells][rows][row bytes]
     CUtensorMap s[2];     // group scales     [cells][rows][groups]
     CUtensorMap b[2];     // group biases
+    CUtensorMap nw[2], ns[2], nb[2];   // the same in the boxes of narrow tiles, twice as wide
 };
 struct UmmaMaps {
     WeightMaps routed[SHRIKE_MAX_POOL_CHUNKS];
@@ -108,8 +124,8 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
           "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
@@ -120,8 +136,8 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
     return p != 0;
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar, uint32_t count = 1) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
@@ -165,15 +181,22 @@ __device__ __forceinline__ void dequant_word(uint32_t w, uint32_t s2, uint32_t z
 }
 
 __device__ __forceinline__ uint32_t half2_dup(float v) {
-    const uint32_t h = __half_as_ushort(__float2half_rn(v));
-    return h | (h << 16);
+    uint32_t h;
+    asm("cvt.rn.f16x2.f32 %0, %1, %1;" : "=r"(h) : "f"(v));
+    return h;
 }
 
-__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-        : "r"(taddr));
+template <int C>
+__device__ __forceinline__ void tmem_ld_issue(uint32_t taddr, uint32_t (&r)[C]) {
+    static_assert(C == 4 || C == 8, "columns");
+    if constexpr (C == 4)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
+    else
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+            : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -203,10 +226,11 @@ __device__ __forceinline__ float glu_epilogue(float gate, float up, uint32_t act
     return __fdividef(gate, 1.0f + __expf(-gate)) * up;
 }
 
-// Bounded wait for the pipeline barriers: these are on the critical path of every K block, so the
-// first polls do not sleep.
-__device__ __forceinline__ bool pipe_wait(uint64_t* bar, uint32_t parity) {
+// Bounded wait for the pipeline barriers: these are on the critical path of every K block, so the first polls do not sleep.
+// False when the time is up, or another role's was. (Inlined: around a call the converters moved their registers.)
+__device__ __forceinline__ bool pipe_wait_or(uint64_t* bar, uint32_t parity, const volatile uint32_t* failed) {
     const uint32_t addr = smem_u32(bar);
+#pragma unroll 1
     for (uint32_t it = 0; it < (1u << 21); ++it) {
         uint32_t ok;
         asm volatile(
@@ -215,9 +239,36 @@ __device__ __forceinline__ bool pipe_wait(uint64_t* bar, uint32_t parity) {
             "selp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
         if (ok) return true;
-        if (it > 256) __nanosleep(32);
+        if (it > 256) {
+            __nanosleep(32);
+            if (*failed) return false;
+        }
     }
     return false;
+}
+// Whether the phase is over, without waiting.
+__device__ __forceinline__ bool pipe_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+
+template <int N>
+__device__ __forceinline__ void load_words(const uint8_t* from, uint32_t (&w)[N]) {
+    static_assert(N == 1 || N == 2 || N == 4, "words");
+    if constexpr (N == 4) {
+        const uint4 v = *(const uint4*)from;
+        w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+    } else if constexpr (N == 2) {
+        const uint2 v = *(const uint2*)from;
+        w[0] = v.x; w[1] = v.y;
+    } else {
+        w[0] = *(const uint32_t*)from;
+    }
 }
 
 // 16-bit field `idx` (0..7) of four registers.
@@ -231,12 +282,9 @@ struct alignas(16) ChunkInstance {  // up to 256 rows that share one expert bloc
     uint32_t kind, slot, first, count;
 };
 
-// The instance's rows as one or two boxes of 16 << i rows (the largest that fits, then the smallest that holds the
-// rest), and the layout of the activation and weight stages. An instance with few rows needs narrow activation tiles and
-// gets more weight stages instead: what paces such a tile is the round trip converters -> tensor core -> converters.
+// The instance's rows as one or two boxes of 16 << i rows (the largest that fits, then the smallest that holds the rest).
 struct TileShape {
-    uint32_t N, n1, b1, n2, b2, b_stage, off_a, a_stages, acc_step;
-    bool in_tmem;   // converted weights: stages of 64 TMEM columns from column 256 on
+    uint32_t N, n1, b1, n2, b2;
     __device__ explicit TileShape(uint32_t count) {
         N = (count + 15u) & ~15u;           // MMA N: rows padded to 16
         n1 = 16; b1 = 0;
@@ -246,68 +294,103 @@ struct TileShape {
             n2 = 16;
             while (n2 < N - n1) { n2 <<= 1; ++b2; }
         }
-        // three layouts: 64, 128 or 256 activation rows a stage
-        b_stage = N <= 64 ? 64u * 128u : N <= 128 ? 128u * 128u : 256u * 128u;
-        off_a = kBStages * b_stage;
-        // Up to 128 rows the accumulators leave TMEM room for the converted weights. From shared memory the tensor core
-        // needs 85 cycles to fetch the weights of an instruction, whatever its N; and the converters' stores and their
-        // fence fall away.
-        in_tmem = N <= 128;
-        acc_step = in_tmem ? 128u : kUmmaMaxN;
-        a_stages = in_tmem ? kMaxAStages : (kOffPk - off_a) / kAStageBytes;
     }
 };
 
-// A persistent block per SM; tiles (instance, 128 or 256 weight rows) come from a counter, in list order. The copy
-// threads run ahead into the next tile while the converters finish this one: as one block per tile, set-up, the first
-// copies' way and the launch gap cost 4 us of every tile's 8 (512 x 16 columns) to 37 (2048 x 256).
-template <int BITS, int GROUP, int META, int PHASE>
+// K blocks of activations in a narrow tile's stage, less one. A copy of activations waits in the SM's copy engine behind the packed
+// weights, 32 KB at a time: with a K block a stage and four stages the tensor core waited 660 cycles for each of 16 rows.
+__device__ __forceinline__ uint32_t narrow_b_mask(uint32_t count) { return count <= 32 ? 3u : count <= 64 ? 1u : 0u; }
+
+// A tile as the weight copy hands it to the other roles: rows r0 and on of the matrix against the rows first .. first + count
+// of the sorted pairs (the shared expert: of the call); count 0 ends the list.
+struct Tile {
+    uint32_t slot, first, r0, count;
+    bool shared, narrow;
+    __device__ Tile() {}
+    __device__ explicit Tile(const uint4& v)
+        : slot(v.x), first(v.y), r0(v.z & 0x7fffffffu), count(v.w), shared(v.z >> 31), narrow(v.w <= kNarrowN) {}
+};
+
+// A persistent block per SM; tiles (instance, 128 or 256 weight rows) come from a counter, in list order: wide ones (129 to 256
+// rows) first. The copy threads run ahead into the next tiles while the converters finish this one: as one block per tile, set-up,
+// the first copies' way and the launch gap cost 4 us of every tile's 8 (512 x 16 columns) to 37 (2048 x 256).
+//
+// Wide tiles are bound by the tensor core, narrow ones by the converters' instructions, and have loops of their own:
+//   wide    all converters on every K block, a thread 32 of a row's 64 weights, into shared memory; both accumulators fill TMEM, so
+//           a tile ends before the next begins;
+//   narrow  the converters in two sets of eight warps on alternate K blocks, a thread all 64 weights of its row, into TMEM: half
+//           the waits, arrivals and scales per weight, and while a set waits the other converts. The tensor core is told of two K
+//           blocks at a time. Up to 64 rows there are two pairs of accumulators, and warps of their own for the epilogues.
+// 10 rows an expert, gate/up and down: 136 + 98 us with all converters on every K block and one loop for both kinds of tile, 121 +
+// 100 in two sets, 106 + 82 with an issuing warp per weight tile (a single one needed 650 cycles for a K block), 101 + 72 with
+// epilogue warps, 93 + 62 with the questions to barriers asked before their answers are needed. Deeper rings of copies, wider
+// boxes and fewer boxes of scales changed nothing: the bytes are there in time.
+// SCT: rows of scales are whole 16-byte units and come by TMA; others (groups % 8 != 0) are read by the converters.
+template <int BITS, int GROUP, int META, int PHASE, bool SCT>
 __global__ void __launch_bounds__(kUmmaThreads, 1)
 umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, uint32_t* __restrict__ n_inst,
                    const uint32_t row_tiles, const __grid_constant__ UmmaMaps maps) {
     constexpr uint32_t kRowBlockBytes = 64 * BITS / 8;  // packed bytes of one row per K block (32 or 64)
     constexpr uint32_t kWordsPerBlock = kRowBlockBytes / 4;
     constexpr uint32_t kGroupsPerBlock = 64 / GROUP;    // 1 (g64) or 2 (g32)
-    constexpr uint32_t kKbPerPk = 64 / kRowBlockBytes;  // K blocks per packed copy (2 or 1)
-    constexpr uint32_t kKbPerSc = 8 / kGroupsPerBlock;  // K blocks per scale copy (8 or 4)
+    constexpr uint32_t kKbPerSc = 8 / kGroupsPerBlock;  // K blocks per eight groups (8 or 4)
+    constexpr uint32_t kWideKbPerPk = 64 / kRowBlockBytes, kNarrowKbPerPk = 2 * kWideKbPerPk;   // K blocks per packed copy
     constexpr float kZero = BITS == 4 ? 8.0f : 128.0f;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     pdl_launch_dependents();
-    // Scale rows that are whole 16-byte units come by TMA; others (groups % 8 != 0) are read by the converters. One way for
-    // all instances: both use the same memory, which the copy thread would fill a tile ahead.
-    const bool sc_tma = PHASE == 0 ? (a.d / GROUP & 7u) == 0 : ((a.f / GROUP | a.f_shared / GROUP) & 7u) == 0;
-
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
     uint64_t* bars = (uint64_t*)(smem + kOffBar);
+    // wide tiles
     uint64_t* a_full = bars;                       // converters -> MMA
-    uint64_t* a_empty = a_full + kMaxAStages;      // MMA -> converters
-    uint64_t* b_full = a_empty + kMaxAStages;      // activation copy -> MMA
-    uint64_t* b_empty = b_full + kBStages;         // MMA -> activation copy
-    uint64_t* pk_full = b_empty + kBStages;        // weight copy -> converters
-    uint64_t* pk_empty = pk_full + kPkSlots;       // converters -> weight copy
-    uint64_t* sc_full = pk_empty + kPkSlots;
+    uint64_t* a_empty = a_full + kWideA;           // MMA -> converters
+    uint64_t* b_full = a_empty + kWideA;           // activation copy -> MMA
+    uint64_t* b_empty = b_full + kWideB;           // MMA -> activation copy
+    uint64_t* pk_full = b_empty + kWideB;          // weight copy -> converters
+    uint64_t* pk_empty = pk_full + kWidePk;        // converters -> weight copy
+    uint64_t* sc_full = pk_empty + kWidePk;
     uint64_t* sc_empty = sc_full + 1;
-    uint64_t* accum = sc_empty + 1;                // all of a tile's MMAs are done
-    uint64_t* next_full = accum + 1;               // [2] weight copy -> everyone: the next tile's number
-    uint64_t* next_empty = next_full + 2;
-    uint64_t* conv = next_empty + 2;               // the converter warps among themselves (a named barrier has no bounded wait)
-    uint32_t* rowid = (uint32_t*)(bars + kNumBars);                 // [2][column] token of a column, tiles in turn
-    float* roww = (float*)(rowid + 2 * kUmmaMaxN);                  // [2][column] route weight (routed) or gate (shared)
-    uint32_t* next_tile = (uint32_t*)(roww + 2 * kUmmaMaxN);        // [2]
-    uint32_t* tmem_slot = next_tile + 2;
+    uint64_t* wide_over = sc_empty + 1;            // MMA -> copies: nothing reads the wide tiles' memory any more
+    // narrow tiles
+    uint64_t* na_full = wide_over + 1;
+    uint64_t* na_empty = na_full + kNarrowA;
+    uint64_t* nb_full = na_empty + kNarrowA;
+    uint64_t* nb_empty = nb_full + kNarrowB;
+    uint64_t* npk_full = nb_empty + kNarrowB;
+    uint64_t* npk_empty = npk_full + kNarrowPk;
+    uint64_t* nsc_full = npk_empty + kNarrowPk;
+    uint64_t* nsc_empty = nsc_full + kNarrowSc;
+    // all
+    uint64_t* accum = nsc_empty + kNarrowSc;       // [kTiles] MMA -> epilogue: all of a tile's MMAs are done, tiles in turn
+    uint64_t* epi_done = accum + kTiles;                // [2] converters -> MMA: a tile's accumulators have been read
+    uint64_t* tile_full = epi_done + 2;            // [kTiles] weight copy -> everyone: the next tile
+    uint64_t* tile_empty = tile_full + kTiles;
+    uint64_t* conv = tile_empty + kTiles;          // the converter warps among themselves (a named barrier has no bounded wait)
+    uint64_t* eids_full = conv + 1;                // the epilogue warps among themselves
+    uint4* next_tile = (uint4*)(smem + kOffTiles);                  // [kTiles]
+    uint32_t* rowid = (uint32_t*)(next_tile + kTiles);              // token of a column: [2][256], tiles in turn, or [4][128]
+    float* roww = (float*)(rowid + 2 * kUmmaMaxN);                  // route weight (routed) or gate (shared)
+    uint32_t* small_id = (uint32_t*)(roww + 2 * kUmmaMaxN);          // the same of a small tile: [2][64], tiles in turn
+    float* small_w = (float*)(small_id + 2 * kSmallN);
+    uint32_t* tmem_slot = (uint32_t*)(small_w + 2 * kSmallN);
     __shared__ uint32_t s_failed;
 
     if (tid == 0) {
-        for (uint32_t s = 0; s < kMaxAStages; ++s) { mbar_init(&a_full[s], kConvWarps); mbar_init(&a_empty[s], 1); }
-        for (uint32_t s = 0; s < kBStages; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
-        for (uint32_t s = 0; s < kPkSlots; ++s) { mbar_init(&pk_full[s], 1); mbar_init(&pk_empty[s], kConvWarps); }
+        for (uint32_t s = 0; s < kWideA; ++s) { mbar_init(&a_full[s], kConvWarps); mbar_init(&a_empty[s], 2); }
+        for (uint32_t s = 0; s < kWideB; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 2); }
+        for (uint32_t s = 0; s < kWidePk; ++s) { mbar_init(&pk_full[s], 1); mbar_init(&pk_empty[s], kConvWarps); }
         mbar_init(sc_full, 1);
         mbar_init(sc_empty, kConvWarps);
-        mbar_init(accum, 1);
+        mbar_init(wide_over, 2);
+        for (uint32_t s = 0; s < kNarrowA; ++s) { mbar_init(&na_full[s], kConvWarps); mbar_init(&na_empty[s], 2); }
+        for (uint32_t s = 0; s < kNarrowB; ++s) { mbar_init(&nb_full[s], 1); mbar_init(&nb_empty[s], 2); }
+        for (uint32_t s = 0; s < kNarrowPk; ++s) { mbar_init(&npk_full[s], 1); mbar_init(&npk_empty[s], kConvWarps); }
+        for (uint32_t s = 0; s < kNarrowSc; ++s) { mbar_init(&nsc_full[s], 1); mbar_init(&nsc_empty[s], kConvWarps); }
+        for (uint32_t s = 0; s < 2; ++s) mbar_init(&epi_done[s], kConvWarps);
+        for (uint32_t s = 0; s < kTiles; ++s) { mbar_init(&accum[s], 2); mbar_init(&tile_full[s], 1); mbar_init(&tile_empty[s], kConvWarps + 3 + kEpiWarps); }
         mbar_init(conv, kConvWarps);
-        for (uint32_t s = 0; s < 2; ++s) { mbar_init(&next_full[s], 1); mbar_init(&next_empty[s], kConvWarps + 2); }
+        mbar_init(eids_full, kEpiWarps);
         fence_mbar_init();
         s_failed = 0;
     }
@@ -318,43 +401,127 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();   // all of the above runs while the last kernel ends
-    const uint32_t n_tiles = n_inst[0] * row_tiles;
     auto give_up = [&]() {
         report_status(a.status, kStatusWaitTimeout);
         *(volatile uint32_t*)&s_failed = 1;
     };
     auto failed = [&]() { return *(volatile uint32_t*)&s_failed != 0; };
-    // Every barrier's use is counted in one bit per stage, kept by each role for itself: full barriers are waited for
-    // with the bit, empty ones with its complement (the first use of a stage finds it empty).
-    // The tile after `turn` others; n_tiles and above: none.
-    auto take_tile = [&](uint32_t turn) -> uint32_t {
-        const uint32_t s = turn & 1;
-        if (!__all_sync(0xffffffffu, pipe_wait(&next_full[s], (turn >> 1) & 1))) { give_up(); return 0xffffffffu; }
-        const uint32_t t = *(volatile uint32_t*)&next_tile[s];
+    auto pipe_wait = [&](uint64_t* bar, uint32_t parity) { return pipe_wait_or(bar, parity, &s_failed); };
+    // Tile number n of this block (all lanes); false: there is none.
+    auto release_tile = [&](uint32_t n) {
         __syncwarp();
-        if (lane == 0) mbar_arrive(&next_empty[s]);
-        return __shfl_sync(0xffffffffu, t, 0);
+        if (lane == 0) mbar_arrive(&tile_empty[n % kTiles]);
     };
-    struct Work {
-        ChunkInstance in;
-        bool shared;
-        uint32_t F, KB, out_rows, r0;
+    auto take_tile = [&](uint32_t n, Tile& t, bool release = true) {
+        const uint32_t s = n % kTiles;
+        if (!__all_sync(0xffffffffu, pipe_wait(&tile_full[s], (n / kTiles) & 1))) { give_up(); return false; }
+        const uint4 v = next_tile[s];
+        if (release) release_tile(n);
+        t = Tile(make_uint4(__shfl_sync(0xffffffffu, v.x, 0), __shfl_sync(0xffffffffu, v.y, 0), __shfl_sync(0xffffffffu, v.z, 0),
+                            __shfl_sync(0xffffffffu, v.w, 0)));
+        return t.count != 0 && !failed();
     };
-    auto open_tile = [&](uint32_t t, Work& w) {   // false: no such rows (a narrower shared or routed expert)
-        const uint32_t ii = t / row_tiles;
-        const uint4 v = __ldg((const uint4*)(inst + ii));
-        w.in.kind = v.x; w.in.slot = v.y; w.in.first = v.z; w.in.count = v.w;
-        w.shared = w.in.kind == 1;
-        w.F = w.shared ? a.f_shared : a.f;
-        w.KB = (PHASE == 0 ? a.d : w.F) / 64;
-        w.out_rows = PHASE == 0 ? w.F : a.d;       // rows of the weight matrix
-        w.r0 = (t - ii * row_tiles) * (PHASE == 0 ? 128u : 256u);
-        return w.r0 < w.out_rows;
+    auto k_blocks = [&](const Tile& t) { return (PHASE == 0 ? a.d : t.shared ? a.f_shared : a.f) / 64; };
+    // Epilogue of tile `e`, the block's n-th, by H x 4 warps: warp w reads TMEM lanes 32*(w & 3) .. +31, every H-th group of C columns
+    // from the h-th on; accumulators at columns acc0 and acc1, the columns' tokens and weights at `ids` and `wts`.
+    auto epilogue = [&](auto width, auto share, uint32_t h, const Tile& e, uint32_t n, uint32_t acc0, uint32_t acc1, const uint32_t* ids, const float* wts) {
+        constexpr int C = decltype(width)::value, H = decltype(share)::value;
+        if (!pipe_wait(&accum[n % kTiles], (n / kTiles) & 1)) give_up();
+        if (failed()) return false;
+        __syncwarp();
+        tc_fence_after();
+        const Offsets3& off = e.shared ? a.shared : a.routed;
+        const uint8_t* base = e.shared ? a.shared_block : pool_cell_base(a.pool, e.slot);
+        const uint32_t F = e.shared ? a.f_shared : a.f, N = (e.count + 15u) & ~15u;
+        // (loops that are not unrolled further: the code runs once per tile, and fetching it takes longer than what
+        // unrolling saves)
+        const uint32_t q = warp & 3;
+        const uint32_t trow = q * 32 + lane;                       // row inside each 128-row tile
+        const uint32_t taddr = tmem_base + ((q * 32) << 16);
+        constexpr uint32_t kColStep = C * H;
+        if (PHASE == 0) {
+            const uint32_t f = e.r0 + trow;
+            float gab = 0.f, uab = 0.f;
+            if (a.expert_bias && f < F) {
+                gab = bf16_bits_to_f32(((const uint16_t*)(base + off.ab[0]))[f]);
+                uab = bf16_bits_to_f32(((const uint16_t*)(base + off.ab[1]))[f]);
+            }
+            uint16_t* const dst = (e.shared ? a.acts_shared : a.acts) + (size_t)e.first * F + perm_index(f, BITS == 4);
+            auto columns = [&](auto glu_of) {
+                bool over = false;
+#pragma unroll 1
+                for (uint32_t c0 = h * C; c0 < N; c0 += kColStep) {
+                    uint32_t g[C], u[C];
+                    tmem_ld_issue<C>(taddr + acc0 + c0, g);
+                    tmem_ld_issue<C>(taddr + acc1 + c0, u);
+                    tmem_ld_wait();
+                    uint16_t* p = dst + (size_t)c0 * F;
+                    const uint32_t live = f < F ? min((uint32_t)C, e.count > c0 ? e.count - c0 : 0u) : 0u;   // rows of this group
+#pragma unroll
+                    for (int j = 0; j < C; j += 2) {
+                        float v[2];
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            v[k] = glu_of(__uint_as_float(g[j + k]) + gab, __uint_as_float(u[j + k]) + uab);
+                            if (fabsf(v[k]) > kHalfMax) {   // false for NaN, which passes through
+                                over |= (uint32_t)(j + k) < live;
+                                v[k] = copysignf(kHalfMax, v[k]);
+                            }
+                        }
+                        const __half2 hv = __floats2half2_rn(v[0], v[1]);
+                        if ((uint32_t)j < live) *p = __half_as_ushort(__low2half(hv));
+                        p += F;
+                        if ((uint32_t)j + 1 < live) *p = __half_as_ushort(__high2half(hv));
+                        p += F;
+                    }
+                }
+                if (over) report_status(a.status, kStatusOperandRange);
+            };
+            if (a.activation == SHRIKE_ACT_CLAMPED_SWIGLU) columns([](float x, float y) { return glu_epilogue(x, y, SHRIKE_ACT_CLAMPED_SWIGLU); });
+            else if (a.activation == SHRIKE_ACT_GELU_TANH) columns([](float x, float y) { return glu_epilogue(x, y, SHRIKE_ACT_GELU_TANH); });
+            else columns([](float x, float y) { return glu_epilogue(x, y, SHRIKE_ACT_SILU); });
+        } else {
+            const uint32_t d0 = e.r0 + trow, d1 = d0 + 128;
+            float ab0 = 0.f, ab1 = 0.f;
+            if (a.expert_bias) {
+                const uint16_t* dab = (const uint16_t*)(base + off.ab[2]);
+                if (d0 < a.d) ab0 = bf16_bits_to_f32(dab[d0]);
+                if (d1 < a.d) ab1 = bf16_bits_to_f32(dab[d1]);
+            }
+            const bool ok0 = d0 < a.d, ok1 = d1 < a.d;
+#pragma unroll 1
+            for (uint32_t c0 = h * C; c0 < N; c0 += kColStep) {
+                uint32_t v0[C], v1[C];
+                tmem_ld_issue<C>(taddr + acc0 + c0, v0);
+                tmem_ld_issue<C>(taddr + acc1 + c0, v1);
+                tmem_ld_wait();
+                const uint32_t live = min((uint32_t)C, e.count > c0 ? e.count - c0 : 0u);
+#pragma unroll
+                for (int j = 0; j < C; ++j) {
+                    if ((uint32_t)j < live) {
+                        // lanes hold consecutive output rows: one 128-byte reduction per warp and column
+                        float* o = a.yacc + (size_t)ids[c0 + j] * a.d + d0;
+                        const float w = wts[c0 + j];
+                        if (ok0) atomicAdd(o, w * (__uint_as_float(v0[j]) + ab0));
+                        if (ok1) atomicAdd(o + 128, w * (__uint_as_float(v1[j]) + ab1));
+                    }
+                }
+            }
+        }
+        tc_fence_before();   // these reads of the accumulators come before the instructions that write them next
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&epi_done[n & 1], kConvWarps / (4 * H));
+        return true;
     };
+    // Barriers' parities: a stage's use n (counted by each role for itself) is waited for with n & 1 at its full barrier, and with the
+    // complement at the empty one. Accumulators and ids: by the number of the tile.
 
     if (warp < kConvWarps) {
-        // ---------------- converters, then the tile's epilogue ----------------
-        uint32_t a_use = 0, pk_use = 0, sc_use = 0, slot = 0, acc_use = 0, conv_use = 0, odd = 0;
+        // ---------------- converters, and the tiles' epilogues ----------------
+        // A lane is a row: the TMEM lanes that a warp reaches. half: of a K block (wide), or which K blocks (narrow).
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConvRegs));
+        const uint32_t tile = (warp >> 2) & 1, r = (warp & 3) * 32 + lane, half = warp >> 3;
+        uint32_t conv_use = 0;
         auto converters_meet = [&]() {
             __syncwarp();
             if (lane == 0) mbar_arrive(conv);
@@ -363,429 +530,666 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             if (!ok) give_up();
             return ok;
         };
-        // Two threads per weight row: thread `half` converts 32 of the K block's 64 weights. A lane is a row: the TMEM lanes
-        // that a warp reaches.
-        const uint32_t tile = (warp >> 2) & 1, r = (warp & 3) * 32 + lane, half = warp >> 3;
-        const uint32_t a_tmem = tmem_base + 256u + (((warp & 3) * 32) << 16) + tile * 32 + half * 16;
-        constexpr uint32_t kWordsPerThread = kWordsPerBlock / 2;   // 4 (int4) or 8 (int8)
-        const uint32_t pk_row = kOffPk + tile * (kPkSlotBytes / 2) + r * 64, pk_xor = (r >> 1) & 3;
-        // What does not change along K: this thread's chunk positions in a packed slot and in the converted
-        // tile (both swizzled by the row).
-        uint32_t pk_off[kKbPerPk * (kWordsPerThread / 4)];
-#pragma unroll
-        for (uint32_t sub = 0; sub < kKbPerPk; ++sub)
-#pragma unroll
-            for (uint32_t q = 0; q < kWordsPerThread / 4; ++q) {
-                // 16-byte chunk of the 64-byte row: the K block's share, then this thread's half of it
-                const uint32_t c = sub * (kRowBlockBytes / 16) + half * (kWordsPerThread / 4) + q;
-                pk_off[sub * (kWordsPerThread / 4) + q] = pk_row + ((c ^ pk_xor) << 4);
-            }
-        uint32_t a_pos[4];
-#pragma unroll
-        for (uint32_t i = 0; i < 4; ++i)   // A row r: 8 chunks of 8 fp16; chunk c lives at position c ^ (r & 7)
-            a_pos[i] = tile * kTileBytes + r * 128 + (((half * 4 + i) ^ (r & 7)) << 4);
-
-        bool wide = false;   // the last tile's accumulators took all of TMEM
-        for (uint32_t turn = 0;; ++turn) {
-            const uint32_t t = take_tile(turn);
-            if (t >= n_tiles || failed()) break;
-            Work wk;
-            if (!open_tile(t, wk)) continue;
-            const ChunkInstance& in = wk.in;
-            const bool shared = wk.shared;
-            const uint32_t F = wk.F, KB = wk.KB, out_rows = wk.out_rows, r0 = wk.r0, G = KB * 64 / GROUP;
-            const TileShape ts(in.count);
-            const Offsets3& off = shared ? a.shared : a.routed;
-            const uint8_t* base = shared ? a.shared_block : pool_cell_base(a.pool, in.slot);
-            uint32_t* const ids = rowid + odd * kUmmaMaxN;
-            float* const wts = roww + odd * kUmmaMaxN;
-            odd ^= 1;
-            // the tokens and route weights of the columns: the epilogue reads them, long after these loads
-            if (PHASE == 1 && tid < kUmmaMaxN) {
-                const uint32_t src = tid < in.count ? tid : 0;
-                if (shared) {
-                    ids[tid] = in.first + src;
-                    wts[tid] = a.shared_gate ? a.shared_gate[in.first + src] : 1.0f;
-                } else {
-                    const uint32_t pair = a.sorted[in.first + src];
-                    ids[tid] = pair / a.top_k;
-                    wts[tid] = a.route_w[pair];
-                }
-            }
-            uint32_t sreg[4] = {0, 0, 0, 0}, breg[4] = {0, 0, 0, 0};
-            uint32_t snext[4] = {0, 0, 0, 0}, bnext[4] = {0, 0, 0, 0};
-            const uint32_t mrow = r0 + (PHASE == 0 ? r : tile * 128 + r);
+        // ---- of the tile at hand ----
+        Tile t;
+        uint32_t KB, G, out_rows, mrow, my_rows;
+        const uint16_t *s_all, *b_all;      // its matrix's scales and biases
+        uint32_t sreg[4] = {0, 0, 0, 0}, breg[4] = {0, 0, 0, 0}, snext[4] = {0, 0, 0, 0}, bnext[4] = {0, 0, 0, 0};
+        uint32_t col_pair = 0;              // the pair (shared: row) behind this thread's column, and its weight
+        float col_w = 0.f;
+        auto open_tile = [&]() {
+            const uint32_t F = t.shared ? a.f_shared : a.f;
+            KB = k_blocks(t);
+            G = KB * 64 / GROUP;
+            out_rows = PHASE == 0 ? F : a.d;       // rows of the weight matrix
+            mrow = t.r0 + (PHASE == 0 ? r : tile * 128 + r);
+            my_rows = t.r0 + (PHASE == 0 ? 0u : tile * 128u) + (warp & 3) * 32 + (lane >> 2);
             const int mat = PHASE == 0 ? (int)tile : 2;
-            const uint16_t* srow = (const uint16_t*)(base + off.s[mat]) + (size_t)mrow * G;
-            const uint16_t* brow = (const uint16_t*)(base + off.b[mat]) + (size_t)mrow * G;
-            // Groups 8*blk .. 8*blk+7 straight from global memory (rows past the matrix and groups past the row read as
-            // zero: the converted weights are then zero). An even number of groups: the warp's 32 rows in 32-bit words, four
-            // lanes a row, handed to the rows' lanes when they are needed; read by each row's threads in 16-bit pieces
-            // they kept L1 busy for 1.3 us per K block of 90-group rows.
-            const bool words = (G & 1u) == 0;
-            const uint32_t my_rows = r0 + (PHASE == 0 ? 0u : tile * 128u) + (warp & 3) * 32 + (lane >> 2);
-            auto fetch_scales = [&](uint32_t blk) {
-                if (words) {
-                    const uint32_t gi = blk * 8 + 2 * (lane & 3);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const uint32_t row = my_rows + 8 * i;
-                        const bool there = row < out_rows && gi < G;
-                        const size_t at = (size_t)row * G + gi;
-                        snext[i] = there ? __ldg((const uint32_t*)((const uint16_t*)(base + off.s[mat]) + at)) : 0u;
-                        bnext[i] = there ? __ldg((const uint32_t*)((const uint16_t*)(base + off.b[mat]) + at)) : 0u;
-                    }
-                    return;
+            const Offsets3& off = t.shared ? a.shared : a.routed;
+            const uint8_t* base = t.shared ? a.shared_block : pool_cell_base(a.pool, t.slot);
+            s_all = (const uint16_t*)(base + off.s[mat]);
+            b_all = (const uint16_t*)(base + off.b[mat]);
+            if (PHASE == 1 && t.count > kSmallN && tid < t.count) col_pair = t.shared ? t.first + tid : a.sorted[t.first + tid];
+        };
+        // The columns' tokens and route weights, for the epilogue: asked for when the tile begins (its weight once the pair is
+        // there), stored when its weights are converted -- a store at the start waits for two trips to L2.
+        auto ask_weight = [&]() {
+            if (PHASE == 1 && tid < t.count) col_w = t.shared ? (a.shared_gate ? a.shared_gate[col_pair] : 1.0f) : a.route_w[col_pair];
+        };
+        auto own_epilogue = [&](auto width, uint32_t n, uint32_t acc1) {
+            const uint32_t at = (n & 1) * kUmmaMaxN;
+            if (PHASE == 1) {
+                if (tid < t.count) {
+                    rowid[at + tid] = t.shared ? col_pair : col_pair / a.top_k;
+                    roww[at + tid] = col_w;
                 }
+                if (!converters_meet()) return false;
+            }
+            return epilogue(width, std::integral_constant<int, 4>(), warp >> 2, t, n, 0u, acc1, rowid + at, roww + at);
+        };
+        // Groups 8*blk .. 8*blk+7 straight from global memory (rows past the matrix and groups past the row read as
+        // zero: the converted weights are then zero). An even number of groups: the warp's 32 rows in 32-bit words, four
+        // lanes a row, handed to the rows' lanes when they are needed; read by each row's threads in 16-bit pieces
+        // they kept L1 busy for 1.3 us per K block of 90-group rows.
+        auto fetch_scales = [&](uint32_t blk) {
+            if ((G & 1u) == 0) {
+                const uint32_t gi = blk * 8 + 2 * (lane & 3);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const uint32_t gi = blk * 8 + 2 * i;
-                    uint32_t sv = 0, bv = 0;
-                    if (mrow < out_rows && gi < G) {
-                        sv = __ldg(srow + gi);
-                        bv = __ldg(brow + gi);
-                        if (gi + 1 < G) {
-                            sv |= (uint32_t)__ldg(srow + gi + 1) << 16;
-                            bv |= (uint32_t)__ldg(brow + gi + 1) << 16;
-                        }
-                    }
-                    snext[i] = sv;
-                    bnext[i] = bv;
+                    const uint32_t row = my_rows + 8 * i;
+                    const bool there = row < out_rows && gi < G;
+                    const size_t at = (size_t)row * G + gi;
+                    snext[i] = there ? __ldg((const uint32_t*)(s_all + at)) : 0u;
+                    bnext[i] = there ? __ldg((const uint32_t*)(b_all + at)) : 0u;
                 }
-            };
-            if (!sc_tma) fetch_scales(0);
-            // A scale block (8 groups of the row) at a time, its K blocks unrolled: the position in the packed slot
-            // and the group of a K block are then constants of the instruction stream.
-            // (a warp may write the stages while others still read the columns that they take of the last accumulators)
-            if (wide && ts.in_tmem && !converters_meet()) break;
-            wide = !ts.in_tmem;
-            uint32_t st = 0;
-            for (uint32_t kb0 = 0; kb0 < KB; kb0 += kKbPerSc) {
-                if (failed()) break;
-                if (sc_tma) {
-                    if (!pipe_wait(sc_full, sc_use)) { give_up(); break; }
-                    sc_use ^= 1;
-                    const uint4 sv = *(const uint4*)(smem + kOffSc + tile * (kScHalfBytes / 2) + r * 16);
-                    const uint4 bv = *(const uint4*)(smem + kOffSc + kScHalfBytes + tile * (kScHalfBytes / 2) + r * 16);
+                return;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t gi = blk * 8 + 2 * i;
+                const size_t at = (size_t)mrow * G + gi;
+                uint32_t sv = 0, bv = 0;
+                if (mrow < out_rows && gi < G) {
+                    sv = __ldg(s_all + at);
+                    bv = __ldg(b_all + at);
+                    if (gi + 1 < G) {
+                        sv |= (uint32_t)__ldg(s_all + at + 1) << 16;
+                        bv |= (uint32_t)__ldg(b_all + at + 1) << 16;
+                    }
+                }
+                snext[i] = sv;
+                bnext[i] = bv;
+            }
+        };
+        // The eight groups fetched one block ago into sreg / breg, and the next ones asked for.
+        auto turn_scales = [&](uint32_t blk) {
+            if ((G & 1u) == 0) {
+                __syncwarp();   // the last block's have been read
+                if constexpr (GROUP == 32) {
+                    // through shared memory: a thread's half has the even or the odd groups, so the two warps of a row write 16
+                    // bits of every word each
+                    uint8_t* const to = smem + kWideOffSc + (tile * 128 + (warp & 3) * 32 + (lane >> 2)) * 16 + (lane & 3) * 4 + half * 2;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        *(uint16_t*)(to + i * 128) = (uint16_t)(half ? snext[i] >> 16 : snext[i]);
+                        *(uint16_t*)(to + kWideScBytes / 2 + i * 128) = (uint16_t)(half ? bnext[i] >> 16 : bnext[i]);
+                    }
+                    __syncwarp();
+                    const uint8_t* const from = smem + kWideOffSc + (tile * 128 + r) * 16;
+                    const uint4 sv = *(const uint4*)from, bv = *(const uint4*)(from + kWideScBytes / 2);
                     sreg[0] = sv.x; sreg[1] = sv.y; sreg[2] = sv.z; sreg[3] = sv.w;
                     breg[0] = bv.x; breg[1] = bv.y; breg[2] = bv.z; breg[3] = bv.w;
-                    // the values are in registers: the copy thread may fetch the next block's
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(sc_empty);
                 } else {
-                    // this block's 8 groups were fetched one block ago; fetch the next block's now
-                    if (words) {
-                        __syncwarp();   // the last block's have been read
-                        if constexpr (GROUP == 32) {
-                            // through the scales' memory: a thread's half has the even or the odd groups, so the two warps
-                            // of a row write 16 bits of every word each
-                            uint8_t* const to = smem + kOffSc + (tile * 128 + (warp & 3) * 32 + (lane >> 2)) * 16 + (lane & 3) * 4 + half * 2;
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                *(uint16_t*)(to + i * 128) = (uint16_t)(half ? snext[i] >> 16 : snext[i]);
-                                *(uint16_t*)(to + kScHalfBytes + i * 128) = (uint16_t)(half ? bnext[i] >> 16 : bnext[i]);
-                            }
-                            __syncwarp();
-                            const uint4 sv = *(const uint4*)(smem + kOffSc + (tile * 128 + r) * 16), bv = *(const uint4*)(smem + kOffSc + kScHalfBytes + (tile * 128 + r) * 16);
-                            sreg[0] = sv.x; sreg[1] = sv.y; sreg[2] = sv.z; sreg[3] = sv.w;
-                            breg[0] = bv.x; breg[1] = bv.y; breg[2] = bv.z; breg[3] = bv.w;
-                        } else {
+                    for (int i = 0; i < 4; ++i) {   // lane 4 (row mod 8) + word of load row / 8
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) {   // lane 4 (row mod 8) + word of load row / 8
-#pragma unroll
-                                for (int w = 0; w < 4; ++w) {
-                                    const uint32_t sv = __shfl_sync(0xffffffffu, snext[i], 4 * (lane & 7) + w);
-                                    const uint32_t bv = __shfl_sync(0xffffffffu, bnext[i], 4 * (lane & 7) + w);
-                                    if ((lane >> 3) == (uint32_t)i) { sreg[w] = sv; breg[w] = bv; }
-                                }
-                            }
+                        for (int w = 0; w < 4; ++w) {
+                            const uint32_t sv = __shfl_sync(0xffffffffu, snext[i], 4 * (lane & 7) + w);
+                            const uint32_t bv = __shfl_sync(0xffffffffu, bnext[i], 4 * (lane & 7) + w);
+                            if ((lane >> 3) == (uint32_t)i) { sreg[w] = sv; breg[w] = bv; }
                         }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) { sreg[i] = snext[i]; breg[i] = bnext[i]; }
                     }
-                    fetch_scales(kb0 / kKbPerSc + 1);
                 }
+            } else {
 #pragma unroll
-                for (uint32_t j = 0; j < kKbPerSc; ++j) {
-                    const uint32_t kb = kb0 + j;
-                    if (kb >= KB) break;
-                    constexpr uint32_t kSubMask = kKbPerPk - 1;
-                    const uint32_t sub = j & kSubMask;         // K block within its packed slot
-                    if (sub == 0 && !pipe_wait(&pk_full[slot], (pk_use >> slot) & 1)) { give_up(); break; }
-                    uint32_t pk[kWordsPerThread];
+                for (int i = 0; i < 4; ++i) { sreg[i] = snext[i]; breg[i] = bnext[i]; }
+            }
+            fetch_scales(blk + 1);
+        };
+        // Narrow tiles of 32-wide groups: a thread multiplies with every second word of its row only, so the same registers
+        // hold two blocks, asked for that much earlier (one block is 2200 cycles, and the loads take longer): lane / 2 is the row.
+        uint32_t own_at[2] = {0, 0};
+        bool own_there[2] = {false, false};
+        auto fetch_own = [&](uint32_t blk, uint32_t* sv, uint32_t* bv) {
+            const uint32_t g0 = blk * 8;
+            const bool inside = g0 + 2 * (2 * (lane & 1) + half) < G;
 #pragma unroll
-                    for (uint32_t q = 0; q < kWordsPerThread / 4; ++q) {
-                        const uint4 v = *(const uint4*)(smem + slot * kPkSlotBytes + pk_off[sub * (kWordsPerThread / 4) + q]);
-                        pk[4 * q] = v.x; pk[4 * q + 1] = v.y; pk[4 * q + 2] = v.z; pk[4 * q + 3] = v.w;
+            for (int i = 0; i < 2; ++i) {
+                const bool there = inside && own_there[i];
+                sv[i] = there ? __ldg((const uint32_t*)(s_all + (own_at[i] + g0))) : 0u;
+                bv[i] = there ? __ldg((const uint32_t*)(b_all + (own_at[i] + g0))) : 0u;
+            }
+        };
+        auto first_scales = [&]() {
+            if (GROUP == 32 && (G & 1u) == 0) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t row = my_rows - (lane >> 2) + (lane >> 1) + 16 * i;
+                    own_there[i] = row < out_rows;
+                    own_at[i] = row * G + 2 * (2 * (lane & 1) + half);
+                }
+                fetch_own(0, snext, bnext);
+                fetch_own(1, snext + 2, bnext + 2);
+            } else {
+                fetch_scales(0);
+            }
+        };
+        // Block blk's scales into sreg / breg: 32-wide groups this thread's two words, else all four.
+        auto narrow_scales = [&](uint32_t blk) {
+            if (GROUP == 32 && (G & 1u) == 0) {
+                uint8_t* const at = smem + kWideOffSc + (tile * 128 + (warp & 3) * 32) * 16 + half * 4;
+                auto exchange = [&](uint32_t* sv, uint32_t* bv) {
+                    __syncwarp();   // the last block's have been read
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        uint8_t* const to = at + ((lane >> 1) + 16 * i) * 16 + (lane & 1) * 8;
+                        *(uint32_t*)to = sv[i];
+                        *(uint32_t*)(to + kWideScBytes / 2) = bv[i];
                     }
-                    // a thread's half of a 64-wide block lies inside one group of 32 or 64
-                    const uint32_t gsel = j * kGroupsPerBlock + (GROUP == 64 ? 0u : half);
-                    const float sc = meta_to_f32<META>(pick16(sreg, gsel));
-                    const float zf = fmaf(kZero, sc, meta_to_f32<META>(pick16(breg, gsel)));
-                    const uint32_t s2 = half2_dup(sc), z2 = half2_dup(zf);
-                    if (!pipe_wait(&a_empty[st], ((a_use >> st) & 1) ^ 1)) { give_up(); break; }
-                    a_use ^= 1u << st;
-                    uint32_t o[16];   // 32 weights
+                    fetch_own(blk + 2, sv, bv);
+                };
+                if (blk & 1) exchange(snext + 2, bnext + 2);
+                else exchange(snext, bnext);
+                __syncwarp();
 #pragma unroll
-                    for (uint32_t i = 0; i < kWordsPerThread; ++i) {
-                        uint32_t w4[4];
-                        dequant_word<BITS>(pk[i], s2, z2, w4);
+                for (int i = 0; i < 2; ++i) {
+                    sreg[i] = *(const uint32_t*)(at + lane * 16 + i * 8);
+                    breg[i] = *(const uint32_t*)(at + kWideScBytes / 2 + lane * 16 + i * 8);
+                }
+                return;
+            }
+            turn_scales(blk);
+            if (GROUP == 32) {   // (turn_scales left all words)
 #pragma unroll
-                        for (uint32_t e = 0; e < 16 / kWordsPerThread; ++e) o[i * (16 / kWordsPerThread) + e] = w4[e];
-                    }
-                    if (ts.in_tmem) {
+                for (int i = 0; i < 2; ++i) {
+                    sreg[i] = half ? sreg[2 * i + 1] : sreg[2 * i];
+                    breg[i] = half ? breg[2 * i + 1] : breg[2 * i];
+                }
+            }
+        };
+        auto scale_words = [&](uint32_t s16, uint32_t b16, uint32_t& s2, uint32_t& z2) {
+            const float sc = meta_to_f32<META>((uint16_t)s16);
+            s2 = half2_dup(sc);
+            z2 = half2_dup(fmaf(kZero, sc, meta_to_f32<META>((uint16_t)b16)));
+        };
+
+        uint32_t n = 0;
+        bool go = take_tile(0, t), was_wide = false;
+        // ---- wide tiles ----
+        {
+            uint32_t a_use = 0, pk_use = 0, sc_use = 0, slot = 0, st = 0;
+            constexpr uint32_t kWordsPerThread = kWordsPerBlock / 2;   // 4 (int4) or 8 (int8)
+            const uint32_t pk_row = kWideOffPk + tile * (kWidePkBytes / 2) + r * 64, pk_xor = (r >> 1) & 3;
+            // What does not change along K: this thread's chunk positions in a packed slot and in the converted
+            // tile (both swizzled by the row).
+            uint32_t pk_off[kWideKbPerPk * (kWordsPerThread / 4)];
+#pragma unroll
+            for (uint32_t sub = 0; sub < kWideKbPerPk; ++sub)
+#pragma unroll
+                for (uint32_t q = 0; q < kWordsPerThread / 4; ++q) {
+                    // 16-byte chunk of the 64-byte row: the K block's share, then this thread's half of it
+                    const uint32_t c = sub * (kRowBlockBytes / 16) + half * (kWordsPerThread / 4) + q;
+                    pk_off[sub * (kWordsPerThread / 4) + q] = pk_row + ((c ^ pk_xor) << 4);
+                }
+            uint32_t a_pos[4];
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i)   // A row r: 8 chunks of 8 fp16; chunk c lives at position c ^ (r & 7)
+                a_pos[i] = tile * kTileBytes + r * 128 + (((half * 4 + i) ^ (r & 7)) << 4);
+            for (; go && !t.narrow; go = take_tile(++n, t)) {
+                was_wide = true;
+                open_tile();
+                if (!SCT) fetch_scales(0);
+                // A scale block (8 groups of the row) at a time, its K blocks unrolled: the position in the packed slot
+                // and the group of a K block are then constants of the instruction stream.
+                for (uint32_t kb0 = 0; kb0 < KB; kb0 += kKbPerSc) {
+                    if (failed()) break;
+                    if (SCT) {
+                        if (!pipe_wait(sc_full, sc_use)) { give_up(); break; }
+                        sc_use ^= 1;
+                        const uint8_t* const from = smem + kWideOffSc + (tile * 128 + r) * 16;
+                        const uint4 sv = *(const uint4*)from;
+                        const uint4 bv = *(const uint4*)(from + kWideScBytes / 2);
+                        sreg[0] = sv.x; sreg[1] = sv.y; sreg[2] = sv.z; sreg[3] = sv.w;
+                        breg[0] = bv.x; breg[1] = bv.y; breg[2] = bv.z; breg[3] = bv.w;
+                        // the values are in registers: the copy thread may fetch the next block's
                         __syncwarp();
-                        tc_fence_after();   // the stage's last readers are done
-                        tmem_st16(a_tmem + st * 64, o);
-                        tc_fence_before();
+                        if (lane == 0) mbar_arrive(sc_empty);
                     } else {
-                        uint8_t* a_stage = smem + ts.off_a + st * kAStageBytes;
+                        turn_scales(kb0 / kKbPerSc);
+                    }
+#pragma unroll
+                    for (uint32_t j = 0; j < kKbPerSc; ++j) {
+                        const uint32_t kb = kb0 + j;
+                        if (kb >= KB) break;
+                        constexpr uint32_t kSubMask = kWideKbPerPk - 1;
+                        const uint32_t sub = j & kSubMask;         // K block within its packed slot
+                        if (sub == 0 && !pipe_wait(&pk_full[slot], (pk_use >> slot) & 1)) { give_up(); break; }
+                        if (j == 2 && kb0 == 0) ask_weight();
+                        uint32_t pk[kWordsPerThread];
+#pragma unroll
+                        for (uint32_t q = 0; q < kWordsPerThread / 4; ++q) {
+                            const uint4 v = *(const uint4*)(smem + slot * kWidePkBytes + pk_off[sub * (kWordsPerThread / 4) + q]);
+                            pk[4 * q] = v.x; pk[4 * q + 1] = v.y; pk[4 * q + 2] = v.z; pk[4 * q + 3] = v.w;
+                        }
+                        // a thread's half of a 64-wide block lies inside one group of 32 or 64
+                        const uint32_t gsel = j * kGroupsPerBlock + (GROUP == 64 ? 0u : half);
+                        uint32_t s2, z2;
+                        scale_words(pick16(sreg, gsel), pick16(breg, gsel), s2, z2);
+                        if (!pipe_wait(&a_empty[st], ((a_use >> st) & 1) ^ 1)) { give_up(); break; }
+                        a_use ^= 1u << st;
+                        uint32_t o[16];   // 32 weights
+#pragma unroll
+                        for (uint32_t i = 0; i < kWordsPerThread; ++i) {
+                            uint32_t w4[4];
+                            dequant_word<BITS>(pk[i], s2, z2, w4);
+#pragma unroll
+                            for (uint32_t e = 0; e < 16 / kWordsPerThread; ++e) o[i * (16 / kWordsPerThread) + e] = w4[e];
+                        }
+                        uint8_t* a_stage = smem + kWideOffA + st * kWideABytes;
 #pragma unroll
                         for (uint32_t i = 0; i < 4; ++i)
                             *(uint4*)(a_stage + a_pos[i]) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
                         fence_async_smem();
-                    }
-                    __syncwarp();
-                    const bool slot_done = sub == kSubMask || kb + 1 == KB;
-                    if (lane == 0) {
-                        // one arrival per warp: 512 arrivals on one barrier word would serialise every K block
-                        mbar_arrive(&a_full[st]);
-                        // The ring slots are handed back only here: by now the values read from them have been
-                        // consumed, so the reads are complete before the copy thread may overwrite the slot.
-                        if (slot_done) mbar_arrive(&pk_empty[slot]);
-                    }
-                    if (slot_done) {
-                        pk_use ^= 1u << slot;
-                        if (++slot == kPkSlots) slot = 0;
-                    }
-                    if (++st == ts.a_stages) st = 0;
-                }
-            }
-            // ---------------- epilogue (warp w: TMEM lanes 32*(w & 3) .. +31, every fourth 16-column group) ----------------
-            bool ok = pipe_wait(accum, acc_use);
-            acc_use ^= 1;
-            if (!ok) give_up();
-            if (failed()) break;
-            tc_fence_after();
-            // the columns' tokens and weights were written by other converter threads at the start of the tile
-            if (PHASE == 1 && !converters_meet()) break;
-            // (eight columns at a time and loops that are not unrolled further: the code runs once per tile, and fetching
-            // it takes longer than what unrolling saves)
-            const uint32_t q = warp & 3, h = warp >> 2, N = ts.N;
-            const uint32_t trow = q * 32 + lane;                       // row inside each 128-row tile
-            const uint32_t taddr = tmem_base + ((q * 32) << 16);
-            constexpr uint32_t kColStep = 8 * (kConvWarps / 4);
-            if (PHASE == 0) {
-                const uint32_t f = r0 + trow;
-                float gab = 0.f, uab = 0.f;
-                if (a.expert_bias && f < F) {
-                    gab = bf16_bits_to_f32(((const uint16_t*)(base + off.ab[0]))[f]);
-                    uab = bf16_bits_to_f32(((const uint16_t*)(base + off.ab[1]))[f]);
-                }
-                uint16_t* const dst = (shared ? a.acts_shared : a.acts) + (size_t)in.first * F + perm_index(f, BITS == 4);
-                auto columns = [&](auto glu_of) {
-                    bool over = false;
-#pragma unroll 1
-                    for (uint32_t c0 = h * 8; c0 < N; c0 += kColStep) {
-                        uint32_t g[8], u[8];
-                        tmem_ld8_issue(taddr + c0, g);
-                        tmem_ld8_issue(taddr + ts.acc_step + c0, u);
-                        tmem_ld_wait();
-                        uint16_t* p = dst + (size_t)c0 * F;
-                        const uint32_t live = f < F ? min(8u, in.count > c0 ? in.count - c0 : 0u) : 0u;   // rows of this group
-#pragma unroll
-                        for (int j = 0; j < 8; j += 2) {
-                            float v[2];
-#pragma unroll
-                            for (int e = 0; e < 2; ++e) {
-                                v[e] = glu_of(__uint_as_float(g[j + e]) + gab, __uint_as_float(u[j + e]) + uab);
-                                if (fabsf(v[e]) > kHalfMax) {   // false for NaN, which passes through
-                                    over |= (uint32_t)(j + e) < live;
-                                    v[e] = copysignf(kHalfMax, v[e]);
-                                }
-                            }
-                            const __half2 hv = __floats2half2_rn(v[0], v[1]);
-                            if ((uint32_t)j < live) *p = __half_as_ushort(__low2half(hv));
-                            p += F;
-                            if ((uint32_t)j + 1 < live) *p = __half_as_ushort(__high2half(hv));
-                            p += F;
+                        __syncwarp();
+                        const bool slot_done = sub == kSubMask || kb + 1 == KB;
+                        if (lane == 0) {
+                            // one arrival per warp: 512 arrivals on one barrier word would serialise every K block
+                            mbar_arrive(&a_full[st]);
+                            // The ring slots are handed back only here: by now the values read from them have been
+                            // consumed, so the reads are complete before the copy thread may overwrite the slot.
+                            if (slot_done) mbar_arrive(&pk_empty[slot]);
                         }
-                    }
-                    if (over) report_status(a.status, kStatusOperandRange);
-                };
-                if (a.activation == SHRIKE_ACT_CLAMPED_SWIGLU) columns([](float x, float y) { return glu_epilogue(x, y, SHRIKE_ACT_CLAMPED_SWIGLU); });
-                else if (a.activation == SHRIKE_ACT_GELU_TANH) columns([](float x, float y) { return glu_epilogue(x, y, SHRIKE_ACT_GELU_TANH); });
-                else columns([](float x, float y) { return glu_epilogue(x, y, SHRIKE_ACT_SILU); });
-            } else {
-                const uint32_t d0 = r0 + trow, d1 = d0 + 128;
-                float ab0 = 0.f, ab1 = 0.f;
-                if (a.expert_bias) {
-                    const uint16_t* dab = (const uint16_t*)(base + off.ab[2]);
-                    if (d0 < a.d) ab0 = bf16_bits_to_f32(dab[d0]);
-                    if (d1 < a.d) ab1 = bf16_bits_to_f32(dab[d1]);
-                }
-                const bool ok0 = d0 < a.d, ok1 = d1 < a.d;
-#pragma unroll 1
-                for (uint32_t c0 = h * 8; c0 < N; c0 += kColStep) {
-                    uint32_t v0[8], v1[8];
-                    tmem_ld8_issue(taddr + c0, v0);
-                    tmem_ld8_issue(taddr + ts.acc_step + c0, v1);
-                    tmem_ld_wait();
-                    const uint32_t live = min(8u, in.count > c0 ? in.count - c0 : 0u);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        if ((uint32_t)j < live) {
-                            // lanes hold consecutive output rows: one 128-byte reduction per warp and column
-                            float* o = a.yacc + (size_t)ids[c0 + j] * a.d + d0;
-                            const float w = wts[c0 + j];
-                            if (ok0) atomicAdd(o, w * (__uint_as_float(v0[j]) + ab0));
-                            if (ok1) atomicAdd(o + 128, w * (__uint_as_float(v1[j]) + ab1));
+                        if (slot_done) {
+                            pk_use ^= 1u << slot;
+                            if (++slot == kWidePk) slot = 0;
                         }
+                        if (++st == kWideA) st = 0;
                     }
                 }
+                if (KB <= 2) ask_weight();
+                if (!own_epilogue(std::integral_constant<int, 8>(), n, kUmmaMaxN)) break;
             }
-            tc_fence_before();   // these reads of the accumulators come before the next tile's instructions
         }
-    } else if (warp == kConvWarps) {
-        // ---------------- MMA issue ----------------
+        // ---- narrow tiles ----
+        // (a warp may write weights and columns while others still read what they take of the last accumulators)
+        if (go && was_wide && !failed()) go = converters_meet();
+        {
+            uint32_t kc = 0, slot = 0, pk_par = 0, ss = 0, sc_par = 0, in_sc = 0;   // pairs of K blocks used before; slots
+            const uint32_t a_tmem = tmem_base + 256u + (((warp & 3) * 32) << 16) + half * 64 + tile * 32;
+            // 16-byte chunks of this thread's K block in its row of 128 packed bytes: the second of int4's two is 64 bytes on
+            constexpr uint32_t kChunks = kRowBlockBytes / 16;
+            uint32_t pk_off[kChunks];
+#pragma unroll
+            for (uint32_t q = 0; q < kChunks; ++q)
+                pk_off[q] = kNarrowOffPk + tile * (kNarrowPkBytes / 2) + r * 128 + (((half * kChunks + q) ^ (r & 7)) << 4);
+            uint32_t pk[kWordsPerBlock];
+            auto load_packed = [&](uint32_t i) {   // of K block i (+ half) in the slot
+#pragma unroll
+                for (uint32_t q = 0; q < kChunks; ++q) {
+                    const uint4 v = *(const uint4*)(smem + slot * kNarrowPkBytes + (pk_off[q] ^ (i * kRowBlockBytes)));
+                    pk[4 * q] = v.x; pk[4 * q + 1] = v.y; pk[4 * q + 2] = v.z; pk[4 * q + 3] = v.w;
+                }
+            };
+            // Eight groups' scales are kRawWords words for each of kSlotsPerSc slots.
+            constexpr uint32_t kRawWords = kNarrowKbPerPk * kGroupsPerBlock / 2, kSlotsPerSc = kKbPerSc / kNarrowKbPerPk, kOwn = kNarrowKbPerPk / 2;
+            const uint32_t sc_row = kNarrowOffSc + (tile * 128 + r) * 32;
+            // What the next slot's first own K block needs, asked for as soon as the slot is there.
+            uint32_t rs[kRawWords], rb[kRawWords];
+            auto open_slot = [&](uint32_t kb0) {
+                if (SCT) {
+                    const uint8_t* const from = smem + sc_row + ss * kNarrowScBytes + in_sc * (kRawWords * 4);
+                    load_words<kRawWords>(from, rs);
+                    load_words<kRawWords>(from + kNarrowScBytes / 2, rb);
+                }
+                if (kb0 + half < KB) load_packed(0);
+            };
+            for (; go; go = take_tile(++n, t)) {
+                open_tile();
+                uint32_t blk = 0, in_blk = 0;   // eight groups; slot of them
+                if (!SCT) first_scales();
+                if (SCT && !pipe_wait(&nsc_full[ss], sc_par)) { give_up(); break; }
+                if (!pipe_wait(&npk_full[slot], pk_par)) { give_up(); break; }
+                open_slot(0);
+                for (uint32_t kb0 = 0; kb0 < KB; kb0 += kNarrowKbPerPk) {
+                    const bool last = kb0 + kNarrowKbPerPk >= KB;
+                    // ---- the slot's scales and biases: own K block i's in sw[i], bw[i] (in the low bits, or both groups') ----
+                    uint32_t sw[kOwn], bw[kOwn];
+                    if constexpr (SCT) {
+#pragma unroll
+                        for (uint32_t i = 0; i < kOwn; ++i) {
+                            if constexpr (GROUP == 32) {
+                                sw[i] = half ? rs[2 * i + 1] : rs[2 * i];
+                                bw[i] = half ? rb[2 * i + 1] : rb[2 * i];
+                            } else {
+                                sw[i] = rs[i] >> (16 * half);
+                                bw[i] = rb[i] >> (16 * half);
+                            }
+                        }
+                    } else {
+                        if (in_blk == 0) narrow_scales(blk++);
+                        else {
+#pragma unroll
+                            for (uint32_t i = 0; i + kOwn < 4; ++i) { sreg[i] = sreg[i + kOwn]; breg[i] = breg[i + kOwn]; }
+                        }
+                        if (++in_blk == kSlotsPerSc) in_blk = 0;
+#pragma unroll
+                        for (uint32_t i = 0; i < kOwn; ++i) {
+                            sw[i] = GROUP == 32 ? sreg[i] : sreg[i] >> (16 * half);
+                            bw[i] = GROUP == 32 ? breg[i] : breg[i] >> (16 * half);
+                        }
+                    }
+                    const uint32_t slot1 = slot + 1 == kNarrowPk ? 0u : slot + 1, pk_par1 = slot1 ? pk_par : pk_par ^ 1;
+                    const bool there = pipe_test(&npk_full[slot1], pk_par1);   // (the answer takes its time: looked at below)
+                    // ---- its K blocks that are this set's ----
+#pragma unroll
+                    for (uint32_t i = 0; i < kOwn; ++i) {
+                        const uint32_t kb = kb0 + 2 * i + half;
+                        if (kb >= KB) break;
+                        const uint32_t c = kc + kb / 2, st = c % kNarrowA, par = ((c / kNarrowA) & 1) ^ 1;
+                        const bool free = pipe_test(&na_empty[st], par);
+                        uint32_t s2, z2;
+                        scale_words(sw[i] & 0xffffu, bw[i] & 0xffffu, s2, z2);
+#pragma unroll
+                        for (uint32_t h = 0; h < 2; ++h) {   // 32 weights, 16 columns at a time: half the registers
+                            if (GROUP == 32 && h) scale_words(sw[i] >> 16, bw[i] >> 16, s2, z2);
+                            uint32_t o[16];
+#pragma unroll
+                            for (uint32_t w = 0; w < kWordsPerBlock / 2; ++w) {
+                                uint32_t w4[4];
+                                dequant_word<BITS>(pk[h * (kWordsPerBlock / 2) + w], s2, z2, w4);
+#pragma unroll
+                                for (uint32_t e = 0; e < 32 / kWordsPerBlock; ++e) o[w * (32 / kWordsPerBlock) + e] = w4[e];
+                            }
+                            if (h == 0) {
+                                if (!free && !pipe_wait(&na_empty[st], par)) { give_up(); break; }
+                                __syncwarp();
+                                tc_fence_after();   // the stage's last readers are done
+                            }
+                            tmem_st16(a_tmem + st * 128 + h * 16, o);
+                        }
+                        if (i + 1 < kOwn && kb + 2 < KB) load_packed(2 * (i + 1));
+                        tmem_st_wait();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&na_full[st]);
+                    }
+                    // handed back only here: the values read from them have been consumed
+                    const bool sc_done = SCT && (++in_sc == 2 * kSlotsPerSc || last);
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&npk_empty[slot]);
+                        if (sc_done) mbar_arrive(&nsc_empty[ss]);
+                    }
+                    if (sc_done) {
+                        in_sc = 0;
+                        if (++ss == kNarrowSc) { ss = 0; sc_par ^= 1; }
+                    }
+                    slot = slot1;
+                    pk_par = pk_par1;
+                    if (!last) {
+                        if (sc_done && !pipe_wait(&nsc_full[ss], sc_par)) { give_up(); break; }
+                        if (!there && !pipe_wait(&npk_full[slot], pk_par)) { give_up(); break; }
+                        open_slot(kb0 + kNarrowKbPerPk);
+                    }
+                    if (kb0 == 0 && t.count > kSmallN) ask_weight();
+                }
+                if (failed()) break;
+                if (half && (KB & 1)) {   // the last pair has no second K block
+                    const uint32_t c = kc + KB / 2;
+                    if (!pipe_wait(&na_empty[c % kNarrowA], ((c / kNarrowA) & 1) ^ 1)) { give_up(); break; }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&na_full[c % kNarrowA]);
+                }
+                kc += (KB + 1) / 2;
+                if (t.count > kSmallN && !own_epilogue(std::integral_constant<int, 4>(), n, 128u)) break;
+            }
+        }
+    } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+    if (warp < kConvWarps + 2) {
+        // ---------------- MMA issue, a warp for each of the two weight tiles ----------------
+        // (one warp for both issued a K block of 16 rows in 650 cycles: it gets a fifth of its scheduler's slots)
+        const uint32_t mt = warp - kConvWarps;
         // The whole warp walks the loop on warp-uniform values and one elected lane issues: behind a branch on the lane
         // number every descriptor was a per-thread value, and all tiles ran at 0.7 us per K block (0.5 now at 16 columns).
-        uint32_t a_use = 0, b_use = 0;
-        for (uint32_t turn = 0;; ++turn) {
-            const uint32_t t = take_tile(turn);
-            if (t >= n_tiles || failed()) break;
-            Work wk;
-            if (!open_tile(t, wk)) continue;
-            const TileShape ts(wk.in.count);
-            const uint32_t idesc = __shfl_sync(0xffffffffu, umma_idesc(ts.N), 0), acc0 = __shfl_sync(0xffffffffu, tmem_base, 0);
-            const uint32_t acc1 = acc0 + __shfl_sync(0xffffffffu, ts.acc_step, 0), stages = __shfl_sync(0xffffffffu, ts.a_stages, 0);
-            const uint32_t b_smem = __shfl_sync(0xffffffffu, smem_base, 0), a_smem = b_smem + __shfl_sync(0xffffffffu, ts.off_a, 0);
-            const uint32_t b_step = __shfl_sync(0xffffffffu, ts.b_stage, 0), n_kb = __shfl_sync(0xffffffffu, wk.KB, 0);
-            const bool in_tmem = __shfl_sync(0xffffffffu, (uint32_t)ts.in_tmem, 0) != 0;
-            uint32_t sa = 0, sb = 0;
-            for (uint32_t kb = 0; kb < n_kb; ++kb) {
-                // (the first stage of converted weights also says that the last tile's accumulators have been read)
-                const bool got = pipe_wait(&b_full[sb], (b_use >> sb) & 1) && pipe_wait(&a_full[sa], (a_use >> sa) & 1);
+        Tile t;
+        uint32_t n = 0;
+        bool go = take_tile(0, t), was_wide = false;
+        const uint32_t acc = __shfl_sync(0xffffffffu, tmem_base, 0), sm0 = __shfl_sync(0xffffffffu, smem_base, 0);
+        {
+            uint32_t a_use = 0, b_use = 0, sa = 0, sb = 0;
+            for (; go && !t.narrow; go = take_tile(++n, t)) {
+                was_wide = true;
+                const uint32_t idesc = umma_idesc((t.count + 15u) & ~15u), n_kb = __shfl_sync(0xffffffffu, k_blocks(t), 0);
+                for (uint32_t kb = 0; kb < n_kb; ++kb) {
+                    // (the first stage of converted weights also says that the last tile's accumulators have been read)
+                    const bool got = pipe_wait(&b_full[sb], (b_use >> sb) & 1) && pipe_wait(&a_full[sa], (a_use >> sa) & 1);
+                    if (!__all_sync(0xffffffffu, got)) {
+                        give_up();
+                        break;
+                    }
+                    a_use ^= 1u << sa;
+                    b_use ^= 1u << sb;
+                    __syncwarp();
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint64_t db = umma_smem_desc(sm0 + sb * kWideBBytes);
+                        const uint64_t da = umma_smem_desc(sm0 + kWideOffA + sa * kWideABytes + mt * kTileBytes);
+                        // 4 x K16 per 64-wide block: 32 bytes further along the row
+#pragma unroll
+                        for (uint32_t k = 0; k < 4; ++k) umma_f16(acc + mt * kUmmaMaxN, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                        umma_commit(&a_empty[sa]);
+                        umma_commit(&b_empty[sb]);
+                    }
+                    __syncwarp();
+                    if (++sa == kWideA) sa = 0;
+                    if (++sb == kWideB) sb = 0;
+                }
+                if (elect_one()) umma_commit(&accum[n % kTiles]);
+                __syncwarp();
+            }
+        }
+        if (was_wide && go) {
+            if (elect_one()) umma_commit(wide_over);
+            __syncwarp();
+        }
+        uint32_t kc = 0, sb = 0, b_par = 0;
+        bool other_small = true;   // the tile before had accumulators of its own
+        for (uint32_t first = n; go; go = take_tile(++n, t)) {
+            const bool small = t.count <= kSmallN;
+            const uint32_t idesc = umma_idesc((t.count + 15u) & ~15u), n_kb = __shfl_sync(0xffffffffu, k_blocks(t), 0);
+            const uint32_t b_mask = narrow_b_mask(t.count), b_step = kNarrowBBytes / (b_mask + 1);
+            const uint32_t acc_at = acc + (small ? (n & 1) * 2 * kSmallN + mt * kSmallN : mt * 128);
+            // the last tiles' epilogues have read these accumulators (a wide tile's: before any narrow weights were converted)
+            bool ok = n < first + 2 || pipe_wait(&epi_done[n & 1], ((n >> 1) & 1) ^ 1);
+            if (n > first && !(small && other_small)) ok = ok && pipe_wait(&epi_done[(n & 1) ^ 1], ((n - 1) >> 1) & 1);
+            if (!__all_sync(0xffffffffu, ok)) { give_up(); break; }
+            other_small = small;
+            for (uint32_t kb = 0; kb < n_kb; kb += 2, ++kc) {
+                const uint32_t st = kc % kNarrowA, here = min(2u, n_kb - kb), in_b = kb & b_mask;   // K block within the activations' stage
+                const uint32_t sb1 = b_mask ? sb : sb + 1 == kNarrowB ? 0u : sb + 1, in_b1 = b_mask ? in_b + 1 : 0u;   // the second one's
+                bool got = in_b || pipe_wait(&nb_full[sb], b_par);
+                if (!b_mask && here == 2) got = got && pipe_wait(&nb_full[sb1], sb1 ? b_par : b_par ^ 1);
+                got = got && pipe_wait(&na_full[st], (kc / kNarrowA) & 1);
                 if (!__all_sync(0xffffffffu, got)) {
                     give_up();
                     break;
                 }
-                a_use ^= 1u << sa;
-                b_use ^= 1u << sb;
-                __syncwarp();
+                const bool b_done = in_b1 == b_mask || kb + 2 >= n_kb;   // (of a stage for several K blocks)
                 tc_fence_after();
                 if (elect_one()) {
-                    const uint64_t db = umma_smem_desc(b_smem + sb * b_step);
-                    if (in_tmem) {
-                        const uint32_t ta = acc0 + 256u + sa * 64;   // 16 of K are eight columns
+                    const uint32_t ta = acc + 256u + st * 128 + mt * 32;   // 16 of K are eight columns
+                    const uint64_t db = umma_smem_desc(sm0 + sb * kNarrowBBytes + in_b * b_step);
 #pragma unroll
-                        for (uint32_t k = 0; k < 4; ++k) {
-                            umma_f16_ts(acc0, ta + 8 * k, db + 2 * k, idesc, (kb | k) != 0);
-                            umma_f16_ts(acc1, ta + 32 + 8 * k, db + 2 * k, idesc, (kb | k) != 0);
-                        }
-                    } else {
-                        const uint64_t da0 = umma_smem_desc(a_smem + sa * kAStageBytes), da1 = umma_smem_desc(a_smem + sa * kAStageBytes + kTileBytes);
-                        // 4 x K16 per 64-wide block: 32 bytes further along the row. The two tiles alternate: consecutive
-                        // instructions then add into different accumulators.
+                    for (uint32_t k = 0; k < 4; ++k) umma_f16_ts(acc_at, ta + 8 * k, db + 2 * k, idesc, (kb | k) != 0);
+                    if (here == 2) {
+                        const uint64_t db1 = umma_smem_desc(sm0 + sb1 * kNarrowBBytes + in_b1 * b_step);
 #pragma unroll
-                        for (uint32_t k = 0; k < 4; ++k) {
-                            umma_f16(acc0, da0 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-                            umma_f16(acc1, da1 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-                        }
+                        for (uint32_t k = 0; k < 4; ++k) umma_f16_ts(acc_at, ta + 64 + 8 * k, db1 + 2 * k, idesc, 1u);
                     }
-                    umma_commit(&a_empty[sa]);
-                    umma_commit(&b_empty[sb]);
+                    umma_commit(&na_empty[st]);
+                    if (b_done) umma_commit(&nb_empty[sb]);
+                    if (!b_mask && here == 2) umma_commit(&nb_empty[sb1]);
                 }
                 __syncwarp();
-                if (++sa == stages) sa = 0;
-                if (++sb == kBStages) sb = 0;
+                for (uint32_t i = b_mask ? (b_done ? 1u : 0u) : here; i; --i)
+                    if (++sb == kNarrowB) { sb = 0; b_par ^= 1; }
             }
-            if (elect_one()) umma_commit(accum);
+            if (elect_one()) umma_commit(&accum[n % kTiles]);
             __syncwarp();
         }
-    } else if (warp == kConvWarps + 1) {
+    } else if (warp == kConvWarps + 2) {
         // ---------------- activation tiles ----------------
         // One or two boxes per K block: these tiles are most of what a block pulls out of L2, and a short instance
         // does not pay for 256 rows, nor one of 80 rows for 128.
-        uint32_t b_use = 0, last_stage = 0;
-        for (uint32_t turn = 0;; ++turn) {
-            const uint32_t t = take_tile(turn);
-            if (t >= n_tiles || failed()) break;
-            Work wk;
-            if (!open_tile(t, wk)) continue;
-            const TileShape ts(wk.in.count);
-            const CUtensorMap* maps_b = wk.shared ? maps.act_shared : maps.act_routed;
+        uint32_t b_use = 0, sb = 0, nsb = 0, b_par = 0;
+        bool was_wide = false, in_wide = true;
+        Tile t;
+        for (uint32_t n = 0; take_tile(n, t); ++n) {
+            const TileShape ts(t.count);
+            const CUtensorMap* maps_b = t.shared ? maps.act_shared : maps.act_routed;
             if (lane == 0) {
-                // Another layout: the last use of the old stages that its stages lie across has to be done. (The stages
-                // themselves are waited for, not the tile: a tile of two K blocks leaves the third stage to the tile before it, so
-                // the tile barrier could still be two phases behind, where its one parity bit reads as passed. By the lane
-                // that copies: with the wait and a vote by the whole warp, 333 rows took 297 us for 291.)
-                const uint32_t over = last_stage && ts.b_stage != last_stage ?
-                                          min(kBStages, (kBStages * ts.b_stage + last_stage - 1) / last_stage) : 0u;
-                last_stage = ts.b_stage;
-#pragma unroll 1
-                for (uint32_t s = 0; s < over; ++s)
-                    if (!pipe_wait(&b_empty[s], ((b_use >> s) & 1) ^ 1)) { give_up(); break; }
-                const uint32_t b_bytes = (ts.n1 + ts.n2) * 128u;
-                uint32_t sb = 0;
-                for (uint32_t kb = 0; kb < wk.KB; ++kb) {
+                const uint32_t KB = k_blocks(t), b_bytes = (ts.n1 + ts.n2) * 128u;
+                if (t.narrow && in_wide) {
+                    in_wide = false;
+                    if (was_wide && !pipe_wait(wide_over, 0)) give_up();
+                }
+                was_wide = in_wide;
+                auto copy = [&](uint32_t dst, uint32_t kb, uint64_t* bar) {
+                    tma_load_2d(dst, &maps_b[ts.b1], (int32_t)(kb * 64), (int32_t)t.first, bar);
+                    if (ts.n2) tma_load_2d(dst + ts.n1 * 128u, &maps_b[ts.b2], (int32_t)(kb * 64), (int32_t)(t.first + ts.n1), bar);
+                };
+                const uint32_t b_mask = narrow_b_mask(t.count), b_step = kNarrowBBytes / (b_mask + 1);
+                for (uint32_t kb = 0; t.narrow && kb < KB; kb += b_mask + 1) {
+                    if (failed()) break;
+                    if (!pipe_wait(&nb_empty[nsb], b_par ^ 1)) { give_up(); break; }
+                    const uint32_t here = min(b_mask + 1, KB - kb);
+                    mbar_expect_tx(&nb_full[nsb], here * b_bytes);
+                    for (uint32_t i = 0; i < here; ++i) copy(smem_base + nsb * kNarrowBBytes + i * b_step, kb + i, &nb_full[nsb]);
+                    if (++nsb == kNarrowB) { nsb = 0; b_par ^= 1; }
+                }
+                for (uint32_t kb = 0; !t.narrow && kb < KB; ++kb) {
                     if (failed()) break;
                     if (!pipe_wait(&b_empty[sb], ((b_use >> sb) & 1) ^ 1)) { give_up(); break; }
                     b_use ^= 1u << sb;
                     mbar_expect_tx(&b_full[sb], b_bytes);
-                    tma_load_2d(smem_base + sb * ts.b_stage, &maps_b[ts.b1], (int32_t)(kb * 64), (int32_t)wk.in.first, &b_full[sb]);
-                    if (ts.n2)
-                        tma_load_2d(smem_base + sb * ts.b_stage + ts.n1 * 128u, &maps_b[ts.b2], (int32_t)(kb * 64),
-                                    (int32_t)(wk.in.first + ts.n1), &b_full[sb]);
-                    if (++sb == kBStages) sb = 0;
+                    copy(smem_base + sb * kWideBBytes, kb, &b_full[sb]);
+                    if (++sb == kWideB) sb = 0;
                 }
             }
             __syncwarp();
         }
+    } else if (warp > kConvWarps + 3) {
+        // ---------------- epilogues of small tiles ----------------
+        // (by the converters between two tiles they took 3000 of a tile's 22,000 cycles at 2048 x 16 rows)
+        const uint32_t et = tid - (kConvWarps + 4) * 32;
+        uint32_t met = 0;
+        Tile t;
+        // A tile is handed back only when its instructions are done, also one that the converters finish: its barrier then is never
+        // more than a phase away from the one that is waited for.
+        for (uint32_t n = 0; take_tile(n, t, false); ++n) {
+            if (t.count > kSmallN) {
+                if (!pipe_wait(&accum[n % kTiles], (n / kTiles) & 1)) { give_up(); break; }
+                release_tile(n);
+                continue;
+            }
+            uint32_t* const ids = small_id + (n & 1) * kSmallN;
+            float* const wts = small_w + (n & 1) * kSmallN;
+            if (PHASE == 1) {
+                if (et < t.count) {
+                    const uint32_t p = t.shared ? t.first + et : a.sorted[t.first + et];
+                    ids[et] = t.shared ? p : p / a.top_k;
+                    wts[et] = t.shared ? (a.shared_gate ? a.shared_gate[p] : 1.0f) : a.route_w[p];
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(eids_full);
+                const bool ok = pipe_wait(eids_full, met);
+                met ^= 1;
+                if (!ok) { give_up(); break; }
+            }
+            const uint32_t at = (n & 1) * 2 * kSmallN;
+            if (!epilogue(std::integral_constant<int, 4>(), std::integral_constant<int, 1>(), 0u, t, n, at, at + kSmallN, ids, wts)) break;
+            release_tile(n);
+        }
     } else if (lane == 0) {
-        // ---------------- tile numbers; packed weights, scales, biases ----------------
-        uint32_t pk_use = 0, sc_use = 0, slot = 0;
-        for (uint32_t turn = 0;; ++turn) {
-            const uint32_t s = turn & 1;
-            const uint32_t t = turn == 0 ? blockIdx.x : gridDim.x + atomicAdd(n_inst + 1 + PHASE, 1u);
-            if (!pipe_wait(&next_empty[s], ((turn >> 1) & 1) ^ 1)) { give_up(); break; }
-            *(volatile uint32_t*)&next_tile[s] = t;
-            mbar_arrive(&next_full[s]);
-            if (t >= n_tiles || failed()) break;
-            Work wk;
-            if (!open_tile(t, wk)) continue;
-            const ChunkInstance& in = wk.in;
-            const WeightMaps* wm = wk.shared ? &maps.shared : &maps.routed[in.slot / a.pool.cells_per_chunk];
-            const int32_t cell = wk.shared ? 0 : (int32_t)(in.slot % a.pool.cells_per_chunk);
-            const int32_t y0 = (int32_t)wk.r0, y1 = (int32_t)(PHASE == 0 ? wk.r0 : wk.r0 + 128);
-            for (uint32_t kb = 0; kb < wk.KB; ++kb) {
+        // ---------------- tiles; packed weights, scales, biases ----------------
+        // The number of the tile after next and the instance of the next one are asked for while this one is copied.
+        const uint32_t n_tiles = n_inst[0] * row_tiles;
+        auto read_inst = [&](uint32_t tile) { return tile < n_tiles ? __ldg((const uint4*)(inst + tile / row_tiles)) : make_uint4(0, 0, 0, 0); };
+        uint32_t now = blockIdx.x, next = gridDim.x + atomicAdd(n_inst + 1 + PHASE, 1u);
+        uint4 v = read_inst(now);
+        uint32_t n = 0, pk_use = 0, sc_use = 0, slot = 0, ss = 0, pk_par = 0, sc_par = 0;
+        bool was_wide = false, in_wide = true;
+        for (;;) {
+            const bool end = now >= n_tiles;
+            const uint4 v_next = end ? v : read_inst(next);
+            const uint32_t after = end ? 0u : gridDim.x + atomicAdd(n_inst + 1 + PHASE, 1u);
+            Tile t;
+            t.shared = v.x == 1;
+            t.slot = v.y; t.first = v.z; t.count = end ? 0u : v.w;
+            t.r0 = (now % row_tiles) * (PHASE == 0 ? 128u : 256u);
+            t.narrow = t.count <= kNarrowN;
+            const uint32_t rows = PHASE == 0 ? (t.shared ? a.f_shared : a.f) : a.d, KB = k_blocks(t);
+            now = next; next = after; v = v_next;
+            if (!end && t.r0 >= rows) continue;   // a narrower shared or routed expert
+            const uint32_t s = n % kTiles;
+            if (!pipe_wait(&tile_empty[s], ((n / kTiles) & 1) ^ 1)) { give_up(); break; }
+            ++n;
+            next_tile[s] = make_uint4(t.slot, t.first, t.r0 | (t.shared ? 0x80000000u : 0u), t.count);
+            mbar_arrive(&tile_full[s]);
+            if (end || failed()) break;
+            const WeightMaps* wm = t.shared ? &maps.shared : &maps.routed[t.slot / a.pool.cells_per_chunk];
+            const int32_t cell = t.shared ? 0 : (int32_t)(t.slot % a.pool.cells_per_chunk);
+            const int32_t y0 = (int32_t)t.r0, y1 = (int32_t)(PHASE == 0 ? t.r0 : t.r0 + 128);
+            if (!t.narrow) {
+                was_wide = true;
+                for (uint32_t kb = 0; kb < KB; ++kb) {
+                    if (failed()) break;
+                    if (SCT && kb % kKbPerSc == 0) {
+                        const int32_t g0 = (int32_t)(kb / kKbPerSc * 8);
+                        if (!pipe_wait(sc_empty, sc_use ^ 1)) { give_up(); break; }
+                        sc_use ^= 1;
+                        mbar_expect_tx(sc_full, kWideScBytes);
+                        const uint32_t dst = smem_base + kWideOffSc;
+                        tma_load_3d(dst, &wm->s[0], g0, y0, cell, sc_full);
+                        tma_load_3d(dst + kWideScBytes / 4, &wm->s[1], g0, y1, cell, sc_full);
+                        tma_load_3d(dst + kWideScBytes / 2, &wm->b[0], g0, y0, cell, sc_full);
+                        tma_load_3d(dst + kWideScBytes / 4 * 3, &wm->b[1], g0, y1, cell, sc_full);
+                    }
+                    if (kb % kWideKbPerPk == 0) {
+                        const int32_t x = (int32_t)(kb / kWideKbPerPk * 64);
+                        if (!pipe_wait(&pk_empty[slot], ((pk_use >> slot) & 1) ^ 1)) { give_up(); break; }
+                        pk_use ^= 1u << slot;
+                        mbar_expect_tx(&pk_full[slot], kWidePkBytes);
+                        const uint32_t dst = smem_base + kWideOffPk + slot * kWidePkBytes;
+                        tma_load_3d(dst, &wm->w[0], x, y0, cell, &pk_full[slot]);
+                        tma_load_3d(dst + kWidePkBytes / 2, &wm->w[1], x, y1, cell, &pk_full[slot]);
+                        if (++slot == kWidePk) slot = 0;
+                    }
+                }
+                continue;
+            }
+            if (in_wide) {
+                in_wide = false;
+                slot = 0;
+                if (was_wide && !pipe_wait(wide_over, 0)) { give_up(); break; }
+            }
+            for (uint32_t kb = 0; kb < KB; kb += kNarrowKbPerPk) {
                 if (failed()) break;
-                if (sc_tma && kb % kKbPerSc == 0) {
+                if (SCT && kb % (2 * kKbPerSc) == 0) {
                     const int32_t g0 = (int32_t)(kb / kKbPerSc * 8);
-                    if (!pipe_wait(sc_empty, sc_use ^ 1)) { give_up(); break; }
-                    sc_use ^= 1;
-                    mbar_expect_tx(sc_full, 2 * kScHalfBytes);
-                    const uint32_t dst = smem_base + kOffSc;
-                    tma_load_3d(dst, &wm->s[0], g0, y0, cell, sc_full);
-                    tma_load_3d(dst + kScHalfBytes / 2, &wm->s[1], g0, y1, cell, sc_full);
-                    tma_load_3d(dst + kScHalfBytes, &wm->b[0], g0, y0, cell, sc_full);
-                    tma_load_3d(dst + kScHalfBytes + kScHalfBytes / 2, &wm->b[1], g0, y1, cell, sc_full);
+                    uint64_t* const bar = &nsc_full[ss];
+                    if (!pipe_wait(&nsc_empty[ss], sc_par ^ 1)) { give_up(); break; }
+                    mbar_expect_tx(bar, kNarrowScBytes);
+                    const uint32_t dst = smem_base + kNarrowOffSc + ss * kNarrowScBytes;
+                    tma_load_3d(dst, &wm->ns[0], g0, y0, cell, bar);
+                    tma_load_3d(dst + kNarrowScBytes / 4, &wm->ns[1], g0, y1, cell, bar);
+                    tma_load_3d(dst + kNarrowScBytes / 2, &wm->nb[0], g0, y0, cell, bar);
+                    tma_load_3d(dst + kNarrowScBytes / 4 * 3, &wm->nb[1], g0, y1, cell, bar);
+                    if (++ss == kNarrowSc) { ss = 0; sc_par ^= 1; }
                 }
-                if (kb % kKbPerPk == 0) {
-                    const int32_t x = (int32_t)(kb / kKbPerPk * 64);
-                    if (!pipe_wait(&pk_empty[slot], ((pk_use >> slot) & 1) ^ 1)) { give_up(); break; }
-                    pk_use ^= 1u << slot;
-                    mbar_expect_tx(&pk_full[slot], kPkSlotBytes);
-                    const uint32_t dst = smem_base + kOffPk + slot * kPkSlotBytes;
-                    tma_load_3d(dst, &wm->w[0], x, y0, cell, &pk_full[slot]);
-                    tma_load_3d(dst + kPkSlotBytes / 2, &wm->w[1], x, y1, cell, &pk_full[slot]);
-                    if (++slot == kPkSlots) slot = 0;
-                }
+                if (!pipe_wait(&npk_empty[slot], pk_par ^ 1)) { give_up(); break; }
+                mbar_expect_tx(&npk_full[slot], kNarrowPkBytes);
+                const uint32_t dst = smem_base + kNarrowOffPk + slot * kNarrowPkBytes;
+                const int32_t x = (int32_t)(kb / kNarrowKbPerPk * 128);
+                tma_load_3d(dst, &wm->nw[0], x, y0, cell, &npk_full[slot]);
+                tma_load_3d(dst + kNarrowPkBytes / 2, &wm->nw[1], x, y1, cell, &npk_full[slot]);
+                if (++slot == kNarrowPk) { slot = 0; pk_par ^= 1; }
             }
         }
     }
-    if (failed() && lane == 0 && warp > kConvWarps) {
+    }
+    if (failed() && lane == 0 && (warp & ~1u) == kConvWarps + 2) {
         // a copy of this block may still be in flight: give it a bounded time to land
         for (int i = 0; i < 200; ++i) __nanosleep(1000);
     }
@@ -797,8 +1201,9 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
     }
 }
 
-// One thread per expert: ceil(count/256) chunk instances each, then the shared expert's.
-// n_inst[0] = instances, [1], [2]: tiles handed out in phase 0, 1.
+// The list of instances: all full ones (256 rows; the shared expert's first), then every expert's rest, most rows first. A tile of
+// 256 rows takes twice the time of one of 16, and a list that ends on long ones leaves SMs idle; and a block then changes the
+// layout of its shared memory twice at most. One thread per expert; n_inst[0] = instances, [1], [2]: tiles handed out in phase 0, 1.
 __global__ void __launch_bounds__(256)
 chunk_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ counts,
                        const uint32_t* __restrict__ slot_of_expert, uint32_t ne, uint32_t T, uint32_t with_shared,
@@ -806,23 +1211,9 @@ chunk_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __r
                        uint32_t* status) {
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ uint32_t warp_sums[8], by_size[256];
+    __shared__ uint32_t warp_sums[8];
     __shared__ __align__(16) uint32_t key[256];
-    // Experts with the most rows first: a tile of 256 rows takes twice the time of one of 16, and a list that ends on long
-    // ones leaves SMs idle (4096 rows: the last ended a tenth after the median SM).
-    key[threadIdx.x] = (threadIdx.x < ne ? counts[threadIdx.x] << 8 : 0u) | (255u - threadIdx.x);
-    __syncthreads();
-    {
-        const uint32_t mine = key[threadIdx.x];
-        uint32_t rank = 0;
-        for (uint32_t j = 0; j < 256; j += 4) {
-            const uint4 v = *(const uint4*)&key[j];
-            rank += (v.x > mine) + (v.y > mine) + (v.z > mine) + (v.w > mine);
-        }
-        by_size[rank] = threadIdx.x;
-    }
-    __syncthreads();
-    const uint32_t e = by_size[threadIdx.x];
+    const uint32_t e = threadIdx.x;
     uint32_t n = 0, slot = SHRIKE_SLOT_MISS, c = 0;
     if (e < ne && counts[e] > 0) {
         c = counts[e];
@@ -831,8 +1222,11 @@ chunk_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __r
             report_status(status, kStatusBadIndex);
             slot = SHRIKE_SLOT_MISS;
         }
-        if (slot != SHRIKE_SLOT_MISS) n = (c + kUmmaMaxN - 1) / kUmmaMaxN;
+        if (slot == SHRIKE_SLOT_MISS) c = 0;
+        n = c / kUmmaMaxN;
     }
+    const uint32_t rest = c % kUmmaMaxN, mine = rest << 8 | (255u - e), shared_rest = with_shared ? T % kUmmaMaxN : 0u;
+    key[e] = mine;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t inc = n;
 #pragma unroll
@@ -841,28 +1235,43 @@ chunk_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __r
         if (lane >= (uint32_t)o) inc += v;
     }
     if (lane == 31) warp_sums[warp] = inc;
-    __syncthreads();
+    const uint32_t before_shared = (uint32_t)__syncthreads_count(rest > shared_rest);   // rests that come before the shared expert's
+    const uint32_t n_rest = (uint32_t)__syncthreads_count(rest != 0) + (shared_rest != 0);
     uint32_t base = 0, total = 0;
     for (uint32_t w = 0; w < 8; ++w) {
         if (w < warp) base += warp_sums[w];
         total += warp_sums[w];
     }
-    // The shared expert's instances come first in the list: they are full (256 rows), and the blocks of the
-    // list's end are the last to start -- a launch that ends on its longest blocks ends late.
-    const uint32_t n_shared = with_shared ? (T + kUmmaMaxN - 1) / kUmmaMaxN : 0;
+    const uint32_t n_shared = with_shared ? T / kUmmaMaxN : 0;
     base += inc - n + n_shared;
+    total += n_shared;
     for (uint32_t j = 0; j < n; ++j) {
         ChunkInstance in;
-        in.kind = 0; in.slot = slot; in.first = offsets[e] + kUmmaMaxN * j; in.count = min(kUmmaMaxN, c - kUmmaMaxN * j);
+        in.kind = 0; in.slot = slot; in.first = offsets[e] + kUmmaMaxN * j; in.count = kUmmaMaxN;
         inst[base + j] = in;
+    }
+    if (rest) {
+        uint32_t rank = rest <= shared_rest ? 1u : 0u;
+        for (uint32_t j = 0; j < 256; j += 4) {
+            const uint4 v = *(const uint4*)&key[j];
+            rank += (v.x > mine) + (v.y > mine) + (v.z > mine) + (v.w > mine);
+        }
+        ChunkInstance in;
+        in.kind = 0; in.slot = slot; in.first = offsets[e] + kUmmaMaxN * n; in.count = rest;
+        inst[total + rank] = in;
     }
     for (uint32_t j = threadIdx.x; j < n_shared; j += blockDim.x) {
         ChunkInstance in;
-        in.kind = 1; in.slot = 0; in.first = kUmmaMaxN * j; in.count = min(kUmmaMaxN, T - kUmmaMaxN * j);
+        in.kind = 1; in.slot = 0; in.first = kUmmaMaxN * j; in.count = kUmmaMaxN;
         inst[j] = in;
     }
     if (threadIdx.x == 0) {
-        n_inst[0] = total + n_shared;
+        if (shared_rest) {
+            ChunkInstance in;
+            in.kind = 1; in.slot = 0; in.first = kUmmaMaxN * n_shared; in.count = shared_rest;
+            inst[total + before_shared] = in;
+        }
+        n_inst[0] = total + n_rest;
         n_inst[1] = n_inst[2] = 0;   // tiles handed out, per phase
     }
 }
@@ -895,19 +1304,19 @@ static bool make_rows_map(CUtensorMap* map, const uint16_t* base, uint64_t cols,
                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// One matrix of every cell of a pool chunk: [cells][rows][row_bytes] bytes (packed weights, 64-byte
-// boxes of 128 rows, 64-byte swizzle) or [cells][rows][groups] 16-bit (scales / biases, 8 per row).
-static bool make_matrix_map(CUtensorMap* map, const uint8_t* base, bool meta, uint64_t row_elems, uint64_t rows,
+// One matrix of every cell of a pool chunk: [cells][rows][row_bytes] bytes (packed weights) or [cells][rows][groups] 16-bit
+// (scales / biases), in boxes of 128 rows: of 64 bytes, swizzled so, or 8 groups, and twice that for narrow tiles.
+static bool make_matrix_map(CUtensorMap* map, const uint8_t* base, bool meta, bool narrow, uint64_t row_elems, uint64_t rows,
                             uint64_t cells, uint64_t cell_stride) {
     const uint64_t esz = meta ? 2 : 1;
     const cuuint64_t dims[3] = {row_elems, rows, cells};
     // a single cell (the shared expert's block) still needs a valid outer pitch
     const cuuint64_t strides[2] = {row_elems * esz, cells > 1 ? cell_stride : row_elems * esz * rows};
-    const cuuint32_t box[3] = {meta ? 8u : 64u, 128, 1};
+    const cuuint32_t box[3] = {(meta ? 8u : 64u) << narrow, 128, 1};
     const cuuint32_t elem[3] = {1, 1, 1};
     return encode_tiled_fn()(map, meta ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, (void*)base,
                              dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             meta ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_64B,
+                             meta ? CU_TENSOR_MAP_SWIZZLE_NONE : narrow ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -916,12 +1325,14 @@ static bool make_weight_maps(WeightMaps* wm, const uint8_t* base, const Offsets3
                              uint32_t rows, uint32_t bits, uint32_t group, uint64_t cells, uint64_t cell_stride) {
     for (int t = 0; t < 2; ++t) {
         const int mat = phase == 0 ? t : 2;
-        if (!make_matrix_map(&wm->w[t], base + off.w[mat], false, (uint64_t)kdim * bits / 8, rows, cells, cell_stride))
+        if (!make_matrix_map(&wm->w[t], base + off.w[mat], false, false, (uint64_t)kdim * bits / 8, rows, cells, cell_stride) ||
+            !make_matrix_map(&wm->nw[t], base + off.w[mat], false, true, (uint64_t)kdim * bits / 8, rows, cells, cell_stride))
             return false;
         if ((kdim / group) % 8 != 0) continue;   // such scale rows are read by the converter threads
-        if (!make_matrix_map(&wm->s[t], base + off.s[mat], true, kdim / group, rows, cells, cell_stride) ||
-            !make_matrix_map(&wm->b[t], base + off.b[mat], true, kdim / group, rows, cells, cell_stride))
-            return false;
+        for (int n = 0; n < 2; ++n)
+            if (!make_matrix_map(n ? &wm->ns[t] : &wm->s[t], base + off.s[mat], true, n, kdim / group, rows, cells, cell_stride) ||
+                !make_matrix_map(n ? &wm->nb[t] : &wm->b[t], base + off.b[mat], true, n, kdim / group, rows, cells, cell_stride))
+                return false;
     }
     return true;
 }
@@ -953,11 +1364,26 @@ cudaError_t umma_prepare(shrike_moe* m) {
     return ok ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+// The converters' setmaxnreg.inc waits for registers that the block was launched with: a build with fewer would wait for good.
+template <int BITS, int GROUP, int META, int PHASE, bool SCT>
+static bool registers_fit() {
+    static const bool fits = [] {
+        cudaFuncAttributes at;
+        return cudaFuncGetAttributes(&at, umma_expert_kernel<BITS, GROUP, META, PHASE, SCT>) == cudaSuccess &&
+               (uint32_t)at.numRegs * kUmmaThreads >= kConverters * kConvRegs + (kUmmaThreads - kConverters) * kOtherRegs;
+    }();
+    return fits;
+}
+
 template <int BITS, int GROUP, int META>
 static cudaError_t launch_umma_t(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, const ChunkInstance* inst,
                                  uint32_t* n_inst, uint32_t max_inst, const UmmaMaps& m0, const UmmaMaps& m1) {
-    auto k0 = umma_expert_kernel<BITS, GROUP, META, 0>;
-    auto k1 = umma_expert_kernel<BITS, GROUP, META, 1>;
+    const bool sct0 = (a.d / GROUP & 7u) == 0, sct1 = ((a.f / GROUP | a.f_shared / GROUP) & 7u) == 0;
+    auto k0 = sct0 ? umma_expert_kernel<BITS, GROUP, META, 0, true> : umma_expert_kernel<BITS, GROUP, META, 0, false>;
+    auto k1 = sct1 ? umma_expert_kernel<BITS, GROUP, META, 1, true> : umma_expert_kernel<BITS, GROUP, META, 1, false>;
+    if (!(sct0 ? registers_fit<BITS, GROUP, META, 0, true>() : registers_fit<BITS, GROUP, META, 0, false>()) ||
+        !(sct1 ? registers_fit<BITS, GROUP, META, 1, true>() : registers_fit<BITS, GROUP, META, 1, false>()))
+        return cudaErrorInvalidConfiguration;
     cudaError_t e = cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUmmaSmemBytes);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUmmaSmemBytes);

@@ -31,6 +31,18 @@ def test_a_short_tile_before_another_layout(cuda_device, kw):
     run_sizes([257] * 24, kw, sample=24)
 
 
+@pytest.mark.parametrize("kw", [
+    dict(d=576, f=64, shared_f=192),                                                # odd numbers of K blocks, one K block
+    dict(d=2112, f=576, shared_f=64, weight_bits=8),                                # odd numbers of groups
+    dict(d=1088, f=320, shared_f=512, weight_bits=4, group_size=32),                # scale rows of 34 and 10 groups
+    dict(d=1024, f=512, shared_f=512, weight_bits=8, group_size=32, meta_dtype=capi.DTYPE_FP16, expert_bias=1),
+], ids=lambda kw: "-".join(f"{k}{v}" for k, v in kw.items()))
+def test_narrow_tiles(cuda_device, kw):
+    """Tiles of up to 128 rows only: on both sides of every number of K blocks in an activation stage (32 and 64 rows) and of the
+    second pair of accumulators (64), with K lengths that end in the middle of a packed slot, a pair of K blocks and a scale block."""
+    run_sizes([128, 113, 112, 65, 64, 49, 33, 32, 31, 17, 16, 15] + [3] * 40, kw)
+
+
 def run_sizes(sizes, kw, sample=None):
     cfg = small_config(num_experts=64, top_k=1, max_tokens=max(1024, sum(sizes)), shared_gated=False, **kw)
     layer = Layer(cfg)
