@@ -667,25 +667,20 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         // Block blk's scales into sreg / breg: 32-wide groups this thread's two words, else all four.
         auto narrow_scales = [&](uint32_t blk) {
             if (GROUP == 32 && (G & 1u) == 0) {
-                uint8_t* const at = smem + kWideOffSc + (tile * 128 + (warp & 3) * 32) * 16 + half * 4;
+                // word j of row `lane` sits in lane 2 (row mod 16) + j of load row / 16
                 auto exchange = [&](uint32_t* sv, uint32_t* bv) {
-                    __syncwarp();   // the last block's have been read
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        uint8_t* const to = at + ((lane >> 1) + 16 * i) * 16 + (lane & 1) * 8;
-                        *(uint32_t*)to = sv[i];
-                        *(uint32_t*)(to + kWideScBytes / 2) = bv[i];
+                    for (int j = 0; j < 2; ++j) {
+                        const uint32_t from = 2 * (lane & 15) + j;
+                        const uint32_t s0 = __shfl_sync(0xffffffffu, sv[0], from), s1 = __shfl_sync(0xffffffffu, sv[1], from);
+                        const uint32_t b0 = __shfl_sync(0xffffffffu, bv[0], from), b1 = __shfl_sync(0xffffffffu, bv[1], from);
+                        sreg[j] = lane & 16 ? s1 : s0;
+                        breg[j] = lane & 16 ? b1 : b0;
                     }
                     fetch_own(blk + 2, sv, bv);
                 };
                 if (blk & 1) exchange(snext + 2, bnext + 2);
                 else exchange(snext, bnext);
-                __syncwarp();
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    sreg[i] = *(const uint32_t*)(at + lane * 16 + i * 8);
-                    breg[i] = *(const uint32_t*)(at + kWideScBytes / 2 + lane * 16 + i * 8);
-                }
                 return;
             }
             turn_scales(blk);
@@ -804,7 +799,9 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         // (a warp may write weights and columns while others still read what they take of the last accumulators)
         if (go && was_wide && !failed()) go = converters_meet();
         {
-            uint32_t kc = 0, slot = 0, pk_par = 0, ss = 0, sc_par = 0, in_sc = 0;   // pairs of K blocks used before; slots
+            static_assert(kNarrowA == 2, "stages in turn");
+            uint32_t a_st = 0, a_par = 1, slot = 0, pk_par = 0, ss = 0, sc_par = 0, in_sc = 0;
+            auto next_pair = [&]() { a_st ^= 1u; a_par ^= a_st ^ 1u; };
             const uint32_t a_tmem = tmem_base + 256u + (((warp & 3) * 32) << 16) + half * 64 + tile * 32;
             // 16-byte chunks of this thread's K block in its row of 128 packed bytes: the second of int4's two is 64 bytes on
             constexpr uint32_t kChunks = kRowBlockBytes / 16;
@@ -875,8 +872,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                     for (uint32_t i = 0; i < kOwn; ++i) {
                         const uint32_t kb = kb0 + 2 * i + half;
                         if (kb >= KB) break;
-                        const uint32_t c = kc + kb / 2, st = c % kNarrowA, par = ((c / kNarrowA) & 1) ^ 1;
-                        const bool free = pipe_test(&na_empty[st], par);
+                        const bool free = pipe_test(&na_empty[a_st], a_par);
                         uint32_t s2, z2;
                         scale_words(sw[i] & 0xffffu, bw[i] & 0xffffu, s2, z2);
 #pragma unroll
@@ -891,17 +887,18 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                                 for (uint32_t e = 0; e < 32 / kWordsPerBlock; ++e) o[w * (32 / kWordsPerBlock) + e] = w4[e];
                             }
                             if (h == 0) {
-                                if (!free && !pipe_wait(&na_empty[st], par)) { give_up(); break; }
+                                if (!free && !pipe_wait(&na_empty[a_st], a_par)) { give_up(); break; }
                                 __syncwarp();
                                 tc_fence_after();   // the stage's last readers are done
                             }
-                            tmem_st16(a_tmem + st * 128 + h * 16, o);
+                            tmem_st16(a_tmem + a_st * 128 + h * 16, o);
                         }
                         if (i + 1 < kOwn && kb + 2 < KB) load_packed(2 * (i + 1));
                         tmem_st_wait();
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(&na_full[st]);
+                        if (lane == 0) mbar_arrive(&na_full[a_st]);
+                        next_pair();
                     }
                     // handed back only here: the values read from them have been consumed
                     const bool sc_done = SCT && (++in_sc == 2 * kSlotsPerSc || last);
@@ -925,12 +922,11 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                 }
                 if (failed()) break;
                 if (half && (KB & 1)) {   // the last pair has no second K block
-                    const uint32_t c = kc + KB / 2;
-                    if (!pipe_wait(&na_empty[c % kNarrowA], ((c / kNarrowA) & 1) ^ 1)) { give_up(); break; }
+                    if (!pipe_wait(&na_empty[a_st], a_par)) { give_up(); break; }
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&na_full[c % kNarrowA]);
+                    if (lane == 0) mbar_arrive(&na_full[a_st]);
+                    next_pair();
                 }
-                kc += (KB + 1) / 2;
                 if (t.count > kSmallN && !own_epilogue(std::integral_constant<int, 4>(), n, 128u)) break;
             }
         }
