@@ -98,7 +98,10 @@ struct StreamArgs {
     void* hidden;
     uint32_t phases;                                 // bit 0, bit 1 (with phase 3); both: this launch routes its rows first
     uint32_t rcp_cpc;                                // ceil(2^32 / cells_per_chunk)
-    uint32_t token_groups;                           // of the logits: a block takes one group's rows against its share of the experts
+    // Reciprocals as quotient() takes them: of the grid, the shared and routed instances' units in phase 1, an instance's in phase
+    // 2, top_k, half a row and the blocks of a token group.
+    uint32_t rcp_grid, rcp_su, rcp_ru, rcp_u2, rcp_top_k, rcp_half, rcp_nbx;
+    uint32_t token_groups_log2;                      // of the logits: a block takes one group's rows against its share of the experts
     RouterArgs r;
     StreamGeom g;
 };
@@ -109,11 +112,16 @@ struct RouteScratch {
     uint32_t mask[kPlanMaxPairs / 32][SHRIKE_MAX_EXPERTS];
     uint64_t word[SHRIKE_MAX_EXPERTS];
     uint32_t cell[SHRIKE_MAX_EXPERTS];
+    RowScratch row[kWarps + kFinish];
 };
 // Bytes of the kernel's static shared memory: the table, the barriers and two words.
 constexpr uint32_t kStaticBytes = (sizeof(StreamTable) + 15) / 16 * 16 + (2 * (kMaxSlots + kMaxSlots2) + 1) * 8 + 24;
 
 namespace {
+
+// v / d by the reciprocal ceil(2^32 / d), exact while v * d < 2^32; 0 stands for d = 1. (A warp's division by a variable
+// takes a few hundred cycles here, the two 64-bit ones of a phase's share a thousand: most of the instructions are waited for.)
+__device__ __forceinline__ uint32_t quotient(uint32_t v, uint32_t rcp) { return rcp ? __umulhi(v, rcp) : v; }
 
 __device__ __forceinline__ bool try_slot(uint32_t addr, uint32_t parity) {
     uint32_t ok;
@@ -422,9 +430,9 @@ __device__ __forceinline__ uint32_t work_list(const StreamArgs& a, uint8_t* dsm,
         // activation rows; what follows the logits every block does for itself: another hand-over between blocks costs
         // more than the work (a row's picks 1 us by one warp, the list 1 us).
         const RouterArgs& r = a.r;
-        const uint32_t rows = r.ne + (r.gate_row ? 1u : 0u), bx = blockIdx.x / a.token_groups, by = blockIdx.x - bx * a.token_groups;
-        const uint32_t nbx = gridDim.x / a.token_groups, e0 = bx < nbx ? rows * bx / nbx : 0u, e1 = bx < nbx ? rows * (bx + 1) / nbx : 0u;
-        const uint32_t t0 = a.T * by / a.token_groups, nt = a.T * (by + 1) / a.token_groups - t0;
+        const uint32_t rows = r.ne + (r.gate_row ? 1u : 0u), tg = a.token_groups_log2, bx = blockIdx.x >> tg, by = blockIdx.x & ((1u << tg) - 1u);
+        const uint32_t nbx = gridDim.x >> tg, e0 = bx < nbx ? quotient(rows * bx, a.rcp_nbx) : 0u, e1 = bx < nbx ? quotient(rows * (bx + 1), a.rcp_nbx) : 0u;
+        const uint32_t t0 = (a.T * by) >> tg, nt = ((a.T * (by + 1)) >> tg) - t0;
         const uint32_t row_bytes = r.bits ? D * r.bits / 8 : D * 4, n_exp = min(e1, r.ne) - min(e0, r.ne), groups = D / 64;
         const bool gate_here = r.gate_row && e1 == rows && e1 > e0;
         const uint32_t gate_at = ring0 + n_exp * row_bytes, sb_at = gate_at + (gate_here ? D * 4 : 0u);
@@ -460,17 +468,22 @@ __device__ __forceinline__ uint32_t work_list(const StreamArgs& a, uint8_t* dsm,
             const uint32_t here = min(room, nt - s0);
             if (s0) __syncthreads();
             if (e1 > e0) {
-#pragma unroll 4
-                for (uint32_t j = tid; j < here * quads; j += kThreads) {
-                    const uint32_t row = j / quads, c = j - row * quads;
-                    float x[4];
-                    load_act4((const uint8_t*)r.hidden + (t0 + s0 + row) * x_stride, c, r.dt, x);
+                for (uint32_t c = tid; c < quads; c += kThreads) {
+                    float es[4] = {1.f, 1.f, 1.f, 1.f};
                     if (r.eff_scale) {
                         const uint2 e = __ldg((const uint2*)r.eff_scale + c);
-                        x[0] = __fmul_rn(x[0], __uint_as_float(e.x << 16)); x[1] = __fmul_rn(x[1], __uint_as_float(e.x & 0xffff0000u));
-                        x[2] = __fmul_rn(x[2], __uint_as_float(e.y << 16)); x[3] = __fmul_rn(x[3], __uint_as_float(e.y & 0xffff0000u));
+                        es[0] = __uint_as_float(e.x << 16); es[1] = __uint_as_float(e.x & 0xffff0000u);
+                        es[2] = __uint_as_float(e.y << 16); es[3] = __uint_as_float(e.y & 0xffff0000u);
                     }
-                    sts128(xs_at + row * x_bytes + c * 16, __float_as_uint(x[0]), __float_as_uint(x[1]), __float_as_uint(x[2]), __float_as_uint(x[3]));
+#pragma unroll 8
+                    for (uint32_t row = 0; row < here; ++row) {
+                        float x[4];
+                        load_act4((const uint8_t*)r.hidden + (t0 + s0 + row) * x_stride, c, r.dt, x);
+                        if (r.eff_scale)
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) x[i] = __fmul_rn(x[i], es[i]);
+                        sts128(xs_at + row * x_bytes + c * 16, __float_as_uint(x[0]), __float_as_uint(x[1]), __float_as_uint(x[2]), __float_as_uint(x[3]));
+                    }
                 }
             }
             if (s0 == 0)   // the fp16 operand copy of all rows, by all blocks
@@ -526,7 +539,7 @@ __device__ __forceinline__ uint32_t work_list(const StreamArgs& a, uint8_t* dsm,
         for (uint32_t row = warp; row < a.T; row += kWarps + kFinish) {
             uint32_t id;
             float w;
-            select_row<true>(r.logits + (size_t)row * r.ne, r, lane, id, w);
+            select_row_ranked<true>(r.logits + (size_t)row * r.ne, r, lane, rs.row[warp], id, w);
             const uint32_t p = row * r.top_k + lane, e = min(id, r.ne - 1u);
             bool live = false;
             if (lane < r.top_k) {
@@ -660,12 +673,13 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
         const uint32_t su = P1 ? a.f_shared / 8 : D / 16, ru = P1 ? a.f / 8 : D / 16, sh_units = n_sh * su;
         // this block's units: [v0, v0 + n) of [shared instances' | routed instances']
         const uint32_t total = sh_units + (n_inst - n_sh) * ru;
-        const uint32_t v0 = (uint32_t)((uint64_t)total * blockIdx.x / gridDim.x);
-        const uint32_t n = (uint32_t)((uint64_t)total * (blockIdx.x + 1) / gridDim.x) - v0;
+        const uint32_t each = quotient(total, a.rcp_grid), over = total - each * gridDim.x;
+        const uint32_t v0 = each * blockIdx.x + min(blockIdx.x, over), n = each + (blockIdx.x < over ? 1u : 0u);
+        const uint32_t rcp_su = P1 ? a.rcp_su : a.rcp_u2, rcp_ru = P1 ? a.rcp_ru : a.rcp_u2;
         auto find = [&](uint32_t j, uint32_t& i, uint32_t& k) {   // unit j -> instance, unit in it
             const uint32_t v = v0 + j;
-            if (v < sh_units) { i = v / su; k = v - i * su; }
-            else { const uint32_t w = v - sh_units, q = w / ru; i = n_sh + q; k = w - q * ru; }
+            if (v < sh_units) { i = quotient(v, rcp_su); k = v - i * su; }
+            else { const uint32_t w = v - sh_units, q = quotient(w, rcp_ru); i = n_sh + q; k = w - q * ru; }
         };
         auto step = [&](uint32_t& i, uint32_t& k) {
             k += pace;
@@ -748,22 +762,26 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
             }
             if (later) __syncthreads();   // the buffers' last readers are done
             later = true;
-            {   // groups of the instances in turn over all warps, two at a time
-                uint32_t ii = i0, j = warp;
-                auto next = [&](const uint16_t*& row, uint32_t& ji, uint32_t& groups, uint32_t& cnt, uint32_t& buf) {
-                    for (;;) {
-                        if (ii >= i1) return false;
-                        groups = (P1 ? D : ii < n_sh ? a.f_shared : a.f) / GROUP;
-                        const uint32_t g4 = (groups + 3) & ~3u;
-                        if (j < g4) break;
+            {   // the instances' groups, in shares of neighbours over all warps (two or more at a time cost registers that the
+                // loops below then spill: 16 rows 500 us over eight layers, 508 and 516)
+                const uint32_t n_s = i0 < n_sh ? min(n_sh, i1) - i0 : 0u;
+                const uint32_t gs = ((P1 ? D : a.f_shared) / GROUP + 3) & ~3u, gr = ((P1 ? D : a.f) / GROUP + 3) & ~3u;
+                const uint32_t all = n_s * gs + (i1 - i0 - n_s) * gr;
+                uint32_t left = all * (warp + 1) / (kWarps + kFinish), ii = i0, j = all * warp / (kWarps + kFinish);
+                left -= j;
+                while (left) {
+                    const bool sh = ii < n_sh;
+                    const uint32_t g4 = sh ? gs : gr;
+                    if (j >= g4) {
                         j -= g4;
                         ++ii;
+                        continue;
                     }
-                    const bool sh = ii < n_sh;
-                    cnt = tab.count[ii];
+                    const uint32_t groups = (P1 ? D : sh ? a.f_shared : a.f) / GROUP, cnt = tab.count[ii];
                     const uint32_t p = pair_of(ii, min(g, cnt - 1u));   // past the count: the last row
+                    const uint16_t* row;
                     if constexpr (P1) {
-                        row = a.xh + (size_t)(sh ? p : p / a.top_k) * D;
+                        row = a.xh + (size_t)(sh ? p : quotient(p, a.rcp_top_k)) * D;
                     } else {
                         const uint32_t F = sh ? a.f_shared : a.f;
                         row = (sh ? a.acts_shared : a.acts) + (size_t)p * F;
@@ -779,22 +797,15 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
                             if (!ok) give_up();
                         }
                     }
-                    ji = j;
-                    buf = dsm0 + __shfl_sync(0xffffffffu, at, ii - i0);
-                    j += kWarps + kFinish;
-                    return true;
-                };
-                for (;;) {
-                    const uint16_t *ra, *rb2;
-                    uint32_t ja, jb, ga, gb, ca, cb, ba, bb;
-                    uint32_t xa[GROUP / 8], xb[GROUP / 8];
-                    if (!next(ra, ja, ga, ca, ba)) break;
-                    if (ja < ga) load_group<GROUP>(ra, ja, t, xa);
-                    const bool two = next(rb2, jb, gb, cb, bb);
-                    if (two && jb < gb) load_group<GROUP>(rb2, jb, t, xb);
-                    stage_group<BITS, GROUP>(xa, ja, ga, ca, ba, BufferLayout(ga, H, ca), lane);
-                    if (!two) break;
-                    stage_group<BITS, GROUP>(xb, jb, gb, cb, bb, BufferLayout(gb, H, cb), lane);
+                    const uint32_t buf = dsm0 + __shfl_sync(0xffffffffu, at, ii - i0);
+                    const BufferLayout lay(groups, H, cnt);
+                    const uint32_t end = min(j + left, g4);
+                    left -= end - j;
+                    for (; j < end; ++j) {
+                        uint32_t x[GROUP / 8];
+                        if (j < groups) load_group<GROUP>(row, j, t, x);
+                        stage_group<BITS, GROUP>(x, j, groups, cnt, buf, lay, lane);
+                    }
                 }
             }
             __syncthreads();
@@ -969,7 +980,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
     uint32_t live = 0;
     float h0 = 0.f, h1 = 0.f;
     if (j < items) {
-        live = tab.live[j / half];
+        live = tab.live[quotient(j, a.rcp_half)];
         if (a.hidden) {
             h0 = load_act(a.hidden, (size_t)j * 2, a.act_dtype);
             h1 = load_act(a.hidden, (size_t)j * 2 + 1, a.act_dtype);
@@ -977,7 +988,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
     }
     if (!grid_sync(a.arrived)) give_up();
     for (bool first = true; j < items; j += stride, first = false) {
-        const uint32_t tk = j / half, c = j - tk * half;
+        const uint32_t tk = quotient(j, a.rcp_half), c = j - tk * half;
         if (!first) live = tab.live[tk];
         float2 s = make_float2(0.f, 0.f), p[SHRIKE_MAX_TOP_K];
         if (n_sh) s = __ldcg((const float2*)(a.parts + ((size_t)a.T * a.top_k + tk) * D) + c);
@@ -1006,6 +1017,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
 namespace {
 
 inline uint32_t align_up(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
+// What quotient() takes for a division by d (nothing is divided by a zero).
+inline uint32_t reciprocal(uint32_t d) { return d < 2 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d); }
 
 // Shared-memory layout; false when the shape does not fit.
 bool stream_geometry(const shrike_moe_config& c, uint32_t smem_optin, StreamGeom& g) {
@@ -1043,6 +1056,9 @@ bool stream_geometry(const shrike_moe_config& c, uint32_t smem_optin, StreamGeom
     };
     if (!team_of(pieces(c.d), g.slot_bytes, kMaxSlots, g.w1, g.n_slots)) return false;
     if (!team_of(most_pieces2, g.w_bytes2 + g.m_bytes2, kMaxSlots2, g.w2, g.n_slots2)) return false;
+    // quotient()'s products: units of all instances times those of one or the blocks, pairs of elements times those of a row
+    const uint64_t units = std::max(std::max(c.f, c.has_shared ? c.shared_f : 0u) / 8, c.d / 16);
+    if (kMaxTable * units * std::max<uint64_t>(units, 4096) >= 1ull << 32 || (uint64_t)SHRIKE_MAX_DECODE_TOKENS * c.d / 2 * (c.d / 2) >= 1ull << 32) return false;
     const uint32_t ring = std::max(g.n_slots * g.slot_bytes, g.n_slots2 * (g.w_bytes2 + g.m_bytes2));
     const uint32_t red = std::max(g.n_slots * g.w1, g.w2 > 1 ? g.n_slots2 * g.w2 : 0u) * kRedWarp * 4;
     if (ring + red + least > budget) return false;
@@ -1100,15 +1116,16 @@ size_t stream_parts_bytes(const shrike_moe_config& c) {
 
 size_t stream_done_bytes() { return kMaxTable * 4; }
 
-// How many groups the call's rows form for the logits: with more rows than two warps' worth a block takes a part of them
-// against more expert rows, since the experts' rows are on the block's chip already and the activations are not. 0 when a
+// How many groups the call's rows form for the logits: with more than a few rows a block takes a part of them against more
+// expert rows. Its own activation rows are what it waits for (us over eight layers, 16 rows: 1 group 529, 2 groups 516, 4 groups 508;
+// over four layers of 32 experts of 2880 x 2880, 64 rows: 4 groups 989, 8 groups 968). 0 when a
 // block's rows of the router do not fit into the ring, or there is no block for every row (block t writes row t's picks): both
 // only on a part of a GPU.
 static uint32_t stream_token_groups(const shrike_moe_config& c, uint32_t sm_count, uint32_t T, uint32_t ring_bytes) {
     const uint32_t rows = c.num_experts + (c.shared_gated ? 1u : 0u), bits = c.router_weight_bits;
     const uint32_t row_bytes = bits ? c.d * bits / 8 + c.d / 64 * 8 : c.d * 4;
     if (T > sm_count) return 0;
-    for (uint32_t n = T <= 16 ? 1 : T <= 32 ? 2 : 4; n; n /= 2) {
+    for (uint32_t n = T <= 2 ? 1 : T <= 4 ? 2 : T <= 16 ? 4 : 8; n; n /= 2) {
         const uint32_t nbx = sm_count / n, most = (rows + nbx - 1) / nbx;
         if (nbx && most * row_bytes + c.d * 4 + 16 + 2 * c.d * 4 <= ring_bytes) return n;
     }
@@ -1135,12 +1152,20 @@ cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const Exp
     a.parts = m->ws.parts; a.sorted = ea.sorted; a.pair_cell = m->ws.pair_cell;
     if (route) {
         a.r = *route;
-        a.token_groups = stream_token_groups(c, m->sm_count, T, a.g.ring_bytes);
-        if (!a.token_groups) return cudaErrorNotSupported;
+        const uint32_t groups = stream_token_groups(c, m->sm_count, T, a.g.ring_bytes);
+        if (!groups) return cudaErrorNotSupported;
+        while ((2u << a.token_groups_log2) <= groups) ++a.token_groups_log2;
+        a.rcp_nbx = reciprocal(m->sm_count / groups);
     }
     a.route_w = ea.route_w; a.shared_gate = ea.shared_gate; a.status = ea.status; a.arrived = m->ws.arrived; a.inst_done = m->ws.inst_done;
     a.T = T; a.y = y; a.hidden = hidden; a.phases = phases;
     a.rcp_cpc = (uint32_t)(((1ull << 32) + cpc - 1) / cpc);
+    a.rcp_grid = reciprocal(m->sm_count);
+    a.rcp_su = reciprocal(a.f_shared / 8);
+    a.rcp_ru = reciprocal(c.f / 8);
+    a.rcp_u2 = reciprocal(c.d / 16);
+    a.rcp_top_k = reciprocal(c.top_k);
+    a.rcp_half = reciprocal(c.d / 2);
     const uint32_t bits = c.weight_bits, grp = c.group_size;
     const bool f16 = c.meta_dtype == SHRIKE_DTYPE_FP16;
     if (bits == 4 && grp == 64 && !f16) return launch_stream_m<4, 64, SHRIKE_DTYPE_BF16>(m, st, a, *maps, pdl);

@@ -86,8 +86,11 @@ __device__ __forceinline__ float selection_weight(const float* lg, const A& a, u
         const float mx = __shfl_sync(0xffffffffu, my_score, 0);
         val = lane < top_k ? exp_det(__fsub_rn(my_score, mx)) : 0.f;
     }
-    float sum = 0.f;
-    for (uint32_t r = 0; r < top_k; ++r) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, val, r));
+    float part[SHRIKE_MAX_TOP_K], sum = 0.f;   // (zeros past top_k leave the sum as it is)
+#pragma unroll
+    for (int r = 0; r < SHRIKE_MAX_TOP_K; ++r) part[r] = __shfl_sync(0xffffffffu, val, r);
+#pragma unroll
+    for (int r = 0; r < SHRIKE_MAX_TOP_K; ++r) sum = __fadd_rn(sum, part[r]);
     float w;
     if (a.sigmoid_scores) w = __fmul_rn(val, __fdiv_rn(a.scaling, __fadd_rn(sum, 1e-20f)));
     else w = __fdiv_rn(val, sum);
@@ -97,34 +100,30 @@ __device__ __forceinline__ float selection_weight(const float* lg, const A& a, u
     return w;
 }
 
-// Top-k of one row by one warp. The (score desc, expert asc) order is total,
-// so K rounds of a warp arg-max give exactly the list the reference's
-// insertion scan builds (moe.metal:436-456). Lane r returns the r-th pick.
-// CG: read the logits past L1 (they were written by other blocks of this launch).
+// The lane's eight experts' selection keys: all logits (and biases) are requested before the first is used.
 template <bool CG, class A>
-__device__ __forceinline__ void select_row(const float* lg, const A& a, uint32_t lane,
-                                           uint32_t& out_id, float& out_w) {
-    const uint32_t ne = a.ne, top_k = a.top_k;
-    // order-preserving integer keys (0 = not a candidate): one warp-wide max and one warp-wide min per pick
-    uint32_t key[8];
-    {
-        // all logits (and biases) are requested before the first is used
-        float raw[8];
-        uint16_t lb[8];
+__device__ __forceinline__ void row_keys(const float* lg, const A& a, uint32_t lane, uint32_t (&key)[8]) {
+    const uint32_t ne = a.ne;
+    float raw[8];
+    uint16_t lb[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t e = lane + 32 * i;
-            raw[i] = e < ne ? (CG ? __ldcg(lg + e) : lg[e]) : 0.f;
-            lb[i] = a.logit_bias && e < ne ? a.logit_bias[e] : (uint16_t)0;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float score = a.sigmoid_scores ? sigmoid_det(raw[i]) : raw[i];
-            key[i] = lane + 32 * i < ne ? key_of_score(__fadd_rn(score, bf16_bits_to_f32(lb[i]))) : 0u;
-        }
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t e = lane + 32 * i;
+        raw[i] = e < ne ? (CG ? __ldcg(lg + e) : lg[e]) : 0.f;
+        lb[i] = a.logit_bias && e < ne ? a.logit_bias[e] : (uint16_t)0;
     }
-    float my_score = 0.f;
-    uint32_t my_id = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float score = a.sigmoid_scores ? sigmoid_det(raw[i]) : raw[i];
+        key[i] = lane + 32 * i < ne ? key_of_score(__fadd_rn(score, bf16_bits_to_f32(lb[i]))) : 0u;
+    }
+}
+// top_k rounds of a warp arg-max (order-preserving integer keys, 0 = not a candidate: one warp-wide max and one warp-wide min
+// per pick). The (score desc, expert asc) order is total, so this is exactly the list the reference's insertion scan builds
+// (moe.metal:436-456). Lane r gets the r-th pick.
+__device__ __forceinline__ void pick_rounds(uint32_t (&key)[8], uint32_t top_k, uint32_t lane, uint32_t& my_key, uint32_t& my_id) {
+    my_key = my_id = 0;
+#pragma unroll 1
     for (uint32_t r = 0; r < top_k; ++r) {
         uint32_t bestk = 0;
 #pragma unroll
@@ -139,28 +138,82 @@ __device__ __forceinline__ void select_row(const float* lg, const A& a, uint32_t
             for (int i = 0; i < 8; ++i) key[i] = (win >> 5) == (uint32_t)i ? 0u : key[i];
         }
         if (lane == r) {
-            my_score = score_of_key(wmax);
+            my_key = wmax;
             my_id = win == 0xffffffffu ? 0u : win;
         }
     }
-    // weights (moe.metal:458-490), sums in rank order
-    float val;
-    if (a.sigmoid_scores) {
-        val = lane < top_k ? sigmoid_det(CG ? __ldcg(lg + my_id) : lg[my_id]) : 0.f;
-    } else {
-        const float mx = __shfl_sync(0xffffffffu, my_score, 0);
-        val = lane < top_k ? exp_det(__fsub_rn(my_score, mx)) : 0.f;
+}
+
+// Top-k of one row by one warp. Lane r returns the r-th pick.
+// CG: read the logits past L1 (they were written by other blocks of this launch).
+template <bool CG, class A>
+__device__ __forceinline__ void select_row(const float* lg, const A& a, uint32_t lane,
+                                           uint32_t& out_id, float& out_w) {
+    uint32_t key[8], my_key;
+    row_keys<CG>(lg, a, lane, key);
+    pick_rounds(key, a.top_k, lane, my_key, out_id);
+    out_w = selection_weight<CG>(lg, a, lane, score_of_key(my_key), out_id);
+}
+
+// The same without the serial rounds, in shared memory of the warp's own: the eighth best of the lanes' best keys is a bound
+// that the eight best experts reach, and few others do. Those are ranked by comparing each with all; more than 32 (ties
+// by the dozen) are left to the rounds. (A row's picks by one warp, 256 experts: 4900 -> 4400 cycles.)
+struct alignas(16) RowScratch {
+    uint32_t best[32];
+    uint2 cand[32];                       // {key, expert}
+    uint2 pick[SHRIKE_MAX_TOP_K];
+};
+template <bool CG, class A>
+__device__ __forceinline__ void select_row_ranked(const float* lg, const A& a, uint32_t lane, RowScratch& rs, uint32_t& out_id,
+                                                  float& out_w) {
+    static_assert(SHRIKE_MAX_TOP_K == 8, "eight lanes' best");
+    uint32_t key[8], best = 0;
+    row_keys<CG>(lg, a, lane, key);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) best = max(best, key[i]);
+    __syncwarp();                         // the last row's entries have been read
+    rs.best[lane] = best;
+    rs.cand[lane] = make_uint2(0u, 0u);
+    if (lane < SHRIKE_MAX_TOP_K) rs.pick[lane] = make_uint2(0u, 0u);
+    __syncwarp();
+    uint32_t rank[2] = {0, 0};
+#pragma unroll
+    for (uint32_t j = 0; j < 32; j += 4) {
+        const uint4 v = *(const uint4*)&rs.best[j];
+        const uint32_t o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) rank[q & 1] += (o[q] > best || (o[q] == best && j + q < lane)) ? 1u : 0u;
     }
-    float sum = 0.f;
-    for (uint32_t r = 0; r < top_k; ++r) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, val, r));
-    float w;
-    if (a.sigmoid_scores) w = __fmul_rn(val, __fdiv_rn(a.scaling, __fadd_rn(sum, 1e-20f)));
-    else w = __fdiv_rn(val, sum);
-    const float pes = a.per_expert_scale ? bf16_bits_to_f32(a.per_expert_scale[my_id]) : 1.0f;
-    w = __fmul_rn(w, pes);
-    if (a.round_f16) w = __half2float(__float2half_rn(w));
+    const uint32_t bound = __shfl_sync(0xffffffffu, best, __ffs(__ballot_sync(0xffffffffu, rank[0] + rank[1] == 7u)) - 1);
+    uint32_t n = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+        const bool in = key[i] != 0u && key[i] >= bound;
+        const uint32_t b = __ballot_sync(0xffffffffu, in), at = n + __popc(b & ((1u << lane) - 1u));
+        if (in && at < 32u) rs.cand[at] = make_uint2(key[i], lane + 32u * i);
+        n += __popc(b);
+    }
+    uint32_t my_key = 0, my_id = 0;
+    if (n <= 32u) {
+        __syncwarp();
+        const uint2 mine = rs.cand[lane];
+        uint32_t r = 0;
+#pragma unroll 4
+        for (uint32_t j = 0; j < n; ++j) {
+            const uint2 o = rs.cand[j];
+            r += (o.x > mine.x || (o.x == mine.x && o.y < mine.y)) ? 1u : 0u;
+        }
+        if (lane < n && r < SHRIKE_MAX_TOP_K) rs.pick[r] = mine;
+        __syncwarp();
+        if (lane < a.top_k) {
+            my_key = rs.pick[lane].x;
+            my_id = rs.pick[lane].y;
+        }
+    } else {
+        pick_rounds(key, a.top_k, lane, my_key, my_id);
+    }
     out_id = my_id;
-    out_w = w;
+    out_w = selection_weight<CG>(lg, a, lane, score_of_key(my_key), my_id);
 }
 
 struct alignas(16) SelectSmem {

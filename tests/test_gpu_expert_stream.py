@@ -83,3 +83,21 @@ def test_blocks_that_end_with_weights(cuda_device):
     for T in (3, 17):
         check_layer(layer, inputs(T, cfg.d, seed=T), fused=True)
     layer.close()
+
+
+@pytest.mark.parametrize("k", [3, 8])
+@pytest.mark.parametrize("alike,left", [(9, 64), (32, 64), (33, 64), (64, 64), (9, 5), (1, 8), (40, 36)])
+def test_picks_among_equal_scores(cuda_device, alike, left, k):
+    """Experts whose router rows are the same score the same: of up to 32 candidates the lower ids win by comparison, of more by
+    rounds. `left` experts have a score at all (the others' bias is minus infinity): fewer than the picks leave id 0."""
+    bias = np.where(np.arange(64) < left, 0.0, -np.inf).astype(np.float32)
+    layer = Layer(small_config(num_experts=64, top_k=k), logit_bias=bias, router_sigma=0.2)
+    at = np.random.default_rng(alike).permutation(64)[:alike]
+    layer.router_w[at] = 3 * layer.router_w[at[0]]
+    layer._rw.copy_(torch.from_numpy(layer.router_w))
+    x = inputs(24, layer.cfg.d, seed=alike)
+    _, ids, w, _ = layer.forward(x, fused=True)
+    ids_ref, w_ref, _ = layer.oracle_route(x)
+    assert (ids == ids_ref).all()
+    assert np.array_equal(w, w_ref, equal_nan=True)
+    layer.close()
