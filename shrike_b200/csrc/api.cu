@@ -1115,7 +1115,7 @@ int shrike_ep_forward(shrike_ep* ep, void* stream, const shrike_pool* local_pool
     if (with_shared) CU(cudaStreamWaitEvent(st, ep->ev_shared, 0));
     if (T)
         CU(launch_ep_combine(m, st, ep->mine + ep->lay.off_ret, ep->row_of, with_shared ? ep->y_home : nullptr, T, ep->world,
-                             ep->cap, y, hidden));
+                             ep->cap, y, hidden, r->ws.yacc, ep->prefix, ep->rank));
     return SHRIKE_OK;
 }
 

@@ -251,7 +251,8 @@ cudaError_t launch_ep_dispatch(const shrike_moe* m, cudaStream_t st, const void*
 cudaError_t launch_ep_local_slots(const shrike_moe* m, cudaStream_t st, const uint32_t* recv_ids,
                                   const uint64_t* table, uint32_t rows, uint32_t* slots);
 cudaError_t launch_ep_combine(const shrike_moe* m, cudaStream_t st, const void* recv_y, const int32_t* row_of,
-                              const void* y_home, uint32_t T, uint32_t world, uint32_t cap, void* y, void* hidden);
+                              const void* y_home, uint32_t T, uint32_t world, uint32_t cap, void* y, void* hidden,
+                              const float* own = nullptr, const uint32_t* own_first = nullptr, uint32_t own_rank = 0);
 }  // namespace shrike
 
 namespace shrike {

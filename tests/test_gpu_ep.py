@@ -381,3 +381,28 @@ def test_int8_shared_expert_beside_int4_routed_experts(cuda_device, T):
     got = y.cpu().numpy()
     assert np.linalg.norm(got - y_ref) / np.linalg.norm(y_ref) <= 1e-3
     layer.close()
+
+
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+def test_output_rows_that_are_not_whole_vectors(cuda_device, dtype):
+    """y and hidden one element into a buffer: combined by single elements, with the results of aligned rows. (The down
+    projection's sums are added in no fixed order: two units of the last place.)"""
+    from shrike_b200 import capi
+    from shrike_b200.moe import RouterOperands
+    cfg = _config(act=capi.DTYPE_FP32 if dtype == "fp32" else capi.DTYPE_BF16)
+    x, router = _problem(40, cfg)
+    layer = _build_layer(cfg, 0, 1, 40, 9, "peer")
+    ops = RouterOperands(weights=torch.from_numpy(router).to(layer.dev))
+    xl = torch.from_numpy(x).to(layer.dev).to(cfg.torch_act_dtype)
+    got = []
+    for skip in (0, 1):
+        y = torch.zeros(xl.numel() + 8, dtype=cfg.torch_y_dtype, device=layer.dev)[skip:skip + xl.numel()].view(xl.shape)
+        h = torch.zeros(xl.numel() + 8, dtype=xl.dtype, device=layer.dev)[skip:skip + xl.numel()].view(xl.shape).copy_(xl)
+        layer.forward(ops, xl, y, h)
+        layer.status()
+        got.append((y.float(), h.float()))
+    layer.close()
+    ulp = 2.0 ** (-22 if dtype == "fp32" else -7)
+    assert not torch.equal(got[0][0], torch.zeros_like(got[0][0]))
+    for a, b in zip(*got):
+        assert ((a - b).abs() <= 2 * ulp * a.abs() + 1e-6 * a.abs().max()).all()
