@@ -439,7 +439,9 @@ typedef struct shrike_stack_layer {
 /* A decode step through stacked MoE layers with host activations in and out: what produceToken's per-layer
  * encodeRoutedLayer calls (RealForwardRunner.swift:2205-2313) amount to for this path when only the MoE
  * halves of the layers are present. The stack owns a device copy of the residual stream,
- * [(layer_count + 1) x max_rows x d] in act_dtype.
+ * [(layer_count + 1) x max_rows x d] in act_dtype, and the launches of a step of max_rows rows as a graph, made with
+ * it: the layers' operand structures are read then too. Steps of fewer rows, and steps whose structures read
+ * differently, launch layer by layer.
  *
  *   rows_host   [(layer_count + 1) x query_count x d]: block 0 is the row set entering layer 0; block l >= 1 is
  *               what the rest of transformer block l (attention, normalisation -- not part of this library)

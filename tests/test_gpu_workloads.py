@@ -206,3 +206,43 @@ def test_decode_stack_host_entry_point_equals_the_layer_calls(cuda_device, T):
     stack.close()
     for L in layers:
         L.close()
+
+
+@pytest.mark.parametrize("T", [1, 5])
+def test_decode_stack_with_other_rows_or_operands(cuda_device, T):
+    """A stack's launches for max_rows are captured when it is made. Calls of fewer rows, and calls after an operand was
+    replaced in the caller's structures, give what a stack made for them gives."""
+    import torch
+    from shrike_b200.moe import DecodeStack
+    cfg = fx.qwen_config(max_tokens=16, d=512, f=256, shared_f=256, num_experts=64, y_dtype=capi.DTYPE_FP32)
+    layers = [Layer(cfg, seed=170 + l, device_fill=True) for l in range(3)]
+
+    def rows(n, seed):
+        return torch.from_numpy(np.stack([fx.round_bf16(inputs(n, cfg.d, seed=seed + l)) for l in range(4)])).to(torch.bfloat16)
+
+    def run(stack, x):
+        out = torch.empty(x.shape[1:], dtype=x.dtype)
+        stack.forward_host(x, out)
+        return out
+
+    def made(n):
+        return DecodeStack([(L.moe, L.pool, L.offsets, 0, L.router_ops, L.shared) for L in layers], n)
+
+    stack, exact = made(T + 1), made(T)
+    x = rows(T, 80)
+    before = run(exact, x)
+    assert torch.equal(run(stack, x), before)
+    # another router, in the structure that the stack points to
+    ops = exact._keep[0]
+    other = layers[0].router_ops.weights.flip(0).contiguous()
+    ops.weights = other.data_ptr()
+    changed = run(exact, x)
+    assert not torch.equal(changed, before)
+    layers[0].router_ops.weights = other
+    fresh = made(T)
+    assert torch.equal(run(fresh, x), changed)
+    for s in (stack, exact, fresh):
+        s.close()
+    for L in layers:
+        L.moe.status()
+        L.close()
