@@ -217,8 +217,9 @@ cudaError_t launch_group_pairs(const shrike_moe* m, cudaStream_t st, const uint3
         if (e != cudaSuccess) return e;
         return cudaMemsetAsync(offsets, 0xff, ne * 4, st);
     }
-    group_hist_kernel<<<nb, 256, 0, st>>>(ids, T, k, ne, m->ws.block_hist, m->ws.status, slots, io_status,
+    cudaError_t eh = launch_after(m, st, group_hist_kernel, dim3(nb), 256, 0, ids, T, k, ne, m->ws.block_hist, m->ws.status, slots, io_status,
                                           m->ws.slot_of_expert);
+    if (eh != cudaSuccess) return eh;
     cudaError_t e = launch_after(m, st, group_scan_kernel, dim3(1), 256, 0, m->ws.block_hist, nb, ne, offsets, counts);
     if (e != cudaSuccess) return e;
     return launch_after(m, st, group_place_kernel, dim3(nb), 256, 0, ids, weights, T, k, ne, m->ws.block_hist, sorted_pairs,

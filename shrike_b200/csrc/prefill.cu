@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(256)
 prefill_xprep_kernel(const void* __restrict__ x, uint32_t T, uint32_t d, uint32_t group, uint32_t act_dtype,
                      uint32_t int4, uint16_t* __restrict__ xh, float* __restrict__ xsum, uint32_t* status,
                      const uint32_t* __restrict__ row_map, const uint32_t* __restrict__ n_rows_dev,
-                     const uint32_t* __restrict__ pos_of_pair, uint32_t top_k, uint16_t* __restrict__ xs) {
+                     const uint32_t* __restrict__ pos_of_pair, uint32_t top_k, uint16_t* __restrict__ xs, float* __restrict__ zero) {
     pdl_wait();
     pdl_launch_dependents();
     const uint32_t items = T * (d / 8);
@@ -77,6 +77,15 @@ prefill_xprep_kernel(const void* __restrict__ x, uint32_t T, uint32_t d, uint32_
     for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < items; i0 += gridDim.x * blockDim.x) {
         const uint32_t i = i0 + threadIdx.x;
         xprep_item(x, row_bytes, d, group, act_dtype, int4 != 0, i, i < items, xh, xsum, status, row_map, n_rows);
+        if (i < items) {   // the rows that the down projection adds into
+            float* const z = zero + (size_t)i * 8;
+            if (((uintptr_t)zero & 15u) == 0) {
+                ((float4*)z)[0] = ((float4*)z)[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+            } else {   // (the caller's own rows)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) z[k] = 0.f;
+            }
+        }
         const uint32_t row = i / (d / 8);
         if (!pos_of_pair || i >= items || row >= n_rows) continue;
         const uint4 v = *(const uint4*)(xh + (size_t)i * 8);   // this thread's own
@@ -110,10 +119,7 @@ cudaError_t launch_prefill_plan(const shrike_moe* m, cudaStream_t st, const uint
                                 const uint32_t* row_map, const uint32_t* n_rows, float* accumulator) {
     const shrike_moe_config& c = m->cfg;
     const Workspace& ws = m->ws;
-    // the rows the down epilogue adds into: the workspace's, or the caller's fp32 output itself
-    cudaError_t e = cudaMemsetAsync(accumulator ? accumulator : ws.yacc, 0, (size_t)T * c.d * 4, st);
-    if (e != cudaSuccess) return e;
-    e = launch_group_pairs(m, st, ids, nullptr, T, nullptr, ws.expert_offsets, ws.expert_counts, slots, io_status);
+    cudaError_t e = launch_group_pairs(m, st, ids, nullptr, T, nullptr, ws.expert_offsets, ws.expert_counts, slots, io_status);
     if (e != cudaSuccess) return e;
     if (warp_mma_instances)   // the tensor-core path builds its own 256-row instances
         prefill_instances_kernel<<<1, 256, 0, st>>>(ws.expert_offsets, ws.expert_counts, ws.slot_of_expert,
@@ -122,7 +128,8 @@ cudaError_t launch_prefill_plan(const shrike_moe* m, cudaStream_t st, const uint
     const uint32_t items = T * (c.d / 8);
     return launch_after(m, st, prefill_xprep_kernel, dim3(min(2048u, (items + 255) / 256)), 256, 0, x, T, c.d, c.group_size, c.act_dtype,
                         c.weight_bits == 4 ? 1u : 0u, ws.xh, ws.xsum, ws.status, row_map, n_rows,
-                        (const uint32_t*)(warp_mma_instances ? nullptr : ws.pos_of_pair), c.top_k, ws.xs);
+                        (const uint32_t*)(warp_mma_instances ? nullptr : ws.pos_of_pair), c.top_k, ws.xs,
+                        accumulator ? accumulator : ws.yacc);   // the rows the down epilogue adds into: the workspace's, or the caller's fp32 output itself
 }
 
 cudaError_t launch_prefill_combine(const shrike_moe* m, cudaStream_t st, uint32_t T, void* y, void* hidden) {

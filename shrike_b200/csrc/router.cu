@@ -68,6 +68,8 @@ __device__ __forceinline__ void logits_body(const RouterArgs& a, Pre pre) {
 
 // grid (ceil((ne + has_gate)/4), token blocks)
 __global__ void __launch_bounds__(kRouterWarps * 32) router_logits_kernel(const RouterArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
     logits_body(a, [] {});
 }
 
@@ -125,6 +127,8 @@ __device__ __forceinline__ void store_tile(const RouterArgs& a, float (&v)[kTile
 }
 
 __global__ void __launch_bounds__(256, 1) router_logits_tiled_kernel(const RouterArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ __align__(16) float tile_smem[];
     float* const w_s = tile_smem;                                           // [2][32][256]
     float* const x_s = tile_smem + 2 * kTileRows * kTileStage;              // [2][32][256]
@@ -262,6 +266,8 @@ constexpr size_t kTile16SmemBytes = (size_t)kTile16Bufs * kTile16Buf;
 
 template <bool FP16>
 __global__ void __launch_bounds__(256, 1) router_logits_tiled16_kernel(const RouterArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ __align__(16) uint8_t tile16_smem[];
     const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(tile16_smem);
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -354,6 +360,8 @@ __global__ void __launch_bounds__(256, 1) router_logits_tiled16_kernel(const Rou
 // warp while the blocks fit the SMs once (333 rows: 8.3 -> 3.5 us), four beyond, where fetching the gate row again costs
 // more (4096 rows: 9 us against 11).
 __global__ void __launch_bounds__(256) router_gate_rows_kernel(const RouterArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t chunks = a.d / 4;
     const size_t esz = a.dt == SHRIKE_DTYPE_FP32 ? 4 : 2;
@@ -367,12 +375,15 @@ __global__ void __launch_bounds__(256) router_gate_rows_kernel(const RouterArgs 
 }
 
 __global__ void __launch_bounds__(128) router_select_kernel(const RouterArgs a) {
+    __shared__ RowScratch rs[4];
+    pdl_wait();
+    pdl_launch_dependents();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t row = blockIdx.x * 4 + warp;
     if (row >= a.T) return;
     uint32_t id;
     float w;
-    select_row<false>(a.logits + (size_t)row * a.ne, a, lane, id, w);
+    select_row_ranked<false>(a.logits + (size_t)row * a.ne, a, lane, rs[warp], id, w);
     if (lane < a.top_k) {
         a.ids[(size_t)row * a.top_k + lane] = id;
         a.weights[(size_t)row * a.top_k + lane] = w;
@@ -518,6 +529,8 @@ __global__ void __launch_bounds__(1024) classify_kernel(const uint32_t* __restri
                                                         uint32_t* __restrict__ miss_exp) {
     __shared__ uint32_t s_miss[1024];
     __shared__ uint32_t s_base;
+    pdl_wait();
+    pdl_launch_dependents();
     auto lookup = [&](uint32_t p, uint32_t& e, uint32_t& slot) {
         e = min(ids[p], ne - 1u);
         const uint64_t word = table[e];
@@ -527,8 +540,9 @@ __global__ void __launch_bounds__(1024) classify_kernel(const uint32_t* __restri
     if (threadIdx.x == 0) s_base = 0;
     __syncthreads();
     uint32_t before_me = 0;
+    const uint32_t earlier = counts || miss_pos || miss_exp ? blockIdx.x : 0u;   // (their misses are asked for)
 #pragma unroll 4
-    for (uint32_t j = 0; j < blockIdx.x; ++j) {
+    for (uint32_t j = 0; j < earlier; ++j) {
         uint32_t e, slot;
         before_me += lookup(j * 1024u + threadIdx.x, e, slot) ? 0u : 1u;
     }
@@ -602,16 +616,14 @@ cudaError_t launch_router(const shrike_moe* m, cudaStream_t st, const shrike_rou
                 if (e != cudaSuccess) return e;
                 attr16_set[dev] = true;
             }
-            if (a.dt == SHRIKE_DTYPE_FP16) router_logits_tiled16_kernel<true><<<grid, 256, kTile16SmemBytes, st>>>(a);
-            else router_logits_tiled16_kernel<false><<<grid, 256, kTile16SmemBytes, st>>>(a);
+            e = launch_after(m, st, a.dt == SHRIKE_DTYPE_FP16 ? router_logits_tiled16_kernel<true> : router_logits_tiled16_kernel<false>, grid, 256,
+                             kTile16SmemBytes, a);
         } else {
-            router_logits_tiled_kernel<<<grid, 256, kTileSmemBytes, st>>>(a);
+            e = launch_after(m, st, router_logits_tiled_kernel, grid, 256, kTileSmemBytes, a);
         }
-        e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         if (a.gate_row) {
-            router_gate_rows_kernel<<<T <= 8u * (uint32_t)m->sm_count ? (T + 7) / 8 : (T + 31) / 32, 256, 0, st>>>(a);
-            e = cudaGetLastError();
+            e = launch_after(m, st, router_gate_rows_kernel, dim3(T <= 8u * (uint32_t)m->sm_count ? (T + 7) / 8 : (T + 31) / 32), 256, 0, a);
             if (e != cudaSuccess) return e;
         }
     } else {
@@ -620,12 +632,10 @@ cudaError_t launch_router(const shrike_moe* m, cudaStream_t st, const shrike_rou
         else if (T > 8) tpb = 4;
         a.tokens_per_block = tpb;
         const dim3 grid((rows + kRouterWarps - 1) / kRouterWarps, (T + tpb - 1) / tpb);
-        router_logits_kernel<<<grid, kRouterWarps * 32, 0, st>>>(a);
-        e = cudaGetLastError();
+        e = launch_after(m, st, router_logits_kernel, grid, kRouterWarps * 32, 0, a);
         if (e != cudaSuccess) return e;
     }
-    router_select_kernel<<<(T + 3) / 4, 128, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_after(m, st, router_select_kernel, dim3((T + 3) / 4), 128, 0, a);
 }
 
 cudaError_t launch_route_fused(const shrike_moe* m, cudaStream_t st, const shrike_router_operands& ops,
@@ -658,9 +668,8 @@ cudaError_t launch_classify(const shrike_moe* m, cudaStream_t st, const uint32_t
                             const uint64_t* table, uint32_t T, uint32_t* slots, uint32_t* counts,
                             uint32_t* miss_pos, uint32_t* miss_exp) {
     const uint32_t n_pairs = T * m->cfg.top_k;
-    classify_kernel<<<n_pairs > 1024u ? (n_pairs + 1023u) / 1024u : 1u, 1024, 0, st>>>(ids, table, n_pairs, m->cfg.num_experts, slots, counts,
-                                                                              miss_pos, miss_exp);
-    return cudaGetLastError();
+    return launch_after(m, st, classify_kernel, dim3(n_pairs > 1024u ? (n_pairs + 1023u) / 1024u : 1u), 1024, 0, ids, table, n_pairs,
+                        m->cfg.num_experts, slots, counts, miss_pos, miss_exp);
 }
 
 }  // namespace shrike
