@@ -417,9 +417,8 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         if (!__all_sync(0xffffffffu, pipe_wait(&tile_full[s], (n / kTiles) & 1))) { give_up(); return false; }
         const uint4 v = next_tile[s];
         if (release) release_tile(n);
-        t = Tile(make_uint4(__shfl_sync(0xffffffffu, v.x, 0), __shfl_sync(0xffffffffu, v.y, 0), __shfl_sync(0xffffffffu, v.z, 0),
-                            __shfl_sync(0xffffffffu, v.w, 0)));
-        return t.count != 0 && !failed();
+        t = Tile(v);
+        return t.count != 0;
     };
     auto k_blocks = [&](const Tile& t) { return (PHASE == 0 ? a.d : t.shared ? a.f_shared : a.f) / 64; };
     // Epilogue of tile `e`, the block's n-th, by H x 4 warps: warp w reads TMEM lanes 32*(w & 3) .. +31, every H-th group of C columns
@@ -946,6 +945,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             uint32_t a_use = 0, b_use = 0, sa = 0, sb = 0;
             for (; go && !t.narrow; go = take_tile(++n, t)) {
                 was_wide = true;
+                t.count = __shfl_sync(0xffffffffu, t.count, 0);
                 const uint32_t idesc = umma_idesc((t.count + 15u) & ~15u), n_kb = __shfl_sync(0xffffffffu, k_blocks(t), 0);
                 for (uint32_t kb = 0; kb < n_kb; ++kb) {
                     // (the first stage of converted weights also says that the last tile's accumulators have been read)
@@ -982,6 +982,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         uint32_t kc = 0, sb = 0, b_par = 0;
         bool other_small = true;   // the tile before had accumulators of its own
         for (uint32_t first = n; go; go = take_tile(++n, t)) {
+            t.count = __shfl_sync(0xffffffffu, t.count, 0);   // (a value that the compiler knows to be uniform)
             const bool small = t.count <= kSmallN;
             const uint32_t idesc = umma_idesc((t.count + 15u) & ~15u), n_kb = __shfl_sync(0xffffffffu, k_blocks(t), 0);
             const uint32_t b_mask = narrow_b_mask(t.count), b_step = kNarrowBBytes / (b_mask + 1);
