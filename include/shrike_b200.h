@@ -275,7 +275,7 @@ int shrike_encode_route_decode(shrike_moe* moe, void* stream, const shrike_route
  * One launch for one row and for 2 to 64 rows. Three launches chained with
  * programmatic dependent launch where the one-launch kernels do not take the
  * shape (an odd number of weight groups in a row, a pool of single-cell chunks,
- * one row too wide for the ring) and for two rows of experts under 4 MB; of
+ * one row too wide for the ring); of
  * those, calls of more than 48 rows on a handle created for prefill
  * (max_tokens > 64) run the router, the classification and the expert-grouped
  * tensor-core path. Results agree within the parity tolerance on every path;

@@ -177,16 +177,13 @@ int fill_expert_args(shrike_moe* m, const shrike_pool* pool, const shrike_expert
 
 
 // Whether the streaming kernel is the faster one for a decode call. A single row has nothing to lay out ahead of the first
-// tile; two rows of small experts are about even (256 experts of 2048 x 512: 29.3 us a layer with the per-tile kernels,
-// 29.7 with it; three rows 34.8 and 33.9; experts of 7 MB at two rows 46.9 and 44.4). Up to 64 rows it also stays ahead of the
-// expert-grouped GEMM, which reads an expert once for all its rows but starts in a dozen launches (us a layer, streaming and
-// grouped, uniform picks; 256 experts of 2048 x 512 int4 | 32 of 2880 x 2880 int4 | 256 of 2304 x 1024 int8):
-//    4 rows  36, 67 |  92, 170 |  62, 123        32 rows   96, 199 | 190, 292 | 186, 322
-//   16 rows  67, 142 | 171, 288 | 130, 234       64 rows  129, 254 | 260, 294 | 251, 413
-// With picks by Zipf(1.1), 64 rows: 85, 124 | 257, 254 | 188, 290.
-bool stream_pays(const shrike_moe_config& c, uint32_t T) {
-    return T > 2 || (T == 2 && (uint64_t)3 * c.d * c.f * c.weight_bits / 8 >= (4u << 20));
-}
+// tile (us a layer, one-row or per-tile kernels and streaming; 256 experts of 2048 x 512 int4 | 32 of 2880 x 2880 int4 | 256 of
+// 2304 x 1024 int8: 17.0, 22.9 | 40.4, 42.0 | 34.0, 36.3); two rows have: 29.3, 27.1 | 88, 57.5 | 46.8, 43.3. Up to 64 rows it also
+// stays ahead of the expert-grouped GEMM, which reads an expert once for all its rows but starts in a dozen launches
+// (streaming and grouped, uniform picks):
+//   17 rows  69, 115 | 179, 253 | 132, 200       64 rows  131, 190 | 245, 255 | 252, 344
+// With picks by Zipf(1.1), 64 rows: 87, 113 | 245, 222 | 192, 246.
+bool stream_pays(uint32_t T) { return T > 1; }
 
 // The expert projections of a decode call's work lists (phases: 1, 2 or 3 = both, a launch each). The streaming kernel takes
 // every shape whose tiles its ring and the tiled copies can hold; the per-tile kernels take the others.
@@ -196,7 +193,7 @@ cudaError_t launch_experts(const shrike_moe* m, cudaStream_t st, const ExpertArg
     const uint32_t mi = max_instances(m->cfg, T);
     for (uint32_t phase = 1; phase <= 2; ++phase) {
         if (!(phases & phase)) continue;
-        cudaError_t e = stream_pays(m->cfg, T) ? launch_expert_stream(m, st, a, T, n_shared, y, hidden, pdl, phase) : cudaErrorNotSupported;
+        cudaError_t e = stream_pays(T) ? launch_expert_stream(m, st, a, T, n_shared, y, hidden, pdl, phase) : cudaErrorNotSupported;
         if (e == cudaErrorNotSupported)
             e = phase == 1 ? launch_phase1(m, st, a, mi, pdl) : launch_phase2(m, st, a, T, mi, y, hidden, pdl);
         if (e != cudaSuccess) return e;
@@ -732,7 +729,7 @@ int shrike_encode_decode_layer(shrike_moe* m, void* stream, const shrike_pool* p
         if (fe != cudaErrorNotSupported) return cuda_fail(m, fe, "launch_fused_layer");
         // a block layout the tiled copies cannot describe: the three launches below
     }
-    if (stream_pays(m->cfg, query_count)) {
+    if (stream_pays(query_count)) {
         // some rows: the same in one launch of the streaming kernel (expert_stream.cu). In three launches the last
         // block of the router ranked every row while the others' SMs idled (8 us of 4 rows' 43, 20 of 16 rows' 92), and
         // the next launch began 3 us later.

@@ -101,3 +101,14 @@ def test_picks_among_equal_scores(cuda_device, alike, left, k):
     assert (ids == ids_ref).all()
     assert np.array_equal(w, w_ref, equal_nan=True)
     layer.close()
+
+
+@pytest.mark.parametrize("kw", [
+    dict(d=256, f=128, shared_f=384),
+    dict(d=384, f=192, shared_f=320, group_size=32, weight_bits=4, meta_dtype=capi.DTYPE_FP16),
+    dict(d=192, f=320, shared_f=64, group_size=32, weight_bits=8, expert_bias=1, activation=capi.ACT_GELU_TANH),
+], ids=lambda kw: "-".join(f"{k}{v}" for k, v in kw.items()))
+@pytest.mark.parametrize("T", [2, 3, 5, 8])
+def test_few_rows(cuda_device, kw, T):
+    """The rows' groups in the router: one, two, four of them, with unequal numbers of rows."""
+    test_stream_edges(cuda_device, kw, T)
