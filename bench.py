@@ -235,10 +235,7 @@ class Workload:
         self.y = torch.zeros((T, cfg.d), dtype=cfg.torch_y_dtype, device=self.dev)
         self.stack = DecodeStack([(self.moes[l], self.pool, self.off, 0, self.routers[l], self.shared[l])
                                   for l in range(layers)], T)
-        # kernels of this library per layer call: one launch, except for two rows of experts under 4 MB (route +
-        # phase 1 + phase 2)
-        small = 3 * cfg.d * cfg.f * cfg.weight_bits // 8 < 4 << 20
-        self.launches_per_step = layers * (3 if T == 2 and small else 1)
+        self.launches_per_step = layers   # a layer call is one kernel
         torch.cuda.synchronize()
 
     def step_resident(self):
@@ -341,8 +338,7 @@ def decode_line(args, rank: int, world: int, local_rank: int):
     hbm, _, src = measured_peaks()
     gbs = layer_bytes / (ms / L * 1e-3) / 1e9
     kernel = ("decode_layer_kernel<4,64,bf16> (router + top-8 + lookup + gate/up + GLU + down + combine of one row, one launch)"
-              if T == 1 else "route_fused_kernel + phase1_kernel<4,64,bf16> + phase2_kernel<4,64,bf16>" if T == 2 else
-              "expert_stream_kernel<4,64,bf16> (the same of 3 to 64 rows, one launch)")
+              if T == 1 else "expert_stream_kernel<4,64,bf16> (the same of 2 to 64 rows, one launch)")
     line = None
     if rank == 0:
         tokens = T * world

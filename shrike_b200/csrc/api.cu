@@ -178,11 +178,12 @@ int fill_expert_args(shrike_moe* m, const shrike_pool* pool, const shrike_expert
 
 // Whether the streaming kernel is the faster one for a decode call. A single row has nothing to lay out ahead of the first
 // tile (us a layer, one-row or per-tile kernels and streaming; 256 experts of 2048 x 512 int4 | 32 of 2880 x 2880 int4 | 256 of
-// 2304 x 1024 int8: 17.0, 22.9 | 40.4, 42.0 | 34.0, 36.3); two rows have: 29.3, 27.1 | 88, 57.5 | 46.8, 43.3. Up to 64 rows it also
-// stays ahead of the expert-grouped GEMM, which reads an expert once for all its rows but starts in a dozen launches
-// (streaming and grouped, uniform picks):
-//   17 rows  69, 115 | 179, 253 | 132, 200       64 rows  131, 190 | 245, 255 | 252, 344
-// With picks by Zipf(1.1), 64 rows: 87, 113 | 245, 222 | 192, 246.
+// 2304 x 1024 int8: 17.0, 22.9 | 40.4, 42.0 | 34.0, 36.3); two rows have: 29.3, 27.1 | 88, 57.5 | 46.8, 43.3. Up to 64 rows it is
+// also ahead of the expert-grouped GEMM, which reads an expert once for all its rows but starts in a dozen launches, unless few
+// large experts get skewed picks, which only the device knows (streaming, when its routing took 5 to 8 us more, and grouped,
+// uniform picks):
+//   17 rows  69, 115 | 179, 253 | 132, 200       64 rows  131, 190 | 262, 255 | 252, 344
+// With picks by Zipf(1.1), 64 rows: 87, 113 | 259, 222 | 192, 246.
 bool stream_pays(uint32_t T) { return T > 1; }
 
 // The expert projections of a decode call's work lists (phases: 1, 2 or 3 = both, a launch each). The streaming kernel takes
