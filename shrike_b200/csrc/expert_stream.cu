@@ -25,10 +25,10 @@
 // All phases run in one launch when the call has them: a block asks for its first phase-2 units before it waits for
 // the other blocks' activations.
 //
-// Measured (256 experts of 2048 x 512, top 8, int4, 16 rows: 181 MB of expert blocks): the whole layer 67 us where router,
-// gate/up and down launches took 101; gate/up reads 121 MB in 19 us (6.3 TB/s), down 60 MB in 11 (5.3 TB/s), the rest is the
-// routing (16 us), the first units' way (6 us), the hand-over between the projections (5 us) and the row sums (7 us). DRAM reads are the
-// algorithmic bytes (184 MB). 64 rows 129 us where the prefill path takes 254.
+// Measured (256 experts of 2048 x 512, top 8, int4, 16 rows: 181 MB of expert blocks): the whole layer 60 us where router,
+// gate/up and down launches took 101; gate/up reads 121 MB in 19 us (6.3 TB/s), down 60 MB in 11 (5.5 TB/s), the rest is the
+// routing (11 us, 16 with divisions, serial picks and all rows in every block), the first units' way (5 us), the hand-over between the
+// projections (5 us) and the row sums (5 us). DRAM reads are the algorithmic bytes (184 MB).
 #include "block_maps.cuh"
 #include "plan.cuh"
 #include "route_args.cuh"
@@ -428,7 +428,7 @@ __device__ __forceinline__ uint32_t work_list(const StreamArgs& a, uint8_t* dsm,
         // ================= router, selection, lookup, work list =================
         // A block has a share of the expert rows (they go to the ring's memory, asked for ahead of the wait) and of the
         // activation rows; what follows the logits every block does for itself: another hand-over between blocks costs
-        // more than the work (a row's picks 1 us by one warp, the list 1 us).
+        // more than the work (a row's picks 2 us by one warp, the list 1 us).
         const RouterArgs& r = a.r;
         const uint32_t rows = r.ne + (r.gate_row ? 1u : 0u), tg = a.token_groups_log2, bx = blockIdx.x >> tg, by = blockIdx.x & ((1u << tg) - 1u);
         const uint32_t nbx = gridDim.x >> tg, e0 = bx < nbx ? quotient(rows * bx, a.rcp_nbx) : 0u, e1 = bx < nbx ? quotient(rows * (bx + 1), a.rcp_nbx) : 0u;
