@@ -426,7 +426,7 @@ int shrike_moe_layer_forward_host(shrike_moe* moe, void* stream, const shrike_po
                                   const void* x_host, uint32_t query_count, void* y_host,
                                   uint32_t* ids_host, float* weights_host);
 
-/* One layer of a decode stack, as shrike_moe_decode_stack_forward_host takes them. */
+/* One layer of a decode stack, as shrike_decode_stack_create takes them. */
 typedef struct shrike_stack_layer {
     shrike_moe*                  moe;                 /* the layer's handle (its own work lists) */
     const shrike_pool*           pool;
@@ -441,7 +441,9 @@ typedef struct shrike_stack_layer {
  * halves of the layers are present. The stack owns a device copy of the residual stream,
  * [(layer_count + 1) x max_rows x d] in act_dtype, and the launches of a step of max_rows rows as a graph, made with
  * it: the layers' operand structures are read then too. Steps of fewer rows, and steps whose structures read
- * differently, launch layer by layer.
+ * differently, launch layer by layer (one Qwen-shape row: 17 us a layer instead of 15); a host whose batch shrinks for long makes
+ * a stack of its size. shrike_decode_stack_runs_graph sets *out to 1 when a step of query_count rows would be the graph as the
+ * structures read now, else to 0: also for max_rows where the calls could not be captured, which creation does not report.
  *
  *   rows_host   [(layer_count + 1) x query_count x d]: block 0 is the row set entering layer 0; block l >= 1 is
  *               what the rest of transformer block l (attention, normalisation -- not part of this library)
@@ -458,6 +460,7 @@ int shrike_decode_stack_create(const shrike_stack_layer* layers, uint32_t layer_
 void shrike_decode_stack_destroy(shrike_decode_stack* stack);
 int shrike_decode_stack_forward_host(shrike_decode_stack* stack, void* stream, const void* rows_host,
                                      uint32_t query_count, void* out_host);
+int shrike_decode_stack_runs_graph(const shrike_decode_stack* stack, uint32_t query_count, int* out);
 
 #ifdef __cplusplus
 }

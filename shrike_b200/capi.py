@@ -113,6 +113,7 @@ SIGNATURES = {
     "shrike_decode_stack_create": (_INT, [C.POINTER(StackLayer), _U32, _U32, C.POINTER(_P)]),
     "shrike_decode_stack_destroy": (None, [_P]),
     "shrike_decode_stack_forward_host": (_INT, [_P, _P, _P, _U32, _P]),
+    "shrike_decode_stack_runs_graph": (_INT, [_P, _U32, C.POINTER(_INT)]),
     "shrike_moe_layer_forward_host": (_INT, [_P, _P, _P, C.POINTER(ExpertOffsets), _P,
                                              C.POINTER(RouterOperands), C.POINTER(SharedExpert),
                                              _P, _U32, _P, _P, _P]),

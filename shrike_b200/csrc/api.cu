@@ -1178,22 +1178,18 @@ struct shrike_decode_stack {
     ~shrike_decode_stack() { delete[] layers; delete[] captured; }
 };
 
-static int encode_stack(shrike_decode_stack* stack, void* stream, uint32_t query_count) {
-    shrike_moe* m = stack->layers[0].moe;
-    const size_t block = (size_t)query_count * m->cfg.d * act_bytes(m->cfg.act_dtype);
-    uint8_t* dev = (uint8_t*)stack->stream_dev;
-    for (uint32_t l = 0; l < stack->layer_count; ++l) {
-        const shrike_stack_layer& ly = stack->layers[l];
-        const int rc = shrike_encode_decode_layer(ly.moe, stream, ly.pool, ly.routed_offsets, ly.residency_table_row,
-                                                  ly.router, ly.shared, dev + (size_t)l * block, query_count, nullptr, nullptr,
-                                                  nullptr, ly.moe->ws.y_dev, dev + (size_t)(l + 1) * block);
-        if (rc) return pass_on(m, ly.moe, rc);
-    }
-    return SHRIKE_OK;
+// Layer l's call for query_count rows of the stack's stream; a failure's text is on the layer's handle.
+static int encode_stack_layer(const shrike_decode_stack* stack, void* stream, uint32_t l, uint32_t query_count) {
+    const shrike_stack_layer& ly = stack->layers[l];
+    const size_t block = (size_t)query_count * ly.moe->cfg.d * act_bytes(ly.moe->cfg.act_dtype);
+    uint8_t* const x = (uint8_t*)stack->stream_dev + (size_t)l * block;
+    return shrike_encode_decode_layer(ly.moe, stream, ly.pool, ly.routed_offsets, ly.residency_table_row, ly.router, ly.shared, x,
+                                      query_count, nullptr, nullptr, nullptr, ly.moe->ws.y_dev, x + block);
 }
 
 // The layer calls of a full step as one graph: a cooperative launch by itself takes 2 to 3 us of a layer's 17, inside a graph nothing.
-// A stack whose calls cannot be captured goes on without.
+// A stack whose calls cannot be captured goes on without, and creation, which succeeds all the same, leaves no failure's text behind:
+// what a layer call refuses, a forward refuses again.
 static void capture_stack(shrike_decode_stack* s) {
     cudaStream_t st;
     if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) {
@@ -1202,8 +1198,15 @@ static void capture_stack(shrike_decode_stack* s) {
     }
     s->captured = new (std::nothrow) StackOperands[s->layer_count];
     if (s->captured && cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        for (uint32_t l = 0; l < s->layer_count; ++l) s->captured[l].read(s->layers[l]);
-        const int rc = encode_stack(s, st, s->max_rows);
+        int rc = SHRIKE_OK;
+        for (uint32_t l = 0; l < s->layer_count && rc == SHRIKE_OK; ++l) {
+            s->captured[l].read(s->layers[l]);
+            shrike_moe* const m = s->layers[l].moe;
+            char text[kErrorText];
+            memcpy(text, m->err, kErrorText);
+            rc = encode_stack_layer(s, st, l, s->max_rows);
+            if (rc) memcpy(m->err, text, kErrorText);
+        }
         cudaGraph_t g = nullptr;
         if (cudaStreamEndCapture(st, &g) == cudaSuccess && g && rc == SHRIKE_OK &&
             (cudaGraphInstantiate(&s->graph, g, 0) != cudaSuccess || cudaGraphUpload(s->graph, st) != cudaSuccess ||
@@ -1215,6 +1218,17 @@ static void capture_stack(shrike_decode_stack* s) {
     }
     cudaStreamDestroy(st);
     cudaGetLastError();
+}
+
+// Whether a step of query_count rows is the captured one: as many rows, and every layer's operands read as they did then.
+static bool stack_runs_graph(const shrike_decode_stack* s, uint32_t query_count) {
+    if (!s->graph || query_count != s->max_rows) return false;
+    for (uint32_t l = 0; l < s->layer_count; ++l) {
+        StackOperands now;
+        now.read(s->layers[l]);
+        if (s->layers[l].moe->beside_others || memcmp(&now, &s->captured[l], sizeof now) != 0) return false;
+    }
+    return true;
 }
 
 int shrike_decode_stack_create(const shrike_stack_layer* layers, uint32_t layer_count, uint32_t max_rows,
@@ -1276,21 +1290,22 @@ int shrike_decode_stack_forward_host(shrike_decode_stack* stack, void* stream, c
     const size_t block = (size_t)query_count * c.d * act_bytes(c.act_dtype);
     uint8_t* dev = (uint8_t*)stack->stream_dev;
     CU(cudaMemcpyAsync(dev, rows_host, (size_t)(L + 1) * block, cudaMemcpyHostToDevice, st));
-    bool same = stack->graph && query_count == stack->max_rows;
-    for (uint32_t l = 0; l < L && same; ++l) {
-        StackOperands now;
-        now.read(stack->layers[l]);
-        same = !stack->layers[l].moe->beside_others && memcmp(&now, &stack->captured[l], sizeof now) == 0;
-    }
     int rc;
-    if (same) {
+    if (stack_runs_graph(stack, query_count)) {
         if ((rc = check_device(m))) return rc;
         CU(cudaGraphLaunch(stack->graph, st));
-    } else if ((rc = encode_stack(stack, stream, query_count))) {
-        return rc;
+    } else {
+        for (uint32_t l = 0; l < L; ++l)
+            if ((rc = encode_stack_layer(stack, stream, l, query_count))) return pass_on(m, stack->layers[l].moe, rc);
     }
     CU(cudaMemcpyAsync(out_host, dev + (size_t)L * block, block, cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));
+    return SHRIKE_OK;
+}
+
+int shrike_decode_stack_runs_graph(const shrike_decode_stack* stack, uint32_t query_count, int* out) {
+    if (!stack || !out) return SHRIKE_EINVAL;
+    *out = stack_runs_graph(stack, query_count);
     return SHRIKE_OK;
 }
 

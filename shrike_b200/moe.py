@@ -321,6 +321,12 @@ class DecodeStack:
         self._first._check(self._lib.shrike_decode_stack_forward_host(
             self._h, _stream(), rows_host.data_ptr(), rows_host.shape[1], out_host.data_ptr()))
 
+    def runs_graph(self, rows: int) -> bool:
+        """Whether a step of this many rows, with the operands as they are, is the graph that was made with the stack."""
+        out = C.c_int()
+        self._first._check(self._lib.shrike_decode_stack_runs_graph(self._h, rows, C.byref(out)))
+        return bool(out.value)
+
 
 def encode_router_static(config: MoEConfig, operands: RouterOperands, hidden: torch.Tensor,
                          out_indices: torch.Tensor, out_weights: torch.Tensor,

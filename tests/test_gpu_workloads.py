@@ -246,3 +246,87 @@ def test_decode_stack_with_other_rows_or_operands(cuda_device, T):
     for L in layers:
         L.moe.status()
         L.close()
+
+
+@pytest.mark.parametrize("T", [1, 5])
+def test_a_full_step_of_a_stack_is_a_graph(cuda_device, T):
+    """A stack reports that its full step is a graph; other rows, and operands that read differently (the router's rows, the
+    experts' offsets, the shared expert's block), take the layer calls and give what a stack made for them gives; operands put back
+    take the graph again."""
+    import torch
+    from shrike_b200.moe import DecodeStack
+    cfg = fx.qwen_config(max_tokens=16, d=512, f=256, shared_f=256, num_experts=64, y_dtype=capi.DTYPE_FP32)
+    layers = [Layer(cfg, seed=180 + l, device_fill=True) for l in range(3)]
+    x = torch.from_numpy(np.stack([fx.round_bf16(inputs(T, cfg.d, seed=90 + l)) for l in range(4)])).to(torch.bfloat16)
+
+    def run(stack):
+        out = torch.empty(x.shape[1:], dtype=x.dtype)
+        stack.forward_host(x, out)
+        return out
+
+    def made():
+        return DecodeStack([(L.moe, L.pool, L.offsets, 0, L.router_ops, L.shared) for L in layers], T)
+
+    stack = made()
+    assert stack.runs_graph(T) and not any(stack.runs_graph(n) for n in range(T + 3) if n != T)
+    before = run(stack)
+    L = layers[1]
+    ops = stack._keep[4]                         # the second layer's structures
+    other = L.router_ops.weights.flip(0).contiguous()
+    offsets = dict(gate_w=L.offsets.up_w, gate_s=L.offsets.up_s, gate_b=L.offsets.up_b,
+                   up_w=L.offsets.gate_w, up_s=L.offsets.gate_s, up_b=L.offsets.gate_b)
+    for struct, changed in ((ops, dict(weights=other.data_ptr())), (L.offsets, offsets),
+                            (L.shared, dict(block=layers[2].shared.block))):
+        kept = {k: getattr(struct, k) for k in changed}
+        for k, v in changed.items():
+            setattr(struct, k, v)
+        assert not stack.runs_graph(T)
+        got = run(stack)
+        assert not torch.equal(got, before)
+        if struct is ops:
+            L.router_ops.weights, other = other, L.router_ops.weights
+        fresh = made()
+        assert fresh.runs_graph(T) and torch.equal(run(fresh), got)
+        fresh.close()
+        if struct is ops:
+            L.router_ops.weights, other = other, L.router_ops.weights
+        for k, v in kept.items():
+            setattr(struct, k, v)
+        assert stack.runs_graph(T) and torch.equal(run(stack), before)
+    stack.close()
+    for L in layers:
+        L.moe.status()
+        L.close()
+
+
+def test_a_stack_that_cannot_be_captured(cuda_device):
+    """Router rows that the layer call refuses (checked on the host): creation succeeds, as it reads no operand for its result, and
+    leaves no text of a failure; the step is no graph, its call reports the operand, and works once that is mended."""
+    import torch
+    from shrike_b200.moe import DecodeStack, ShrikeError
+    cfg = fx.qwen_config(max_tokens=16, d=512, f=256, shared_f=256, num_experts=64, y_dtype=capi.DTYPE_FP32)
+    layers = [Layer(cfg, seed=190 + l, device_fill=True) for l in range(2)]
+    x = torch.from_numpy(np.stack([fx.round_bf16(inputs(2, cfg.d, seed=95 + l)) for l in range(3)])).to(torch.bfloat16)
+    out, want = torch.empty(x.shape[1:], dtype=x.dtype), torch.empty(x.shape[1:], dtype=x.dtype)
+
+    def made():
+        return DecodeStack([(L.moe, L.pool, L.offsets, 0, L.router_ops, L.shared) for L in layers], 2)
+
+    whole = made()
+    whole.forward_host(x, want)
+    rows = layers[1].router_ops.weights
+    layers[1].router_ops.weights = torch.zeros(rows.numel() + 1, device=rows.device)[1:].view_as(rows)
+    stack = made()
+    assert all(L.moe._lib.shrike_last_error(L.moe._h) == b"" for L in layers)
+    assert not stack.runs_graph(2)
+    with pytest.raises(ShrikeError) as err:
+        stack.forward_host(x, out)
+    assert err.value.code == capi.EINVAL and "aligned" in str(err.value)
+    stack._keep[4].weights = rows.data_ptr()
+    stack.forward_host(x, out)
+    assert torch.equal(out, want) and not stack.runs_graph(2)
+    for s in (whole, stack):
+        s.close()
+    for L in layers:
+        L.moe.status()
+        L.close()
