@@ -406,3 +406,90 @@ def test_output_rows_that_are_not_whole_vectors(cuda_device, dtype):
     assert not torch.equal(got[0][0], torch.zeros_like(got[0][0]))
     for a, b in zip(*got):
         assert ((a - b).abs() <= 2 * ulp * a.abs() + 1e-6 * a.abs().max()).all()
+
+
+def _view(address, nbytes):
+    """The device memory at an address, as a byte tensor over it."""
+    class Memory:
+        __cuda_array_interface__ = dict(shape=(nbytes,), typestr="|u1", data=(address, False), version=3)
+    return torch.as_tensor(Memory(), device="cuda")
+
+
+def _exchange_areas(cfg, world, cap, buf):
+    """A rank's exchange buffer by its areas, each a multiple of 256 bytes: rows, ids and weights received from every rank,
+    partial rows returned, and the two arrival words."""
+    at, areas = 0, []
+    for shape, dtype in (((world, cap, cfg.d), cfg.torch_act_dtype), ((world, cap, cfg.top_k), torch.int32),
+                         ((world, cap, cfg.top_k), torch.float32), ((world, cap, cfg.d), cfg.torch_y_dtype),
+                         ((world,), torch.int64), ((world,), torch.int64)):
+        n = int(np.prod(shape)) * torch.empty((), dtype=dtype).element_size()
+        areas.append(buf[at:at + n].view(dtype).view(shape))
+        at = (at + n + 255) // 256 * 256
+    assert at == buf.numel()
+    return areas
+
+
+@pytest.mark.parametrize("T,dtype", [(1, "fp32"), (37, "fp32"), (37, "bf16"), (90, "bf16")])
+def test_both_ranks_rows_beside_words_that_are_there(cuda_device, T, dtype):
+    """Rank 0 of a two-rank world, and rank 1 made on the host: before the call its rows, its partial rows and both of its
+    arrival words are in rank 0's buffer, so no wait waits. Rank 0's y are its own picks, the returned rows and the shared
+    expert; what it sends and returns is in rank 1's buffer, and nothing in its own return area."""
+    import ep_reference as R
+    import fixtures as fx
+    import oracle_lib as O
+    from shrike_b200 import capi
+    from shrike_b200.ep import ExpertParallelLayer
+    from shrike_b200.moe import RouterOperands, expert_offsets
+    cfg, seed, world = _config(act=capi.DTYPE_FP32 if dtype == "fp32" else capi.DTYPE_BF16), 26, 2
+    x, router = _problem(world * T, cfg)
+    ids, w, y_ref = _oracle(cfg, x, router, seed)
+    layer = ExpertParallelLayer(cfg, 0, world, 0, T, None, exchange="peer", connect=False)
+    epr = layer.epr
+    for e in range(layer.lo, layer.hi):
+        layer.pool.upload(e - layer.lo, fx.synth_block(cfg, seed, 0, e))
+    sh = torch.from_numpy(fx.synth_block(cfg, seed, 0, 100000, shared=True).copy()).cuda()
+    layer.set_shared(capi.SharedExpert(sh.data_ptr(), expert_offsets(cfg, shared=True)[0]))
+    base, nbytes = layer.buffer()
+    peer = torch.zeros(nbytes, dtype=torch.uint8, device="cuda")
+    layer.connect_pointers([base, peer.data_ptr()])
+    mine, theirs = _exchange_areas(cfg, world, T, _view(base, nbytes)), _exchange_areas(cfg, world, T, peer)
+    blocks = {e: fx.synth_block(cfg, seed, 0, e) for e in range(cfg.num_experts)}
+    lcfg = O.layer_cfg(O.expert_cfg(cfg.d, cfg.f), None, False)
+
+    def partial(rank, rows):   # the rows' picks on a rank, added in fp32
+        return O.moe_layer(lcfg, blocks, None, None, x[rows], ids[rows], np.where(ids[rows] // epr == rank, w[rows], np.float32(0)))
+
+    home, away = np.arange(T), np.arange(T, 2 * T)   # rank 0's rows, rank 1's
+    sent, back = R.pack(x[home], ids[home], w[home], world, epr, T), R.pack(x[away], ids[away], w[away], world, epr, T)
+    on_1, from_1 = (ids[home] // epr == 1).any(axis=1), (ids[away] // epr == 0).any(axis=1)
+    ops = RouterOperands(weights=torch.from_numpy(router).cuda())
+    xd = torch.from_numpy(x[home]).cuda().to(cfg.torch_act_dtype)
+    y, h = torch.empty((T, cfg.d), dtype=cfg.torch_y_dtype, device="cuda"), torch.empty_like(xd)
+    tol = 1e-3 if dtype == "fp32" else 1e-3 + 3 * 2.0 ** -9   # bf16: both partial rows and their sum are rounded
+    for call in (1, 2):
+        mine[0][1, :from_1.sum()] = torch.from_numpy(back[0][0, :from_1.sum()]).cuda().to(cfg.torch_act_dtype)
+        mine[1][1] = torch.from_numpy(back[1][0].view(np.int32)).cuda()
+        mine[2][1] = torch.from_numpy(back[2][0]).cuda()
+        mine[3].fill_(7.0)
+        mine[3][1, :on_1.sum()] = torch.from_numpy(partial(1, home[on_1])).cuda().to(cfg.torch_y_dtype)
+        mine[4][1] = call << 32 | int(from_1.sum())
+        mine[5][1] = call << 32
+        theirs[3].fill_(-7.0)
+        h.copy_(xd)
+        torch.cuda.synchronize()
+        layer.forward(ops, xd, y, h)
+        layer.status()
+        got = y.float().cpu().numpy()
+        assert np.linalg.norm(got - y_ref[home]) <= tol * np.linalg.norm(y_ref[home])
+        assert torch.equal(h, (xd.float() + y.float()).to(h.dtype))
+        n = int(sent[3][1])
+        assert int(theirs[4][0]) == call << 32 | n and int(theirs[5][0]) == call << 32
+        assert torch.equal(theirs[0][0, :n].float().cpu(), torch.from_numpy(sent[0][1, :n]))
+        assert (theirs[1][0, :n].cpu().numpy().view(np.uint32) == sent[1][1, :n]).all()
+        assert (theirs[2][0, :n].cpu().numpy() == sent[2][1, :n]).all()
+        n = int(from_1.sum())
+        want = partial(0, away[from_1])
+        assert np.linalg.norm(theirs[3][0, :n].float().cpu().numpy() - want) <= tol * np.linalg.norm(want)
+        assert (theirs[3][0, n:] == -7.0).all() and (theirs[3][1] == -7.0).all() and (mine[3][0] == 7.0).all()
+        assert layer.last_counts()[0] == [int(sent[3][0]), int(sent[3][1])] and layer.last_counts()[1] == int(sent[3][0]) + n
+    layer.close()
