@@ -186,14 +186,6 @@ int fill_expert_args(shrike_moe* m, const shrike_pool* pool, const shrike_expert
 // With picks by Zipf(1.1), 64 rows: 87, 113 | 259, 222 | 192, 246.
 bool stream_pays(uint32_t T) { return T > 1; }
 
-// The same for projections that are launches of their own: each has the streaming kernel's set-up to pay, and not the router to
-// gain. Plan and both projections, us, per-tile kernels and streaming (experts of 1.6 MB | 7.1 MB | 12.4 MB):
-//   2 rows  30.3, 32.8 | 45.9, 49.3 | 85.0, 62.0      3 rows  34.4, 37.0 | 60.2, 57.5 | 113, 76      4 rows  41.1, 39.9 | 72, 66 | 138, 82
-bool stream_phase_pays(const shrike_moe_config& c, uint32_t T) {
-    const uint64_t bytes = (uint64_t)3 * c.d * c.f * c.weight_bits / 8;
-    return T > 3 || (T == 3 && bytes >= (4u << 20)) || (T == 2 && bytes >= (8u << 20));
-}
-
 // The expert projections of a decode call's work lists (phases: 1, 2 or 3 = both, a launch each). The streaming kernel takes
 // every shape whose tiles its ring and the tiled copies can hold; the per-tile kernels take the others.
 cudaError_t launch_experts(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, uint32_t T, uint32_t phases, void* y,
@@ -202,7 +194,7 @@ cudaError_t launch_experts(const shrike_moe* m, cudaStream_t st, const ExpertArg
     const uint32_t mi = max_instances(m->cfg, T);
     for (uint32_t phase = 1; phase <= 2; ++phase) {
         if (!(phases & phase)) continue;
-        cudaError_t e = stream_phase_pays(m->cfg, T) ? launch_expert_stream(m, st, a, T, n_shared, y, hidden, pdl, phase) : cudaErrorNotSupported;
+        cudaError_t e = stream_pays(T) ? launch_expert_stream(m, st, a, T, n_shared, y, hidden, pdl, phase) : cudaErrorNotSupported;
         if (e == cudaErrorNotSupported)
             e = phase == 1 ? launch_phase1(m, st, a, mi, pdl) : launch_phase2(m, st, a, T, mi, y, hidden, pdl);
         if (e != cudaSuccess) return e;

@@ -201,32 +201,6 @@ class Layer:
         return O.moe_layer(lcfg, blocks, self.shared_block_host, self.gate_w, xr, ids, weights, threads=threads)
 
 
-def captured_kernels(call) -> list[int]:
-    """The kernels (addresses of their functions) that a call on the current stream launches, in no order: the nodes of its graph."""
-    rt = C.CDLL("libcudart.so.12")
-    torch.cuda.synchronize()
-    stream = torch.cuda.Stream()
-    graph, n = C.c_void_p(), C.c_size_t()
-    with torch.cuda.stream(stream):
-        assert rt.cudaStreamBeginCapture(C.c_void_p(stream.cuda_stream), 1) == 0   # 1: this thread's calls
-        try:
-            call()
-        finally:
-            assert rt.cudaStreamEndCapture(C.c_void_p(stream.cuda_stream), C.byref(graph)) == 0
-    assert rt.cudaGraphGetNodes(graph, None, C.byref(n)) == 0
-    nodes = (C.c_void_p * n.value)()
-    assert rt.cudaGraphGetNodes(graph, nodes, C.byref(n)) == 0
-    kernels = []
-    for node in nodes:
-        kind, params = C.c_int(), (C.c_uint64 * 7)()   # cudaKernelNodeParams: the function, grid, block, bytes, arguments
-        assert rt.cudaGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
-        if kind.value == 0:
-            assert rt.cudaGraphKernelNodeGetParams(C.c_void_p(node), params) == 0
-            kernels.append(params[0])
-    assert rt.cudaGraphDestroy(graph) == 0
-    return kernels
-
-
 def small_config(**kw) -> MoEConfig:
     base = dict(d=128, f=64, num_experts=16, top_k=4, weight_bits=4, group_size=64, act_dtype=capi.DTYPE_FP32,
                 has_shared=True, shared_gated=True, shared_f=64, max_tokens=64)

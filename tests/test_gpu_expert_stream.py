@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from shrike_b200 import capi
-from gpu_harness import Layer, captured_kernels, inputs, rel_l2, small_config, to_act_tensor
+from gpu_harness import Layer, inputs, rel_l2, small_config, to_act_tensor
 from test_gpu_parity import TOL, check_layer
 
 pytestmark = pytest.mark.gpu
@@ -112,34 +112,3 @@ def test_picks_among_equal_scores(cuda_device, alike, left, k):
 def test_few_rows(cuda_device, kw, T):
     """The rows' groups in the router: one, two, four of them, with unequal numbers of rows."""
     test_stream_edges(cuda_device, kw, T)
-
-
-@pytest.mark.parametrize("kw,tiles", [
-    (dict(d=256, f=128, shared_f=128), 3),                                                # experts below 4 MB
-    (dict(d=2304, f=1024, shared_f=1024, weight_bits=8, num_experts=4, top_k=2), 2),      # below 8 MB
-    (dict(d=2880, f=2880, group_size=32, num_experts=4, top_k=2, has_shared=False, shared_gated=False), 1),
-], ids=["small", "middle", "large"])
-def test_projections_of_few_rows_as_calls_of_their_own(cuda_device, kw, tiles):
-    """One row's kernels take up to three rows of small experts, two of middle ones; the streaming kernel the others. Layer calls
-    are the streaming kernel's from two rows on."""
-    layer = Layer(small_config(**kw))
-    x = inputs(4, kw["d"], seed=6)
-    x_dev = to_act_tensor(x, layer.cfg.act_dtype, layer.device)
-    ids, w, gate = layer.route(x_dev)
-    slots, _ = layer.classify(ids)
-    y = torch.empty_like(x_dev)
-
-    def separate(T):
-        layer.moe.encode_decode(layer.pool, layer.offsets, slots[:T], w[:T], x_dev[:T], y[:T], None, layer.shared,
-                                gate if gate is None else gate[:T])
-
-    def whole(T):
-        layer.moe.encode_decode_layer(layer.pool, layer.offsets, 0, layer.router_ops, x_dev[:T], y[:T], None, layer.shared)
-
-    separate(4)
-    one = set(captured_kernels(lambda: separate(1)))
-    assert [set(captured_kernels(lambda T=T: separate(T))) == one for T in (2, 3, 4)] == [T <= tiles for T in (2, 3, 4)]
-    assert len(one) == 3 and all(len(captured_kernels(lambda T=T: whole(T))) == 1 for T in (2, 3, 4))
-    for T in (2, 3):
-        check_layer(layer, x[:T])
-    layer.close()
