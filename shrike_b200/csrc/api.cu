@@ -184,6 +184,9 @@ int fill_expert_args(shrike_moe* m, const shrike_pool* pool, const shrike_expert
 // uniform picks):
 //   17 rows  69, 115 | 179, 253 | 132, 200       64 rows  131, 190 | 262, 255 | 252, 344
 // With picks by Zipf(1.1), 64 rows: 87, 113 | 259, 222 | 192, 246.
+// The projections as calls of their own follow the same rule, so that they give a layer call's rows bit for bit. Each pays the
+// kernel's set-up, with no router to share: plan and both of them, us, per-tile kernels and streaming, 30.3, 32.8 | 85, 62 | 45.9,
+// 49.3 at two rows, 34.4, 37.0 | 113, 76 | 60.2, 57.5 at three, 41.1, 39.9 | 138, 82 | 72, 66 at four.
 bool stream_pays(uint32_t T) { return T > 1; }
 
 // The expert projections of a decode call's work lists (phases: 1, 2 or 3 = both, a launch each). The streaming kernel takes

@@ -7,7 +7,7 @@ import torch
 
 from shrike_b200 import capi
 from gpu_harness import Layer, inputs, rel_l2, small_config, to_act_tensor
-from test_gpu_parity import TOL, check_layer
+from test_gpu_parity import TOL, check_layer, test_fused_decode_layer_equals_the_separate_calls as equals_the_separate_calls
 
 pytestmark = pytest.mark.gpu
 
@@ -112,3 +112,12 @@ def test_picks_among_equal_scores(cuda_device, alike, left, k):
 def test_few_rows(cuda_device, kw, T):
     """The rows' groups in the router: one, two, four of them, with unequal numbers of rows."""
     test_stream_edges(cuda_device, kw, T)
+
+
+@pytest.mark.parametrize("kw", [
+    dict(),
+    dict(weight_bits=8, router_weight_bits=8, router_kind=capi.ROUTER_SIGMOID, routed_scaling=2.446, shared_gated=False),
+], ids=["int4", "int8"])
+def test_two_rows_are_the_separate_calls_rows(cuda_device, kw):
+    """The smallest number of rows that layer calls and projections of their own both give to this kernel: bit for bit the same."""
+    equals_the_separate_calls(cuda_device, 2, kw)
