@@ -531,20 +531,27 @@ __global__ void __launch_bounds__(1024) classify_kernel(const uint32_t* __restri
     __shared__ uint32_t s_base;
     pdl_wait();
     pdl_launch_dependents();
-    auto lookup = [&](uint32_t p, uint32_t& e, uint32_t& slot) {
-        e = min(ids[p], ne - 1u);
-        const uint64_t word = table[e];
-        slot = (uint32_t)(word & 0xffffffffu);
-        return (uint32_t)(word >> 32) == 2u && slot != SHRIKE_SLOT_MISS;
+    auto slot_of = [](uint64_t word) {   // or SHRIKE_SLOT_MISS
+        return (uint32_t)(word >> 32) == 2u ? (uint32_t)(word & 0xffffffffu) : SHRIKE_SLOT_MISS;
     };
     if (threadIdx.x == 0) s_base = 0;
     __syncthreads();
     uint32_t before_me = 0;
-    const uint32_t earlier = counts || miss_pos || miss_exp ? blockIdx.x : 0u;   // (their misses are asked for)
-#pragma unroll 4
-    for (uint32_t j = 0; j < earlier; ++j) {
-        uint32_t e, slot;
-        before_me += lookup(j * 1024u + threadIdx.x, e, slot) ? 0u : 1u;
+    if (counts || miss_pos || miss_exp) {   // the misses are asked for
+        // Eight pairs of a thread at a time, written out: a lookup is two loads one after the other, and the compiler took the pairs
+        // of a loop one by one (4096 rows of eight picks, caches cold: 17.8 us, so 9.4).
+        constexpr uint32_t N = 8;
+#pragma unroll 1
+        for (uint32_t j = 0; j < blockIdx.x; j += N) {
+            uint32_t e[N];
+            uint64_t word[N];
+#pragma unroll
+            for (uint32_t q = 0; q < N; ++q) e[q] = j + q < blockIdx.x ? ids[(j + q) * 1024u + threadIdx.x] : 0u;
+#pragma unroll
+            for (uint32_t q = 0; q < N; ++q) word[q] = table[min(e[q], ne - 1u)];
+#pragma unroll
+            for (uint32_t q = 0; q < N; ++q) before_me += j + q < blockIdx.x && slot_of(word[q]) == SHRIKE_SLOT_MISS ? 1u : 0u;
+        }
     }
     for (int o = 16; o; o >>= 1) before_me += __shfl_xor_sync(0xffffffffu, before_me, o);
     if ((threadIdx.x & 31u) == 0 && before_me) atomicAdd(&s_base, before_me);
@@ -552,10 +559,10 @@ __global__ void __launch_bounds__(1024) classify_kernel(const uint32_t* __restri
     bool miss = false;
     uint32_t e = 0;
     if (p < n_pairs) {
-        uint32_t slot;
-        const bool hit = lookup(p, e, slot);
-        slots[p] = hit ? slot : SHRIKE_SLOT_MISS;
-        miss = !hit;
+        e = min(ids[p], ne - 1u);
+        const uint32_t slot = slot_of(table[e]);
+        slots[p] = slot;
+        miss = slot == SHRIKE_SLOT_MISS;
     }
     s_miss[threadIdx.x] = miss ? 1u : 0u;
     const uint32_t chunk = __syncthreads_count(miss);

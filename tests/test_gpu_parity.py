@@ -242,6 +242,32 @@ def test_router_strided_hidden_equals_dense(cuda_device):
     layer.close()
 
 
+@pytest.mark.parametrize("T", [256, 2048, 2305, 4100])
+def test_miss_lists_of_many_blocks(cuda_device, T):
+    """A block counts the misses before its own eight blocks of pairs at a time: with one, eight, ten and seventeen blocks the lists
+    hold every miss in the picks' order, whichever of them are asked for."""
+    layer = Layer(small_config(max_tokens=T))
+    for e in (2, 3, 11):
+        layer.moe.residency_set(0, e, 0, 1)
+    ids_np = np.random.default_rng(T).integers(0, 16, (T, 4)).astype(np.int32)
+    ids = torch.from_numpy(ids_np).to(layer.device)
+    missing = np.isin(ids_np, (2, 3, 11)).ravel()
+    pos = np.flatnonzero(missing)
+    for asked in ("counts", "miss_positions", "miss_experts"):
+        out = dict(counts=None, miss_positions=None, miss_experts=None)
+        out[asked] = torch.full((2 if asked == "counts" else T * 4,), -7, dtype=torch.int32, device=layer.device)
+        slots = torch.empty_like(ids)
+        layer.moe.encode_residency_classification(ids, 0, slots, **out)
+        layer.moe.status()
+        assert (slots.cpu().numpy().ravel() == np.where(missing, -1, ids_np.ravel())).all()
+        got = out[asked].cpu().numpy()
+        if asked == "counts":
+            assert got.tolist() == [T * 4 - len(pos), len(pos)]
+        else:
+            assert (got[:len(pos)] == (pos if asked == "miss_positions" else ids_np.ravel()[pos])).all() and (got[len(pos):] == -7).all()
+    layer.close()
+
+
 @pytest.mark.parametrize("T", [32, 700])
 def test_residency_classification_and_misses(cuda_device, T):
     """T = 700: 2800 pairs, three blocks of the classification kernel, the miss lists still in router order."""
