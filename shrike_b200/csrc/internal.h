@@ -96,7 +96,7 @@ struct Workspace {
     uint32_t* n_chunk_inst = nullptr; // [0] instances, [1], [2] tiles handed out per phase
     uint32_t* pos_of_pair = nullptr; // prefill: place of every pair in the expert-sorted order, or 0xffffffff
     uint16_t* xs = nullptr;         // prefill: fp16 activation rows in expert-sorted order [max_tokens x top_k x d]
-    void* tensor_maps = nullptr;    // host: the TMA descriptors of xs, acts, xh, acts_shared
+    void* tensor_maps = nullptr;    // host: the TMA descriptors of xs, acts, xh, acts_shared and of the last prefill's pool and shared block
     // one-row decode layer in one launch (fused_layer.cu)
     void* fused_geom = nullptr;       // host: sizes of the shared-memory ring, or NULL when the shape does not fit
     void* fused_maps = nullptr;       // host: cached tensor maps of the last call's pool and shared block

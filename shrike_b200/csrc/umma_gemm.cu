@@ -1325,10 +1325,10 @@ static bool make_matrix_map(CUtensorMap* map, const uint8_t* base, bool meta, bo
                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The two tiles of one phase: gate + up (phase 0) or down twice (phase 1).
+// The two tiles of one phase: gate + up (phase 0) or down twice (phase 1: the same maps).
 static bool make_weight_maps(WeightMaps* wm, const uint8_t* base, const Offsets3& off, int phase, uint32_t kdim,
                              uint32_t rows, uint32_t bits, uint32_t group, uint64_t cells, uint64_t cell_stride) {
-    for (int t = 0; t < 2; ++t) {
+    for (int t = 0; t < (phase == 0 ? 2 : 1); ++t) {
         const int mat = phase == 0 ? t : 2;
         if (!make_matrix_map(&wm->w[t], base + off.w[mat], false, false, (uint64_t)kdim * bits / 8, rows, cells, cell_stride) ||
             !make_matrix_map(&wm->nw[t], base + off.w[mat], false, true, (uint64_t)kdim * bits / 8, rows, cells, cell_stride))
@@ -1339,6 +1339,8 @@ static bool make_weight_maps(WeightMaps* wm, const uint8_t* base, const Offsets3
                 !make_matrix_map(n ? &wm->nb[t] : &wm->b[t], base + off.b[mat], true, n, kdim / group, rows, cells, cell_stride))
                 return false;
     }
+    if (phase == 1)
+        for (CUtensorMap* both : {wm->w, wm->s, wm->b, wm->nw, wm->ns, wm->nb}) both[1] = both[0];
     return true;
 }
 
@@ -1349,13 +1351,24 @@ bool umma_supported(const shrike_moe_config& c) {
     return encode_tiled_fn() != nullptr;
 }
 
+// A handle's maps: of its activation operands, and of the pool and shared block of its last call with what they were made from.
+struct UmmaMapCache {
+    CUtensorMap act[4 * kActBoxes];   // operands xs, acts, xh, acts_shared; boxes of 16, 32, 64, 128, 256 rows
+    UmmaMaps phase[2];
+    PoolView pool;
+    Offsets3 routed, shared;
+    const uint8_t* shared_block;
+    bool valid;
+};
+
 // Called once per handle, after the workspace exists: the activation operands' maps.
 cudaError_t umma_prepare(shrike_moe* m) {
     const shrike_moe_config& c = m->cfg;
     Workspace& ws = m->ws;
+    UmmaMapCache* const cache = (UmmaMapCache*)ws.tensor_maps;
+    memset(cache, 0, sizeof *cache);
     if (!ws.xs || !umma_supported(c)) return cudaSuccess;
-    // maps[operand][box]: operands xs, acts, xh, acts_shared; boxes of 16, 32, 64, 128, 256 rows
-    CUtensorMap* am = (CUtensorMap*)ws.tensor_maps;
+    CUtensorMap* am = cache->act;
     const uint64_t pairs = (uint64_t)c.max_tokens * c.top_k;
     bool ok = true;
     for (int bi = 0; bi < kActBoxes && ok; ++bi) {
@@ -1409,7 +1422,46 @@ uint32_t umma_max_chunk_instances(const shrike_moe_config& c, uint32_t T) {
 }
 
 size_t umma_chunk_instance_bytes() { return sizeof(ChunkInstance); }
-size_t umma_tensor_map_bytes() { return 4 * kActBoxes * sizeof(CUtensorMap); }
+size_t umma_tensor_map_bytes() { return (sizeof(UmmaMapCache) + 63) / 64 * 64; }
+
+// The maps of a call's pool and shared block; NULL when one cannot be encoded. They change only when the host changes the pool, the
+// offsets or the shared block: encoded on every call, a pool of eight chunks with a shared expert took 216 of them (36 us of host
+// work a call of 65 rows, 33 before narrow tiles had boxes of their own; 23 with the maps kept).
+static const UmmaMaps* umma_maps_for(const shrike_moe* m, const ExpertArgs& a) {
+    const shrike_moe_config& c = m->cfg;
+    UmmaMapCache* const cache = (UmmaMapCache*)m->ws.tensor_maps;
+    if (cache->valid && memcmp(&cache->pool, &a.pool, sizeof(PoolView)) == 0 && memcmp(&cache->routed, &a.routed, sizeof(Offsets3)) == 0 &&
+        memcmp(&cache->shared, &a.shared, sizeof(Offsets3)) == 0 && cache->shared_block == a.shared_block)
+        return cache->phase;
+    cache->valid = false;
+    memset(cache->phase, 0, sizeof cache->phase);
+    for (int phase = 0; phase < 2; ++phase) {
+        UmmaMaps& mp = cache->phase[phase];
+        const uint32_t kdim = phase == 0 ? c.d : c.f, rows = phase == 0 ? c.f : c.d;
+        uint32_t left = a.pool.cells;
+        for (uint32_t ch = 0; ch < SHRIKE_MAX_POOL_CHUNKS && a.pool.base[ch] && left; ++ch) {
+            const uint32_t cells = left < a.pool.cells_per_chunk ? left : a.pool.cells_per_chunk;
+            if (!make_weight_maps(&mp.routed[ch], a.pool.base[ch], a.routed, phase, kdim, rows, c.weight_bits,
+                                  c.group_size, cells, a.pool.stride))
+                return nullptr;
+            left -= cells;
+        }
+        for (int bi = 0; bi < kActBoxes; ++bi) mp.act_routed[bi] = cache->act[phase * kActBoxes + bi];
+        if (c.has_shared) {
+            const uint32_t kds = phase == 0 ? c.d : c.shared_f, rws = phase == 0 ? c.shared_f : c.d;
+            if (!make_weight_maps(&mp.shared, a.shared_block, a.shared, phase, kds, rws, c.weight_bits, c.group_size, 1,
+                                  16))
+                return nullptr;
+            for (int bi = 0; bi < kActBoxes; ++bi) mp.act_shared[bi] = cache->act[(2 + phase) * kActBoxes + bi];
+        } else {
+            mp.shared = mp.routed[0];
+            for (int bi = 0; bi < kActBoxes; ++bi) mp.act_shared[bi] = mp.act_routed[bi];
+        }
+    }
+    cache->pool = a.pool; cache->routed = a.routed; cache->shared = a.shared; cache->shared_block = a.shared_block;
+    cache->valid = true;
+    return cache->phase;
+}
 
 // Gate/up + GLU, then down, for the instances built from the grouping the
 // prefill plan left in the workspace.
@@ -1417,34 +1469,9 @@ cudaError_t launch_umma_prefill(const shrike_moe* m, cudaStream_t st, const Expe
                                 uint32_t pool_cells) {
     const shrike_moe_config& c = m->cfg;
     const Workspace& ws = m->ws;
-    const CUtensorMap* am = (const CUtensorMap*)ws.tensor_maps;
-    if (!am || !umma_supported(c)) return cudaErrorNotSupported;
-    // descriptors of this call's pool and shared block (host work only)
-    UmmaMaps maps[2];
-    for (int phase = 0; phase < 2; ++phase) {
-        UmmaMaps& mp = maps[phase];
-        memset(&mp, 0, sizeof mp);
-        const uint32_t kdim = phase == 0 ? c.d : c.f, rows = phase == 0 ? c.f : c.d;
-        uint32_t left = a.pool.cells;
-        for (uint32_t ch = 0; ch < SHRIKE_MAX_POOL_CHUNKS && a.pool.base[ch] && left; ++ch) {
-            const uint32_t cells = left < a.pool.cells_per_chunk ? left : a.pool.cells_per_chunk;
-            if (!make_weight_maps(&mp.routed[ch], a.pool.base[ch], a.routed, phase, kdim, rows, c.weight_bits,
-                                  c.group_size, cells, a.pool.stride))
-                return cudaErrorInvalidValue;
-            left -= cells;
-        }
-        for (int bi = 0; bi < kActBoxes; ++bi) mp.act_routed[bi] = am[phase * kActBoxes + bi];
-        if (c.has_shared) {
-            const uint32_t kds = phase == 0 ? c.d : c.shared_f, rws = phase == 0 ? c.shared_f : c.d;
-            if (!make_weight_maps(&mp.shared, a.shared_block, a.shared, phase, kds, rws, c.weight_bits, c.group_size, 1,
-                                  16))
-                return cudaErrorInvalidValue;
-            for (int bi = 0; bi < kActBoxes; ++bi) mp.act_shared[bi] = am[(2 + phase) * kActBoxes + bi];
-        } else {
-            mp.shared = mp.routed[0];
-            for (int bi = 0; bi < kActBoxes; ++bi) mp.act_shared[bi] = mp.act_routed[bi];
-        }
-    }
+    if (!ws.tensor_maps || !umma_supported(c)) return cudaErrorNotSupported;
+    const UmmaMaps* const maps = umma_maps_for(m, a);
+    if (!maps) return cudaErrorInvalidValue;
     ChunkInstance* inst = (ChunkInstance*)ws.chunk_inst;
     const uint32_t max_inst = umma_max_chunk_instances(c, T);
     cudaError_t e = launch_after(m, st, chunk_instances_kernel, dim3(1), 256, 0, ws.expert_offsets, ws.expert_counts, ws.slot_of_expert,

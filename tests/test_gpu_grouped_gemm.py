@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from shrike_b200 import capi
+from shrike_b200.moe import MoE
 from gpu_harness import Layer, inputs, rel_l2, small_config, to_act_tensor
 
 pytestmark = pytest.mark.gpu
@@ -41,6 +42,48 @@ def test_narrow_tiles(cuda_device, kw):
     """Tiles of up to 128 rows only: on both sides of every number of K blocks in an activation stage (32 and 64 rows) and of the
     second pair of accumulators (64), with K lengths that end in the middle of a packed slot, a pair of K blocks and a scale block."""
     run_sizes([128, 113, 112, 65, 64, 49, 33, 32, 31, 17, 16, 15] + [3] * 40, kw)
+
+
+def test_a_handle_whose_pool_offsets_or_shared_block_change(cuda_device):
+    """A handle keeps the maps of its last call's operands: another pool (of other chunks), another shared block, other offsets in
+    the same structure, and the first ones again give what a handle of their own gives. (A row's two sums are added to zero: in
+    either order the same.)"""
+    cfg = small_config(d=256, f=192, shared_f=128, num_experts=24, top_k=1, max_tokens=300, shared_gated=False)
+    layers = [Layer(cfg, seed=s, chunks=n) for s, n in ((1, 1), (2, 8))]
+    first, second = layers
+    ids = torch.from_numpy(np.random.default_rng(3).integers(0, 24, (300, 1)).astype(np.int32)).cuda()
+    w = torch.rand((300, 1), generator=torch.Generator().manual_seed(4)).cuda()
+    x = to_act_tensor(inputs(300, cfg.d, seed=5), cfg.act_dtype, first.device)
+    slots, _ = first.classify(ids)
+
+    def run(moe, pool, offsets, shared):
+        y = torch.empty(x.shape, dtype=cfg.torch_y_dtype, device=x.device)
+        moe.encode_prefill(pool, offsets, ids, slots, w, x, y, None, shared)
+        moe.status()
+        return y
+
+    def alone(*operands):
+        moe = MoE(cfg)
+        y = run(moe, *operands)
+        moe.close()
+        return y
+
+    seen = []
+    for pool, shared in ((first.pool, first.shared), (second.pool, second.shared), (second.pool, first.shared),
+                         (first.pool, first.shared)):
+        got = run(first.moe, pool, first.offsets, shared)
+        assert torch.equal(got, alone(pool, first.offsets, shared))
+        seen.append(got)
+    assert torch.equal(seen[0], seen[3]) and not any(torch.equal(a, b) for a, b in zip(seen, seen[1:]))
+    o = first.offsets
+    for part in ("w", "s", "b"):
+        gate, up = getattr(o, f"gate_{part}"), getattr(o, f"up_{part}")
+        setattr(o, f"gate_{part}", up)
+        setattr(o, f"up_{part}", gate)
+    got = run(first.moe, first.pool, o, first.shared)
+    assert torch.equal(got, alone(first.pool, o, first.shared)) and not torch.equal(got, seen[0])
+    for L in layers:
+        L.close()
 
 
 def run_sizes(sizes, kw, sample=None):
