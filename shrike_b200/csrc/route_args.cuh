@@ -24,7 +24,6 @@ struct RouterArgs {
     float* weights;
     float* gate_out;
     uint32_t tokens_per_block;
-    uint32_t row_base;             // first row of this launch (the tiled prefill router leaves only the gate row)
     // fused decode tail (route_fused_kernel only)
     const uint64_t* table;
     uint32_t pool_cells;

@@ -28,7 +28,7 @@ constexpr int kRouterWarps = 8;       // expert rows per block (router_gemv_r4 h
 template <int N, bool PRED, typename Pre>
 __device__ __forceinline__ void logits_rows(const RouterArgs& a, Pre pre) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t e = a.row_base + blockIdx.x * kRouterWarps + warp;
+    const uint32_t e = blockIdx.x * kRouterWarps + warp;
     const bool is_gate = a.gate_row != nullptr && e == a.ne;
     const bool active = e < a.ne || is_gate;
     const bool f32row = a.bits == 0 || is_gate;

@@ -66,14 +66,6 @@ __device__ __forceinline__ uint32_t selection_key_of(float raw, float bias, cons
     return key_of_score(__fadd_rn(a.sigmoid_scores ? sigmoid_det(raw) : raw, bias));
 }
 
-template <bool CG, class A>
-__device__ __forceinline__ uint32_t selection_key(const float* lg, const A& a, uint32_t e) {
-    if (e >= a.ne) return 0u;
-    const float raw = CG ? __ldcg(lg + e) : lg[e];
-    const float bias = a.logit_bias ? bf16_bits_to_f32(a.logit_bias[e]) : 0.0f;
-    return selection_key_of(raw, bias, a);
-}
-
 // Route weights of the picks (lane r holds the r-th pick): moe.metal:458-490, sums in rank order.
 template <bool CG, class A>
 __device__ __forceinline__ float selection_weight(const float* lg, const A& a, uint32_t lane, float my_score,

@@ -574,11 +574,11 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             return epilogue(width, std::integral_constant<int, 4>(), warp >> 2, t, n, 0u, acc1, rowid + at, roww + at);
         };
         // Groups 8*blk .. 8*blk+7 straight from global memory (rows past the matrix and groups past the row read as
-        // zero: the converted weights are then zero). An even number of groups: the warp's 32 rows in 32-bit words, four
+        // zero: the converted weights are then zero). An even number of groups (32-wide ones always): the warp's 32 rows in 32-bit words, four
         // lanes a row, handed to the rows' lanes when they are needed; read by each row's threads in 16-bit pieces
         // they kept L1 busy for 1.3 us per K block of 90-group rows.
         auto fetch_scales = [&](uint32_t blk) {
-            if ((G & 1u) == 0) {
+            if (GROUP == 32 || (G & 1u) == 0) {
                 const uint32_t gi = blk * 8 + 2 * (lane & 3);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -609,7 +609,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         };
         // The eight groups fetched one block ago into sreg / breg, and the next ones asked for.
         auto turn_scales = [&](uint32_t blk) {
-            if ((G & 1u) == 0) {
+            if (GROUP == 32 || (G & 1u) == 0) {
                 __syncwarp();   // the last block's have been read
                 if constexpr (GROUP == 32) {
                     // through shared memory: a thread's half has the even or the odd groups, so the two warps of a row write 16
@@ -657,7 +657,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             }
         };
         auto first_scales = [&]() {
-            if (GROUP == 32 && (G & 1u) == 0) {
+            if constexpr (GROUP == 32) {
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     const uint32_t row = my_rows - (lane >> 2) + (lane >> 1) + 16 * i;
@@ -672,7 +672,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         };
         // Block blk's scales into sreg / breg: 32-wide groups this thread's two words, else all four.
         auto narrow_scales = [&](uint32_t blk) {
-            if (GROUP == 32 && (G & 1u) == 0) {
+            if constexpr (GROUP == 32) {
                 // word j of row `lane` sits in lane 2 (row mod 16) + j of load row / 16
                 auto exchange = [&](uint32_t* sv, uint32_t* bv) {
 #pragma unroll
@@ -687,15 +687,8 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                 };
                 if (blk & 1) exchange(snext + 2, bnext + 2);
                 else exchange(snext, bnext);
-                return;
-            }
-            turn_scales(blk);
-            if (GROUP == 32) {   // (turn_scales left all words)
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    sreg[i] = half ? sreg[2 * i + 1] : sreg[2 * i];
-                    breg[i] = half ? breg[2 * i + 1] : breg[2 * i];
-                }
+            } else {
+                turn_scales(blk);
             }
         };
         auto scale_words = [&](uint32_t s16, uint32_t b16, uint32_t& s2, uint32_t& z2) {
