@@ -1,7 +1,7 @@
 """The expert-grouped GEMM with more tiles than SMs, against the oracle: instances on both sides of every stage layout
 (1, 16, 64, 65, 128, 129 and 256 rows and one more than 256) follow one another on an SM, shared and routed experts have
-different numbers of row tiles, and the last ones are partial. Tiles of two K blocks, which use two of the three activation stages,
-between longer ones and another layout."""
+different numbers of row tiles, and the last ones are partial. Wide tiles of two K blocks, which use two of the three activation stages,
+before narrow ones; narrow tiles alone, more of them on an SM than it has places for tiles."""
 import numpy as np
 import pytest
 import torch
@@ -27,8 +27,8 @@ def test_tiles_of_every_layout(cuda_device, kw):
     dict(d=2048, f=128, shared_f=192, weight_bits=8, group_size=32),
 ], ids=lambda kw: "-".join(f"{k}{v}" for k, v in kw.items()))
 def test_a_short_tile_before_another_layout(cuda_device, kw):
-    """The shared expert's last instance has 24 rows and three or six K blocks in the down projection, the routed experts two:
-    on many SMs a remainder of one row follows it, which leaves the third stage to it, and then a tile of 256 rows."""
+    """The routed experts' wide tiles have two K blocks in the down projection, the shared expert's three or six: the tiles of one and
+    of 24 rows that follow on the same SMs have the other layout, while the accumulators of the last wide tile are still read."""
     run_sizes([257] * 24, kw, sample=24)
 
 
@@ -39,9 +39,20 @@ def test_a_short_tile_before_another_layout(cuda_device, kw):
     dict(d=1024, f=512, shared_f=512, weight_bits=8, group_size=32, meta_dtype=capi.DTYPE_FP16, expert_bias=1),
 ], ids=lambda kw: "-".join(f"{k}{v}" for k, v in kw.items()))
 def test_narrow_tiles(cuda_device, kw):
-    """Tiles of up to 128 rows only: on both sides of every number of K blocks in an activation stage (32 and 64 rows) and of the
-    second pair of accumulators (64), with K lengths that end in the middle of a packed slot, a pair of K blocks and a scale block."""
+    """The routed experts' tiles have up to 128 rows (the shared expert's full ones come before them): on both sides of every number
+    of K blocks in an activation stage (32 and 64 rows) and of the second pair of accumulators (64), with K lengths that end in the middle of a packed slot, a pair of K blocks and a scale block."""
     run_sizes([128, 113, 112, 65, 64, 49, 33, 32, 31, 17, 16, 15] + [3] * 40, kw)
+
+
+@pytest.mark.parametrize("kw", [
+    dict(d=640, f=640),
+    dict(d=704, f=576, group_size=32, expert_bias=1),
+], ids=lambda kw: "-".join(f"{k}{v}" for k, v in kw.items()))
+def test_narrow_tiles_alone(cuda_device, kw):
+    """No wide tile and no shared expert: 768 tiles and more in both projections, five and more on an SM of 148, so that the four
+    places for tiles, the accumulators' barriers and both kinds of narrow tile come round again."""
+    sizes = [128, 97, 96, 80, 72, 66, 65, 64, 63, 48, 33, 32, 17, 16] + [1 + 7 * e % 24 for e in range(242)]
+    run_sizes(sizes, dict(kw, num_experts=256, has_shared=False, shared_f=0), sample=100)
 
 
 def test_a_handle_whose_pool_offsets_or_shared_block_change(cuda_device):
@@ -87,7 +98,7 @@ def test_a_handle_whose_pool_offsets_or_shared_block_change(cuda_device):
 
 
 def run_sizes(sizes, kw, sample=None):
-    cfg = small_config(num_experts=64, top_k=1, max_tokens=max(1024, sum(sizes)), shared_gated=False, **kw)
+    cfg = small_config(**dict(dict(num_experts=64, top_k=1, max_tokens=max(1024, sum(sizes)), shared_gated=False), **kw))
     layer = Layer(cfg)
     ids = np.concatenate([np.full(n, e, np.uint32) for e, n in enumerate(sizes)])
     ids = np.random.default_rng(3).permutation(ids)[:, None]
