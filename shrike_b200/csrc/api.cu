@@ -180,10 +180,10 @@ int fill_expert_args(shrike_moe* m, const shrike_pool* pool, const shrike_expert
 // tile (us a layer, one-row or per-tile kernels and streaming; 256 experts of 2048 x 512 int4 | 32 of 2880 x 2880 int4 | 256 of
 // 2304 x 1024 int8: 17.0, 22.9 | 40.4, 42.0 | 34.0, 36.3); two rows have: 29.3, 27.1 | 88, 57.5 | 46.8, 43.3. Up to 64 rows it is
 // also ahead of the expert-grouped GEMM, which reads an expert once for all its rows but starts in a dozen launches, unless few
-// large experts get skewed picks, which only the device knows (streaming, when its routing took 5 to 8 us more, and grouped,
-// uniform picks):
-//   17 rows  69, 115 | 179, 253 | 132, 200       64 rows  131, 190 | 262, 255 | 252, 344
-// With picks by Zipf(1.1), 64 rows: 87, 113 | 259, 222 | 192, 246.
+// large experts get many rows (streaming and grouped, uniform picks):
+//   17 rows  65, 96 | 152, 214 | 136, 186     48 rows  109, 151 | 191, 220 | 226, 292     64 rows  123, 166 | 241, 220 | 252, 324
+// With picks by Zipf(1.1), 48 rows: 68, 83 | 211, 201 | 160, 194; 64 rows: 80, 92 | 241, 198 | 182, 204. There too its rows are sums in
+// a fixed order, which the grouped GEMM's are not, and those of the separate calls.
 // The projections as calls of their own follow the same rule, so that they give a layer call's rows bit for bit. Each pays the
 // kernel's set-up, with no router to share: plan and both of them, us, per-tile kernels and streaming, 30.3, 32.8 | 85, 62 | 45.9,
 // 49.3 at two rows, 34.4, 37.0 | 113, 76 | 60.2, 57.5 at three, 41.1, 39.9 | 138, 82 | 72, 66 at four.
@@ -229,8 +229,8 @@ int encode_prefill(shrike_moe* m, void* stream, const shrike_pool* pool,
     // every expert on the 8-row warp-MMA tiles (the decode kernels); SHRIKE_PREFILL_PATH=mma in the
     // environment of shrike_moe_create forces them for a handle (a test switch).
     const bool warp_mma = m->force_warp_mma || !umma_supported(m->cfg);
-    // fp32 rows out and no residual to add: the down epilogue adds straight into y (zeroed by the plan; x is read
-    // after that, so not when y is x) and no pass over the rows follows
+    // fp32 rows out and no residual to add: the down epilogue adds straight into y and no pass over the rows follows. The
+    // kernel that reads x clears y, block by block: not when y is x (they must not overlap otherwise)
     const bool direct = m->cfg.y_dtype == SHRIKE_DTYPE_FP32 && !hidden && y != x;
     if (direct) a.yacc = (float*)y;
     CU(launch_prefill_plan(m, st, topk_indices, resolved_slots, x, query_count, m->cfg.has_shared != 0,
@@ -756,11 +756,13 @@ int shrike_encode_decode_layer(shrike_moe* m, void* stream, const shrike_pool* p
     }
     // Shapes that the streaming kernel does not take, with many rows, on a handle that owns the prefill operands: the
     // expert-grouped GEMM reads every expert once for all its rows, where the 8-row tiles read it once per 8. The dozen
-    // launches around it pay from about 50 rows on (us a layer, tiles and grouped, odd numbers of groups, picks uniform or by Zipf(1.1);
+    // launches around it pay from 24 to 50 rows on, by the number of experts; the line is where no shape loses (us a layer, tiles and
+    // grouped, odd numbers of groups, picks uniform or by Zipf(1.1);
     // 256 experts of 2048 x 576 int4 | 256 of 2304 x 1088 int8 | 32 of 2880 x 2880 int4 in groups of 64):
-    //   17 rows  120, 167 | 191, 256 | 240, 378     Zipf   62, 91 | 150, 221 | 161, 268
-    //   48 rows  226, 266 | 351, 414 | 302, 384     Zipf  124, 119 | 260, 290 | 301, 324
-    //   64 rows  263, 297 | 410, 459 | 374, 386     Zipf  157, 130 | 311, 301 | 368, 321
+    //   17 rows  119, 116 | 199, 200 | 231, 295     Zipf   63, 71 | 151, 162 | 158, 248
+    //   32 rows  176, 156 | 281, 257 | 260, 303     Zipf   89, 79 | 194, 182 | 240, 251
+    //   48 rows  223, 182 | 361, 318 | 301, 304     Zipf  128, 92 | 254, 214 | 304, 278
+    //   64 rows  259, 202 | 413, 349 | 369, 304     Zipf  161, 100 | 298, 224 | 364, 277
     if (query_count > 48 && w.xs && umma_supported(m->cfg) && !m->force_warp_mma) {
         int rcg = shrike_encode_router(m, stream, router, x, query_count, m->cfg.d, ids, wt, gate);
         if (rcg) return rcg;

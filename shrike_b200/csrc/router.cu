@@ -442,7 +442,8 @@ __global__ void __launch_bounds__(kRouterWarps * 32) route_fused_kernel(const Ro
         }
     } else {
         // several rows: a warp per row, the rows side by side (the same picks and weights: both forms build the
-        // list of the reference's insertion scan)
+        // list of the reference's insertion scan). By rounds: ranked by comparison, as in the streaming kernel, this launch
+        // takes 14.8 us instead of 15.8 for 16 rows of 256 experts, but 11.1 instead of 10.4 for 4 rows of 32.
         for (uint32_t row = warp; row < a.T; row += kRouterWarps) {
             uint32_t id;
             float w;

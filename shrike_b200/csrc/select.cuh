@@ -136,7 +136,7 @@ __device__ __forceinline__ void pick_rounds(uint32_t (&key)[8], uint32_t top_k, 
     }
 }
 
-// Top-k of one row by one warp. Lane r returns the r-th pick.
+// Top-k of one row by one warp, for the kernel that routes in a launch of its own. Lane r returns the r-th pick.
 // CG: read the logits past L1 (they were written by other blocks of this launch).
 template <bool CG, class A>
 __device__ __forceinline__ void select_row(const float* lg, const A& a, uint32_t lane,

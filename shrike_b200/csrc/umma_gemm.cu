@@ -36,8 +36,8 @@
 //          weighted reduce, with no per-(row, rank) partial rows in between).
 //
 // What bounds it (256 experts of 2048 x 512, int4): at 256 rows a K block takes 0.74 to 0.76 us. That is 8.39 MFLOP on each of 148
-// SMs: 1.63 to 1.68 PFLOP/s, as fast as the measured burst rate of a library GEMM (1.67). What is left of full tiles lies outside
-// the K loop: 9 of a down tile's 14 us. With few rows the issue slots of the converters (70 % taken at 10 rows an expert; fp16
+// SMs: 1.63 to 1.68 PFLOP/s, as fast as the measured burst rate of a library GEMM (1.63). What is left of full tiles lies outside
+// the K loop: 12,600 of a down tile's 25,800 cycles. With few rows the issue slots of the converters (70 % taken at 10 rows an expert; fp16
 // arithmetic and logic run at half the rate there); 10 rows an expert take 93 us for gate/up and 62 for down, 2.9 TB/s.
 //
 // Every wait is bounded; a wait that gives up sets the status word and the
@@ -369,7 +369,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
     uint64_t* conv = tile_empty + kTiles;          // the converter warps among themselves (a named barrier has no bounded wait)
     uint64_t* eids_full = conv + 1;                // the epilogue warps among themselves
     uint4* next_tile = (uint4*)(smem + kOffTiles);                  // [kTiles]
-    uint32_t* rowid = (uint32_t*)(next_tile + kTiles);              // token of a column: [2][256], tiles in turn, or [4][128]
+    uint32_t* rowid = (uint32_t*)(next_tile + kTiles);              // token of a column: [2][256], tiles in turn
     float* roww = (float*)(rowid + 2 * kUmmaMaxN);                  // route weight (routed) or gate (shared)
     uint32_t* small_id = (uint32_t*)(roww + 2 * kUmmaMaxN);          // the same of a small tile: [2][64], tiles in turn
     float* small_w = (float*)(small_id + 2 * kSmallN);
@@ -402,8 +402,8 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
     const uint32_t tmem_base = *tmem_slot;
     // All of the above runs while the last kernel ends. The down projection takes its first tiles and converts their weights
     // meanwhile: of what comes before, only the activations are the gate/up launch's, and the warp that copies them waits. The list, the
-    // pairs and the cleared rows were there when that launch let this one start (they are read past L1). 333 rows 196 -> 189 us a
-    // call, 4096 rows 494 -> 475.
+    // pairs and the cleared rows were there when that launch let this one start (they are read past L1). 333 rows 196 -> 187 us a
+    // call, 4096 rows 498 -> 490.
     if (PHASE == 0) {
         pdl_wait();
         pdl_launch_dependents();
@@ -1200,8 +1200,8 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
 }
 
 // The list of instances: all full ones (256 rows; the shared expert's first), then every expert's rest, most rows first. A tile of
-// 256 rows takes twice the time of one of 16, and a list that ends on long ones leaves SMs idle; and a block then changes the
-// layout of its shared memory twice at most. One thread per expert; n_inst[0] = instances, [1], [2]: tiles handed out in phase 0, 1.
+// 256 rows takes twice the time of one of 16, and a list that ends on long ones leaves SMs idle. All tiles of more than 128 rows come before the
+// others, so a block changes the layout of its shared memory once at most: the barrier wide_over has one phase for it. One thread per expert; n_inst[0] = instances, [1], [2]: tiles handed out in phase 0, 1.
 __global__ void __launch_bounds__(256)
 chunk_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ counts,
                        const uint32_t* __restrict__ slot_of_expert, uint32_t ne, uint32_t T, uint32_t with_shared,
