@@ -493,3 +493,29 @@ def test_both_ranks_rows_beside_words_that_are_there(cuda_device, T, dtype):
         assert (theirs[3][0, n:] == -7.0).all() and (theirs[3][1] == -7.0).all() and (mine[3][0] == 7.0).all()
         assert layer.last_counts()[0] == [int(sent[3][0]), int(sent[3][1])] and layer.last_counts()[1] == int(sent[3][0]) + n
     layer.close()
+
+
+@pytest.mark.parametrize("T,world,skip", [(1, 1, 0), (5, 3, 1), (37, 8, 0), (65536 + 37, 2, 0), (65536 + 3, 2, 1)])
+def test_combine_matches_the_protocol(cuda_device, T, world, skip):
+    """More rows than one launch numbers, ranks in whole and broken fours, rows that are not whole vectors: the sums in rank order."""
+    import ep_reference as R
+    from shrike_b200.moe import MoE, _ptr, _stream
+    cfg = dataclasses.replace(_config(), d=64)
+    moe = MoE(cfg)
+    rng = np.random.default_rng(T)
+    cap = min(T, 300)
+    recv = rng.normal(0, 1, (world, cap, 64)).astype(np.float32)
+    row_of = rng.integers(-1, cap, (T, world)).astype(np.int32)
+    home, x = rng.normal(0, 1, (T, 64)).astype(np.float32), rng.normal(0, 1, (T, 64)).astype(np.float32)
+    y, h = (torch.zeros(T * 64 + 8, device="cuda")[skip:skip + T * 64].view(T, 64) for _ in range(2))
+    h.copy_(torch.from_numpy(x))
+    operands = [torch.from_numpy(v).cuda() for v in (recv, row_of, home)]   # (held until the call is over)
+    moe._check(moe._lib.shrike_ep_encode_combine(moe._h, _stream(), *map(_ptr, operands), T, world, cap, _ptr(y), _ptr(h)))
+    moe.status()
+    want = home.copy()
+    for g in range(world):
+        want += np.where(row_of[:, g, None] >= 0, recv[g][np.maximum(row_of[:, g], 0)], np.float32(0))
+    if T < 100:
+        assert np.array_equal(want, R.combine(recv, row_of, home))
+    assert (y.cpu().numpy() == want).all() and (h.cpu().numpy() == x + want).all()
+    moe.close()
