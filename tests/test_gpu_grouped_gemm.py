@@ -97,6 +97,23 @@ def test_a_handle_whose_pool_offsets_or_shared_block_change(cuda_device):
         L.close()
 
 
+@pytest.mark.parametrize("T", [1, 100])
+def test_rows_in_place(cuda_device, T):
+    """y is x: the down projection may not add into rows that are still read, so the call takes the rows of its own."""
+    cfg = small_config(d=256, f=192, shared_f=128, num_experts=24, top_k=1, max_tokens=100, shared_gated=False)
+    layer = Layer(cfg)
+    ids = torch.from_numpy(np.random.default_rng(3).integers(0, 24, (T, 1)).astype(np.int32)).cuda()
+    w = torch.rand((T, 1), generator=torch.Generator().manual_seed(4)).cuda()
+    x = to_act_tensor(inputs(T, cfg.d, seed=5), cfg.act_dtype, layer.device)
+    slots, _ = layer.classify(ids)
+    y, same = torch.empty_like(x), x.clone()
+    for rows, out in ((x, y), (same, same)):
+        layer.moe.encode_prefill(layer.pool, layer.offsets, ids, slots, w, rows, out, None, layer.shared)
+        layer.moe.status()
+    assert torch.equal(y, same) and not torch.equal(y, x)
+    layer.close()
+
+
 def run_sizes(sizes, kw, sample=None):
     cfg = small_config(**dict(dict(num_experts=64, top_k=1, max_tokens=max(1024, sum(sizes)), shared_gated=False), **kw))
     layer = Layer(cfg)
