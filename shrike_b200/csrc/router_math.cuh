@@ -111,7 +111,7 @@ __device__ __forceinline__ float lane_dot_f32(const float4 (&wr)[N], uint32_t ch
 }
 
 // router_gemv_body (moe.metal:324-364): lane l takes elements 64g+2l, 64g+2l+1 of every group g.
-// The operands of eight groups are requested before the first is used (one memory round trip per
+// The operands of eight groups are requested, as they are in memory, before the first is used (one memory round trip per
 // eight groups instead of one per group); the arithmetic and its order are the shader's.
 __device__ __forceinline__ float lane_dot_affine(const uint8_t* row, const uint16_t* s_row,
                                                  const uint16_t* b_row, uint32_t bits, uint32_t groups,
@@ -119,42 +119,38 @@ __device__ __forceinline__ float lane_dot_affine(const uint8_t* row, const uint1
                                                  const uint16_t* eff_scale) {
     float acc = 0.f;
     constexpr uint32_t kBatch = 8;
+#pragma unroll 1
     for (uint32_t g0 = 0; g0 < groups; g0 += kBatch) {
         uint16_t sr[kBatch], br[kBatch];
         uint32_t qr[kBatch], er[kBatch];
-        float x0r[kBatch], x1r[kBatch];
+        uint2 xr[kBatch];
 #pragma unroll
         for (uint32_t j = 0; j < kBatch; ++j) {
-            const uint32_t gi = g0 + j;
-            if (gi < groups) {
-                const uint32_t idx = gi * 64 + lane * 2;
-                sr[j] = s_row[gi];
-                br[j] = b_row[gi];
-                // both elements: one byte (int4) or two bytes (int8), the low one first
-                qr[j] = bits == 4 ? (uint32_t)row[idx >> 1] : (uint32_t)*(const uint16_t*)(row + idx);
-                if (dt == SHRIKE_DTYPE_FP32) {
-                    const float2 v = *(const float2*)((const float*)xrow + idx);
-                    x0r[j] = v.x; x1r[j] = v.y;
-                } else {
-                    const uint32_t v = *(const uint32_t*)((const uint16_t*)xrow + idx);
-                    if (dt == SHRIKE_DTYPE_FP16) {
-                        x0r[j] = f16_bits_to_f32(v & 0xffff); x1r[j] = f16_bits_to_f32(v >> 16);
-                    } else {
-                        x0r[j] = __uint_as_float(v << 16); x1r[j] = __uint_as_float(v & 0xffff0000u);
-                    }
-                }
-                er[j] = eff_scale ? *(const uint32_t*)(eff_scale + idx) : 0x3f803f80u;
-            }
+            const uint32_t gi = min(g0 + j, groups - 1), idx = gi * 64 + lane * 2;   // (past the end: the last group again, unused)
+            sr[j] = s_row[gi];
+            br[j] = b_row[gi];
+            // both elements: one byte (int4) or two bytes (int8), the low one first
+            qr[j] = bits == 4 ? (uint32_t)row[idx >> 1] : (uint32_t)*(const uint16_t*)(row + idx);
+            xr[j] = make_uint2(0u, 0u);
+            if (dt == SHRIKE_DTYPE_FP32) xr[j] = *(const uint2*)((const float*)xrow + idx);
+            else xr[j].x = *(const uint32_t*)((const uint16_t*)xrow + idx);
+            er[j] = eff_scale ? *(const uint32_t*)(eff_scale + idx) : 0x3f803f80u;
         }
 #pragma unroll
         for (uint32_t j = 0; j < kBatch; ++j) {
-            const uint32_t gi = g0 + j;
-            if (gi < groups) {
+            if (g0 + j < groups) {
                 const float sc = bf16_bits_to_f32(sr[j]);
                 const float bi = bf16_bits_to_f32(br[j]);
                 const float q0 = (float)(bits == 4 ? (qr[j] & 0xfu) : (qr[j] & 0xffu));
                 const float q1 = (float)(bits == 4 ? (qr[j] >> 4) : (qr[j] >> 8));
-                float x0 = x0r[j], x1 = x1r[j];
+                float x0, x1;
+                if (dt == SHRIKE_DTYPE_FP32) {
+                    x0 = __uint_as_float(xr[j].x); x1 = __uint_as_float(xr[j].y);
+                } else if (dt == SHRIKE_DTYPE_FP16) {
+                    x0 = f16_bits_to_f32(xr[j].x & 0xffff); x1 = f16_bits_to_f32(xr[j].x >> 16);
+                } else {
+                    x0 = __uint_as_float(xr[j].x << 16); x1 = __uint_as_float(xr[j].x & 0xffff0000u);
+                }
                 if (eff_scale) {
                     x0 = __fmul_rn(x0, __uint_as_float(er[j] << 16));
                     x1 = __fmul_rn(x1, __uint_as_float(er[j] & 0xffff0000u));
