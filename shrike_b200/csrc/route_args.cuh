@@ -44,5 +44,8 @@ struct RouterArgs {
 
 RouterArgs make_router_args(const shrike_moe* m, const shrike_router_operands& ops, const void* hidden, uint32_t T,
                             uint32_t stride, uint32_t* ids, float* weights, float* shared_gate);
+// router_tile.cu: the logits (and gate values) of a call of many rows; whether it takes these operands
+bool router_tiles_take(const RouterArgs& a);
+cudaError_t launch_router_tiles(const shrike_moe* m, cudaStream_t st, const RouterArgs& a);
 
 }  // namespace shrike

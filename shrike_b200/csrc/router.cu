@@ -73,307 +73,6 @@ __global__ void __launch_bounds__(kRouterWarps * 32) router_logits_kernel(const 
     logits_body(a, [] {});
 }
 
-// ---- prefill router: register-tiled logits ---------------------------------------
-//
-// Hundreds of rows against the same fp32 router matrix: the warp-per-row kernel
-// above re-reads every activation row once per expert row and stalls on those
-// loads. Here a block owns 32 expert rows x 32 tokens, stages both operands in
-// shared memory (activations converted to fp32 once per block), and a warp
-// accumulates an 8 x 16 register tile. Lane l still owns the float4 chunks
-// l, l+32, ... of every row and walks them in order with one fused multiply-add
-// per element, and the 32 lane sums still meet in the xor 16..1 butterfly, so
-// each logit is the same sequence of roundings as in the warp-per-row kernel.
-// Chunks past the end of a row are staged as zeros: adding +0 changes nothing.
-constexpr int kTileRows = 32, kTileTokens = 32, kTileStage = 256;   // 256 elements of K per stage
-constexpr int kTileWarpRows = 8, kTileWarpTokens = 16;
-constexpr size_t kTileSmemBytes = 2 * (size_t)(kTileRows + kTileTokens) * kTileStage * sizeof(float);
-
-__device__ __forceinline__ void cp_async_16_zfill(uint32_t smem_addr, const void* gptr, bool valid) {
-    const uint32_t n = valid ? 16u : 0u;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr), "l"(gptr), "r"(n) : "memory");
-}
-
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-    uint64_t v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
-    return v;
-}
-
-// The lane sums of a warp's tile, [token][row], meet in the xor 16..1 order of butterfly_sum, each lane keeping half of the
-// values at every step (124 exchanges instead of 640; an addition does not care which side it is on). Lane l ends with
-// values 4l .. 4l + 3: rows 4 (l & 1) and on of token l / 2.
-__device__ __forceinline__ void store_tile(const RouterArgs& a, float (&v)[kTileWarpTokens * kTileWarpRows], uint32_t e, uint32_t tok, uint32_t lane) {
-    static_assert(kTileWarpTokens * kTileWarpRows == 128 && kTileWarpRows == 8, "four values a lane");
-#pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) {
-        const bool up = (lane & m) != 0;
-#pragma unroll
-        for (int i = 0; i < 4 * m; ++i) {
-            const float keep = up ? v[i + 4 * m] : v[i], send = up ? v[i] : v[i + 4 * m];
-            v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, m));
-        }
-    }
-    tok += lane >> 1;
-    e += (lane & 1) * 4;
-    if (tok >= a.T) return;
-    float* const dst = a.logits + (size_t)tok * a.ne + e;
-    if (e + 4 <= a.ne && (a.ne & 3u) == 0) {
-        *(float4*)dst = make_float4(v[0], v[1], v[2], v[3]);
-    } else {
-#pragma unroll
-        for (uint32_t i = 0; i < 4; ++i)
-            if (e + i < a.ne) dst[i] = v[i];
-    }
-}
-
-__global__ void __launch_bounds__(256, 1) router_logits_tiled_kernel(const RouterArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
-    extern __shared__ __align__(16) float tile_smem[];
-    float* const w_s = tile_smem;                                           // [2][32][256]
-    float* const x_s = tile_smem + 2 * kTileRows * kTileStage;              // [2][32][256]
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t e0 = blockIdx.x * kTileRows, t0 = blockIdx.y * kTileTokens;
-    const uint32_t chunks = a.d / 4;
-    const uint32_t stages = (a.d + kTileStage - 1) / kTileStage;
-    const size_t esz = a.dt == SHRIKE_DTYPE_FP32 ? 4 : 2;
-
-    // staging roles: thread -> (row, 8 chunks of 4 floats) of each operand tile
-    const uint32_t srow = tid >> 3, sc0 = (tid & 7) * 8;                    // 32 rows x 8 threads x 8 chunks
-    const uint32_t wrow = min(e0 + srow, a.ne - 1), xtok = min(t0 + srow, a.T - 1);
-    const float* const wsrc = (const float*)a.w + (size_t)wrow * a.d;
-    const uint8_t* const xsrc = (const uint8_t*)a.hidden + (size_t)xtok * a.stride * esz;
-
-    uint4 xr[8];   // the next stage's activations: 32 elements (16-bit) or 2 x 16 (fp32)
-    auto fetch_w = [&](uint32_t s, uint32_t buf) {
-        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(w_s + ((size_t)buf * kTileRows + srow) * kTileStage);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint32_t c = s * (kTileStage / 4) + sc0 + j;
-            cp_async_16_zfill(dst + (sc0 + j) * 16, wsrc + (size_t)min(c, chunks - 1) * 4, c < chunks);
-        }
-        cp_async_commit();
-    };
-    auto fetch_x = [&](uint32_t s) {
-        if (a.dt == SHRIKE_DTYPE_FP32) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint32_t c = s * (kTileStage / 4) + sc0 + j;
-                xr[j] = c < chunks ? __ldg((const uint4*)xsrc + c) : make_uint4(0, 0, 0, 0);
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t c = s * (kTileStage / 4) + sc0 + 2 * j;       // two chunks per 16 bytes
-                xr[j] = c < chunks ? __ldg((const uint4*)xsrc + c / 2) : make_uint4(0, 0, 0, 0);
-            }
-        }
-    };
-    auto store_x = [&](uint32_t s, uint32_t buf) {
-        float4* const dst = (float4*)(x_s + ((size_t)buf * kTileTokens + srow) * kTileStage) + sc0;
-        const uint2* const es = a.eff_scale ? (const uint2*)a.eff_scale + s * (kTileStage / 4) + sc0 : nullptr;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            float4 v;
-            if (a.dt == SHRIKE_DTYPE_FP32) {
-                v = make_float4(__uint_as_float(xr[j].x), __uint_as_float(xr[j].y), __uint_as_float(xr[j].z),
-                                __uint_as_float(xr[j].w));
-            } else {
-                const uint32_t lo = (j & 1) ? xr[j / 2].z : xr[j / 2].x, hi = (j & 1) ? xr[j / 2].w : xr[j / 2].y;
-                if (a.dt == SHRIKE_DTYPE_FP16)
-                    v = make_float4(f16_bits_to_f32(lo & 0xffff), f16_bits_to_f32(lo >> 16), f16_bits_to_f32(hi & 0xffff),
-                                    f16_bits_to_f32(hi >> 16));
-                else
-                    v = make_float4(__uint_as_float(lo << 16), __uint_as_float(lo & 0xffff0000u),
-                                    __uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u));
-            }
-            if (es && s * (kTileStage / 4) + sc0 + j < chunks) {
-                const uint2 q = __ldg(es + j);
-                v.x = __fmul_rn(v.x, __uint_as_float(q.x << 16));
-                v.y = __fmul_rn(v.y, __uint_as_float(q.x & 0xffff0000u));
-                v.z = __fmul_rn(v.z, __uint_as_float(q.y << 16));
-                v.w = __fmul_rn(v.w, __uint_as_float(q.y & 0xffff0000u));
-            }
-            dst[j] = v;
-        }
-    };
-
-    float acc[kTileWarpRows][kTileWarpTokens];
-#pragma unroll
-    for (int r = 0; r < kTileWarpRows; ++r)
-#pragma unroll
-        for (int t = 0; t < kTileWarpTokens; ++t) acc[r][t] = 0.f;
-
-    fetch_w(0, 0);
-    fetch_x(0);
-    store_x(0, 0);
-    cp_async_wait<0>();
-    __syncthreads();
-
-    const uint32_t rg = warp & 3, tg = warp >> 2;
-    for (uint32_t s = 0; s < stages; ++s) {
-        const uint32_t buf = s & 1;
-        const bool more = s + 1 < stages;
-        if (more) {
-            fetch_w(s + 1, buf ^ 1);
-            fetch_x(s + 1);
-        }
-        const float4* const wb = (const float4*)(w_s + ((size_t)buf * kTileRows + rg * kTileWarpRows) * kTileStage);
-        const float4* const xb = (const float4*)(x_s + ((size_t)buf * kTileTokens + tg * kTileWarpTokens) * kTileStage);
-#pragma unroll
-        for (int ii = 0; ii < kTileStage / 128; ++ii) {
-            float4 wv[kTileWarpRows];
-#pragma unroll
-            for (int r = 0; r < kTileWarpRows; ++r) wv[r] = wb[r * (kTileStage / 4) + ii * 32 + lane];
-#pragma unroll
-            for (int t = 0; t < kTileWarpTokens; ++t) {
-                const float4 xv = xb[t * (kTileStage / 4) + ii * 32 + lane];
-#pragma unroll
-                for (int r = 0; r < kTileWarpRows; ++r) {
-                    float v = acc[r][t];
-                    v = __fmaf_rn(wv[r].x, xv.x, v);
-                    v = __fmaf_rn(wv[r].y, xv.y, v);
-                    v = __fmaf_rn(wv[r].z, xv.z, v);
-                    v = __fmaf_rn(wv[r].w, xv.w, v);
-                    acc[r][t] = v;
-                }
-            }
-        }
-        if (more) {
-            store_x(s + 1, buf ^ 1);
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-    }
-
-    float sums[kTileWarpTokens * kTileWarpRows];
-#pragma unroll
-    for (int t = 0; t < kTileWarpTokens; ++t)
-#pragma unroll
-        for (int r = 0; r < kTileWarpRows; ++r) sums[t * kTileWarpRows + r] = acc[r][t];
-    store_tile(a, sums, e0 + rg * kTileWarpRows, t0 + tg * kTileWarpTokens, lane);
-}
-
-// The same tile for 16-bit activations without a per-column scale (the common case): both operands go to
-// shared memory by cp.async, three stages deep, the activations as they are (half the bytes), and are widened
-// where they are multiplied -- exact, so the logits are unchanged. Thread t of a row's eight copies 16-byte
-// units t, t + 8, ...: a warp's copies land 128 bytes a row, free of bank conflicts. (The kernel above holds
-// the next stage's activations in registers across the multiply loop; the compiler sinks those loads to their
-// use, and a block of 8 warps then waits for L2 once per stage.)
-constexpr uint32_t kTile16WBytes = kTileRows * kTileStage * 4, kTile16XBytes = kTileTokens * kTileStage * 2;
-constexpr uint32_t kTile16Buf = kTile16WBytes + kTile16XBytes, kTile16Bufs = 3;
-constexpr size_t kTile16SmemBytes = (size_t)kTile16Bufs * kTile16Buf;
-
-template <bool FP16>
-__global__ void __launch_bounds__(256, 1) router_logits_tiled16_kernel(const RouterArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
-    extern __shared__ __align__(16) uint8_t tile16_smem[];
-    const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(tile16_smem);
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t e0 = blockIdx.x * kTileRows, t0 = blockIdx.y * kTileTokens;
-    const uint32_t chunks = a.d / 4, units = a.d / 8;   // float4 chunks of a weight row, 16-byte units of an activation row
-    const uint32_t stages = (a.d + kTileStage - 1) / kTileStage;
-    const uint32_t srow = tid >> 3, l8 = tid & 7;
-    const float* const wsrc = (const float*)a.w + (size_t)min(e0 + srow, a.ne - 1) * a.d;
-    const uint8_t* const xsrc = (const uint8_t*)a.hidden + (size_t)min(t0 + srow, a.T - 1) * a.stride * 2;
-
-    auto fetch = [&](uint32_t s, uint32_t buf) {
-        const uint32_t wdst = smem0 + buf * kTile16Buf + srow * (kTileStage * 4);
-#pragma unroll
-        for (uint32_t j = 0; j < 8; ++j) {
-            const uint32_t u = j * 8 + l8, c = s * (kTileStage / 4) + u;
-            cp_async_16_zfill(wdst + u * 16, wsrc + (size_t)min(c, chunks - 1) * 4, c < chunks);
-        }
-        const uint32_t xdst = smem0 + buf * kTile16Buf + kTile16WBytes + srow * (kTileStage * 2);
-#pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-            const uint32_t u = j * 8 + l8, c = s * (kTileStage / 8) + u;
-            cp_async_16_zfill(xdst + u * 16, xsrc + (size_t)min(c, units - 1) * 16, c < units);
-        }
-        cp_async_commit();
-    };
-
-    // [row][token pair]: one packed instruction does a fused multiply-add for each of two tokens, each rounded as ever
-    uint64_t acc[kTileWarpRows][kTileWarpTokens / 2];
-#pragma unroll
-    for (int r = 0; r < kTileWarpRows; ++r)
-#pragma unroll
-        for (int t = 0; t < kTileWarpTokens / 2; ++t) acc[r][t] = 0;
-
-    fetch(0, 0);
-    if (stages > 1) fetch(1, 1);
-    const uint32_t rg = warp & 3, tg = warp >> 2;
-    for (uint32_t s = 0; s < stages; ++s) {
-        const uint32_t buf = s % kTile16Bufs;
-        if (s + 1 < stages) cp_async_wait<1>();
-        else cp_async_wait<0>();
-        __syncthreads();   // stage s has landed for every thread, and every warp is done with stage s - 1
-        if (s + 2 < stages) fetch(s + 2, (s + 2) % kTile16Bufs);
-        const float4* const wb = (const float4*)(tile16_smem + (size_t)buf * kTile16Buf) + rg * kTileWarpRows * (kTileStage / 4);
-        const uint2* const xb = (const uint2*)(tile16_smem + (size_t)buf * kTile16Buf + kTile16WBytes) + tg * kTileWarpTokens * (kTileStage / 4);
-#pragma unroll
-        for (int ii = 0; ii < kTileStage / 128; ++ii) {
-            uint64_t wv[kTileWarpRows][4];
-#pragma unroll
-            for (int r = 0; r < kTileWarpRows; ++r) {
-                const float4 v = wb[r * (kTileStage / 4) + ii * 32 + lane];
-                wv[r][0] = pack2(v.x, v.x); wv[r][1] = pack2(v.y, v.y); wv[r][2] = pack2(v.z, v.z); wv[r][3] = pack2(v.w, v.w);
-            }
-#pragma unroll
-            for (int t = 0; t < kTileWarpTokens / 2; ++t) {
-                float x[2][4];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const uint2 q = xb[(2 * t + u) * (kTileStage / 4) + ii * 32 + lane];
-                    if (FP16) {
-                        x[u][0] = f16_bits_to_f32(q.x & 0xffff); x[u][1] = f16_bits_to_f32(q.x >> 16);
-                        x[u][2] = f16_bits_to_f32(q.y & 0xffff); x[u][3] = f16_bits_to_f32(q.y >> 16);
-                    } else {
-                        x[u][0] = __uint_as_float(q.x << 16); x[u][1] = __uint_as_float(q.x & 0xffff0000u);
-                        x[u][2] = __uint_as_float(q.y << 16); x[u][3] = __uint_as_float(q.y & 0xffff0000u);
-                    }
-                }
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const uint64_t xv = pack2(x[0][c], x[1][c]);
-#pragma unroll
-                    for (int r = 0; r < kTileWarpRows; ++r)
-                        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[r][t]) : "l"(wv[r][c]), "l"(xv));
-                }
-            }
-        }
-    }
-
-    float sums[kTileWarpTokens * kTileWarpRows];
-#pragma unroll
-    for (int t = 0; t < kTileWarpTokens / 2; ++t)
-#pragma unroll
-        for (int r = 0; r < kTileWarpRows; ++r)
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(sums[2 * t * kTileWarpRows + r]), "=f"(sums[(2 * t + 1) * kTileWarpRows + r]) : "l"(acc[r][t]));
-    store_tile(a, sums, e0 + rg * kTileWarpRows, t0 + tg * kTileWarpTokens, lane);
-}
-
-// The shared expert's scalar gate for many rows (the tiled router covers the expert rows only): one
-// warp per row of activations at a time, the gate row held in registers, the same lane order, fused
-// multiply-adds and butterfly as everywhere else. A warp's rows follow one another at an L2 round trip each: a row per
-// warp while the blocks fit the SMs once (333 rows: 8.3 -> 3.5 us), four beyond, where fetching the gate row again costs
-// more (4096 rows: 9 us against 11).
-__global__ void __launch_bounds__(256) router_gate_rows_kernel(const RouterArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t chunks = a.d / 4;
-    const size_t esz = a.dt == SHRIKE_DTYPE_FP32 ? 4 : 2;
-    float4 wr[kRouterMaxChunks];
-    load_row_f32<kRouterMaxChunks, true>(a.gate_row, chunks, lane, wr);
-    for (uint32_t tk = blockIdx.x * 8 + warp; tk < a.T; tk += gridDim.x * 8) {
-        const void* xrow = (const uint8_t*)a.hidden + (size_t)tk * a.stride * esz;
-        const float acc = butterfly_sum(lane_dot_f32<kRouterMaxChunks, true>(wr, chunks, lane, xrow, a.dt, nullptr));
-        if (lane == 0) a.gate_out[tk] = sigmoid_det(acc);
-    }
-}
-
 __global__ void __launch_bounds__(128) router_select_kernel(const RouterArgs a) {
     __shared__ RowScratch rs[4];
     pdl_wait();
@@ -600,40 +299,11 @@ cudaError_t launch_router(const shrike_moe* m, cudaStream_t st, const shrike_rou
     RouterArgs a = make_router_args(m, ops, hidden, T, stride, ids, weights, shared_gate);
     const uint32_t rows = a.ne + (a.gate_row ? 1u : 0u);
     cudaError_t e;
-    if (T > 256 && a.bits == 0 && a.d % 8 == 0 && stride % 8 == 0 && ((uintptr_t)hidden & 15u) == 0 &&
-        ((uintptr_t)a.w & 15u) == 0) {
-        // tiled logits for the expert rows; the warp-per-row kernel keeps the gate row
-        static bool attr_set[64] = {};
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (dev < 64 && !attr_set[dev]) {
-            e = cudaFuncSetAttribute(router_logits_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kTileSmemBytes);
-            if (e != cudaSuccess) return e;
-            attr_set[dev] = true;
-        }
-        const dim3 grid((a.ne + kTileRows - 1) / kTileRows, (T + kTileTokens - 1) / kTileTokens);
-        if (a.dt != SHRIKE_DTYPE_FP32 && !a.eff_scale) {
-            static bool attr16_set[64] = {};
-            if (dev < 64 && !attr16_set[dev]) {
-                e = cudaFuncSetAttribute(router_logits_tiled16_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kTile16SmemBytes);
-                if (e == cudaSuccess)
-                    e = cudaFuncSetAttribute(router_logits_tiled16_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)kTile16SmemBytes);
-                if (e != cudaSuccess) return e;
-                attr16_set[dev] = true;
-            }
-            e = launch_after(m, st, a.dt == SHRIKE_DTYPE_FP16 ? router_logits_tiled16_kernel<true> : router_logits_tiled16_kernel<false>, grid, 256,
-                             kTile16SmemBytes, a);
-        } else {
-            e = launch_after(m, st, router_logits_tiled_kernel, grid, 256, kTileSmemBytes, a);
-        }
+    // A warp per row re-reads the activations for every expert row: ahead up to eight rows (the logits of 256 experts of 2048 columns, us:
+    // 4 rows 2.8 against the tiles' 5.4, 8 rows 4.5 / 5.4, 16 rows 5.8 / 5.2, 64 rows 19 / 5.4; int8 rows 5.0 / 9.0, 9.0 / 9.0, 16 / 9, 60 / 9).
+    if (T > 8 && router_tiles_take(a)) {
+        e = launch_router_tiles(m, st, a);
         if (e != cudaSuccess) return e;
-        if (a.gate_row) {
-            e = launch_after(m, st, router_gate_rows_kernel, dim3(T <= 8u * (uint32_t)m->sm_count ? (T + 7) / 8 : (T + 31) / 32), 256, 0, a);
-            if (e != cudaSuccess) return e;
-        }
     } else {
         uint32_t tpb = 1;
         if (T > 64) tpb = 32;
