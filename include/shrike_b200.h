@@ -365,6 +365,8 @@ int shrike_ep_encode_combine(shrike_moe* moe, void* stream, const void* recv_y, 
  *                      once per layer step. The call enqueues on `stream` and on the handle's own second
  *                      stream (joined before it returns control of `stream`'s order); it is not capturable
  *                      in a CUDA graph (the epoch of the arrival words is a host counter).
+ *                      A world of one has nobody to exchange with: `home` runs the call as its own layer call, on
+ *                      `stream` alone, unless its weight format is not the routed experts' or y lies across x.
  *                      A rank whose peer never arrives waits about a second per exchange, then the next
  *                      shrike_ep_status returns SHRIKE_ETIMEDOUT; the rows of that peer are missing from y.
  *   wait_polls         0 = the default limit (about one second); tests pass a small number. */

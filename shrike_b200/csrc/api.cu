@@ -1052,6 +1052,37 @@ int shrike_ep_set_wait_polls(shrike_ep* ep, uint32_t wait_polls) {
     return SHRIKE_OK;
 }
 
+// Whether a forward has nobody to exchange rows with and can be the home handle's own layer call, which knows the number of its rows
+// on the host, keeps them where they are and runs on one stream. What that call does not take goes the general way: formats of the
+// routed experts that the home handle does not describe, one row whose y is not 16-byte aligned, y across x. Through the exchange buffer,
+// in some twenty launches, and as the layer call, us: 256 experts of 2048 x 512 int4, 4 rows 119 / 36; 32 of 2880 x 2880 int4, 3 rows 164 / 76,
+// 144 rows 396 / 222; 256 of 2304 x 1024 int8, 39 rows 348 / 199, 2064 rows 697 / 630.
+static bool ep_alone(const shrike_ep* ep, uint32_t T, const void* x, const void* y, const void* hidden) {
+    const shrike_moe_config &c = ep->home->cfg, &r = ep->routed->cfg;
+    if (ep->world != 1 || T == 0 || r.weight_bits != c.weight_bits || r.group_size != c.group_size || r.meta_dtype != c.meta_dtype) return false;
+    if (T == 1 && (!aligned_to(y, 16) || !aligned_to(hidden, 16))) return false;
+    const uintptr_t x0 = (uintptr_t)x, y0 = (uintptr_t)y, elems = (uintptr_t)T * c.d;
+    return x0 == y0 || x0 + elems * act_bytes(c.act_dtype) <= y0 || y0 + elems * act_bytes(c.y_dtype) <= x0;
+}
+
+static int ep_forward_alone(shrike_ep* ep, void* stream, const shrike_pool* pool, const shrike_expert_offsets* routed_offsets,
+                            const uint64_t* residency_row, const shrike_router_operands* router, const shrike_shared_expert* shared,
+                            const void* x, uint32_t T, void* y, void* hidden) {
+    shrike_moe* m = ep->home;
+    int rc;
+    if (T <= SHRIKE_MAX_DECODE_TOKENS) {
+        rc = shrike_encode_decode_layer(m, stream, pool, routed_offsets, residency_row, router, shared, x, T, nullptr, ep->ids, ep->w, y, hidden);
+    } else {
+        float* gate = m->cfg.shared_gated ? ep->gate : nullptr;
+        rc = shrike_encode_router(m, stream, router, x, T, m->cfg.d, ep->ids, ep->w, gate);
+        if (!rc) rc = shrike_encode_residency_classification(m, stream, ep->ids, residency_row, T, ep->c_slots, nullptr, nullptr, nullptr);
+        if (!rc) rc = encode_prefill(m, stream, pool, routed_offsets, ep->ids, ep->c_slots, ep->w, x, T, shared, gate, nullptr, y, hidden);
+    }
+    if (rc) return rc;
+    CU(launch_ep_alone_counts(m, (cudaStream_t)stream, T, ep->send_counts, ep->prefix, ep->n_rows));
+    return SHRIKE_OK;
+}
+
 int shrike_ep_forward(shrike_ep* ep, void* stream, const shrike_pool* local_pool,
                       const shrike_expert_offsets* routed_offsets, const uint64_t* local_residency_row,
                       const shrike_router_operands* router, const shrike_shared_expert* shared, const void* x,
@@ -1067,6 +1098,8 @@ int shrike_ep_forward(shrike_ep* ep, void* stream, const shrike_pool* local_pool
     cudaStream_t st = (cudaStream_t)stream;
     int rc;
     if ((rc = check_device(m))) return rc;
+    if (ep_alone(ep, query_count, x, y, hidden))
+        return ep_forward_alone(ep, stream, local_pool, routed_offsets, local_residency_row, router, shared, x, query_count, y, hidden);
     // the call's two streams run beside each other; outside of it the handles launch as any other
     struct Beside {
         shrike_moe *a, *b;

@@ -244,6 +244,8 @@ cudaError_t launch_ep_return(const shrike_moe* routed, cudaStream_t st, const ui
                              const EpLayout& lay, uint32_t epoch);
 cudaError_t launch_ep_wait_returns(const shrike_moe* home, cudaStream_t st, const uint8_t* mine, const EpLayout& lay,
                                    uint32_t world, uint32_t cap, uint32_t epoch, uint32_t max_polls);
+cudaError_t launch_ep_alone_counts(const shrike_moe* m, cudaStream_t st, uint32_t rows, uint32_t* send_counts, uint32_t* prefix,
+                                   uint32_t* n_rows);
 cudaError_t launch_ep_dispatch(const shrike_moe* m, cudaStream_t st, const void* x, const uint32_t* ids,
                                const float* weights, uint32_t T, uint32_t world, uint32_t experts_per_rank,
                                uint32_t cap, void* send_x, uint32_t* send_ids, float* send_w,

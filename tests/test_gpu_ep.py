@@ -519,3 +519,70 @@ def test_combine_matches_the_protocol(cuda_device, T, world, skip):
         assert np.array_equal(want, R.combine(recv, row_of, home))
     assert (y.cpu().numpy() == want).all() and (h.cpu().numpy() == x + want).all()
     moe.close()
+
+
+@pytest.mark.parametrize("T", [1, 2, 64, 65, 200])
+@pytest.mark.parametrize("shared", [True, False])
+def test_a_rank_alone_gives_what_the_exchange_gives(cuda_device, T, shared):
+    """A world of one runs the home handle's layer call; rows whose y begins inside x take the general way through the exchange
+    buffer. Both against the oracle, the residual and the counters."""
+    from shrike_b200.moe import RouterOperands
+    seed = 31
+    cfg = dataclasses.replace(_config(), **({} if shared else dict(has_shared=False, shared_f=0)))
+    x, router = _problem(T, cfg)
+    ids, w, y_ref = _oracle(_config(), x, router, seed)
+    if not shared:
+        import fixtures as fx
+        import oracle_lib as O
+        ecfg = O.expert_cfg(cfg.d, cfg.f)
+        y_ref = O.moe_layer(O.layer_cfg(ecfg, None, False), {int(e): fx.synth_block(cfg, seed, 0, int(e)) for e in np.unique(ids)}, None, None,
+                            x, ids, w)
+    layer = _build_alone(cfg, T, seed)
+    ops = RouterOperands(weights=torch.from_numpy(router).to(layer.dev))
+    for across in (False, True):
+        buf = torch.zeros((2 * T + 1, cfg.d), device=layer.dev)
+        xd, y = buf[:T], buf[1:T + 1] if across else buf[T:2 * T]
+        xd.copy_(torch.from_numpy(x))
+        h = torch.from_numpy(x).to(layer.dev)
+        layer.forward(ops, xd, y, h)
+        layer.status()
+        got = y.cpu().numpy()
+        assert np.linalg.norm(got - y_ref) / np.linalg.norm(y_ref) <= 1e-3
+        assert np.abs(h.cpu().numpy() - (x + got)).max() <= 1e-5 * np.abs(x).max()
+        assert layer.last_counts() == ([T], T, 0)
+    layer.close()
+
+
+def _build_alone(cfg, T, seed):
+    import fixtures as fx
+    from shrike_b200.ep import ExpertParallelLayer
+    if cfg.has_shared:
+        return _build_layer(cfg, 0, 1, T, seed, "peer")
+    layer = ExpertParallelLayer(cfg, 0, 1, 0, T)
+    for e in range(layer.lo, layer.hi):
+        layer.pool.upload(e, fx.synth_block(cfg, seed, 0, e))
+    return layer
+
+
+def test_a_replayed_forward_counts_its_own_rows(cuda_device):
+    from shrike_b200.moe import RouterOperands
+    cfg = _config()
+    x, router = _problem(8, cfg)
+    layer = _build_layer(cfg, 0, 1, 8, 32, "peer")
+    ops = RouterOperands(weights=torch.from_numpy(router).to(layer.dev))
+    xd = torch.from_numpy(x).to(layer.dev)
+    y, y4 = torch.zeros_like(xd), torch.zeros_like(xd[:4])
+    layer.forward(ops, xd, y)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        layer.forward(ops, xd, y)
+    want = y.clone()
+    layer.forward(ops, xd[:4], y4)
+    torch.cuda.synchronize()
+    assert layer.last_counts()[:2] == ([4], 4)
+    y.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert layer.last_counts()[:2] == ([8], 8) and torch.equal(y, want)
+    layer.close()
