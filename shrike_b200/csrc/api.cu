@@ -239,7 +239,7 @@ int encode_prefill(shrike_moe* m, void* stream, const shrike_pool* pool,
         CU(launch_phase1(m, st, a, mi, false));
         CU(launch_phase2_accumulate(m, st, a, mi));
     } else {
-        CU(launch_umma_prefill(m, st, a, query_count, pool->view.cells));
+        CU(launch_umma_prefill(m, st, a, query_count));
     }
     if (!direct) CU(launch_prefill_combine(m, st, query_count, y, hidden));
     return SHRIKE_OK;
@@ -327,6 +327,7 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
     A(&w.done_counter, 4);
     A(&w.arrived, 8);
     A(&w.fused_epoch, 4);
+    A(&w.plan_ticket, 4);
     const size_t zeroed = small_bytes;
     A(&w.logits, T * c.num_experts * 4);
     A(&w.xh, T * c.d * 2);
@@ -345,7 +346,7 @@ int shrike_moe_create(const shrike_moe_config* config, int device, shrike_moe** 
     A(&w.yacc, T > SHRIKE_MAX_DECODE_TOKENS ? T * c.d * 4 : 0);
     A(&w.chunk_inst, T > SHRIKE_MAX_DECODE_TOKENS ? umma_max_chunk_instances(c, c.max_tokens) * umma_chunk_instance_bytes() : 0);
     A(&w.n_chunk_inst, 16);
-    if (T > SHRIKE_MAX_DECODE_TOKENS) A(&w.pos_of_pair, T * K * 4);
+    if (T > SHRIKE_MAX_DECODE_TOKENS) A(&w.rank_of_pair, T * K * 4);
     if (T > SHRIKE_MAX_DECODE_TOKENS) A(&w.xs, T * K * c.d * 2);   // prefill operands
     A(&w.x_dev, T * c.d * ab);
     A(&w.y_dev, T * c.d * yb);
@@ -1143,7 +1144,7 @@ int shrike_ep_forward(shrike_ep* ep, void* stream, const shrike_pool* local_pool
             CU(launch_phase1(r, st, a, mi, false));
             CU(launch_phase2_accumulate(r, st, a, mi));
         } else {
-            CU(launch_umma_prefill(r, st, a, ep->t_max, local_pool->view.cells));
+            CU(launch_umma_prefill(r, st, a, ep->t_max));
         }
     }
     CU(launch_ep_return(r, st, ep->row_map, ep->n_rows, ep->t_max, ep->world, ep->rank, ep->cap, ep->peer, ep->lay, epoch));

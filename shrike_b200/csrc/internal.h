@@ -16,6 +16,13 @@ struct Instance {
     uint32_t pair[8];  // routed: row*top_k + rank of each of the `count` rows; shared: the row
 };
 
+constexpr uint32_t kChunkRows = 256;   // rows of the expert-grouped GEMM's instances
+struct alignas(16) ChunkInstance {     // up to that many rows that share one expert block
+    uint32_t kind, slot, first, count;
+};
+
+constexpr uint32_t kGroupTokens = 128;  // rows of a block of the prefill grouping
+
 // PoolBases (moe.metal:297-300) by value as a kernel argument.
 struct PoolView {
     const uint8_t* base[SHRIKE_MAX_POOL_CHUNKS];
@@ -94,7 +101,8 @@ struct Workspace {
     float* yacc = nullptr;          // prefill: fp32 output accumulator [max_tokens x d]
     void* chunk_inst = nullptr;     // prefill: instances of up to 256 rows (tensor-core path)
     uint32_t* n_chunk_inst = nullptr; // [0] instances, [1], [2] tiles handed out per phase
-    uint32_t* pos_of_pair = nullptr; // prefill: place of every pair in the expert-sorted order, or 0xffffffff
+    uint32_t* rank_of_pair = nullptr; // prefill: earlier rows of the pair's block of rows with its expert, or 0xffffffff: no row is needed
+    uint32_t* plan_ticket = nullptr; // blocks finished, prefill plan
     uint16_t* xs = nullptr;         // prefill: fp16 activation rows in expert-sorted order [max_tokens x top_k x d]
     void* tensor_maps = nullptr;    // host: the TMA descriptors of xs, acts, xh, acts_shared and of the last prefill's pool and shared block
     // one-row decode layer in one launch (fused_layer.cu)
@@ -177,8 +185,9 @@ cudaError_t launch_decode_plan(const shrike_moe* m, cudaStream_t st, const uint3
                                bool with_shared, uint32_t pool_cells);
 cudaError_t launch_group_pairs(const shrike_moe* m, cudaStream_t st, const uint32_t* ids,
                                const float* weights, uint32_t T, uint32_t* sorted_pairs,
-                               uint32_t* offsets, uint32_t* counts, const uint32_t* slots = nullptr,
-                               const uint32_t* io_status = nullptr);
+                               uint32_t* offsets, uint32_t* counts);
+cudaError_t launch_group_plan(const shrike_moe* m, cudaStream_t st, const uint32_t* ids, uint32_t T, const uint32_t* slots,
+                              const uint32_t* io_status, bool with_shared, uint32_t pool_cells);
 // decode.cu
 cudaError_t launch_phase1(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a,
                           uint32_t max_inst, bool pdl);
@@ -281,6 +290,5 @@ size_t umma_chunk_instance_bytes();
 size_t umma_tensor_map_bytes();
 cudaError_t umma_prepare(shrike_moe* m);
 bool umma_supported(const shrike_moe_config& c);
-cudaError_t launch_umma_prefill(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, uint32_t T,
-                                uint32_t pool_cells);
+cudaError_t launch_umma_prefill(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, uint32_t T);
 }  // namespace shrike

@@ -86,34 +86,24 @@ cudaError_t launch_decode_plan(const shrike_moe* m, cudaStream_t st, const uint3
 
 // ---- prefill grouping -------------------------------------------------------
 
-constexpr uint32_t kGroupTokens = 128;  // rows per block
+using GroupBits = uint32_t[SHRIKE_MAX_EXPERTS][kGroupTokens / 32];
 
-// Step 1: per block, a bitmap of the rows that chose each expert; writes the
-// per-(block, expert) counts and, given the pairs' cells, the cell of every expert that has a pair (a streamed batch
-// whose status word is not READY, moe_io_ready, moe.metal:36-39, leaves every expert without one).
+// Step 1: per block, a bitmap of the rows that chose each expert; writes the per-(block, expert) counts.
 __global__ void __launch_bounds__(256)
 group_hist_kernel(const uint32_t* __restrict__ ids, uint32_t T, uint32_t top_k, uint32_t ne,
-                  uint32_t* __restrict__ block_hist, uint32_t* status, const uint32_t* __restrict__ slots,
-                  const uint32_t* __restrict__ io_status, uint32_t* __restrict__ slot_of_expert) {
+                  uint32_t* __restrict__ block_hist, uint32_t* status) {
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ uint32_t bits[SHRIKE_MAX_EXPERTS][kGroupTokens / 32];
+    __shared__ GroupBits bits;
     const uint32_t t0 = blockIdx.x * kGroupTokens;
     for (uint32_t i = threadIdx.x; i < SHRIKE_MAX_EXPERTS * (kGroupTokens / 32); i += blockDim.x)
         (&bits[0][0])[i] = 0;
-    bool ready = true;
-    if (io_status) {
-        const uint32_t s = *io_status;
-        ready = s == 1u || s == 3u;
-    }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < kGroupTokens * top_k; i += blockDim.x) {
         const uint32_t tl = i / top_k, t = t0 + tl;
         if (t < T) {
-            const size_t p = (size_t)t * top_k + (i - tl * top_k);
-            const uint32_t e = ids[p];
+            const uint32_t e = ids[(size_t)t * top_k + (i - tl * top_k)];
             if (e < ne) {
-                if (slots) slot_of_expert[e] = ready ? slots[p] : SHRIKE_SLOT_MISS;
                 // a row that names one expert twice (no top-k router does) is counted once and reported
                 const uint32_t bit = 1u << (tl & 31);
                 if (atomicOr(&bits[e][tl >> 5], bit) & bit) report_status(status, kStatusBadIndex);
@@ -133,30 +123,57 @@ group_hist_kernel(const uint32_t* __restrict__ ids, uint32_t T, uint32_t top_k, 
     }
 }
 
+// Rows before row tl of the block that chose expert e.
+__device__ __forceinline__ uint32_t rows_before(const GroupBits& bits, uint32_t e, uint32_t tl) {
+    uint32_t before = 0;
+    const uint32_t word = tl >> 5;
+    for (uint32_t w = 0; w < word; ++w) before += __popc(bits[e][w]);
+    return before + __popc(bits[e][word] & ((1u << (tl & 31)) - 1u));
+}
+
 // Step 2 (one block): per-expert totals, exclusive scan over experts, and the
 // running base of every (block, expert) cell.
-__global__ void __launch_bounds__(256)
-group_scan_kernel(uint32_t* __restrict__ block_hist, uint32_t n_blocks, uint32_t ne,
-                  uint32_t* __restrict__ offsets, uint32_t* __restrict__ counts) {
-    pdl_wait();
-    pdl_launch_dependents();
-    __shared__ uint32_t warp_sums[8];
+__device__ __forceinline__ void group_scan(uint32_t* warp_sums, uint32_t* block_hist, uint32_t n_blocks, uint32_t ne,
+                                           uint32_t* __restrict__ offsets, uint32_t* __restrict__ counts, uint32_t& total, uint32_t& base) {
     const uint32_t e = threadIdx.x;
-    uint32_t total = 0;
-    if (e < ne)
-        for (uint32_t b = 0; b < n_blocks; ++b) total += block_hist[(size_t)b * ne + e];
+    constexpr uint32_t kKept = 8;   // blocks' counts that a second look does not ask L2 for again
+    uint32_t kept[kKept];
+    total = 0;
+#pragma unroll
+    for (uint32_t b = 0; b < kKept; ++b) kept[b] = b < n_blocks && e < ne ? __ldcg(block_hist + (size_t)b * ne + e) : 0u;
+#pragma unroll
+    for (uint32_t b = 0; b < kKept; ++b) total += kept[b];
+    if (e < ne) {
+#pragma unroll 8
+        for (uint32_t b = kKept; b < n_blocks; ++b) total += __ldcg(block_hist + (size_t)b * ne + e);
+    }
     uint32_t all;
-    const uint32_t base = block_exclusive_scan(e < ne ? total : 0u, warp_sums, all);
+    base = block_exclusive_scan(total, warp_sums, all);
     if (e < ne) {
         counts[e] = total;
         offsets[e] = total ? base : 0xffffffffu;
         uint32_t run = base;
-        for (uint32_t b = 0; b < n_blocks; ++b) {
-            const uint32_t c = block_hist[(size_t)b * ne + e];
+#pragma unroll
+        for (uint32_t b = 0; b < kKept; ++b) {
+            if (b < n_blocks) block_hist[(size_t)b * ne + e] = run;
+            run += kept[b];
+        }
+#pragma unroll 8
+        for (uint32_t b = kKept; b < n_blocks; ++b) {
+            const uint32_t c = __ldcg(block_hist + (size_t)b * ne + e);
             block_hist[(size_t)b * ne + e] = run;
             run += c;
         }
     }
+}
+__global__ void __launch_bounds__(256)
+group_scan_kernel(uint32_t* block_hist, uint32_t n_blocks, uint32_t ne,
+                  uint32_t* __restrict__ offsets, uint32_t* __restrict__ counts) {
+    pdl_wait();
+    pdl_launch_dependents();
+    __shared__ uint32_t warp_sums[8];
+    uint32_t total, base;
+    group_scan(warp_sums, block_hist, n_blocks, ne, offsets, counts, total, base);
 }
 
 // Step 3: place every pair at base(block, expert) + number of earlier rows of
@@ -164,8 +181,7 @@ group_scan_kernel(uint32_t* __restrict__ block_hist, uint32_t n_blocks, uint32_t
 __global__ void __launch_bounds__(256)
 group_place_kernel(const uint32_t* __restrict__ ids, const float* __restrict__ weights, uint32_t T,
                    uint32_t top_k, uint32_t ne, const uint32_t* __restrict__ block_base,
-                   uint32_t* __restrict__ sorted_pairs, uint32_t* __restrict__ sorted_ids,
-                   const uint32_t* __restrict__ slots, uint32_t* __restrict__ pos_of_pair) {
+                   uint32_t* __restrict__ sorted_pairs) {
     pdl_wait();
     pdl_launch_dependents();
     __shared__ uint32_t bits[SHRIKE_MAX_EXPERTS][kGroupTokens / 32];
@@ -185,31 +201,128 @@ group_place_kernel(const uint32_t* __restrict__ ids, const float* __restrict__ w
         const uint32_t tl = i / top_k, t = t0 + tl, r = i - tl * top_k;
         if (t >= T) continue;
         const uint32_t e = ids[(size_t)t * top_k + r];
-        if (e >= ne) {
-            if (pos_of_pair) pos_of_pair[(size_t)t * top_k + r] = 0xffffffffu;
-            continue;
-        }
-        uint32_t before = 0;
-        const uint32_t word = tl >> 5;
-        for (uint32_t w = 0; w < word; ++w) before += __popc(bits[e][w]);
-        before += __popc(bits[e][word] & ((1u << (tl & 31)) - 1u));
-        const uint32_t pos = block_base[(size_t)blockIdx.x * ne + e] + before;
-        if (sorted_pairs) {
-            uint4 p;
-            p.x = t; p.y = e; p.z = r;
-            // weight bits as the reference stores them: fp16 in the low half
-            p.w = weights ? (uint32_t)__half_as_ushort(__float2half_rn(weights[(size_t)t * top_k + r])) : 0u;
-            ((uint4*)sorted_pairs)[pos] = p;
-        }
-        if (sorted_ids) sorted_ids[pos] = t * top_k + r;
-        // (no row is needed where the expert has no cell)
-        if (pos_of_pair) pos_of_pair[(size_t)t * top_k + r] = slots[(size_t)t * top_k + r] == SHRIKE_SLOT_MISS ? 0xffffffffu : pos;
+        if (e >= ne) continue;
+        const uint32_t pos = block_base[(size_t)blockIdx.x * ne + e] + rows_before(bits, e, tl);
+        uint4 p;
+        p.x = t; p.y = e; p.z = r;
+        // weight bits as the reference stores them: fp16 in the low half
+        p.w = weights ? (uint32_t)__half_as_ushort(__float2half_rn(weights[(size_t)t * top_k + r])) : 0u;
+        ((uint4*)sorted_pairs)[pos] = p;
     }
+}
+
+// The list of instances: all full ones (256 rows; the shared expert's first), then every expert's rest, most rows first. A tile of
+// 256 rows takes twice the time of one of 16, and a list that ends on long ones leaves SMs idle. All tiles of more than 128 rows come before the
+// others, so a block changes the layout of its shared memory once at most. Thread e has expert e's `c` rows, which begin at `first`
+// in the sorted order; n_inst[0] = instances, [1], [2]: tiles handed out in phase 0, 1.
+__device__ __forceinline__ void chunk_instances(uint32_t* warp_sums, uint32_t (&key)[256], uint32_t c, uint32_t first, uint32_t slot, uint32_t T,
+                                                uint32_t with_shared, ChunkInstance* __restrict__ inst, uint32_t* __restrict__ n_inst) {
+    const uint32_t e = threadIdx.x, n = c / kChunkRows, rest = c % kChunkRows, mine = rest << 8 | (255u - e);
+    const uint32_t shared_rest = with_shared ? T % kChunkRows : 0u, n_shared = with_shared ? T / kChunkRows : 0u;
+    key[e] = mine;
+    uint32_t total;
+    uint32_t base = block_exclusive_scan(n, warp_sums, total);
+    const uint32_t before_shared = (uint32_t)__syncthreads_count(rest > shared_rest);   // rests that come before the shared expert's
+    const uint32_t n_rest = (uint32_t)__syncthreads_count(rest != 0) + (shared_rest != 0);
+    base += n_shared;
+    total += n_shared;
+    auto put = [&](uint32_t at, uint32_t kind, uint32_t cell, uint32_t from, uint32_t count) {
+        *(uint4*)(inst + at) = make_uint4(kind, cell, from, count);
+    };
+    for (uint32_t j = 0; j < n; ++j) put(base + j, 0, slot, first + kChunkRows * j, kChunkRows);
+    if (rest) {
+        uint32_t rank = rest <= shared_rest ? 1u : 0u;
+        for (uint32_t j = 0; j < 256; j += 4) {
+            const uint4 v = *(const uint4*)&key[j];
+            rank += (v.x > mine) + (v.y > mine) + (v.z > mine) + (v.w > mine);
+        }
+        put(total + rank, 0, slot, first + kChunkRows * n, rest);
+    }
+    for (uint32_t j = e; j < n_shared; j += blockDim.x) put(j, 1, 0, kChunkRows * j, kChunkRows);
+    if (e == 0) {
+        if (shared_rest) put(total + before_shared, 1, 0, kChunkRows * n_shared, shared_rest);
+        n_inst[0] = total + n_rest;
+        n_inst[1] = n_inst[2] = 0;   // tiles handed out, per phase
+    }
+}
+
+// The prefill plan in one launch: step 1, and every pair's rows before it in its block of rows; the block that finishes last
+// takes step 2 and lists the instances. The pairs' places follow from the two where the rows are converted. Bound by a chain of trips
+// to L2 (ids, counts, ticket, counts again, list). Counting, scan, places and list as launches of their own, and this: a call of 70 rows
+// 155.9 -> 150.1 us, 333 rows 181.5 -> 177.6, 1134 rows 247.9 -> 243.2.
+__global__ void __launch_bounds__(256)
+group_plan_kernel(const uint32_t* __restrict__ ids, uint32_t T, uint32_t top_k, uint32_t ne, uint32_t* block_hist, uint32_t* status,
+                  const uint32_t* __restrict__ slots, const uint32_t* __restrict__ io_status, uint32_t* slot_of_expert,
+                  uint32_t* __restrict__ rank_of_pair, uint32_t* __restrict__ offsets, uint32_t* __restrict__ counts, uint32_t* ticket,
+                  uint32_t with_shared, uint32_t pool_cells, ChunkInstance* __restrict__ inst, uint32_t* __restrict__ n_inst) {
+    pdl_wait();
+    pdl_launch_dependents();
+    __shared__ GroupBits bits;
+    __shared__ uint32_t warp_sums[8], s_last;
+    __shared__ __align__(16) uint32_t key[256];
+    // a thread's pairs, asked for at once and kept
+    constexpr uint32_t N = kGroupTokens * SHRIKE_MAX_TOP_K / 256;
+    const uint32_t t0 = blockIdx.x * kGroupTokens, n = min(T - t0, kGroupTokens) * top_k, io = io_status ? *io_status : 1u;
+    const bool ready = io == 1u || io == 3u;
+    uint32_t e[N], cell[N];
+#pragma unroll
+    for (uint32_t j = 0; j < N; ++j) {
+        const uint32_t i = j * 256 + threadIdx.x;
+        e[j] = i < n ? ids[(size_t)t0 * top_k + i] : 0xffffffffu;
+        cell[j] = i < n ? slots[(size_t)t0 * top_k + i] : SHRIKE_SLOT_MISS;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < sizeof(GroupBits) / 4 / 256; ++j) (&bits[0][0])[j * 256 + threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll
+    for (uint32_t j = 0; j < N; ++j) {
+        const uint32_t tl = (j * 256 + threadIdx.x) / top_k, bit = 1u << (tl & 31);
+        if (e[j] < ne) {
+            slot_of_expert[e[j]] = ready ? cell[j] : SHRIKE_SLOT_MISS;
+            // a row that names one expert twice (no top-k router does) is counted once and reported
+            if (atomicOr(&bits[e[j]][tl >> 5], bit) & bit) report_status(status, kStatusBadIndex);
+        } else if (e[j] != 0xffffffffu) {
+            report_status(status, kStatusBadIndex);   // out of range: dropped (0xffffffff: the pick lives on another rank)
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < ne) {
+        uint32_t c = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kGroupTokens / 32; ++w) c += __popc(bits[threadIdx.x][w]);
+        block_hist[(size_t)blockIdx.x * ne + threadIdx.x] = c;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < N; ++j) {
+        const uint32_t i = j * 256 + threadIdx.x;
+        // (no row is needed where the expert has no cell)
+        if (i < n) rank_of_pair[(size_t)t0 * top_k + i] = e[j] >= ne || cell[j] == SHRIKE_SLOT_MISS ? 0xffffffffu : rows_before(bits, e[j], i / top_k);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
+        if (s_last) *ticket = 0;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    uint32_t total, base;
+    group_scan(warp_sums, block_hist, gridDim.x, ne, offsets, counts, total, base);
+    uint32_t slot = SHRIKE_SLOT_MISS;
+    if (threadIdx.x < ne && total) {
+        slot = __ldcg(slot_of_expert + threadIdx.x);
+        if (slot != SHRIKE_SLOT_MISS && slot >= pool_cells) {
+            report_status(status, kStatusBadIndex);
+            slot = SHRIKE_SLOT_MISS;
+        }
+    }
+    chunk_instances(warp_sums, key, slot == SHRIKE_SLOT_MISS ? 0u : total, base, slot, T, with_shared, inst, n_inst);
 }
 
 cudaError_t launch_group_pairs(const shrike_moe* m, cudaStream_t st, const uint32_t* ids,
                                const float* weights, uint32_t T, uint32_t* sorted_pairs,
-                               uint32_t* offsets, uint32_t* counts, const uint32_t* slots, const uint32_t* io_status) {
+                               uint32_t* offsets, uint32_t* counts) {
     const uint32_t nb = (T + kGroupTokens - 1) / kGroupTokens;
     const uint32_t ne = m->cfg.num_experts, k = m->cfg.top_k;
     if (nb == 0) {
@@ -217,13 +330,19 @@ cudaError_t launch_group_pairs(const shrike_moe* m, cudaStream_t st, const uint3
         if (e != cudaSuccess) return e;
         return cudaMemsetAsync(offsets, 0xff, ne * 4, st);
     }
-    cudaError_t eh = launch_after(m, st, group_hist_kernel, dim3(nb), 256, 0, ids, T, k, ne, m->ws.block_hist, m->ws.status, slots, io_status,
-                                          m->ws.slot_of_expert);
-    if (eh != cudaSuccess) return eh;
-    cudaError_t e = launch_after(m, st, group_scan_kernel, dim3(1), 256, 0, m->ws.block_hist, nb, ne, offsets, counts);
+    cudaError_t e = launch_after(m, st, group_hist_kernel, dim3(nb), 256, 0, ids, T, k, ne, m->ws.block_hist, m->ws.status);
     if (e != cudaSuccess) return e;
-    return launch_after(m, st, group_place_kernel, dim3(nb), 256, 0, ids, weights, T, k, ne, m->ws.block_hist, sorted_pairs,
-                        m->ws.sorted, slots, slots ? m->ws.pos_of_pair : nullptr);
+    e = launch_after(m, st, group_scan_kernel, dim3(1), 256, 0, m->ws.block_hist, nb, ne, offsets, counts);
+    if (e != cudaSuccess) return e;
+    return launch_after(m, st, group_place_kernel, dim3(nb), 256, 0, ids, weights, T, k, ne, m->ws.block_hist, sorted_pairs);
+}
+
+cudaError_t launch_group_plan(const shrike_moe* m, cudaStream_t st, const uint32_t* ids, uint32_t T, const uint32_t* slots,
+                              const uint32_t* io_status, bool with_shared, uint32_t pool_cells) {
+    const Workspace& ws = m->ws;
+    return launch_after(m, st, group_plan_kernel, dim3((T + kGroupTokens - 1) / kGroupTokens), 256, 0, ids, T, m->cfg.top_k, m->cfg.num_experts,
+                        ws.block_hist, ws.status, slots, io_status, ws.slot_of_expert, ws.rank_of_pair, ws.expert_offsets, ws.expert_counts,
+                        ws.plan_ticket, with_shared ? 1u : 0u, pool_cells, (ChunkInstance*)ws.chunk_inst, ws.n_chunk_inst);
 }
 
 }  // namespace shrike

@@ -61,23 +61,42 @@ prefill_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* _
     if (threadIdx.x == 0) *n_inst = total + n_shared;
 }
 
-// x -> fp16 operand layout and per-group sums, all rows; given the pairs' places, also into the expert-sorted rows that the
-// grouped GEMM copies its tiles from. (Bound by the sorted rows' bytes, top_k times x's: as a kernel of its own that read
+// x -> fp16 operand layout and per-group sums, all rows; the pairs in expert-sorted order; given `xs`, the rows in that order too, which
+// the grouped GEMM copies its tiles from. (Bound by the sorted rows' bytes, top_k times x's: as a kernel of its own that read
 // them back, the gather took 28 us of a 4096-row call beside 11 here.)
 __global__ void __launch_bounds__(256)
 prefill_xprep_kernel(const void* __restrict__ x, uint32_t T, uint32_t d, uint32_t group, uint32_t act_dtype,
                      uint32_t int4, uint16_t* __restrict__ xh, float* __restrict__ xsum, uint32_t* status,
                      const uint32_t* __restrict__ row_map, const uint32_t* __restrict__ n_rows_dev,
-                     const uint32_t* __restrict__ pos_of_pair, uint32_t top_k, uint16_t* __restrict__ xs, float* __restrict__ zero) {
+                     const uint32_t* __restrict__ ids, const uint32_t* __restrict__ rank_of_pair,
+                     const uint32_t* __restrict__ block_base, uint32_t ne, uint32_t top_k, uint32_t* __restrict__ sorted,
+                     uint16_t* __restrict__ xs, float* __restrict__ zero) {
     pdl_wait();
     pdl_launch_dependents();
     const uint32_t items = T * (d / 8);
     const size_t row_bytes = (size_t)d * (act_dtype == SHRIKE_DTYPE_FP32 ? 4 : 2);
     const uint32_t n_rows = n_rows_dev ? *n_rows_dev : T;
     for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < items; i0 += gridDim.x * blockDim.x) {
-        const uint32_t i = i0 + threadIdx.x;
-        xprep_item(x, row_bytes, d, group, act_dtype, int4 != 0, i, i < items, xh, xsum, status, row_map, n_rows);
-        if (i < items) {   // the rows that the down projection adds into
+        const uint32_t i = i0 + threadIdx.x, row = i / (d / 8), col = (i - row * (d / 8)) * 8;
+        const bool there = i < items;
+        // the pairs' places: the first of their expert's rows in this block of rows, and those before them in the block (asked for
+        // ahead of the row itself: two trips to L2)
+        uint32_t pos[SHRIKE_MAX_TOP_K];
+#pragma unroll
+        for (uint32_t r = 0; r < SHRIKE_MAX_TOP_K; ++r) pos[r] = 0xffffffffu;
+        if (there && row < n_rows && (xs || col == 0)) {
+            uint32_t rank[SHRIKE_MAX_TOP_K], e[SHRIKE_MAX_TOP_K];
+#pragma unroll
+            for (uint32_t r = 0; r < SHRIKE_MAX_TOP_K; ++r) {
+                rank[r] = r < top_k ? rank_of_pair[row * top_k + r] : 0xffffffffu;
+                e[r] = r < top_k ? ids[row * top_k + r] : 0u;
+            }
+#pragma unroll
+            for (uint32_t r = 0; r < SHRIKE_MAX_TOP_K; ++r)
+                if (rank[r] != 0xffffffffu) pos[r] = block_base[(size_t)(row / kGroupTokens) * ne + e[r]] + rank[r];
+        }
+        xprep_item(x, row_bytes, d, group, act_dtype, int4 != 0, i, there, xh, xsum, status, row_map, n_rows);
+        if (there) {   // the rows that the down projection adds into
             float* const z = zero + (size_t)i * 8;
             if (((uintptr_t)zero & 15u) == 0) {
                 ((float4*)z)[0] = ((float4*)z)[1] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -86,14 +105,17 @@ prefill_xprep_kernel(const void* __restrict__ x, uint32_t T, uint32_t d, uint32_
                 for (int k = 0; k < 8; ++k) z[k] = 0.f;
             }
         }
-        const uint32_t row = i / (d / 8);
-        if (!pos_of_pair || i >= items || row >= n_rows) continue;
-        const uint4 v = *(const uint4*)(xh + (size_t)i * 8);   // this thread's own
-        const uint32_t col = (i - row * (d / 8)) * 8;
-        for (uint32_t r = 0; r < top_k; ++r) {
-            const uint32_t pos = pos_of_pair[(size_t)row * top_k + r];
-            if (pos != 0xffffffffu) *(uint4*)(xs + (size_t)pos * d + col) = v;
+        if (!there || row >= n_rows) continue;
+        if (col == 0) {
+#pragma unroll
+            for (uint32_t r = 0; r < SHRIKE_MAX_TOP_K; ++r)
+                if (pos[r] != 0xffffffffu) sorted[pos[r]] = row * top_k + r;
         }
+        if (!xs) continue;
+        const uint4 v = *(const uint4*)(xh + (size_t)i * 8);   // this thread's own
+#pragma unroll
+        for (uint32_t r = 0; r < SHRIKE_MAX_TOP_K; ++r)
+            if (pos[r] != 0xffffffffu) *(uint4*)(xs + (size_t)pos[r] * d + col) = v;
     }
 }
 
@@ -119,17 +141,20 @@ cudaError_t launch_prefill_plan(const shrike_moe* m, cudaStream_t st, const uint
                                 const uint32_t* row_map, const uint32_t* n_rows, float* accumulator) {
     const shrike_moe_config& c = m->cfg;
     const Workspace& ws = m->ws;
-    cudaError_t e = launch_group_pairs(m, st, ids, nullptr, T, nullptr, ws.expert_offsets, ws.expert_counts, slots, io_status);
+    cudaError_t e = launch_group_plan(m, st, ids, T, slots, io_status, with_shared, pool_cells);
     if (e != cudaSuccess) return e;
-    if (warp_mma_instances)   // the tensor-core path builds its own 256-row instances
+    const uint32_t items = T * (c.d / 8);
+    e = launch_after(m, st, prefill_xprep_kernel, dim3(min(2048u, (items + 255) / 256)), 256, 0, x, T, c.d, c.group_size, c.act_dtype,
+                     c.weight_bits == 4 ? 1u : 0u, ws.xh, ws.xsum, ws.status, row_map, n_rows, ids, ws.rank_of_pair, ws.block_hist,
+                     c.num_experts, c.top_k, ws.sorted, warp_mma_instances ? nullptr : ws.xs,
+                     accumulator ? accumulator : ws.yacc);   // the rows the down epilogue adds into: the workspace's, or the caller's fp32 output itself
+    if (e == cudaSuccess && warp_mma_instances) {   // the tensor-core path has its 256-row instances from the plan
         prefill_instances_kernel<<<1, 256, 0, st>>>(ws.expert_offsets, ws.expert_counts, ws.slot_of_expert,
                                                     c.num_experts, T, with_shared ? 1u : 0u, pool_cells, ws.sorted,
                                                     ws.inst, ws.n_inst, ws.status);
-    const uint32_t items = T * (c.d / 8);
-    return launch_after(m, st, prefill_xprep_kernel, dim3(min(2048u, (items + 255) / 256)), 256, 0, x, T, c.d, c.group_size, c.act_dtype,
-                        c.weight_bits == 4 ? 1u : 0u, ws.xh, ws.xsum, ws.status, row_map, n_rows,
-                        (const uint32_t*)(warp_mma_instances ? nullptr : ws.pos_of_pair), c.top_k, ws.xs,
-                        accumulator ? accumulator : ws.yacc);   // the rows the down epilogue adds into: the workspace's, or the caller's fp32 output itself
+        e = cudaGetLastError();
+    }
+    return e;
 }
 
 cudaError_t launch_prefill_combine(const shrike_moe* m, cudaStream_t st, uint32_t T, void* y, void* hidden) {

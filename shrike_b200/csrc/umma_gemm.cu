@@ -50,7 +50,7 @@
 
 namespace shrike {
 
-constexpr uint32_t kUmmaMaxN = 256;
+constexpr uint32_t kUmmaMaxN = kChunkRows;
 constexpr int kActBoxes = 5;
 constexpr uint32_t kConverters = 512;                  // two threads per weight row
 constexpr uint32_t kConvWarps = kConverters / 32;
@@ -277,10 +277,6 @@ __device__ __forceinline__ uint16_t pick16(const uint32_t (&v)[4], uint32_t idx)
     const uint32_t w = (idx & 4u) ? hi : lo;
     return (uint16_t)((idx & 1u) ? (w >> 16) : (w & 0xffffu));
 }
-
-struct alignas(16) ChunkInstance {  // up to 256 rows that share one expert block
-    uint32_t kind, slot, first, count;
-};
 
 // The instance's rows as one or two boxes of 16 << i rows (the largest that fits, then the smallest that holds the rest).
 struct TileShape {
@@ -1199,81 +1195,6 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
     }
 }
 
-// The list of instances: all full ones (256 rows; the shared expert's first), then every expert's rest, most rows first. A tile of
-// 256 rows takes twice the time of one of 16, and a list that ends on long ones leaves SMs idle. All tiles of more than 128 rows come before the
-// others, so a block changes the layout of its shared memory once at most: the barrier wide_over has one phase for it. One thread per expert; n_inst[0] = instances, [1], [2]: tiles handed out in phase 0, 1.
-__global__ void __launch_bounds__(256)
-chunk_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ counts,
-                       const uint32_t* __restrict__ slot_of_expert, uint32_t ne, uint32_t T, uint32_t with_shared,
-                       uint32_t pool_cells, ChunkInstance* __restrict__ inst, uint32_t* __restrict__ n_inst,
-                       uint32_t* status) {
-    pdl_wait();
-    pdl_launch_dependents();
-    __shared__ uint32_t warp_sums[8];
-    __shared__ __align__(16) uint32_t key[256];
-    const uint32_t e = threadIdx.x;
-    uint32_t n = 0, slot = SHRIKE_SLOT_MISS, c = 0;
-    if (e < ne && counts[e] > 0) {
-        c = counts[e];
-        slot = slot_of_expert[e];
-        if (slot != SHRIKE_SLOT_MISS && slot >= pool_cells) {
-            report_status(status, kStatusBadIndex);
-            slot = SHRIKE_SLOT_MISS;
-        }
-        if (slot == SHRIKE_SLOT_MISS) c = 0;
-        n = c / kUmmaMaxN;
-    }
-    const uint32_t rest = c % kUmmaMaxN, mine = rest << 8 | (255u - e), shared_rest = with_shared ? T % kUmmaMaxN : 0u;
-    key[e] = mine;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t inc = n;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= (uint32_t)o) inc += v;
-    }
-    if (lane == 31) warp_sums[warp] = inc;
-    const uint32_t before_shared = (uint32_t)__syncthreads_count(rest > shared_rest);   // rests that come before the shared expert's
-    const uint32_t n_rest = (uint32_t)__syncthreads_count(rest != 0) + (shared_rest != 0);
-    uint32_t base = 0, total = 0;
-    for (uint32_t w = 0; w < 8; ++w) {
-        if (w < warp) base += warp_sums[w];
-        total += warp_sums[w];
-    }
-    const uint32_t n_shared = with_shared ? T / kUmmaMaxN : 0;
-    base += inc - n + n_shared;
-    total += n_shared;
-    for (uint32_t j = 0; j < n; ++j) {
-        ChunkInstance in;
-        in.kind = 0; in.slot = slot; in.first = offsets[e] + kUmmaMaxN * j; in.count = kUmmaMaxN;
-        inst[base + j] = in;
-    }
-    if (rest) {
-        uint32_t rank = rest <= shared_rest ? 1u : 0u;
-        for (uint32_t j = 0; j < 256; j += 4) {
-            const uint4 v = *(const uint4*)&key[j];
-            rank += (v.x > mine) + (v.y > mine) + (v.z > mine) + (v.w > mine);
-        }
-        ChunkInstance in;
-        in.kind = 0; in.slot = slot; in.first = offsets[e] + kUmmaMaxN * n; in.count = rest;
-        inst[total + rank] = in;
-    }
-    for (uint32_t j = threadIdx.x; j < n_shared; j += blockDim.x) {
-        ChunkInstance in;
-        in.kind = 1; in.slot = 0; in.first = kUmmaMaxN * j; in.count = kUmmaMaxN;
-        inst[j] = in;
-    }
-    if (threadIdx.x == 0) {
-        if (shared_rest) {
-            ChunkInstance in;
-            in.kind = 1; in.slot = 0; in.first = kUmmaMaxN * n_shared; in.count = shared_rest;
-            inst[total + before_shared] = in;
-        }
-        n_inst[0] = total + n_rest;
-        n_inst[1] = n_inst[2] = 0;   // tiles handed out, per phase
-    }
-}
-
 // ---- tensor maps -------------------------------------------------------------------
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1456,20 +1377,15 @@ static const UmmaMaps* umma_maps_for(const shrike_moe* m, const ExpertArgs& a) {
     return cache->phase;
 }
 
-// Gate/up + GLU, then down, for the instances built from the grouping the
-// prefill plan left in the workspace.
-cudaError_t launch_umma_prefill(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, uint32_t T,
-                                uint32_t pool_cells) {
+// Gate/up + GLU, then down, for the instances that the prefill plan left in the workspace.
+cudaError_t launch_umma_prefill(const shrike_moe* m, cudaStream_t st, const ExpertArgs& a, uint32_t T) {
     const shrike_moe_config& c = m->cfg;
     const Workspace& ws = m->ws;
     if (!ws.tensor_maps || !umma_supported(c)) return cudaErrorNotSupported;
     const UmmaMaps* const maps = umma_maps_for(m, a);
     if (!maps) return cudaErrorInvalidValue;
-    ChunkInstance* inst = (ChunkInstance*)ws.chunk_inst;
+    const ChunkInstance* const inst = (const ChunkInstance*)ws.chunk_inst;
     const uint32_t max_inst = umma_max_chunk_instances(c, T);
-    cudaError_t e = launch_after(m, st, chunk_instances_kernel, dim3(1), 256, 0, ws.expert_offsets, ws.expert_counts, ws.slot_of_expert,
-                                 c.num_experts, T, (uint32_t)c.has_shared, pool_cells, inst, ws.n_chunk_inst, ws.status);
-    if (e != cudaSuccess) return e;
     const uint32_t bits = c.weight_bits, grp = c.group_size;
     const bool f16 = c.meta_dtype == SHRIKE_DTYPE_FP16;
 #define SHRIKE_UMMA(B, G, M) \
