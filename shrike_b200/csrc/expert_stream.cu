@@ -215,14 +215,17 @@ __device__ __forceinline__ void column_sums(const uint32_t (&b)[GROUP / 8], floa
 __device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
+__device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
+    asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory");
+}
 // Bytes of an instance buffer and its parts: [group][half][column][t] 16 bytes of operands, [quad][column][t] sums,
-// [group][t] initial values.
+// [group][t] 8 bytes of initial values (columns 2t and 2t + 1; a tile's rows have the same).
 struct BufferLayout {
     uint32_t z_off, cq_off, bytes;
     __device__ BufferLayout(uint32_t groups, uint32_t halves, uint32_t count) {
         z_off = groups * halves * count * 64;
         cq_off = z_off + (groups + 3) / 4 * count * 64;
-        bytes = cq_off + groups * 64;
+        bytes = (cq_off + groups * 32 + 15u) & ~15u;
     }
 };
 
@@ -247,8 +250,7 @@ __device__ __forceinline__ void stage_group(const uint32_t (&b)[GROUP / 8], uint
             if (g < count) sts128(buf + (j * (GROUP / 32) + h) * count * 64 + lane * 16, b[4 * h], b[4 * h + 1], b[4 * h + 2], b[4 * h + 3]);
         float r[4];
         column_sums<BITS, GROUP>(b, r);
-        if (lane < 4)
-            sts128(buf + lay.cq_off + j * 64 + lane * 16, __float_as_uint(-r[2]), __float_as_uint(-r[3]), __float_as_uint(-r[2]), __float_as_uint(-r[3]));
+        if (lane < 4) sts64(buf + lay.cq_off + j * 32 + lane * 8, __float_as_uint(-r[2]), __float_as_uint(-r[3]));
         // column g's sum sits in lane g / 2
         const float v0 = __shfl_sync(0xffffffffu, r[0], g >> 1), v1 = __shfl_sync(0xffffffffu, r[1], g >> 1);
         mine = (g & 1u) ? v1 : v0;
@@ -319,9 +321,9 @@ __device__ __forceinline__ void piece_tiles(uint32_t w, uint32_t sc, uint32_t d_
                 b += sB;
                 bf[e][4 * h] = v.x; bf[e][4 * h + 1] = v.y; bf[e][4 * h + 2] = v.z; bf[e][4 * h + 3] = v.w;
             }
-            const uint4 v = lds128(cq + (i + e) * 64);
-            c0[e][0] = __uint_as_float(v.x); c0[e][1] = __uint_as_float(v.y);
-            c0[e][2] = __uint_as_float(v.z); c0[e][3] = __uint_as_float(v.w);
+            const uint2 v = lds64(cq + (i + e) * 32);
+            c0[e][0] = c0[e][2] = __uint_as_float(v.x);
+            c0[e][1] = c0[e][3] = __uint_as_float(v.y);
         }
 #pragma unroll
         for (int m = 0; m < Q::kMmas; ++m) {
@@ -625,6 +627,10 @@ template <int BITS, int GROUP, int META, bool AL>
 __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid_constant__ StreamArgs a, const __grid_constant__ PieceMaps maps) {
     using Q = FQ<BITS, GROUP>;
     constexpr uint32_t GP = 128 / Q::kGroupBytes, H = GROUP / 32;   // groups of a piece; 16-byte operand parts of a group
+    // The warps of a team share a row by whole pieces, or by halves of pieces of eight groups where rows end within a piece: of 12
+    // pieces (2880 columns in groups of 32) eight warps have one or two, of 23 halves two or three. 32 experts of 2880 x 2880, 64 rows, us
+    // over four layers: 972 by pieces, 852 by halves and with initial values of 8 bytes (half of the loops' cycles are reads of shared memory).
+    constexpr uint32_t kHalves = GP == 8 && !AL ? 2 : 1;
     extern __shared__ __align__(128) uint8_t dsm_raw[];
     uint8_t* const dsm = dsm_raw + ((1024u - (smem_u32(dsm_raw) & 1023u)) & 1023u);   // the swizzle follows the address
     __shared__ uint64_t full1[kMaxSlots], done1[kMaxSlots], full2[kMaxSlots2], done2[kMaxSlots2];
@@ -813,7 +819,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
             // that role's registers): multiplies, finishes, or, in a team of one, both.
             auto units = [&](auto role) {
                 constexpr bool MUL = decltype(role)::value != 1, FIN = decltype(role)::value != 0, ONE = MUL && FIN;
-                uint32_t cur = 0xffffffffu, count = 0, groups_left = 0, pieces = 0;
+                uint32_t cur = 0xffffffffu, count = 0, groups_left = 0, pieces = 0, first_half = 0;
                 uint32_t b0 = 0, cq0 = 0, z0 = 0, sB = 0, w_at = 0, s_at = 0, ab_at = 0, d_s = 0, d_z = 0, k0 = 0;
                 uint16_t* dst = nullptr;   // gate/up: where column g's activations go
                 float* out0 = nullptr;     // down: where the rows of column g (ONE: columns 2t and 2t + 1) go, and their weights
@@ -833,18 +839,19 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
                     count = tab.count[i];
                     const uint32_t col = min(g, count - 1u);
                     if constexpr (MUL) {
-                        const uint32_t K = P1 ? D : sh ? a.f_shared : a.f, P = (K * BITS / 8 + 127) / 128, G2 = K / GROUP;
-                        const uint32_t p0 = P * wi / W;
-                        pieces = P * (wi + 1) / W - p0;
-                        groups_left = G2 - min(G2, p0 * GP);
+                        const uint32_t K = P1 ? D : sh ? a.f_shared : a.f, G2 = K / GROUP, P = (G2 + GP / kHalves - 1) / (GP / kHalves);
+                        const uint32_t h0 = P * wi / W, h1 = P * (wi + 1) / W, p0 = h0 / kHalves;
+                        first_half = h0 % kHalves;
+                        pieces = h1 > h0 ? (h1 + kHalves - 1) / kHalves - p0 : 0u;
+                        groups_left = (kHalves == 1 ? G2 : min(G2, h1 * 4)) - min(G2, h0 * (GP / kHalves));
                         const BufferLayout lay(G2, H, count);
                         sB = count * 64;
-                        b0 = buf + col * 64 + t * 16 + p0 * GP * H * sB;
-                        cq0 = buf + lay.cq_off + t * 16 + p0 * GP * 64;
-                        z0 = buf + lay.z_off + col * 64 + t * 16 + (GP == 2 ? p0 / 2 : p0 * (GP / 4)) * sB;
-                        k0 = GP == 2 ? 2 * (p0 & 1) : 0u;
-                        w_at = ring0 + w_lane + p0 * 2048;
-                        s_at = meta0 + (pr * G2 + p0 * GP) * 2;
+                        b0 = buf + col * 64 + t * 16 + h0 * (GP / kHalves) * H * sB;
+                        cq0 = buf + lay.cq_off + t * 8 + h0 * (GP / kHalves) * 32;
+                        z0 = buf + lay.z_off + col * 64 + t * 16 + (GP == 2 ? h0 / 2 : h0 * (GP / kHalves / 4)) * sB;
+                        k0 = GP == 2 ? 2 * (h0 & 1) : 0u;
+                        w_at = (ring0 + w_lane + p0 * 2048) ^ (first_half * 64);
+                        s_at = meta0 + (pr * G2 + h0 * (GP / kHalves)) * 2;
                         d_s = P1 ? 32 * G2 : 16 * G2;
                         d_z = P1 ? 16 * G2 : 32 * G2;
                         ab_at = meta0 - (P1 ? G.meta_off : 0u) + (P1 ? G.ab_off : G.ab_off2[sh]) + pr * 2;
@@ -879,20 +886,22 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
                             acc[2] = acc[3] = bf16_bits_to_f32((uint16_t)lds16(ab_at + mo + 16));
                         }
                         uint32_t w = w_at + slot * (P1 ? G.slot_bytes : G.w_bytes2), sc = s_at + mo, b = b0, cq = cq0, z = z0, kk = k0, left = groups_left;
+                        uint32_t cap = kHalves == 2 && first_half ? GP / 2 : GP;   // groups from here to the piece's end
 #pragma unroll 1
                         for (uint32_t p = 0; p < pieces; ++p) {
-                            piece_tiles<BITS, GROUP, META, !AL>(w, sc, d_s, d_z, b, cq, z, sB, min(GP, left), kk, t, acc);
-                            w += 2048;
-                            sc += 2 * GP;
-                            b += GP * H * sB;
-                            cq += GP * 64;
+                            piece_tiles<BITS, GROUP, META, !AL>(w, sc, d_s, d_z, b, cq, z, sB, min(cap, left), kk, t, acc);
+                            w = (kHalves == 2 && cap != GP ? w ^ 64u : w) + 2048;
+                            sc += 2 * cap;
+                            b += cap * H * sB;
+                            cq += cap * 32;
                             if constexpr (GP == 2) {
                                 kk ^= 2u;
                                 z += kk ? 0u : sB;
                             } else {
-                                z += GP / 4 * sB;
+                                z += cap / 4 * sB;
                             }
-                            left -= GP;
+                            left -= cap;
+                            if constexpr (kHalves == 2) cap = GP;
                         }
                         if (P1 || !ONE) {
                             const uint32_t to = rb + wi * (kRedWarp * 4) + my_red;
@@ -1026,7 +1035,7 @@ bool stream_geometry(const shrike_moe_config& c, uint32_t smem_optin, StreamGeom
     const uint32_t G1 = c.d / c.group_size, G2 = c.f / c.group_size, Gs = c.has_shared ? c.shared_f / c.group_size : 0;
     if ((G1 | G2 | Gs) & 1u) return false;   // rows of scales are read as 32-bit words
     auto pieces = [&](uint32_t K) { return (K * c.weight_bits / 8 + 127) / 128; };
-    auto buffer = [&](uint32_t groups) { return groups * (c.group_size / 32) * 512 + (groups + 3) / 4 * 512 + groups * 64; };   // eight columns
+    auto buffer = [&](uint32_t groups) { return groups * (c.group_size / 32) * 512 + (groups + 3) / 4 * 512 + (groups * 32 + 15) / 16 * 16; };   // eight columns
     g.meta_off = 2048 * pieces(c.d);
     g.ab_off = align_up(g.meta_off + 64 * G1, 128);
     g.slot_bytes = align_up(g.ab_off + (c.expert_bias ? 128 : 0), 1024);

@@ -18,6 +18,7 @@ pytestmark = pytest.mark.gpu
     dict(d=384, f=640, shared_f=128),                                    # a piece of two groups at the end
     dict(d=320, f=192, shared_f=192),                                    # odd numbers of groups: the per-tile kernels
     dict(d=128, f=128, has_shared=0, shared_gated=0, num_experts=4, top_k=2),   # many instances of the same experts
+    dict(d=1216, f=1344, shared_f=2880, group_size=32),                  # two and four warps to a row, some from the middle of a piece
     dict(d=384, f=192, shared_f=320, group_size=32, weight_bits=4, meta_dtype=capi.DTYPE_FP16),
     dict(d=128, f=384, shared_f=128, group_size=64, weight_bits=8),
     dict(d=192, f=320, shared_f=64, group_size=32, weight_bits=8, expert_bias=1, activation=capi.ACT_GELU_TANH),
