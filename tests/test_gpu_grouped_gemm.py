@@ -8,6 +8,7 @@ import torch
 
 from shrike_b200 import capi
 from shrike_b200.moe import MoE
+import fixtures as fx
 from gpu_harness import Layer, inputs, rel_l2, small_config, to_act_tensor
 
 pytestmark = pytest.mark.gpu
@@ -114,9 +115,39 @@ def test_rows_in_place(cuda_device, T):
     layer.close()
 
 
-def run_sizes(sizes, kw, sample=None):
+class LayerOfLargeScales(Layer):
+    """Expert blocks whose groups' scales and biases are up to 2^6 (gate, up) and 2^20 (down) times the fixture's: from 0.0013,
+    or 2^-14 for bytes, to where a converted weight still is an fp16 number. Most rows keep some groups as they are."""
+
+    def block(self, e):
+        if e not in self._blocks:
+            b = fx.synth_block(self.cfg, self.seed, self.layer, e)
+            o, cfg, rng = self.offsets, self.cfg, np.random.default_rng(e)
+            for name, rows, cols, most in (("gate", cfg.f, cfg.d, 6), ("up", cfg.f, cfg.d, 6), ("down", cfg.d, cfg.f, 20)):
+                n = rows * cols // cfg.group_size
+                by = 2.0 ** (rng.integers(0, most + 1, n) * rng.integers(0, 2, n))
+                for part in "sb":
+                    at = getattr(o, f"{name}_{part}")
+                    v = b[at:at + 2 * n].view(np.uint16)
+                    v[:] = fx.meta_bits(fx.meta_to_f32(v, cfg.meta_dtype) * by, cfg.meta_dtype)
+            self._blocks[e] = b
+        return self._blocks[e]
+
+
+@pytest.mark.parametrize("kw", [
+    dict(d=640, f=192),
+    dict(d=704, f=192, group_size=32),
+    dict(d=512, f=256, weight_bits=8, meta_dtype=capi.DTYPE_FP16),
+    dict(d=576, f=192, weight_bits=8, group_size=32),
+], ids=lambda kw: "-".join(f"{k}{v}" for k, v in kw.items()))
+def test_large_scales(cuda_device, kw):
+    """Scales that leave fp16's range when they are multiplied up for integers below its normal range, beside ones that do not."""
+    run_sizes([257, 129, 65, 17] + [3] * 10, dict(kw, num_experts=16, has_shared=False, shared_f=0), layer_of=LayerOfLargeScales)
+
+
+def run_sizes(sizes, kw, sample=None, layer_of=Layer):
     cfg = small_config(**dict(dict(num_experts=64, top_k=1, max_tokens=max(1024, sum(sizes)), shared_gated=False), **kw))
-    layer = Layer(cfg)
+    layer = layer_of(cfg)
     ids = np.concatenate([np.full(n, e, np.uint32) for e, n in enumerate(sizes)])
     ids = np.random.default_rng(3).permutation(ids)[:, None]
     x = inputs(len(ids), kw["d"], seed=5)
