@@ -10,10 +10,10 @@
 // reads each activation byte once per 256 weight rows and dequantises each
 // weight once per 256 activation rows.
 //
-//   warp 19    one thread takes tiles, streams the packed weights (64 or, for narrow tiles, 128
+//   warp 19    takes tiles, streams the packed weights (64 or, for narrow tiles, 128
 //              bytes of every row per copy: a 3-D TMA box of 128 rows of one matrix of one pool
 //              cell, swizzled) and the group scales / biases (16 or 32 bytes
-//              of every row per copy) into shared-memory rings. Whole-line TMA
+//              of every row per copy, or words of every row) into shared-memory rings. Whole-line TMA
 //              requests keep the packed experts streaming at HBM speed where
 //              per-thread 32-byte loads ran out of outstanding requests.
 //   warp 18    one thread copies the activation tiles: one or two boxes of 64 x
@@ -57,7 +57,7 @@ constexpr uint32_t kConvWarps = kConverters / 32;
 constexpr uint32_t kEpiWarps = 4;
 constexpr uint32_t kUmmaThreads = kConverters + 128 + kEpiWarps * 32;   // + two MMA warps, activation-copy warp, weight-copy warp, epilogue warps
 constexpr uint32_t kSmallN = 64;                       // rows up to which TMEM holds two pairs of accumulators
-constexpr uint32_t kConvRegs = 96, kOtherRegs = 48;    // of the 80 that 768 threads are launched with
+constexpr uint32_t kConvRegs = 88, kOtherRegs = 64;    // of the 80 that 768 threads are launched with
 static_assert(kConverters * kConvRegs + (kUmmaThreads - kConverters) * kOtherRegs <= kUmmaThreads * 80, "registers of a block");
 constexpr uint32_t kTileBytes = 128 * 128;             // 128 rows x 64 fp16, one swizzle-128B K block
 constexpr uint32_t kTiles = 4;                         // tiles that the copies may be ahead
@@ -75,12 +75,14 @@ constexpr uint32_t kNarrowBBytes = kNarrowN * 128;     // a K block of 128 rows,
 constexpr uint32_t kNarrowPkBytes = 256 * 128;         // 128 packed bytes of 256 rows
 constexpr uint32_t kNarrowScBytes = 2 * 256 * 32;      // 16 scales and biases of 256 rows
 constexpr uint32_t kNarrowOffPk = kNarrowB * kNarrowBBytes, kNarrowOffSc = kNarrowOffPk + kNarrowPk * kNarrowPkBytes;
-constexpr uint32_t kOffBar = kWideOffSc + kWideScBytes;
-static_assert(kNarrowOffSc + kNarrowSc * kNarrowScBytes <= kWideOffSc, "the converters' own scales lie beside the narrow tiles' ring");
+// Rows of an odd number of scales: every odd row's word past its scale block, [stage][scales, biases][128] (wide tiles: a stage).
+constexpr uint32_t kOffPast = kWideOffSc + kWideScBytes, kPastBytes = 128 * 4;
+static_assert(kNarrowOffSc + kNarrowSc * kNarrowScBytes <= kOffPast, "narrow tiles' scales");
+constexpr uint32_t kOffBar = kOffPast + kNarrowSc * 2 * kPastBytes;
 constexpr uint32_t kNumBars = 2 * (kWideB + kWideA + kWidePk + 1) + 1 + 2 * (kNarrowA + kNarrowB + kNarrowPk + kNarrowSc) + 2 + 3 * kTiles + 2;
 constexpr uint32_t kOffTiles = (kOffBar + kNumBars * 8 + 15) / 16 * 16;
 constexpr uint32_t kUmmaSmemBytes = kOffTiles + kTiles * 16 + 4 * kUmmaMaxN * 4 + 4 * kSmallN * 4 + 16 + 1024 /*alignment slack*/;
-static_assert(kUmmaSmemBytes + 64 <= 227 * 1024, "shared memory of a block");
+static_assert(kUmmaSmemBytes + 1024 <= 227 * 1024, "shared memory of a block");
 
 struct WeightMaps {       // TMA descriptors of the two 128-row tiles of a block
     CUtensorMap w[2];     // packed weights   [cells][rows][row bytes]
@@ -340,7 +342,10 @@ struct Tile {
 // 100 in two sets, 106 + 82 with an issuing warp per weight tile (a single one needed 650 cycles for a K block), 101 + 72 with
 // epilogue warps, 93 + 62 with the questions to barriers asked before their answers are needed. Deeper rings of copies, wider
 // boxes and fewer boxes of scales changed nothing: the bytes are there in time.
-// SCT: rows of scales are whole 16-byte units and come by TMA; others (groups % 8 != 0) are read by the converters.
+// SCT: rows of scales are whole 16-byte units and come by TMA; others (groups % 8 != 0) word by word (cp.async), into the same places.
+// Read by the converters themselves, a block ahead and through registers, their waits for a stage were waits for DRAM too: 32
+// experts of 2880 x 2880 in groups of 32 took 900 cycles for a K block and 6000 until a tile's first one, now 780 and 350 (host
+// call of 777 rows 519 -> 492 us).
 template <int BITS, int GROUP, int META, int PHASE, bool SCT>
 __global__ void __launch_bounds__(kUmmaThreads, 1)
 umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, uint32_t* __restrict__ n_inst,
@@ -394,13 +399,13 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         for (uint32_t s = 0; s < kWideA; ++s) { mbar_init(&a_full[s], kConvWarps); mbar_init(&a_empty[s], 2); }
         for (uint32_t s = 0; s < kWideB; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 2); }
         for (uint32_t s = 0; s < kWidePk; ++s) { mbar_init(&pk_full[s], 1); mbar_init(&pk_empty[s], kConvWarps); }
-        mbar_init(sc_full, 1);
+        mbar_init(sc_full, SCT ? 1 : 32);
         mbar_init(sc_empty, kConvWarps);
         mbar_init(wide_over, 2);
         for (uint32_t s = 0; s < kNarrowA; ++s) { mbar_init(&na_full[s], kConvWarps); mbar_init(&na_empty[s], 2); }
         for (uint32_t s = 0; s < kNarrowB; ++s) { mbar_init(&nb_full[s], 1); mbar_init(&nb_empty[s], 2); }
         for (uint32_t s = 0; s < kNarrowPk; ++s) { mbar_init(&npk_full[s], 1); mbar_init(&npk_empty[s], kConvWarps); }
-        for (uint32_t s = 0; s < kNarrowSc; ++s) { mbar_init(&nsc_full[s], 1); mbar_init(&nsc_empty[s], kConvWarps); }
+        for (uint32_t s = 0; s < kNarrowSc; ++s) { mbar_init(&nsc_full[s], SCT ? 1 : 32); mbar_init(&nsc_empty[s], kConvWarps); }
         for (uint32_t s = 0; s < 2; ++s) mbar_init(&epi_done[s], kConvWarps);
         for (uint32_t s = 0; s < kTiles; ++s) { mbar_init(&accum[s], 2); mbar_init(&tile_full[s], 1); mbar_init(&tile_empty[s], kConvWarps + 3 + kEpiWarps); }
         mbar_init(conv, kConvWarps);
@@ -552,23 +557,11 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         };
         // ---- of the tile at hand ----
         Tile t;
-        uint32_t KB, G, out_rows, mrow, my_rows;
-        const uint16_t *s_all, *b_all;      // its matrix's scales and biases
-        uint32_t sreg[4] = {0, 0, 0, 0}, breg[4] = {0, 0, 0, 0}, snext[4] = {0, 0, 0, 0}, bnext[4] = {0, 0, 0, 0};
+        uint32_t KB;
         uint32_t col_pair = 0;              // the pair (shared: row) behind this thread's column, and its weight
         float col_w = 0.f;
         auto open_tile = [&]() {
-            const uint32_t F = t.shared ? a.f_shared : a.f;
             KB = k_blocks(t);
-            G = KB * 64 / GROUP;
-            out_rows = PHASE == 0 ? F : a.d;       // rows of the weight matrix
-            mrow = t.r0 + (PHASE == 0 ? r : tile * 128 + r);
-            my_rows = t.r0 + (PHASE == 0 ? 0u : tile * 128u) + (warp & 3) * 32 + (lane >> 2);
-            const int mat = PHASE == 0 ? (int)tile : 2;
-            const Offsets3& off = t.shared ? a.shared : a.routed;
-            const uint8_t* base = t.shared ? a.shared_block : pool_cell_base(a.pool, t.slot);
-            s_all = (const uint16_t*)(base + off.s[mat]);
-            b_all = (const uint16_t*)(base + off.b[mat]);
             if (PHASE == 1 && t.count > kSmallN && tid < t.count) col_pair = t.shared ? t.first + tid : __ldcg(a.sorted + t.first + tid);
         };
         // The columns' tokens and route weights, for the epilogue: asked for when the tile begins (its weight once the pair is
@@ -587,123 +580,13 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             }
             return epilogue(width, std::integral_constant<int, 4>(), warp >> 2, t, n, 0u, acc1, rowid + at, roww + at);
         };
-        // Groups 8*blk .. 8*blk+7 straight from global memory (rows past the matrix and groups past the row read as
-        // zero: the converted weights are then zero). An even number of groups (32-wide ones always): the warp's 32 rows in 32-bit words, four
-        // lanes a row, handed to the rows' lanes when they are needed; read by each row's threads in 16-bit pieces
-        // they kept L1 busy for 1.3 us per K block of 90-group rows.
-        auto fetch_scales = [&](uint32_t blk) {
-            if (GROUP == 32 || (G & 1u) == 0) {
-                const uint32_t gi = blk * 8 + 2 * (lane & 3);
+        // Whether this row's scales begin with one of the row before: an odd row of an odd number of them.
+        auto past = [&]() { return !SCT && GROUP == 64 && (KB & r & 1u) != 0; };
+        // N words of scales become those that begin a half later.
+        auto shift_in = [&](auto& v, uint32_t next) {
+            constexpr int N = sizeof v / 4;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint32_t row = my_rows + 8 * i;
-                    const bool there = row < out_rows && gi < G;
-                    const size_t at = (size_t)row * G + gi;
-                    snext[i] = there ? __ldg((const uint32_t*)(s_all + at)) : 0u;
-                    bnext[i] = there ? __ldg((const uint32_t*)(b_all + at)) : 0u;
-                }
-                return;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint32_t gi = blk * 8 + 2 * i;
-                const size_t at = (size_t)mrow * G + gi;
-                uint32_t sv = 0, bv = 0;
-                if (mrow < out_rows && gi < G) {
-                    sv = __ldg(s_all + at);
-                    bv = __ldg(b_all + at);
-                    if (gi + 1 < G) {
-                        sv |= (uint32_t)__ldg(s_all + at + 1) << 16;
-                        bv |= (uint32_t)__ldg(b_all + at + 1) << 16;
-                    }
-                }
-                snext[i] = sv;
-                bnext[i] = bv;
-            }
-        };
-        // The eight groups fetched one block ago into sreg / breg, and the next ones asked for.
-        auto turn_scales = [&](uint32_t blk) {
-            if (GROUP == 32 || (G & 1u) == 0) {
-                __syncwarp();   // the last block's have been read
-                if constexpr (GROUP == 32) {
-                    // through shared memory: a thread's half has the even or the odd groups, so the two warps of a row write 16
-                    // bits of every word each
-                    uint8_t* const to = smem + kWideOffSc + (tile * 128 + (warp & 3) * 32 + (lane >> 2)) * 16 + (lane & 3) * 4 + half * 2;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        *(uint16_t*)(to + i * 128) = (uint16_t)(half ? snext[i] >> 16 : snext[i]);
-                        *(uint16_t*)(to + kWideScBytes / 2 + i * 128) = (uint16_t)(half ? bnext[i] >> 16 : bnext[i]);
-                    }
-                    __syncwarp();
-                    const uint8_t* const from = smem + kWideOffSc + (tile * 128 + r) * 16;
-                    const uint4 sv = *(const uint4*)from, bv = *(const uint4*)(from + kWideScBytes / 2);
-                    sreg[0] = sv.x; sreg[1] = sv.y; sreg[2] = sv.z; sreg[3] = sv.w;
-                    breg[0] = bv.x; breg[1] = bv.y; breg[2] = bv.z; breg[3] = bv.w;
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {   // lane 4 (row mod 8) + word of load row / 8
-#pragma unroll
-                        for (int w = 0; w < 4; ++w) {
-                            const uint32_t sv = __shfl_sync(0xffffffffu, snext[i], 4 * (lane & 7) + w);
-                            const uint32_t bv = __shfl_sync(0xffffffffu, bnext[i], 4 * (lane & 7) + w);
-                            if ((lane >> 3) == (uint32_t)i) { sreg[w] = sv; breg[w] = bv; }
-                        }
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) { sreg[i] = snext[i]; breg[i] = bnext[i]; }
-            }
-            fetch_scales(blk + 1);
-        };
-        // Narrow tiles of 32-wide groups: a thread multiplies with every second word of its row only, so the same registers
-        // hold two blocks, asked for that much earlier (one block is 2200 cycles, and the loads take longer): lane / 2 is the row.
-        uint32_t own_at[2] = {0, 0};
-        bool own_there[2] = {false, false};
-        auto fetch_own = [&](uint32_t blk, uint32_t* sv, uint32_t* bv) {
-            const uint32_t g0 = blk * 8;
-            const bool inside = g0 + 2 * (2 * (lane & 1) + half) < G;
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const bool there = inside && own_there[i];
-                sv[i] = there ? __ldg((const uint32_t*)(s_all + (own_at[i] + g0))) : 0u;
-                bv[i] = there ? __ldg((const uint32_t*)(b_all + (own_at[i] + g0))) : 0u;
-            }
-        };
-        auto first_scales = [&]() {
-            if constexpr (GROUP == 32) {
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const uint32_t row = my_rows - (lane >> 2) + (lane >> 1) + 16 * i;
-                    own_there[i] = row < out_rows;
-                    own_at[i] = row * G + 2 * (2 * (lane & 1) + half);
-                }
-                fetch_own(0, snext, bnext);
-                fetch_own(1, snext + 2, bnext + 2);
-            } else {
-                fetch_scales(0);
-            }
-        };
-        // Block blk's scales into sreg / breg: 32-wide groups this thread's two words, else all four.
-        auto narrow_scales = [&](uint32_t blk) {
-            if constexpr (GROUP == 32) {
-                // word j of row `lane` sits in lane 2 (row mod 16) + j of load row / 16
-                auto exchange = [&](uint32_t* sv, uint32_t* bv) {
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const uint32_t from = 2 * (lane & 15) + j;
-                        const uint32_t s0 = __shfl_sync(0xffffffffu, sv[0], from), s1 = __shfl_sync(0xffffffffu, sv[1], from);
-                        const uint32_t b0 = __shfl_sync(0xffffffffu, bv[0], from), b1 = __shfl_sync(0xffffffffu, bv[1], from);
-                        sreg[j] = lane & 16 ? s1 : s0;
-                        breg[j] = lane & 16 ? b1 : b0;
-                    }
-                    fetch_own(blk + 2, sv, bv);
-                };
-                if (blk & 1) exchange(snext + 2, bnext + 2);
-                else exchange(snext, bnext);
-            } else {
-                turn_scales(blk);
-            }
+            for (int i = 0; i < N; ++i) v[i] = __funnelshift_r(v[i], i + 1 < N ? v[i + 1 < N ? i + 1 : i] : next, 16);
         };
         // True for the warp when a lane's scale is too large for dequant_word(): the weights then take scale_weights() as well.
         auto scale_words = [&](uint32_t s16, uint32_t b16, uint32_t& s2, uint32_t& z2) {
@@ -748,25 +631,24 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             for (; go && !t.narrow; go = take_tile(++n, t)) {
                 was_wide = true;
                 open_tile();
-                if (!SCT) fetch_scales(0);
                 // A scale block (8 groups of the row) at a time, its K blocks unrolled: the position in the packed slot
                 // and the group of a K block are then constants of the instruction stream.
                 for (uint32_t kb0 = 0; kb0 < KB; kb0 += kKbPerSc) {
                     if (failed()) break;
-                    if (SCT) {
-                        if (!pipe_wait(sc_full, sc_use)) { give_up(); break; }
-                        sc_use ^= 1;
-                        const uint8_t* const from = smem + kWideOffSc + (tile * 128 + r) * 16;
-                        const uint4 sv = *(const uint4*)from;
-                        const uint4 bv = *(const uint4*)(from + kWideScBytes / 2);
-                        sreg[0] = sv.x; sreg[1] = sv.y; sreg[2] = sv.z; sreg[3] = sv.w;
-                        breg[0] = bv.x; breg[1] = bv.y; breg[2] = bv.z; breg[3] = bv.w;
-                        // the values are in registers: the copy thread may fetch the next block's
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(sc_empty);
-                    } else {
-                        turn_scales(kb0 / kKbPerSc);
+                    if (!pipe_wait(sc_full, sc_use)) { give_up(); break; }
+                    sc_use ^= 1;
+                    const uint8_t* const from = smem + kWideOffSc + (tile * 128 + r) * 16;
+                    uint32_t sreg[4], breg[4];
+                    load_words<4>(from, sreg);
+                    load_words<4>(from + kWideScBytes / 2, breg);
+                    if (past()) {
+                        const uint32_t* const more = (const uint32_t*)(smem + kOffPast) + (tile * 128 + r) / 2;
+                        shift_in(sreg, more[0]);
+                        shift_in(breg, more[kPastBytes / 4]);
                     }
+                    // the values are in registers: the copy thread may fetch the next block's
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(sc_empty);
 #pragma unroll
                     for (uint32_t j = 0; j < kKbPerSc; ++j) {
                         const uint32_t kb = kb0 + j;
@@ -850,46 +732,34 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             // What the next slot's first own K block needs, asked for as soon as the slot is there.
             uint32_t rs[kRawWords], rb[kRawWords];
             auto open_slot = [&](uint32_t kb0) {
-                if (SCT) {
-                    const uint8_t* const from = smem + sc_row + ss * kNarrowScBytes + in_sc * (kRawWords * 4);
-                    load_words<kRawWords>(from, rs);
-                    load_words<kRawWords>(from + kNarrowScBytes / 2, rb);
+                const uint8_t* const from = smem + sc_row + ss * kNarrowScBytes + in_sc * (kRawWords * 4);
+                load_words<kRawWords>(from, rs);
+                load_words<kRawWords>(from + kNarrowScBytes / 2, rb);
+                if (past()) {
+                    const bool end = (in_sc + 1) * kRawWords == 8;
+                    const uint8_t* const more = end ? smem + kOffPast + ss * 2 * kPastBytes + (tile * 128 + r) / 2 * 4 : from + kRawWords * 4;
+                    shift_in(rs, *(const uint32_t*)more);
+                    shift_in(rb, *(const uint32_t*)(more + (end ? kPastBytes : kNarrowScBytes / 2)));
                 }
                 if (kb0 + half < KB) load_packed(0);
             };
             for (; go; go = take_tile(++n, t)) {
                 open_tile();
-                uint32_t blk = 0, in_blk = 0;   // eight groups; slot of them
-                if (!SCT) first_scales();
-                if (SCT && !pipe_wait(&nsc_full[ss], sc_par)) { give_up(); break; }
+                if (!pipe_wait(&nsc_full[ss], sc_par)) { give_up(); break; }
                 if (!pipe_wait(&npk_full[slot], pk_par)) { give_up(); break; }
                 open_slot(0);
                 for (uint32_t kb0 = 0; kb0 < KB; kb0 += kNarrowKbPerPk) {
                     const bool last = kb0 + kNarrowKbPerPk >= KB;
                     // ---- the slot's scales and biases: own K block i's in sw[i], bw[i] (in the low bits, or both groups') ----
                     uint32_t sw[kOwn], bw[kOwn];
-                    if constexpr (SCT) {
 #pragma unroll
-                        for (uint32_t i = 0; i < kOwn; ++i) {
-                            if constexpr (GROUP == 32) {
-                                sw[i] = half ? rs[2 * i + 1] : rs[2 * i];
-                                bw[i] = half ? rb[2 * i + 1] : rb[2 * i];
-                            } else {
-                                sw[i] = rs[i] >> (16 * half);
-                                bw[i] = rb[i] >> (16 * half);
-                            }
-                        }
-                    } else {
-                        if (in_blk == 0) narrow_scales(blk++);
-                        else {
-#pragma unroll
-                            for (uint32_t i = 0; i + kOwn < 4; ++i) { sreg[i] = sreg[i + kOwn]; breg[i] = breg[i + kOwn]; }
-                        }
-                        if (++in_blk == kSlotsPerSc) in_blk = 0;
-#pragma unroll
-                        for (uint32_t i = 0; i < kOwn; ++i) {
-                            sw[i] = GROUP == 32 ? sreg[i] : sreg[i] >> (16 * half);
-                            bw[i] = GROUP == 32 ? breg[i] : breg[i] >> (16 * half);
+                    for (uint32_t i = 0; i < kOwn; ++i) {
+                        if constexpr (GROUP == 32) {
+                            sw[i] = half ? rs[2 * i + 1] : rs[2 * i];
+                            bw[i] = half ? rb[2 * i + 1] : rb[2 * i];
+                        } else {
+                            sw[i] = rs[i] >> (16 * half);
+                            bw[i] = rb[i] >> (16 * half);
                         }
                     }
                     const uint32_t slot1 = slot + 1 == kNarrowPk ? 0u : slot + 1, pk_par1 = slot1 ? pk_par : pk_par ^ 1;
@@ -929,7 +799,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                         next_pair();
                     }
                     // handed back only here: the values read from them have been consumed
-                    const bool sc_done = SCT && (++in_sc == 2 * kSlotsPerSc || last);
+                    const bool sc_done = ++in_sc == 2 * kSlotsPerSc || last;
                     __syncwarp();
                     if (lane == 0) {
                         mbar_arrive(&npk_empty[slot]);
@@ -1038,13 +908,14 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                     const uint64_t db = umma_smem_desc(sm0 + sb * kNarrowBBytes + in_b * b_step);
 #pragma unroll
                     for (uint32_t k = 0; k < 4; ++k) umma_f16_ts(acc_at, ta + 8 * k, db + 2 * k, idesc, (kb | k) != 0);
+                    if (!b_mask) umma_commit(&nb_empty[sb]);   // (its next copy need not wait for the other K block)
                     if (here == 2) {
                         const uint64_t db1 = umma_smem_desc(sm0 + sb1 * kNarrowBBytes + in_b1 * b_step);
 #pragma unroll
                         for (uint32_t k = 0; k < 4; ++k) umma_f16_ts(acc_at, ta + 64 + 8 * k, db1 + 2 * k, idesc, 1u);
                     }
                     umma_commit(&na_empty[st]);
-                    if (b_done) umma_commit(&nb_empty[sb]);
+                    if (b_mask && b_done) umma_commit(&nb_empty[sb]);
                     if (!b_mask && here == 2) umma_commit(&nb_empty[sb1]);
                 }
                 __syncwarp();
@@ -1128,19 +999,63 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             if (!epilogue(std::integral_constant<int, 4>(), std::integral_constant<int, 1>(), 0u, t, n, at, at + kSmallN, ids, wts)) break;
             release_tile(n);
         }
-    } else if (lane == 0) {
+    } else {
         // ---------------- tiles; packed weights, scales, biases ----------------
+        // The whole warp walks the loop: one lane asks for the TMA copies, all copy words of scales where those do not come by TMA.
+        auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, pipe_wait(bar, parity)) != 0; };
+        auto any_failed = [&]() { return __any_sync(0xffffffffu, failed()) != 0; };
+        // W words of every row's scales and biases from group g0 on, rows y0 .. y0 + 127 and y1 .. y1 + 127 of the tile's matrices of G
+        // groups a row; of an odd row of an odd number of groups, from the word that the first one shares with the row before, and a word
+        // more. What lies past the matrix reads as zero.
+        auto copy_scales = [&](auto width, const Tile& t, uint32_t g0, uint32_t y0, uint32_t y1, uint32_t to, uint32_t to_past, uint64_t* bar) {
+            constexpr uint32_t W = decltype(width)::value, kStep = 32 / W, kBias = 256 * W * 4;
+            const Offsets3& off = t.shared ? a.shared : a.routed;
+            const uint8_t* const base = t.shared ? a.shared_block : pool_cell_base(a.pool, t.slot);
+            const uint32_t G = k_blocks(t) * 64 / GROUP, odd = G & 1u, stride = kStep * G * 2;
+            const int32_t total = (int32_t)((PHASE == 0 ? t.shared ? a.f_shared : a.f : a.d) * G);
+            auto word = [&](uint32_t dst, const uint8_t* sp, const uint8_t* bp, int32_t at, uint32_t bias_dst) {
+                const uint32_t n = (uint32_t)max(0, min(2 * (total - at), 4));
+                const size_t from = n ? (size_t)at * 2 : 0;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(sp + from), "r"(n) : "memory");
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + bias_dst), "l"(bp + from), "r"(n) : "memory");
+            };
+#pragma unroll 1
+            for (uint32_t m = 0; m < 2; ++m) {
+                const int mat = PHASE == 0 ? (int)m : 2;
+                const uint8_t *const sp = base + off.s[mat], *const bp = base + off.b[mat];
+                const uint32_t row0 = m ? y1 : y0, row = lane / W, dst = to + (m * 128 * W + lane) * 4;
+                const int32_t at = (int32_t)((row0 + row) * G + g0 + 2 * (lane % W) - (row & odd));
+                if ((int32_t)((row0 + 127) * G + g0 + 2 * W) <= total) {   // (most of the warp's instructions; the copies of weights wait for them)
+                    const uint8_t *s_at = sp + (size_t)at * 2, *b_at = bp + (size_t)at * 2;
+#pragma unroll 8
+                    for (uint32_t q = 0; q < 128 / kStep; ++q, s_at += stride, b_at += stride) {
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + q * 128), "l"(s_at) : "memory");
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + q * 128 + kBias), "l"(b_at) : "memory");
+                    }
+                } else {
+#pragma unroll 1
+                    for (uint32_t q = 0; q < 128 / kStep; ++q) word(dst + q * 128, sp, bp, at + (int32_t)(q * kStep * G), kBias);
+                }
+                if (odd)
+#pragma unroll 1
+                    for (uint32_t i = lane; i < 64; i += 32)
+                        word(to_past + (m * 64 + i) * 4, sp, bp, (int32_t)((row0 + 2 * i + 1) * G + g0 + 2 * W - 1), kPastBytes);
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+        };
         // The number of the tile after next and the instance of the next one are asked for while this one is copied.
         const uint32_t n_tiles = __ldcg(n_inst) * row_tiles;
         auto read_inst = [&](uint32_t tile) { return tile < n_tiles ? __ldcg((const uint4*)(inst + tile / row_tiles)) : make_uint4(0, 0, 0, 0); };
-        uint32_t now = blockIdx.x, next = gridDim.x + atomicAdd(n_inst + 1 + PHASE, 1u);
+        auto number = [&]() { return lane == 0 ? gridDim.x + atomicAdd(n_inst + 1 + PHASE, 1u) : 0u; };   // (of lane 0)
+        uint32_t now = blockIdx.x, next = number();
         uint4 v = read_inst(now);
         uint32_t n = 0, pk_use = 0, sc_use = 0, slot = 0, ss = 0, pk_par = 0, sc_par = 0;
         bool was_wide = false, in_wide = true;
         for (;;) {
             const bool end = now >= n_tiles;
+            next = __shfl_sync(0xffffffffu, next, 0);
             const uint4 v_next = end ? v : read_inst(next);
-            const uint32_t after = end ? 0u : gridDim.x + atomicAdd(n_inst + 1 + PHASE, 1u);
+            const uint32_t after = end ? 0u : number();
             Tile t;
             t.shared = v.x == 1;
             t.slot = v.y; t.first = v.z; t.count = end ? 0u : v.w;
@@ -1150,37 +1065,45 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             now = next; next = after; v = v_next;
             if (!end && t.r0 >= rows) continue;   // a narrower shared or routed expert
             const uint32_t s = n % kTiles;
-            if (!pipe_wait(&tile_empty[s], ((n / kTiles) & 1) ^ 1)) { give_up(); break; }
+            if (!wait(&tile_empty[s], ((n / kTiles) & 1) ^ 1)) { give_up(); break; }
             ++n;
-            next_tile[s] = make_uint4(t.slot, t.first, t.r0 | (t.shared ? 0x80000000u : 0u), t.count);
-            mbar_arrive(&tile_full[s]);
-            if (end || failed()) break;
+            if (lane == 0) {
+                next_tile[s] = make_uint4(t.slot, t.first, t.r0 | (t.shared ? 0x80000000u : 0u), t.count);
+                mbar_arrive(&tile_full[s]);
+            }
+            if (end || any_failed()) break;
             const WeightMaps* wm = t.shared ? &maps.shared : &maps.routed[t.slot / a.pool.cells_per_chunk];
             const int32_t cell = t.shared ? 0 : (int32_t)(t.slot % a.pool.cells_per_chunk);
             const int32_t y0 = (int32_t)t.r0, y1 = (int32_t)(PHASE == 0 ? t.r0 : t.r0 + 128);
             if (!t.narrow) {
                 was_wide = true;
                 for (uint32_t kb = 0; kb < KB; ++kb) {
-                    if (failed()) break;
-                    if (SCT && kb % kKbPerSc == 0) {
+                    if (any_failed()) break;
+                    if (kb % kKbPerSc == 0) {
                         const int32_t g0 = (int32_t)(kb / kKbPerSc * 8);
-                        if (!pipe_wait(sc_empty, sc_use ^ 1)) { give_up(); break; }
+                        if (!wait(sc_empty, sc_use ^ 1)) { give_up(); break; }
                         sc_use ^= 1;
-                        mbar_expect_tx(sc_full, kWideScBytes);
                         const uint32_t dst = smem_base + kWideOffSc;
-                        tma_load_3d(dst, &wm->s[0], g0, y0, cell, sc_full);
-                        tma_load_3d(dst + kWideScBytes / 4, &wm->s[1], g0, y1, cell, sc_full);
-                        tma_load_3d(dst + kWideScBytes / 2, &wm->b[0], g0, y0, cell, sc_full);
-                        tma_load_3d(dst + kWideScBytes / 4 * 3, &wm->b[1], g0, y1, cell, sc_full);
+                        if (!SCT) {
+                            copy_scales(std::integral_constant<uint32_t, 4>(), t, (uint32_t)g0, (uint32_t)y0, (uint32_t)y1, dst, smem_base + kOffPast, sc_full);
+                        } else if (lane == 0) {
+                            mbar_expect_tx(sc_full, kWideScBytes);
+                            tma_load_3d(dst, &wm->s[0], g0, y0, cell, sc_full);
+                            tma_load_3d(dst + kWideScBytes / 4, &wm->s[1], g0, y1, cell, sc_full);
+                            tma_load_3d(dst + kWideScBytes / 2, &wm->b[0], g0, y0, cell, sc_full);
+                            tma_load_3d(dst + kWideScBytes / 4 * 3, &wm->b[1], g0, y1, cell, sc_full);
+                        }
                     }
                     if (kb % kWideKbPerPk == 0) {
                         const int32_t x = (int32_t)(kb / kWideKbPerPk * 64);
-                        if (!pipe_wait(&pk_empty[slot], ((pk_use >> slot) & 1) ^ 1)) { give_up(); break; }
+                        if (!wait(&pk_empty[slot], ((pk_use >> slot) & 1) ^ 1)) { give_up(); break; }
                         pk_use ^= 1u << slot;
-                        mbar_expect_tx(&pk_full[slot], kWidePkBytes);
-                        const uint32_t dst = smem_base + kWideOffPk + slot * kWidePkBytes;
-                        tma_load_3d(dst, &wm->w[0], x, y0, cell, &pk_full[slot]);
-                        tma_load_3d(dst + kWidePkBytes / 2, &wm->w[1], x, y1, cell, &pk_full[slot]);
+                        if (lane == 0) {
+                            mbar_expect_tx(&pk_full[slot], kWidePkBytes);
+                            const uint32_t dst = smem_base + kWideOffPk + slot * kWidePkBytes;
+                            tma_load_3d(dst, &wm->w[0], x, y0, cell, &pk_full[slot]);
+                            tma_load_3d(dst + kWidePkBytes / 2, &wm->w[1], x, y1, cell, &pk_full[slot]);
+                        }
                         if (++slot == kWidePk) slot = 0;
                     }
                 }
@@ -1189,28 +1112,35 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
             if (in_wide) {
                 in_wide = false;
                 slot = 0;
-                if (was_wide && !pipe_wait(wide_over, 0)) { give_up(); break; }
+                if (was_wide && !wait(wide_over, 0)) { give_up(); break; }
             }
             for (uint32_t kb = 0; kb < KB; kb += kNarrowKbPerPk) {
-                if (failed()) break;
-                if (SCT && kb % (2 * kKbPerSc) == 0) {
+                if (any_failed()) break;
+                if (kb % (2 * kKbPerSc) == 0) {
                     const int32_t g0 = (int32_t)(kb / kKbPerSc * 8);
                     uint64_t* const bar = &nsc_full[ss];
-                    if (!pipe_wait(&nsc_empty[ss], sc_par ^ 1)) { give_up(); break; }
-                    mbar_expect_tx(bar, kNarrowScBytes);
+                    if (!wait(&nsc_empty[ss], sc_par ^ 1)) { give_up(); break; }
                     const uint32_t dst = smem_base + kNarrowOffSc + ss * kNarrowScBytes;
-                    tma_load_3d(dst, &wm->ns[0], g0, y0, cell, bar);
-                    tma_load_3d(dst + kNarrowScBytes / 4, &wm->ns[1], g0, y1, cell, bar);
-                    tma_load_3d(dst + kNarrowScBytes / 2, &wm->nb[0], g0, y0, cell, bar);
-                    tma_load_3d(dst + kNarrowScBytes / 4 * 3, &wm->nb[1], g0, y1, cell, bar);
+                    if (!SCT) {
+                        copy_scales(std::integral_constant<uint32_t, 8>(), t, (uint32_t)g0, (uint32_t)y0, (uint32_t)y1, dst,
+                                    smem_base + kOffPast + ss * 2 * kPastBytes, bar);
+                    } else if (lane == 0) {
+                        mbar_expect_tx(bar, kNarrowScBytes);
+                        tma_load_3d(dst, &wm->ns[0], g0, y0, cell, bar);
+                        tma_load_3d(dst + kNarrowScBytes / 4, &wm->ns[1], g0, y1, cell, bar);
+                        tma_load_3d(dst + kNarrowScBytes / 2, &wm->nb[0], g0, y0, cell, bar);
+                        tma_load_3d(dst + kNarrowScBytes / 4 * 3, &wm->nb[1], g0, y1, cell, bar);
+                    }
                     if (++ss == kNarrowSc) { ss = 0; sc_par ^= 1; }
                 }
-                if (!pipe_wait(&npk_empty[slot], pk_par ^ 1)) { give_up(); break; }
-                mbar_expect_tx(&npk_full[slot], kNarrowPkBytes);
-                const uint32_t dst = smem_base + kNarrowOffPk + slot * kNarrowPkBytes;
-                const int32_t x = (int32_t)(kb / kNarrowKbPerPk * 128);
-                tma_load_3d(dst, &wm->nw[0], x, y0, cell, &npk_full[slot]);
-                tma_load_3d(dst + kNarrowPkBytes / 2, &wm->nw[1], x, y1, cell, &npk_full[slot]);
+                if (!wait(&npk_empty[slot], pk_par ^ 1)) { give_up(); break; }
+                if (lane == 0) {
+                    mbar_expect_tx(&npk_full[slot], kNarrowPkBytes);
+                    const uint32_t dst = smem_base + kNarrowOffPk + slot * kNarrowPkBytes;
+                    const int32_t x = (int32_t)(kb / kNarrowKbPerPk * 128);
+                    tma_load_3d(dst, &wm->nw[0], x, y0, cell, &npk_full[slot]);
+                    tma_load_3d(dst + kNarrowPkBytes / 2, &wm->nw[1], x, y1, cell, &npk_full[slot]);
+                }
                 if (++slot == kNarrowPk) { slot = 0; pk_par ^= 1; }
             }
         }
@@ -1280,7 +1210,7 @@ static bool make_weight_maps(WeightMaps* wm, const uint8_t* base, const Offsets3
         if (!make_matrix_map(&wm->w[t], base + off.w[mat], false, false, (uint64_t)kdim * bits / 8, rows, cells, cell_stride) ||
             !make_matrix_map(&wm->nw[t], base + off.w[mat], false, true, (uint64_t)kdim * bits / 8, rows, cells, cell_stride))
             return false;
-        if ((kdim / group) % 8 != 0) continue;   // such scale rows are read by the converter threads
+        if ((kdim / group) % 8 != 0) continue;   // such scale rows are copied word by word
         for (int n = 0; n < 2; ++n)
             if (!make_matrix_map(n ? &wm->ns[t] : &wm->s[t], base + off.s[mat], true, n, kdim / group, rows, cells, cell_stride) ||
                 !make_matrix_map(n ? &wm->nb[t] : &wm->b[t], base + off.b[mat], true, n, kdim / group, rows, cells, cell_stride))
