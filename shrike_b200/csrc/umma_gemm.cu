@@ -16,7 +16,7 @@
 //              of every row per copy, or words of every row) into shared-memory rings. Whole-line TMA
 //              requests keep the packed experts streaming at HBM speed where
 //              per-thread 32-byte loads ran out of outstanding requests.
-//   warp 18    one thread copies the activation tiles: one or two boxes of 64 x
+//   warp 18    copies the activation tiles: one or two boxes of 64 x
 //              16 to 256 of the expert-sorted fp16 rows per K block, 128-byte
 //              swizzle.
 //   warps 0-15 converters: they turn the packed nibbles/bytes of a 64-wide K block into fp16
@@ -399,13 +399,13 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         for (uint32_t s = 0; s < kWideA; ++s) { mbar_init(&a_full[s], kConvWarps); mbar_init(&a_empty[s], 2); }
         for (uint32_t s = 0; s < kWideB; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 2); }
         for (uint32_t s = 0; s < kWidePk; ++s) { mbar_init(&pk_full[s], 1); mbar_init(&pk_empty[s], kConvWarps); }
-        mbar_init(sc_full, SCT ? 1 : 32);
+        mbar_init(sc_full, SCT ? 1 : 64);
         mbar_init(sc_empty, kConvWarps);
         mbar_init(wide_over, 2);
         for (uint32_t s = 0; s < kNarrowA; ++s) { mbar_init(&na_full[s], kConvWarps); mbar_init(&na_empty[s], 2); }
         for (uint32_t s = 0; s < kNarrowB; ++s) { mbar_init(&nb_full[s], 1); mbar_init(&nb_empty[s], 2); }
         for (uint32_t s = 0; s < kNarrowPk; ++s) { mbar_init(&npk_full[s], 1); mbar_init(&npk_empty[s], kConvWarps); }
-        for (uint32_t s = 0; s < kNarrowSc; ++s) { mbar_init(&nsc_full[s], SCT ? 1 : 32); mbar_init(&nsc_empty[s], kConvWarps); }
+        for (uint32_t s = 0; s < kNarrowSc; ++s) { mbar_init(&nsc_full[s], SCT ? 1 : 64); mbar_init(&nsc_empty[s], kConvWarps); }
         for (uint32_t s = 0; s < 2; ++s) mbar_init(&epi_done[s], kConvWarps);
         for (uint32_t s = 0; s < kTiles; ++s) { mbar_init(&accum[s], 2); mbar_init(&tile_full[s], 1); mbar_init(&tile_empty[s], kConvWarps + 3 + kEpiWarps); }
         mbar_init(conv, kConvWarps);
@@ -830,6 +830,44 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         }
     } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, pipe_wait(bar, parity)) != 0; };
+    auto any_failed = [&]() { return __any_sync(0xffffffffu, failed()) != 0; };
+    // Weight tile m: W words of every row's scales and biases from group g0 on, 128 rows from row0 on; of an odd row of an odd number
+    // of groups, from the word that the first one shares with the row before, and a word more. What lies past the matrix reads
+    // as zero. (By one warp for both weight tiles: 100 rows of 32 experts of 2880 x 2880 239 us a call, by a warp each 197.)
+    auto copy_scales = [&](auto width, uint32_t m, const Tile& t, uint32_t g0, uint32_t row0, uint32_t to, uint32_t to_past, uint64_t* bar) {
+        constexpr uint32_t W = decltype(width)::value, kStep = 32 / W, kBias = 256 * W * 4;
+        const Offsets3& off = t.shared ? a.shared : a.routed;
+        const uint8_t* const base = t.shared ? a.shared_block : pool_cell_base(a.pool, t.slot);
+        const uint32_t G = k_blocks(t) * 64 / GROUP, odd = G & 1u, stride = kStep * G * 2;
+        const int32_t total = (int32_t)((PHASE == 0 ? t.shared ? a.f_shared : a.f : a.d) * G);
+        auto word = [&](uint32_t dst, const uint8_t* sp, const uint8_t* bp, int32_t at, uint32_t bias_dst) {
+            const uint32_t n = (uint32_t)max(0, min(2 * (total - at), 4));
+            const size_t from = n ? (size_t)at * 2 : 0;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(sp + from), "r"(n) : "memory");
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + bias_dst), "l"(bp + from), "r"(n) : "memory");
+        };
+        const int mat = PHASE == 0 ? (int)m : 2;
+        const uint8_t *const sp = base + off.s[mat], *const bp = base + off.b[mat];
+        const uint32_t row = lane / W, dst = to + (m * 128 * W + lane) * 4;
+        const int32_t at = (int32_t)((row0 + row) * G + g0 + 2 * (lane % W) - (row & odd));
+        if ((int32_t)((row0 + 127) * G + g0 + 2 * W) <= total) {   // (most of the warp's instructions; the copies of weights wait for them)
+            const uint8_t *s_at = sp + (size_t)at * 2, *b_at = bp + (size_t)at * 2;
+#pragma unroll 8
+            for (uint32_t q = 0; q < 128 / kStep; ++q, s_at += stride, b_at += stride) {
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + q * 128), "l"(s_at) : "memory");
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + q * 128 + kBias), "l"(b_at) : "memory");
+            }
+        } else {
+#pragma unroll 1
+            for (uint32_t q = 0; q < 128 / kStep; ++q) word(dst + q * 128, sp, bp, at + (int32_t)(q * kStep * G), kBias);
+        }
+        if (odd)
+#pragma unroll 1
+            for (uint32_t i = lane; i < 64; i += 32)
+                word(to_past + (m * 64 + i) * 4, sp, bp, (int32_t)((row0 + 2 * i + 1) * G + g0 + 2 * W - 1), kPastBytes);
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+    };
     if (warp < kConvWarps + 2) {
         // ---------------- MMA issue, a warp for each of the two weight tiles ----------------
         // (one warp for both issued a K block of 16 rows in 650 cycles: it gets a fifth of its scheduler's slots)
@@ -929,44 +967,58 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         // ---------------- activation tiles ----------------
         // One or two boxes per K block: these tiles are most of what a block pulls out of L2, and a short instance
         // does not pay for 256 rows, nor one of 80 rows for 128.
-        uint32_t b_use = 0, sb = 0, nsb = 0, b_par = 0;
-        bool was_wide = false, in_wide = true;
+        uint32_t b_use = 0, sb = 0, nsb = 0, b_par = 0, ss = 0, sc_par = 0, sc_use = 0;
+        bool was_wide = false, in_wide = true, waited = PHASE == 0;
         Tile t;
-        if (PHASE == 1) pdl_wait();
         for (uint32_t n = 0; take_tile(n, t); ++n) {
             const TileShape ts(t.count);
             const CUtensorMap* maps_b = t.shared ? maps.act_shared : maps.act_routed;
-            if (lane == 0) {
-                const uint32_t KB = k_blocks(t), b_bytes = (ts.n1 + ts.n2) * 128u;
-                if (t.narrow && in_wide) {
-                    in_wide = false;
-                    if (was_wide && !pipe_wait(wide_over, 0)) give_up();
+            const uint32_t KB = k_blocks(t), b_bytes = (ts.n1 + ts.n2) * 128u, y1 = PHASE == 0 ? t.r0 : t.r0 + 128;
+            if (t.narrow && in_wide) {
+                in_wide = false;
+                if (was_wide && !wait(wide_over, 0)) give_up();
+            }
+            was_wide = in_wide;
+            auto copy = [&](uint32_t dst, uint32_t kb, uint64_t* bar) {
+                tma_load_2d(dst, &maps_b[ts.b1], (int32_t)(kb * 64), (int32_t)t.first, bar);
+                if (ts.n2) tma_load_2d(dst + ts.n1 * 128u, &maps_b[ts.b2], (int32_t)(kb * 64), (int32_t)(t.first + ts.n1), bar);
+            };
+            const uint32_t b_mask = narrow_b_mask(t.count), b_step = kNarrowBBytes / (b_mask + 1);
+            for (uint32_t kb = 0; t.narrow && kb < KB; kb += b_mask + 1) {
+                if (any_failed()) break;
+                if (!SCT && kb % (2 * kKbPerSc) == 0) {
+                    if (!wait(&nsc_empty[ss], sc_par ^ 1)) { give_up(); break; }
+                    copy_scales(std::integral_constant<uint32_t, 8>(), 1, t, kb * kGroupsPerBlock, y1, smem_base + kNarrowOffSc + ss * kNarrowScBytes,
+                                smem_base + kOffPast + ss * 2 * kPastBytes, &nsc_full[ss]);
+                    if (++ss == kNarrowSc) { ss = 0; sc_par ^= 1; }
                 }
-                was_wide = in_wide;
-                auto copy = [&](uint32_t dst, uint32_t kb, uint64_t* bar) {
-                    tma_load_2d(dst, &maps_b[ts.b1], (int32_t)(kb * 64), (int32_t)t.first, bar);
-                    if (ts.n2) tma_load_2d(dst + ts.n1 * 128u, &maps_b[ts.b2], (int32_t)(kb * 64), (int32_t)(t.first + ts.n1), bar);
-                };
-                const uint32_t b_mask = narrow_b_mask(t.count), b_step = kNarrowBBytes / (b_mask + 1);
-                for (uint32_t kb = 0; t.narrow && kb < KB; kb += b_mask + 1) {
-                    if (failed()) break;
-                    if (!pipe_wait(&nb_empty[nsb], b_par ^ 1)) { give_up(); break; }
+                if (!waited) { pdl_wait(); waited = true; }   // the scales are there before the gate/up launch ends
+                if (!wait(&nb_empty[nsb], b_par ^ 1)) { give_up(); break; }
+                if (lane == 0) {
                     const uint32_t here = min(b_mask + 1, KB - kb);
                     mbar_expect_tx(&nb_full[nsb], here * b_bytes);
                     for (uint32_t i = 0; i < here; ++i) copy(smem_base + nsb * kNarrowBBytes + i * b_step, kb + i, &nb_full[nsb]);
-                    if (++nsb == kNarrowB) { nsb = 0; b_par ^= 1; }
                 }
-                for (uint32_t kb = 0; !t.narrow && kb < KB; ++kb) {
-                    if (failed()) break;
-                    if (!pipe_wait(&b_empty[sb], ((b_use >> sb) & 1) ^ 1)) { give_up(); break; }
-                    b_use ^= 1u << sb;
+                if (++nsb == kNarrowB) { nsb = 0; b_par ^= 1; }
+            }
+            for (uint32_t kb = 0; !t.narrow && kb < KB; ++kb) {
+                if (any_failed()) break;
+                if (!SCT && kb % kKbPerSc == 0) {
+                    if (!wait(sc_empty, sc_use ^ 1)) { give_up(); break; }
+                    sc_use ^= 1;
+                    copy_scales(std::integral_constant<uint32_t, 4>(), 1, t, kb * kGroupsPerBlock, y1, smem_base + kWideOffSc, smem_base + kOffPast, sc_full);
+                }
+                if (!waited) { pdl_wait(); waited = true; }
+                if (!wait(&b_empty[sb], ((b_use >> sb) & 1) ^ 1)) { give_up(); break; }
+                b_use ^= 1u << sb;
+                if (lane == 0) {
                     mbar_expect_tx(&b_full[sb], b_bytes);
                     copy(smem_base + sb * kWideBBytes, kb, &b_full[sb]);
-                    if (++sb == kWideB) sb = 0;
                 }
+                if (++sb == kWideB) sb = 0;
             }
-            __syncwarp();
         }
+        if (!waited) pdl_wait();   // (no tile here: the launch still ends after the one before)
     } else if (warp > kConvWarps + 3) {
         // ---------------- epilogues of small tiles ----------------
         // (by the converters between two tiles they took 3000 of a tile's 22,000 cycles at 2048 x 16 rows)
@@ -1001,48 +1053,6 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
         }
     } else {
         // ---------------- tiles; packed weights, scales, biases ----------------
-        // The whole warp walks the loop: one lane asks for the TMA copies, all copy words of scales where those do not come by TMA.
-        auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, pipe_wait(bar, parity)) != 0; };
-        auto any_failed = [&]() { return __any_sync(0xffffffffu, failed()) != 0; };
-        // W words of every row's scales and biases from group g0 on, rows y0 .. y0 + 127 and y1 .. y1 + 127 of the tile's matrices of G
-        // groups a row; of an odd row of an odd number of groups, from the word that the first one shares with the row before, and a word
-        // more. What lies past the matrix reads as zero.
-        auto copy_scales = [&](auto width, const Tile& t, uint32_t g0, uint32_t y0, uint32_t y1, uint32_t to, uint32_t to_past, uint64_t* bar) {
-            constexpr uint32_t W = decltype(width)::value, kStep = 32 / W, kBias = 256 * W * 4;
-            const Offsets3& off = t.shared ? a.shared : a.routed;
-            const uint8_t* const base = t.shared ? a.shared_block : pool_cell_base(a.pool, t.slot);
-            const uint32_t G = k_blocks(t) * 64 / GROUP, odd = G & 1u, stride = kStep * G * 2;
-            const int32_t total = (int32_t)((PHASE == 0 ? t.shared ? a.f_shared : a.f : a.d) * G);
-            auto word = [&](uint32_t dst, const uint8_t* sp, const uint8_t* bp, int32_t at, uint32_t bias_dst) {
-                const uint32_t n = (uint32_t)max(0, min(2 * (total - at), 4));
-                const size_t from = n ? (size_t)at * 2 : 0;
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(sp + from), "r"(n) : "memory");
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + bias_dst), "l"(bp + from), "r"(n) : "memory");
-            };
-#pragma unroll 1
-            for (uint32_t m = 0; m < 2; ++m) {
-                const int mat = PHASE == 0 ? (int)m : 2;
-                const uint8_t *const sp = base + off.s[mat], *const bp = base + off.b[mat];
-                const uint32_t row0 = m ? y1 : y0, row = lane / W, dst = to + (m * 128 * W + lane) * 4;
-                const int32_t at = (int32_t)((row0 + row) * G + g0 + 2 * (lane % W) - (row & odd));
-                if ((int32_t)((row0 + 127) * G + g0 + 2 * W) <= total) {   // (most of the warp's instructions; the copies of weights wait for them)
-                    const uint8_t *s_at = sp + (size_t)at * 2, *b_at = bp + (size_t)at * 2;
-#pragma unroll 8
-                    for (uint32_t q = 0; q < 128 / kStep; ++q, s_at += stride, b_at += stride) {
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + q * 128), "l"(s_at) : "memory");
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + q * 128 + kBias), "l"(b_at) : "memory");
-                    }
-                } else {
-#pragma unroll 1
-                    for (uint32_t q = 0; q < 128 / kStep; ++q) word(dst + q * 128, sp, bp, at + (int32_t)(q * kStep * G), kBias);
-                }
-                if (odd)
-#pragma unroll 1
-                    for (uint32_t i = lane; i < 64; i += 32)
-                        word(to_past + (m * 64 + i) * 4, sp, bp, (int32_t)((row0 + 2 * i + 1) * G + g0 + 2 * W - 1), kPastBytes);
-            }
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-        };
         // The number of the tile after next and the instance of the next one are asked for while this one is copied.
         const uint32_t n_tiles = __ldcg(n_inst) * row_tiles;
         auto read_inst = [&](uint32_t tile) { return tile < n_tiles ? __ldcg((const uint4*)(inst + tile / row_tiles)) : make_uint4(0, 0, 0, 0); };
@@ -1085,7 +1095,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                         sc_use ^= 1;
                         const uint32_t dst = smem_base + kWideOffSc;
                         if (!SCT) {
-                            copy_scales(std::integral_constant<uint32_t, 4>(), t, (uint32_t)g0, (uint32_t)y0, (uint32_t)y1, dst, smem_base + kOffPast, sc_full);
+                            copy_scales(std::integral_constant<uint32_t, 4>(), 0, t, (uint32_t)g0, (uint32_t)y0, dst, smem_base + kOffPast, sc_full);
                         } else if (lane == 0) {
                             mbar_expect_tx(sc_full, kWideScBytes);
                             tma_load_3d(dst, &wm->s[0], g0, y0, cell, sc_full);
@@ -1122,8 +1132,7 @@ umma_expert_kernel(const ExpertArgs a, const ChunkInstance* __restrict__ inst, u
                     if (!wait(&nsc_empty[ss], sc_par ^ 1)) { give_up(); break; }
                     const uint32_t dst = smem_base + kNarrowOffSc + ss * kNarrowScBytes;
                     if (!SCT) {
-                        copy_scales(std::integral_constant<uint32_t, 8>(), t, (uint32_t)g0, (uint32_t)y0, (uint32_t)y1, dst,
-                                    smem_base + kOffPast + ss * 2 * kPastBytes, bar);
+                        copy_scales(std::integral_constant<uint32_t, 8>(), 0, t, (uint32_t)g0, (uint32_t)y0, dst, smem_base + kOffPast + ss * 2 * kPastBytes, bar);
                     } else if (lane == 0) {
                         mbar_expect_tx(bar, kNarrowScBytes);
                         tma_load_3d(dst, &wm->ns[0], g0, y0, cell, bar);
