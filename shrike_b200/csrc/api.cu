@@ -181,9 +181,10 @@ int fill_expert_args(shrike_moe* m, const shrike_pool* pool, const shrike_expert
 // 2304 x 1024 int8: 17.0, 22.9 | 40.4, 42.0 | 34.0, 36.3); two rows have: 29.3, 27.1 | 88, 57.5 | 46.8, 43.3. Up to 64 rows it is
 // also ahead of the expert-grouped GEMM, which reads an expert once for all its rows but starts in a dozen launches, unless few
 // large experts get many rows (streaming and grouped, uniform picks):
-//   17 rows  65, 96 | 152, 214 | 136, 186     48 rows  109, 151 | 191, 220 | 226, 292     64 rows  123, 166 | 241, 220 | 252, 324
-// With picks by Zipf(1.1), 48 rows: 68, 83 | 211, 201 | 160, 194; 64 rows: 80, 92 | 241, 198 | 182, 204. There too its rows are sums in
-// a fixed order, which the grouped GEMM's are not, and those of the separate calls.
+//   17 rows  65, 92 | 130, 187 | 134, 176     48 rows  110, 134 | 170, 191 | 210, 246     64 rows  121, 145 | 210, 192 | 240, 266
+// With picks by Zipf(1.1), 48 rows: 67, 69 | 173, 172 | 152, 163; 64 rows: 79, 72 | 218, 179 | 179, 174. There too its rows are sums in
+// a fixed order, which the grouped GEMM's are not, those of the separate calls, and of products with the packed integers as they are, where
+// the grouped GEMM rounds a weight to fp16.
 // The projections as calls of their own follow the same rule, so that they give a layer call's rows bit for bit. Each pays the
 // kernel's set-up, with no router to share: plan and both of them, us, per-tile kernels and streaming, 30.3, 32.8 | 85, 62 | 45.9,
 // 49.3 at two rows, 34.4, 37.0 | 113, 76 | 60.2, 57.5 at three, 41.1, 39.9 | 138, 82 | 72, 66 at four.
@@ -759,13 +760,13 @@ int shrike_encode_decode_layer(shrike_moe* m, void* stream, const shrike_pool* p
     }
     // Shapes that the streaming kernel does not take, with many rows, on a handle that owns the prefill operands: the
     // expert-grouped GEMM reads every expert once for all its rows, where the 8-row tiles read it once per 8. The dozen
-    // launches around it pay from 24 to 50 rows on, by the number of experts; the line is where no shape loses (us a layer, tiles and
-    // grouped, odd numbers of groups, picks uniform or by Zipf(1.1);
+    // launches around it pay from 17 rows on (us a layer, tiles and grouped, odd numbers of groups, picks uniform or by Zipf(1.1);
     // 256 experts of 2048 x 576 int4 | 256 of 2304 x 1088 int8 | 32 of 2880 x 2880 int4 in groups of 64):
-    //   17 rows  119, 116 | 199, 200 | 231, 295     Zipf   63, 71 | 151, 162 | 158, 248
-    //   32 rows  176, 156 | 281, 257 | 260, 303     Zipf   89, 79 | 194, 182 | 240, 251
-    //   48 rows  223, 182 | 361, 318 | 301, 304     Zipf  128, 92 | 254, 214 | 304, 278
-    //   64 rows  259, 202 | 413, 349 | 369, 304     Zipf  161, 100 | 298, 224 | 364, 277
+    //   17 rows  119, 107 | 209, 198 | 227, 181     Zipf   62, 64 | 160, 155 | 165, 148
+    //   32 rows  175, 139 | 286, 250 | 265, 183     Zipf   89, 69 | 205, 176 | 253, 160
+    //   48 rows  228, 164 | 349, 286 | 298, 184     Zipf  122, 76 | 255, 187 | 300, 165
+    //   64 rows  261, 174 | 399, 308 | 369, 185     Zipf  151, 78 | 305, 200 | 390, 172
+    // The line stays: below it a row's sums have a fixed order and its weights are not rounded.
     if (query_count > 48 && w.xs && umma_supported(m->cfg) && !m->force_warp_mma) {
         int rcg = shrike_encode_router(m, stream, router, x, query_count, m->cfg.d, ids, wt, gate);
         if (rcg) return rcg;
