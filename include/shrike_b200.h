@@ -294,7 +294,8 @@ int shrike_encode_decode_layer(shrike_moe* moe, void* stream, const shrike_pool*
  * (PrefillSharedExpert.swift:105-161), encodeReduceTokenMajor (PrefillMoE.swift:11-20)
  * and the two residual adds (RealForwardRunner.swift:4658-4665). Same
  * arithmetic contract as the decode call; rows are grouped by topk_indices
- * (the expert ids), and every pair of one expert must resolve to one cell.
+ * (the expert ids), and every pair of one expert that has a cell must have the
+ * same one. A pair whose slot is SHRIKE_SLOT_MISS contributes nothing.
  * y may be x; rows that overlap in another way are not supported. */
 int shrike_encode_moe_prefill(shrike_moe* moe, void* stream, const shrike_pool* pool,
                               const shrike_expert_offsets* routed_offsets,

@@ -101,7 +101,7 @@ struct Workspace {
     float* yacc = nullptr;          // prefill: fp32 output accumulator [max_tokens x d]
     void* chunk_inst = nullptr;     // prefill: instances of up to 256 rows (tensor-core path)
     uint32_t* n_chunk_inst = nullptr; // [0] instances, [1], [2] tiles handed out per phase
-    uint32_t* rank_of_pair = nullptr; // prefill: earlier rows of the pair's block of rows with its expert, or 0xffffffff: no row is needed
+    uint32_t* rank_of_pair = nullptr; // prefill: earlier rows of its block of rows with a cell for its expert, or 0xffffffff: the pair has no cell
     uint32_t* plan_ticket = nullptr; // blocks finished, prefill plan
     uint16_t* xs = nullptr;         // prefill: fp16 activation rows in expert-sorted order [max_tokens x top_k x d]
     void* tensor_maps = nullptr;    // host: the TMA descriptors of xs, acts, xh, acts_shared and of the last prefill's pool and shared block

@@ -247,7 +247,8 @@ __device__ __forceinline__ void chunk_instances(uint32_t* warp_sums, uint32_t (&
 }
 
 // The prefill plan in one launch: step 1, and every pair's rows before it in its block of rows; the block that finishes last
-// takes step 2 and lists the instances. The pairs' places follow from the two where the rows are converted. Bound by a chain of trips
+// takes step 2 and lists the instances. Only pairs with a cell are counted and placed, so that every place an instance covers is
+// written, whatever the slots say: an expert that becomes resident while they are looked up has pairs of both kinds. The pairs' places follow from the two where the rows are converted. Bound by a chain of trips
 // to L2 (ids, counts, ticket, counts again, list). Counting, scan, places and list as launches of their own, and this: a call of 70 rows
 // 155.9 -> 150.1 us, 333 rows 181.5 -> 177.6, 1134 rows 247.9 -> 243.2.
 __global__ void __launch_bounds__(256)
@@ -257,7 +258,7 @@ group_plan_kernel(const uint32_t* __restrict__ ids, uint32_t T, uint32_t top_k, 
                   uint32_t with_shared, uint32_t pool_cells, ChunkInstance* __restrict__ inst, uint32_t* __restrict__ n_inst) {
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ GroupBits bits;
+    __shared__ GroupBits named, bits;   // the rows that name each expert; those that have a cell for it
     __shared__ uint32_t warp_sums[8], s_last;
     __shared__ __align__(16) uint32_t key[256];
     // a thread's pairs, asked for at once and kept
@@ -272,15 +273,23 @@ group_plan_kernel(const uint32_t* __restrict__ ids, uint32_t T, uint32_t top_k, 
         cell[j] = i < n ? slots[(size_t)t0 * top_k + i] : SHRIKE_SLOT_MISS;
     }
 #pragma unroll
-    for (uint32_t j = 0; j < sizeof(GroupBits) / 4 / 256; ++j) (&bits[0][0])[j * 256 + threadIdx.x] = 0;
+    for (uint32_t j = 0; j < sizeof(GroupBits) / 4 / 256; ++j) (&named[0][0])[j * 256 + threadIdx.x] = (&bits[0][0])[j * 256 + threadIdx.x] = 0;
     __syncthreads();
 #pragma unroll
     for (uint32_t j = 0; j < N; ++j) {
         const uint32_t tl = (j * 256 + threadIdx.x) / top_k, bit = 1u << (tl & 31);
         if (e[j] < ne) {
-            slot_of_expert[e[j]] = ready ? cell[j] : SHRIKE_SLOT_MISS;
             // a row that names one expert twice (no top-k router does) is counted once and reported
-            if (atomicOr(&bits[e[j]][tl >> 5], bit) & bit) report_status(status, kStatusBadIndex);
+            if (atomicOr(&named[e[j]][tl >> 5], bit) & bit) report_status(status, kStatusBadIndex);
+            if (!ready) cell[j] = SHRIKE_SLOT_MISS;
+            if (cell[j] != SHRIKE_SLOT_MISS && cell[j] >= pool_cells) {
+                report_status(status, kStatusBadIndex);
+                cell[j] = SHRIKE_SLOT_MISS;
+            }
+            if (cell[j] != SHRIKE_SLOT_MISS) {
+                atomicOr(&bits[e[j]][tl >> 5], bit);
+                slot_of_expert[e[j]] = cell[j];   // (of an expert with two cells either)
+            }
         } else if (e[j] != 0xffffffffu) {
             report_status(status, kStatusBadIndex);   // out of range: dropped (0xffffffff: the pick lives on another rank)
         }
@@ -295,7 +304,6 @@ group_plan_kernel(const uint32_t* __restrict__ ids, uint32_t T, uint32_t top_k, 
 #pragma unroll
     for (uint32_t j = 0; j < N; ++j) {
         const uint32_t i = j * 256 + threadIdx.x;
-        // (no row is needed where the expert has no cell)
         if (i < n) rank_of_pair[(size_t)t0 * top_k + i] = e[j] >= ne || cell[j] == SHRIKE_SLOT_MISS ? 0xffffffffu : rows_before(bits, e[j], i / top_k);
     }
     __threadfence();
@@ -309,15 +317,8 @@ group_plan_kernel(const uint32_t* __restrict__ ids, uint32_t T, uint32_t top_k, 
     __threadfence();
     uint32_t total, base;
     group_scan(warp_sums, block_hist, gridDim.x, ne, offsets, counts, total, base);
-    uint32_t slot = SHRIKE_SLOT_MISS;
-    if (threadIdx.x < ne && total) {
-        slot = __ldcg(slot_of_expert + threadIdx.x);
-        if (slot != SHRIKE_SLOT_MISS && slot >= pool_cells) {
-            report_status(status, kStatusBadIndex);
-            slot = SHRIKE_SLOT_MISS;
-        }
-    }
-    chunk_instances(warp_sums, key, slot == SHRIKE_SLOT_MISS ? 0u : total, base, slot, T, with_shared, inst, n_inst);
+    const uint32_t slot = threadIdx.x < ne && total ? __ldcg(slot_of_expert + threadIdx.x) : SHRIKE_SLOT_MISS;
+    chunk_instances(warp_sums, key, total, base, slot, T, with_shared, inst, n_inst);
 }
 
 cudaError_t launch_group_pairs(const shrike_moe* m, cudaStream_t st, const uint32_t* ids,

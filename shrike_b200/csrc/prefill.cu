@@ -14,20 +14,15 @@ namespace shrike {
 __global__ void __launch_bounds__(256)
 prefill_instances_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ counts,
                          const uint32_t* __restrict__ slot_of_expert, uint32_t ne, uint32_t T,
-                         uint32_t with_shared, uint32_t pool_cells,
-                         const uint32_t* __restrict__ sorted, Instance* __restrict__ inst,
-                         uint32_t* __restrict__ n_inst, uint32_t* status) {
+                         uint32_t with_shared, const uint32_t* __restrict__ sorted, Instance* __restrict__ inst,
+                         uint32_t* __restrict__ n_inst) {
     __shared__ uint32_t warp_sums[8];
     const uint32_t e = threadIdx.x;
     uint32_t n = 0, slot = SHRIKE_SLOT_MISS, c = 0;
-    if (e < ne && counts[e] > 0) {
+    if (e < ne && counts[e] > 0) {   // (of pairs with a cell)
         c = counts[e];
         slot = slot_of_expert[e];
-        if (slot != SHRIKE_SLOT_MISS && slot >= pool_cells) {
-            report_status(status, kStatusBadIndex);
-            slot = SHRIKE_SLOT_MISS;
-        }
-        if (slot != SHRIKE_SLOT_MISS) n = (c + 7) / 8;
+        n = (c + 7) / 8;
     }
     // exclusive scan over 256 threads
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -150,8 +145,8 @@ cudaError_t launch_prefill_plan(const shrike_moe* m, cudaStream_t st, const uint
                      accumulator ? accumulator : ws.yacc);   // the rows the down epilogue adds into: the workspace's, or the caller's fp32 output itself
     if (e == cudaSuccess && warp_mma_instances) {   // the tensor-core path has its 256-row instances from the plan
         prefill_instances_kernel<<<1, 256, 0, st>>>(ws.expert_offsets, ws.expert_counts, ws.slot_of_expert,
-                                                    c.num_experts, T, with_shared ? 1u : 0u, pool_cells, ws.sorted,
-                                                    ws.inst, ws.n_inst, ws.status);
+                                                    c.num_experts, T, with_shared ? 1u : 0u, ws.sorted,
+                                                    ws.inst, ws.n_inst);
         e = cudaGetLastError();
     }
     return e;

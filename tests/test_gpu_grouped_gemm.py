@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from shrike_b200 import capi
-from shrike_b200.moe import MoE
+from shrike_b200.moe import MoE, ShrikeError
 import fixtures as fx
 from gpu_harness import Layer, inputs, rel_l2, small_config, to_act_tensor
 
@@ -112,6 +112,44 @@ def test_rows_in_place(cuda_device, T):
         layer.moe.encode_prefill(layer.pool, layer.offsets, ids, slots, w, rows, out, None, layer.shared)
         layer.moe.status()
     assert torch.equal(y, same) and not torch.equal(y, x)
+    layer.close()
+
+
+@pytest.mark.parametrize("path", ["umma", "mma"])
+@pytest.mark.parametrize("T", [65, 300])
+def test_experts_with_pairs_that_miss(cuda_device, monkeypatch, path, T):
+    """Pairs at SLOT_MISS, and outside the pool, of experts whose other pairs have a cell, after a larger call on the same handle:
+    they contribute nothing, what the larger call left in the order of the pairs is not followed, and nothing is added behind y."""
+    if path == "mma":
+        monkeypatch.setenv("SHRIKE_PREFILL_PATH", "mma")
+    cfg = small_config(d=256, f=192, shared_f=128, num_experts=12, top_k=4, max_tokens=700, shared_gated=False)
+    layer = Layer(cfg, router_sigma=0.05)
+    layer.forward(inputs(700, cfg.d, seed=1))
+    x = inputs(T, cfg.d, seed=2)
+    x_dev = to_act_tensor(x, cfg.act_dtype, layer.device)
+    ids, w, _ = layer.route(x_dev)
+    slots, _ = layer.classify(ids)
+    ids_np, w_np = ids.cpu().numpy().astype(np.uint32), w.cpu().numpy()
+    missing = np.random.default_rng(3).random((T, 4)) < 0.4
+    missing[ids_np == 3] = True     # no pair with a cell
+    missing[ids_np == 7] = False    # every pair
+    for e, at in ((0, -1), (1, 0)):   # only the last, only the first pair misses
+        rows = np.flatnonzero((ids_np == e).any(axis=1))
+        missing[ids_np == e] = False
+        missing[rows[at], ids_np[rows[at]] == e] = True
+    y_ref = layer.oracle_forward(x, ids_np, np.where(missing, np.float32(0), w_np))
+    for cell in (-1, cfg.num_experts + 5):
+        slots_in = torch.where(torch.from_numpy(missing).cuda(), torch.full_like(slots, cell), slots)
+        out = torch.full((700, cfg.d), 7.0, device=layer.device)
+        layer.moe.encode_prefill(layer.pool, layer.offsets, ids, slots_in, w, x_dev, out[:T], None, layer.shared)
+        if cell < 0:
+            layer.moe.status()
+        else:
+            with pytest.raises(ShrikeError) as err:
+                layer.moe.status()
+            assert err.value.code == capi.ERANGE
+        assert rel_l2(out[:T].cpu().numpy(), y_ref) <= 1e-3
+        assert (out[T:] == 7.0).all()
     layer.close()
 
 
