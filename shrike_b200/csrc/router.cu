@@ -47,8 +47,10 @@ __device__ __forceinline__ void logits_rows(const RouterArgs& a, Pre pre) {
         if (f32row) {
             acc = lane_dot_f32<N, PRED>(wr, chunks, lane, xrow, a.dt, is_gate ? nullptr : a.eff_scale);
         } else {
-            acc = lane_dot_affine((const uint8_t*)a.w + (size_t)e * (a.d * a.bits / 8), a.scales + (size_t)e * groups,
-                                  a.biases + (size_t)e * groups, a.bits, groups, lane, xrow, a.dt, a.eff_scale);
+            const uint8_t* const row = (const uint8_t*)a.w + (size_t)e * (a.d * a.bits / 8);
+            const uint16_t *const s_row = a.scales + (size_t)e * groups, *const b_row = a.biases + (size_t)e * groups;
+            if (a.dt == SHRIKE_DTYPE_FP32) acc = lane_dot_affine_f32(row, s_row, b_row, a.bits, groups, lane, (const float*)xrow, a.eff_scale);
+            else acc = lane_dot_affine(row, s_row, b_row, a.bits, groups, lane, xrow, a.dt, a.eff_scale);
         }
         acc = butterfly_sum(acc);
         if (lane == 0) {

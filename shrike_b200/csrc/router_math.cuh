@@ -110,6 +110,14 @@ __device__ __forceinline__ float lane_dot_f32(const float4 (&wr)[N], uint32_t ch
     return acc;
 }
 
+// acc plus an affine group's share of a lane: its scale and bias, the two packed elements q (the low one first), their activations.
+__device__ __forceinline__ float add_affine(float acc, uint32_t bits, uint16_t s, uint16_t b, uint32_t q, float x0, float x1) {
+    const float q0 = (float)(bits == 4 ? (q & 0xfu) : (q & 0xffu));
+    const float q1 = (float)(bits == 4 ? (q >> 4) : (q >> 8));
+    acc = __fmaf_rn(bf16_bits_to_f32(s), __fadd_rn(__fmul_rn(q0, x0), __fmul_rn(q1, x1)), acc);
+    return __fmaf_rn(bf16_bits_to_f32(b), __fadd_rn(x0, x1), acc);
+}
+
 // router_gemv_body (moe.metal:324-364): lane l takes elements 64g+2l, 64g+2l+1 of every group g.
 // The operands of eight groups are requested, as they are in memory, before the first is used (one memory round trip per
 // eight groups instead of one per group); the arithmetic and its order are the shader's.
@@ -139,10 +147,6 @@ __device__ __forceinline__ float lane_dot_affine(const uint8_t* row, const uint1
 #pragma unroll
         for (uint32_t j = 0; j < kBatch; ++j) {
             if (g0 + j < groups) {
-                const float sc = bf16_bits_to_f32(sr[j]);
-                const float bi = bf16_bits_to_f32(br[j]);
-                const float q0 = (float)(bits == 4 ? (qr[j] & 0xfu) : (qr[j] & 0xffu));
-                const float q1 = (float)(bits == 4 ? (qr[j] >> 4) : (qr[j] >> 8));
                 float x0, x1;
                 if (dt == SHRIKE_DTYPE_FP32) {
                     x0 = __uint_as_float(xr[j].x); x1 = __uint_as_float(xr[j].y);
@@ -155,8 +159,45 @@ __device__ __forceinline__ float lane_dot_affine(const uint8_t* row, const uint1
                     x0 = __fmul_rn(x0, __uint_as_float(er[j] << 16));
                     x1 = __fmul_rn(x1, __uint_as_float(er[j] & 0xffff0000u));
                 }
-                acc = __fmaf_rn(sc, __fadd_rn(__fmul_rn(q0, x0), __fmul_rn(q1, x1)), acc);
-                acc = __fmaf_rn(bi, __fadd_rn(x0, x1), acc);
+                acc = add_affine(acc, bits, sr[j], br[j], qr[j], x0, x1);
+            }
+        }
+    }
+    return acc;
+}
+
+// The same of fp32 activations, which nothing has to convert behind their loads: the compiler may run the batches into one another and
+// leaves out what lies past the last group. (The router of 256 experts, as above and this, us: int4 rows, 8 rows of 128 columns
+// 6.1, 5.8; 2048 columns 11.6, 9.7; 2880 columns 15.0, 12.1. The one-row layer keeps the shorter code: its blocks wait for instructions.)
+__device__ __forceinline__ float lane_dot_affine_f32(const uint8_t* row, const uint16_t* s_row, const uint16_t* b_row, uint32_t bits,
+                                                     uint32_t groups, uint32_t lane, const float* xrow, const uint16_t* eff_scale) {
+    float acc = 0.f;
+    constexpr uint32_t kBatch = 8;
+    for (uint32_t g0 = 0; g0 < groups; g0 += kBatch) {
+        uint16_t sr[kBatch], br[kBatch];
+        uint32_t qr[kBatch], er[kBatch];
+        float2 xr[kBatch];
+#pragma unroll
+        for (uint32_t j = 0; j < kBatch; ++j) {
+            const uint32_t gi = g0 + j;
+            if (gi < groups) {
+                const uint32_t idx = gi * 64 + lane * 2;
+                sr[j] = s_row[gi];
+                br[j] = b_row[gi];
+                qr[j] = bits == 4 ? (uint32_t)row[idx >> 1] : (uint32_t)*(const uint16_t*)(row + idx);
+                xr[j] = *(const float2*)(xrow + idx);
+                er[j] = eff_scale ? *(const uint32_t*)(eff_scale + idx) : 0x3f803f80u;
+            }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kBatch; ++j) {
+            if (g0 + j < groups) {
+                float x0 = xr[j].x, x1 = xr[j].y;
+                if (eff_scale) {
+                    x0 = __fmul_rn(x0, __uint_as_float(er[j] << 16));
+                    x1 = __fmul_rn(x1, __uint_as_float(er[j] & 0xffff0000u));
+                }
+                acc = add_affine(acc, bits, sr[j], br[j], qr[j], x0, x1);
             }
         }
     }
