@@ -303,7 +303,12 @@ cudaError_t launch_router(const shrike_moe* m, cudaStream_t st, const shrike_rou
     cudaError_t e;
     // A warp per row re-reads the activations for every expert row: ahead up to eight rows (the logits of 256 experts of 2048 columns, us:
     // 4 rows 2.8 against the tiles' 5.4, 8 rows 4.5 / 5.4, 16 rows 5.8 / 5.2, 64 rows 19 / 5.4; int8 rows 5.0 / 9.0, 9.0 / 9.0, 16 / 9, 60 / 9).
-    if (T > 8 && router_tiles_take(a)) {
+    // fp32 rows of 2048 and 2304 columns have straight-line code, and while its blocks run at once it keeps ahead of
+    // tiles that are a few at most (4 experts of 2048 columns, 9 to 64 rows, us: bf16 6.7 / 7.1, fp32 7.2 / 8.2), of fp32 activations
+    // at 2048 columns whatever the experts (16 experts 7.8 / 8.1; 128 experts, 9 rows 8.0 / 8.4, 40 rows, more than a block an SM, 12.5 / 8.5).
+    const bool straight = a.bits == 0 && (a.d == 2048 || a.d == 2304) && (rows + kRouterWarps - 1) / kRouterWarps * ((T + 3) / 4) <= (uint32_t)m->sm_count &&
+                          (a.ne < kRouterWarps || (a.d == 2048 && a.dt == SHRIKE_DTYPE_FP32));
+    if (T > 8 && !(T <= 64 && straight) && router_tiles_take(a)) {
         e = launch_router_tiles(m, st, a);
         if (e != cudaSuccess) return e;
     } else {

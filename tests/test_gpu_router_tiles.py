@@ -13,7 +13,7 @@ ACTS = [capi.DTYPE_FP32, capi.DTYPE_BF16, capi.DTYPE_FP16]
 
 
 def make(bits, act, d, ne, T, **kw):
-    cfg = small_config(d=d, num_experts=ne, top_k=8, act_dtype=act, router_weight_bits=bits, max_tokens=T, **kw)
+    cfg = small_config(d=d, num_experts=ne, top_k=min(8, ne), act_dtype=act, router_weight_bits=bits, max_tokens=T, **kw)
     layer = Layer(cfg, router_sigma=0.05, device_fill=True)
     x = inputs(T, d, seed=T)
     return layer, x.astype(np.float16).astype(np.float32) if act == capi.DTYPE_FP16 else x
@@ -22,7 +22,8 @@ def make(bits, act, d, ne, T, **kw):
 # tiles of 4 x 8 up to 96 Ki logits (9, 77, 383 rows), of 8 x 8 (fp32 activations) or 8 x 16 beyond; 1,100 rows: above 256 Ki
 @pytest.mark.parametrize("act", ACTS)
 @pytest.mark.parametrize("bits", [0, 8, 4])
-@pytest.mark.parametrize("d,ne,T", [(320, 250, 9), (2880, 31, 77), (64, 256, 383), (192, 256, 401), (320, 250, 1100)])
+@pytest.mark.parametrize("d,ne,T", [(320, 250, 9), (2880, 31, 77), (64, 256, 383), (192, 256, 401), (320, 250, 1100),
+                                    (2048, 5, 64), (2048, 16, 33), (2304, 7, 12)])   # (rows of few experts: by a warp each)
 def test_ids_and_weights_are_the_oracles(cuda_device, bits, act, d, ne, T):
     layer, x = make(bits, act, d, ne, T)
     ids, w, gate = layer.route(to_act_tensor(x, act, layer.device))
