@@ -38,10 +38,10 @@ def test_ids_and_weights_are_the_oracles(cuda_device, bits, act, d, ne, T):
 
 
 @pytest.mark.parametrize("act", ACTS)
-@pytest.mark.parametrize("bits", [0, 8])
+@pytest.mark.parametrize("bits", [0, 8, 4])
 def test_strides_column_scales_and_values_that_are_no_numbers(cuda_device, bits, act):
     """Rows a stride apart with a scale per column, NaN, infinities and zeros among them: the tiles (a stride of whole 16 bytes)
-    and the kernel of a warp per expert row (any other) give the same."""
+    and the kernel of a warp per expert row (any other stride of 16-bit rows, and eight rows at a time) give the same."""
     d, ne, T = 192, 40, 70
     layer, x = make(bits, act, d, ne, T)
     x[3, 17] = np.nan
@@ -54,10 +54,11 @@ def test_strides_column_scales_and_values_that_are_no_numbers(cuda_device, bits,
         wide = np.full((T, d + pad), 3.0, dtype=np.float32)
         wide[:, :d] = x
         got.append(layer.route(to_act_tensor(wide, act, layer.device), stride=d + pad))
-    assert act == capi.DTYPE_FP32 or (d + 4) * 2 % 16 != 0
+    assert act == capi.DTYPE_FP32 or (d + 4) * 2 % 16 != 0   # (every stride of fp32 rows is whole 16 bytes)
     for a, b in zip(*got):
         assert torch.equal(a.view(torch.int32), b.view(torch.int32))
-    few = layer.route(to_act_tensor(x[8:16], act, layer.device))
-    for a, b in zip(few, got[0]):
-        assert torch.equal(a.view(torch.int32), b[8:16].view(torch.int32))
+    for t0 in [*range(0, T - 8, 8), T - 8]:
+        few = layer.route(to_act_tensor(x[t0:t0 + 8], act, layer.device))
+        for a, b in zip(few, got[0]):
+            assert torch.equal(a.view(torch.int32), b[t0:t0 + 8].view(torch.int32))
     layer.close()
