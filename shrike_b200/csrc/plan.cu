@@ -5,9 +5,11 @@
 // a block, and the activation rows are copied to the fp16 operand layout.
 //
 // Prefill: PrefillMoEGrouping.groupTokenExpertPairs
-// (PrefillMoEGrouping.swift:269-370) as a three-step counting sort by expert
-// id that keeps (token, rank) order inside an expert, in place of the host
-// sort the reference runs between two GPU syncs (RealForwardRunner.swift:4305).
+// (PrefillMoEGrouping.swift:269-370) as a counting sort by expert id that
+// keeps (token, rank) order inside an expert, in place of the host sort the
+// reference runs between two GPU syncs (RealForwardRunner.swift:4305): three
+// launches for the grouping as a call of its own, one for a prefill call,
+// whose rows are placed where they are converted (prefill.cu).
 #include "plan.cuh"
 
 namespace shrike {
@@ -88,6 +90,30 @@ cudaError_t launch_decode_plan(const shrike_moe* m, cudaStream_t st, const uint3
 
 using GroupBits = uint32_t[SHRIKE_MAX_EXPERTS][kGroupTokens / 32];
 
+// Row tl of the block names expert e. False: there is no such expert.
+__device__ __forceinline__ bool name_expert(GroupBits& named, uint32_t e, uint32_t ne, uint32_t tl, uint32_t* status) {
+    if (e >= ne) {
+        // out of range: the pair is dropped and reported (0xffffffff is the expert-parallel layer's
+        // "this pick lives on another rank" and is dropped silently)
+        if (e != 0xffffffffu) report_status(status, kStatusBadIndex);
+        return false;
+    }
+    // a row that names one expert twice (no top-k router does) is counted once and reported
+    const uint32_t bit = 1u << (tl & 31);
+    if (atomicOr(&named[e][tl >> 5], bit) & bit) report_status(status, kStatusBadIndex);
+    return true;
+}
+
+// The block's rows of each expert (block_hist: [block][expert]).
+__device__ __forceinline__ void count_rows(const GroupBits& bits, uint32_t ne, uint32_t* block_hist) {
+    for (uint32_t e = threadIdx.x; e < ne; e += blockDim.x) {
+        uint32_t c = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kGroupTokens / 32; ++w) c += __popc(bits[e][w]);
+        block_hist[(size_t)blockIdx.x * ne + e] = c;
+    }
+}
+
 // Step 1: per block, a bitmap of the rows that chose each expert; writes the per-(block, expert) counts.
 __global__ void __launch_bounds__(256)
 group_hist_kernel(const uint32_t* __restrict__ ids, uint32_t T, uint32_t top_k, uint32_t ne,
@@ -101,26 +127,10 @@ group_hist_kernel(const uint32_t* __restrict__ ids, uint32_t T, uint32_t top_k, 
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < kGroupTokens * top_k; i += blockDim.x) {
         const uint32_t tl = i / top_k, t = t0 + tl;
-        if (t < T) {
-            const uint32_t e = ids[(size_t)t * top_k + (i - tl * top_k)];
-            if (e < ne) {
-                // a row that names one expert twice (no top-k router does) is counted once and reported
-                const uint32_t bit = 1u << (tl & 31);
-                if (atomicOr(&bits[e][tl >> 5], bit) & bit) report_status(status, kStatusBadIndex);
-            } else if (e != 0xffffffffu) {
-                // out of range: the pair is dropped and reported (0xffffffff is the expert-parallel layer's
-                // "this pick lives on another rank" and is dropped silently)
-                report_status(status, kStatusBadIndex);
-            }
-        }
+        if (t < T) name_expert(bits, ids[(size_t)t * top_k + (i - tl * top_k)], ne, tl, status);
     }
     __syncthreads();
-    for (uint32_t e = threadIdx.x; e < ne; e += blockDim.x) {
-        uint32_t c = 0;
-#pragma unroll
-        for (int w = 0; w < (int)(kGroupTokens / 32); ++w) c += __popc(bits[e][w]);
-        block_hist[(size_t)blockIdx.x * ne + e] = c;
-    }
+    count_rows(bits, ne, block_hist);
 }
 
 // Rows before row tl of the block that chose expert e.
@@ -277,34 +287,23 @@ group_plan_kernel(const uint32_t* __restrict__ ids, uint32_t T, uint32_t top_k, 
     __syncthreads();
 #pragma unroll
     for (uint32_t j = 0; j < N; ++j) {
-        const uint32_t tl = (j * 256 + threadIdx.x) / top_k, bit = 1u << (tl & 31);
-        if (e[j] < ne) {
-            // a row that names one expert twice (no top-k router does) is counted once and reported
-            if (atomicOr(&named[e[j]][tl >> 5], bit) & bit) report_status(status, kStatusBadIndex);
-            if (!ready) cell[j] = SHRIKE_SLOT_MISS;
-            if (cell[j] != SHRIKE_SLOT_MISS && cell[j] >= pool_cells) {
-                report_status(status, kStatusBadIndex);
-                cell[j] = SHRIKE_SLOT_MISS;
-            }
-            if (cell[j] != SHRIKE_SLOT_MISS) {
-                atomicOr(&bits[e[j]][tl >> 5], bit);
-                slot_of_expert[e[j]] = cell[j];   // (of an expert with two cells either)
-            }
-        } else if (e[j] != 0xffffffffu) {
-            report_status(status, kStatusBadIndex);   // out of range: dropped (0xffffffff: the pick lives on another rank)
+        const uint32_t tl = (j * 256 + threadIdx.x) / top_k;
+        if (!name_expert(named, e[j], ne, tl, status) || !ready) cell[j] = SHRIKE_SLOT_MISS;
+        if (cell[j] != SHRIKE_SLOT_MISS && cell[j] >= pool_cells) {
+            report_status(status, kStatusBadIndex);
+            cell[j] = SHRIKE_SLOT_MISS;
+        }
+        if (cell[j] != SHRIKE_SLOT_MISS) {
+            atomicOr(&bits[e[j]][tl >> 5], 1u << (tl & 31));
+            slot_of_expert[e[j]] = cell[j];   // (of an expert with two cells either)
         }
     }
     __syncthreads();
-    if (threadIdx.x < ne) {
-        uint32_t c = 0;
-#pragma unroll
-        for (uint32_t w = 0; w < kGroupTokens / 32; ++w) c += __popc(bits[threadIdx.x][w]);
-        block_hist[(size_t)blockIdx.x * ne + threadIdx.x] = c;
-    }
+    count_rows(bits, ne, block_hist);
 #pragma unroll
     for (uint32_t j = 0; j < N; ++j) {
         const uint32_t i = j * 256 + threadIdx.x;
-        if (i < n) rank_of_pair[(size_t)t0 * top_k + i] = e[j] >= ne || cell[j] == SHRIKE_SLOT_MISS ? 0xffffffffu : rows_before(bits, e[j], i / top_k);
+        if (i < n) rank_of_pair[(size_t)t0 * top_k + i] = cell[j] == SHRIKE_SLOT_MISS ? 0xffffffffu : rows_before(bits, e[j], i / top_k);
     }
     __threadfence();
     __syncthreads();

@@ -150,6 +150,13 @@ def test_experts_with_pairs_that_miss(cuda_device, monkeypatch, path, T):
             assert err.value.code == capi.ERANGE
         assert rel_l2(out[:T].cpu().numpy(), y_ref) <= 1e-3
         assert (out[T:] == 7.0).all()
+    ids[5, 1] = ids[5, 0]   # a row that names an expert twice is reported, whatever its slots are
+    for cells in ((-1, -1), (-1, 2), (2, -1), (2, 2)):
+        slots[5, 0], slots[5, 1] = cells
+        layer.moe.encode_prefill(layer.pool, layer.offsets, ids, slots, w, x_dev, out[:T], None, layer.shared)
+        with pytest.raises(ShrikeError) as err:
+            layer.moe.status()
+        assert err.value.code == capi.ERANGE
     layer.close()
 
 
