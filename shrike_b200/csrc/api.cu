@@ -1058,9 +1058,9 @@ int shrike_ep_set_wait_polls(shrike_ep* ep, uint32_t wait_polls) {
 
 // Whether a forward has nobody to exchange rows with and can be the home handle's own layer call, which knows the number of its rows
 // on the host, keeps them where they are and runs on one stream. What that call does not take goes the general way: formats of the
-// routed experts that the home handle does not describe, one row whose y is not 16-byte aligned, y across x. Through the exchange buffer,
-// in some twenty launches, and as the layer call, us: 256 experts of 2048 x 512 int4, 4 rows 119 / 36; 32 of 2880 x 2880 int4, 3 rows 164 / 76,
-// 144 rows 396 / 222; 256 of 2304 x 1024 int8, 39 rows 348 / 199, 2064 rows 697 / 630.
+// routed experts that the home handle does not describe, one row whose y or hidden is not 16-byte aligned, y across x. Through the
+// exchange buffer, in some twenty launches, and as the layer call, calls one after the other, us: 256 experts of 2048 x 512 int4, 4 rows 104 / 34; 32 of
+// 2880 x 2880 int4, 3 rows 152 / 72, 144 rows 248 / 195; 256 of 2304 x 1024 int8, 39 rows 318 / 195, 2064 rows 662 / 613.
 static bool ep_alone(const shrike_ep* ep, uint32_t T, const void* x, const void* y, const void* hidden) {
     const shrike_moe_config &c = ep->home->cfg, &r = ep->routed->cfg;
     if (ep->world != 1 || T == 0 || r.weight_bits != c.weight_bits || r.group_size != c.group_size || r.meta_dtype != c.meta_dtype) return false;

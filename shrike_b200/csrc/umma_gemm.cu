@@ -160,7 +160,7 @@ __device__ __forceinline__ uint32_t umma_idesc(uint32_t n) {
 
 // 8 packed nibbles -> 8 fp16 weights in operand order {0,4,1,5,2,6,3,7}; 4 bytes -> 4 fp16 in order. A byte q in a half's low bits is
 // the fp16 number q x 2^-24, below the normal range and exact: it is multiplied as it lies there, by a scale of 2^24 times the
-// group's, with one rounding in all and no subtraction of an offset (256 experts of 2304 x 1024, 2064 rows, 710 -> 690 us a call).
+// group's, with one rounding in all and no subtraction of an offset (256 experts of 2304 x 1024, 2064 rows, 707 -> 695 us a call).
 // (Nibbles the same way, at bit 4: no faster, 333 rows 177 us with the subtractions, 180 without.)
 template <int BITS>
 __device__ __forceinline__ void dequant_word(uint32_t w, uint32_t s2, uint32_t z2, uint32_t* out) {
