@@ -7,7 +7,8 @@ combine.
 exchange="peer" (default): the whole layer is `shrike_ep_forward` of the C ABI. Rows travel as plain stores
 into the destination rank's exchange buffer over NVLink (opened through CUDA IPC handles that this class
 passes around with `torch.distributed.all_gather_object`), only the routed rows move, and the shared expert
-runs on a second stream beside the exchange. torch.distributed is used once, to hand the 64-byte tokens round.
+runs on a second stream beside the exchange. A rank alone runs the home handle's layer call where that takes the
+operands (include/shrike_b200.h says which it does not). torch.distributed is used once, to hand the 64-byte tokens round.
 
 exchange="nccl": the earlier form, kept as the checker of the peer path -- the library's pack / local-slots /
 combine kernels around fixed-capacity `all_to_all_single` calls over the process group.
