@@ -1060,11 +1060,14 @@ int shrike_ep_set_wait_polls(shrike_ep* ep, uint32_t wait_polls) {
 // on the host, keeps them where they are and runs on one stream. What that call does not take goes the general way: formats of the
 // routed experts that the home handle does not describe, one row whose y or hidden is not 16-byte aligned, y across x. Through the
 // exchange buffer, in some twenty launches, and as the layer call, calls one after the other, us: 256 experts of 2048 x 512 int4, 4 rows 104 / 34; 32 of
-// 2880 x 2880 int4, 3 rows 152 / 72, 144 rows 248 / 195; 256 of 2304 x 1024 int8, 39 rows 318 / 195, 2064 rows 662 / 613.
+// 2880 x 2880 int4, 3 rows 152 / 72, 144 rows 248 / 195; 256 of 2304 x 1024 int8, 39 rows 318 / 195, 2064 rows 662 / 613. Nor is it the faster way for more than 48 rows of shapes that end up on
+// the per-tile kernels, on a home handle without prefill operands (32 experts of 2880 x 2880 int4 in groups of 64, 64 rows, picks uniform or by Zipf(1.1): 235 /
+// 343, 229 / 392; 256 of 2048 x 576 int4 228 / 244, 133 / 152; at 48 rows 210 / 203, 131 / 119 the last).
 static bool ep_alone(const shrike_ep* ep, uint32_t T, const void* x, const void* y, const void* hidden) {
     const shrike_moe_config &c = ep->home->cfg, &r = ep->routed->cfg;
     if (ep->world != 1 || T == 0 || r.weight_bits != c.weight_bits || r.group_size != c.group_size || r.meta_dtype != c.meta_dtype) return false;
     if (T == 1 && (!aligned_to(y, 16) || !aligned_to(hidden, 16))) return false;
+    if (T > 48 && T <= SHRIKE_MAX_DECODE_TOKENS && !ep->home->ws.xs && !stream_takes_shape(ep->home)) return false;
     const uintptr_t x0 = (uintptr_t)x, y0 = (uintptr_t)y, elems = (uintptr_t)T * c.d;
     return x0 == y0 || x0 + elems * act_bytes(c.act_dtype) <= y0 || y0 + elems * act_bytes(c.y_dtype) <= x0;
 }

@@ -1119,6 +1119,12 @@ cudaError_t launch_stream_m(const shrike_moe* m, cudaStream_t st, const StreamAr
 
 }  // namespace
 
+// Whether calls of some rows run here, pools of single-cell chunks and parts of a GPU aside.
+bool stream_takes_shape(const shrike_moe* m) {
+    StreamGeom g;
+    return stream_geometry(m->cfg, m->smem_optin, g);
+}
+
 size_t stream_parts_bytes(const shrike_moe_config& c) {
     const size_t T = std::min(c.max_tokens, (uint32_t)SHRIKE_MAX_DECODE_TOKENS);
     return T * (c.top_k + (c.has_shared ? 1u : 0u)) * c.d * 4;

@@ -213,6 +213,7 @@ cudaError_t launch_after(const shrike_moe* m, cudaStream_t st, void (*k)(P...), 
 struct RouterArgs;
 cudaError_t launch_expert_stream(const shrike_moe* m, cudaStream_t st, const ExpertArgs& ea, uint32_t T, uint32_t n_shared,
                                  void* y, void* hidden, bool pdl, uint32_t phases, const RouterArgs* route = nullptr);
+bool stream_takes_shape(const shrike_moe* m);
 size_t stream_parts_bytes(const shrike_moe_config& c);
 size_t stream_done_bytes();
 // synth.cu

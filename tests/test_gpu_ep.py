@@ -580,6 +580,24 @@ def test_a_rank_alone_gives_what_the_exchange_gives(cuda_device, T, shared):
     layer.close()
 
 
+@pytest.mark.parametrize("T,exchanges", [(48, 0), (49, 1), (64, 1)])
+def test_more_than_48_rows_of_odd_groups_exchange(cuda_device, T, exchanges):
+    """An odd number of groups, a home handle of up to 64 rows: per-tile kernels up to 48 rows, beyond them the exchange, whose experts
+    run on the grouped GEMM."""
+    from shrike_b200.moe import RouterOperands
+    cfg = dataclasses.replace(_config(), f=192, shared_f=192)
+    x, router = _problem(T, cfg)
+    _, _, y_ref = _oracle(cfg, x, router, 33)
+    layer = _build_layer(cfg, 0, 1, 64, 33, "peer")
+    xd, y = _rows(cfg, x, layer.dev, across=False)
+    layer.forward(RouterOperands(weights=torch.from_numpy(router).to(layer.dev)), xd, y)
+    layer.status()
+    assert _exchanges(layer) == exchanges
+    assert np.linalg.norm(y.cpu().numpy() - y_ref) / np.linalg.norm(y_ref) <= 1e-3
+    assert layer.last_counts() == ([T], T, 0)
+    layer.close()
+
+
 def _build_alone(cfg, T, seed):
     import fixtures as fx
     from shrike_b200.ep import ExpertParallelLayer
