@@ -1,7 +1,6 @@
 """Expert parallelism on GPUs: the expert-parallel layer against the oracle -- over peer memory (the C ABI's
 shrike_ep_*) and over NCCL all-to-all (the checker) -- with one rank always, with two ranks when the box has
-two GPUs. (One rank alone exchanges with itself where its layer call does not take the operands, such as a y that begins inside
-x; most tests of one rank hand in such rows.) The pack kernel against the numpy protocol; the full-size mixed batch; and a wait that runs out
+two GPUs; the pack kernel against the numpy protocol; the full-size mixed batch; and a wait that runs out
 because nothing ever writes its word (a peer that never answers, made on the host)."""
 import dataclasses
 import os
@@ -66,43 +65,6 @@ def _build_layer(cfg, rank, world, per, seed, exchange, group=None):
     return layer
 
 
-def _view(address, nbytes):
-    """The device memory at an address, as a byte tensor over it."""
-    class Memory:
-        __cuda_array_interface__ = dict(shape=(nbytes,), typestr="|u1", data=(address, False), version=3)
-    return torch.as_tensor(Memory(), device="cuda")
-
-
-def _exchange_areas(cfg, world, cap, buf):
-    """A rank's exchange buffer by its areas, each a multiple of 256 bytes: rows, ids and weights received from every rank,
-    partial rows returned, and the two arrival words."""
-    at, areas = 0, []
-    for shape, dtype in (((world, cap, cfg.d), cfg.torch_act_dtype), ((world, cap, cfg.top_k), torch.int32),
-                         ((world, cap, cfg.top_k), torch.float32), ((world, cap, cfg.d), cfg.torch_y_dtype),
-                         ((world,), torch.int64), ((world,), torch.int64)):
-        n = int(np.prod(shape)) * torch.empty((), dtype=dtype).element_size()
-        areas.append(buf[at:at + n].view(dtype).view(shape))
-        at = (at + n + 255) // 256 * 256
-    assert at == buf.numel()
-    return areas
-
-
-def _exchanges(layer):
-    """Forwards that went through the exchange buffer: the epoch of this rank's arrival word for itself."""
-    torch.cuda.synchronize()
-    return int(_exchange_areas(layer.cfg, layer.world, layer.cap, _view(*layer.buffer()))[4][layer.rank]) >> 32
-
-
-def _rows(cfg, x, dev, across, skip=0):
-    """x on the device and y: rows of their own, or beginning 16 bytes into x, `skip` elements further on."""
-    n_x, n_y = x.size * (4 if cfg.torch_act_dtype == torch.float32 else 2), x.size * (4 if cfg.torch_y_dtype == torch.float32 else 2)
-    buf = torch.zeros(n_x + n_y + 64, dtype=torch.uint8, device=dev)
-    at = (16 if across else (n_x + 15) // 16 * 16) + skip * (n_y // x.size)
-    xd, y = buf[:n_x].view(cfg.torch_act_dtype).view(x.shape), buf[at:at + n_y].view(cfg.torch_y_dtype).view(x.shape)
-    xd.copy_(torch.from_numpy(x))
-    return xd, y
-
-
 def _run_rank(rank, world, port, T, seed, out_path, exchange="peer"):
     """One EP rank: builds its shard, runs the layer twice on its rows, saves y, hidden and the routing."""
     import torch.distributed as dist
@@ -120,17 +82,15 @@ def _run_rank(rank, world, port, T, seed, out_path, exchange="peer"):
     layer = _build_layer(cfg, rank, world, per, seed, exchange, group)
     dev = layer.dev
     ops = RouterOperands(weights=torch.from_numpy(router).to(dev))
-    mine = x[rank * per:(rank + 1) * per].copy()
-    xl, y = _rows(cfg, mine, dev, across=world == 1 and exchange == "peer")
+    xl = torch.from_numpy(x[rank * per:(rank + 1) * per].copy()).to(dev)
+    y = torch.empty_like(xl)
     h = xl.clone()
     for _ in range(2):  # a second pass reuses every buffer
-        xl.copy_(torch.from_numpy(mine))
         h.copy_(xl)
         layer.forward(ops, xl, y, h)
     layer.status()
-    assert exchange != "peer" or _exchanges(layer) == 2
     np.save(out_path, np.stack([y.cpu().numpy(), h.cpu().numpy()]))
-    ids, _ = layer.routing(ops, torch.from_numpy(mine).to(dev))
+    ids, _ = layer.routing(ops, xl)
     np.save(out_path + ".ids.npy", ids.cpu().numpy().astype(np.uint32))
     if exchange == "peer":
         sent, received, nbytes = layer.last_counts()
@@ -181,7 +141,7 @@ def _edges(call):
 
 
 def test_handles_launch_as_before_once_a_forward_is_over(cuda_device):
-    """An expert-parallel forward that exchanges launches its kernels without overlap of successive ones; the handles' own prefill
+    """An expert-parallel forward launches its kernels without overlap of successive ones; the handles' own prefill
     calls have it before the layer is made, after a forward, and after the layer has gone."""
     from shrike_b200.moe import RouterOperands
     cfg, T = _config(), 96
@@ -199,13 +159,9 @@ def test_handles_launch_as_before_once_a_forward_is_over(cuda_device):
 
     prefill()
     before = _edges(prefill)
-    x_in, y_across = _rows(cfg, x_np, layer.dev, across=True)
-    layer.forward(ops, x_in, y_across)
+    layer.forward(ops, x, y)
     layer.status()
-    assert _exchanges(layer) == 1
     assert before[1] > 0 and _edges(prefill) == before
-    edges = _edges(lambda: layer.forward(ops, x_in, y_across))   # (looked at, never run)
-    assert edges[0] > 0 and edges[1] == 0 and _edges(prefill) == before
     layer._lib.shrike_ep_destroy(layer._ep)
     layer._ep = None
     assert _edges(prefill) == before
@@ -270,12 +226,10 @@ def test_cuda_dispatch_matches_the_protocol(cuda_device):
     moe.close()
 
 
-@pytest.mark.parametrize("across", [False, True])
-def test_full_size_mixed_batch_on_one_rank(cuda_device, across):
+def test_full_size_mixed_batch_on_one_rank(cuda_device):
     """The expert-parallel workload at its full per-rank size: 16 decode rows + one 2048-row prefill chunk of the
     Kimi-Linear shape (int8 g64, 256 experts top-8 sigmoid with a selection bias, shared expert), bf16 rows in,
-    fp32 rows out, every expert on this rank: as a layer call, and (y across x) through the exchange buffer; sampled rows against
-    the oracle."""
+    fp32 rows out, through the peer-memory layer with every expert on this rank; sampled rows against the oracle."""
     import fixtures as fx
     import oracle_lib as O
     from shrike_b200 import capi
@@ -295,11 +249,11 @@ def test_full_size_mixed_batch_on_one_rank(cuda_device, across):
     correction = rng.uniform(-0.1, 0.1, cfg.num_experts).astype(np.float32)
     xr = fx.round_bf16(rng.normal(0, 1, (rows, cfg.d)).astype(np.float32))
     ops = RouterOperands(weights=torch.from_numpy(router).to(dev), logit_bias=bf16_tensor(correction, dev))
-    x, y = _rows(cfg, xr, dev, across)
+    x = torch.from_numpy(xr).to(torch.bfloat16).to(dev)
+    y = torch.empty((rows, cfg.d), dtype=torch.float32, device=dev)
     layer.forward(ops, x, y)
     layer.status()
-    assert _exchanges(layer) == across
-    ids, w = layer.routing(ops, torch.from_numpy(xr).to(torch.bfloat16).to(dev))
+    ids, w = layer.routing(ops, x)
     ids, w = ids.cpu().numpy().astype(np.uint32), w.cpu().numpy()
     assert all(len(set(r)) == cfg.top_k for r in ids[:64].tolist())
     sample = np.sort(rng.choice(rows, 40, replace=False))
@@ -439,19 +393,40 @@ def test_output_rows_that_are_not_whole_vectors(cuda_device, dtype):
     x, router = _problem(40, cfg)
     layer = _build_layer(cfg, 0, 1, 40, 9, "peer")
     ops = RouterOperands(weights=torch.from_numpy(router).to(layer.dev))
+    xl = torch.from_numpy(x).to(layer.dev).to(cfg.torch_act_dtype)
     got = []
     for skip in (0, 1):
-        xl, y = _rows(cfg, x, layer.dev, across=True, skip=skip)
+        y = torch.zeros(xl.numel() + 8, dtype=cfg.torch_y_dtype, device=layer.dev)[skip:skip + xl.numel()].view(xl.shape)
         h = torch.zeros(xl.numel() + 8, dtype=xl.dtype, device=layer.dev)[skip:skip + xl.numel()].view(xl.shape).copy_(xl)
         layer.forward(ops, xl, y, h)
         layer.status()
         got.append((y.float(), h.float()))
-    assert _exchanges(layer) == 2
     layer.close()
     ulp = 2.0 ** (-22 if dtype == "fp32" else -7)
     assert not torch.equal(got[0][0], torch.zeros_like(got[0][0]))
     for a, b in zip(*got):
         assert ((a - b).abs() <= 2 * ulp * a.abs() + 1e-6 * a.abs().max()).all()
+
+
+def _view(address, nbytes):
+    """The device memory at an address, as a byte tensor over it."""
+    class Memory:
+        __cuda_array_interface__ = dict(shape=(nbytes,), typestr="|u1", data=(address, False), version=3)
+    return torch.as_tensor(Memory(), device="cuda")
+
+
+def _exchange_areas(cfg, world, cap, buf):
+    """A rank's exchange buffer by its areas, each a multiple of 256 bytes: rows, ids and weights received from every rank,
+    partial rows returned, and the two arrival words."""
+    at, areas = 0, []
+    for shape, dtype in (((world, cap, cfg.d), cfg.torch_act_dtype), ((world, cap, cfg.top_k), torch.int32),
+                         ((world, cap, cfg.top_k), torch.float32), ((world, cap, cfg.d), cfg.torch_y_dtype),
+                         ((world,), torch.int64), ((world,), torch.int64)):
+        n = int(np.prod(shape)) * torch.empty((), dtype=dtype).element_size()
+        areas.append(buf[at:at + n].view(dtype).view(shape))
+        at = (at + n + 255) // 256 * 256
+    assert at == buf.numel()
+    return areas
 
 
 @pytest.mark.parametrize("T,dtype", [(1, "fp32"), (37, "fp32"), (37, "bf16"), (90, "bf16")])
@@ -549,8 +524,8 @@ def test_combine_matches_the_protocol(cuda_device, T, world, skip):
 @pytest.mark.parametrize("T", [1, 2, 64, 65, 200])
 @pytest.mark.parametrize("shared", [True, False])
 def test_a_rank_alone_gives_what_the_exchange_gives(cuda_device, T, shared):
-    """A world of one runs the home handle's layer call; rows whose y begins inside x, and one row whose y or hidden is not 16-byte
-    aligned, take the general way through the exchange buffer. Both against the oracle, the residual and the counters."""
+    """A world of one runs the home handle's layer call; rows whose y begins inside x take the general way through the exchange
+    buffer. Both against the oracle, the residual and the counters."""
     from shrike_b200.moe import RouterOperands
     seed = 31
     cfg = dataclasses.replace(_config(), **({} if shared else dict(has_shared=False, shared_f=0)))
@@ -564,37 +539,17 @@ def test_a_rank_alone_gives_what_the_exchange_gives(cuda_device, T, shared):
                             x, ids, w)
     layer = _build_alone(cfg, T, seed)
     ops = RouterOperands(weights=torch.from_numpy(router).to(layer.dev))
-    exchanges = 0
-    for across, skip_y, skip_h in ((False, 0, 0), (True, 0, 0), (False, 1, 0), (False, 0, 1)):
-        xd, y = _rows(cfg, x, layer.dev, across, skip_y)
-        h = torch.zeros(x.size + 8, device=layer.dev)[skip_h:skip_h + x.size].view(x.shape)
-        h.copy_(torch.from_numpy(x))
+    for across in (False, True):
+        buf = torch.zeros((2 * T + 1, cfg.d), device=layer.dev)
+        xd, y = buf[:T], buf[1:T + 1] if across else buf[T:2 * T]
+        xd.copy_(torch.from_numpy(x))
+        h = torch.from_numpy(x).to(layer.dev)
         layer.forward(ops, xd, y, h)
         layer.status()
-        exchanges += across or (T == 1 and skip_y + skip_h > 0)
-        assert _exchanges(layer) == exchanges
         got = y.cpu().numpy()
         assert np.linalg.norm(got - y_ref) / np.linalg.norm(y_ref) <= 1e-3
         assert np.abs(h.cpu().numpy() - (x + got)).max() <= 1e-5 * np.abs(x).max()
         assert layer.last_counts() == ([T], T, 0)
-    layer.close()
-
-
-@pytest.mark.parametrize("T,exchanges", [(48, 0), (49, 1), (64, 1)])
-def test_more_than_48_rows_of_odd_groups_exchange(cuda_device, T, exchanges):
-    """An odd number of groups, a home handle of up to 64 rows: per-tile kernels up to 48 rows, beyond them the exchange, whose experts
-    run on the grouped GEMM."""
-    from shrike_b200.moe import RouterOperands
-    cfg = dataclasses.replace(_config(), f=192, shared_f=192)
-    x, router = _problem(T, cfg)
-    _, _, y_ref = _oracle(cfg, x, router, 33)
-    layer = _build_layer(cfg, 0, 1, 64, 33, "peer")
-    xd, y = _rows(cfg, x, layer.dev, across=False)
-    layer.forward(RouterOperands(weights=torch.from_numpy(router).to(layer.dev)), xd, y)
-    layer.status()
-    assert _exchanges(layer) == exchanges
-    assert np.linalg.norm(y.cpu().numpy() - y_ref) / np.linalg.norm(y_ref) <= 1e-3
-    assert layer.last_counts() == ([T], T, 0)
     layer.close()
 
 
@@ -630,4 +585,108 @@ def test_a_replayed_forward_counts_its_own_rows(cuda_device):
     graph.replay()
     torch.cuda.synchronize()
     assert layer.last_counts()[:2] == ([8], 8) and torch.equal(y, want)
+    layer.close()
+
+
+def _exchanges(layer):
+    """Forwards that went through the exchange buffer: the epoch of this rank's arrival word for itself."""
+    torch.cuda.synchronize()
+    return int(_exchange_areas(layer.cfg, layer.world, layer.cap, _view(*layer.buffer()))[4][layer.rank]) >> 32
+
+
+def _rows(cfg, x, across, skip=0):
+    """x, and y: rows of their own, or beginning 16 bytes into x, `skip` elements further on."""
+    esz = torch.empty((), dtype=cfg.torch_y_dtype).element_size()
+    n_x, n_y = x.numel() * x.element_size(), x.numel() * esz
+    buf = torch.zeros(n_x + n_y + 64, dtype=torch.uint8, device=x.device)
+    at = (16 if across else (n_x + 15) // 16 * 16) + skip * esz
+    xd, y = buf[:n_x].view(x.dtype).view(x.shape), buf[at:at + n_y].view(cfg.torch_y_dtype).view(x.shape)
+    return xd.copy_(x), y
+
+
+@pytest.fixture
+def exchanged(monkeypatch):
+    """A world of one exchanges with itself where its layer call does not take the rows: every forward's y begins inside x
+    here, as far from a whole 16 bytes as the test's own."""
+    from shrike_b200.ep import ExpertParallelLayer
+    inner = ExpertParallelLayer.forward
+
+    def forward(self, router, x, y, hidden=None):
+        xd, yd = _rows(self.cfg, x, True, y.data_ptr() % 16 // y.element_size())
+        before = _exchanges(self)
+        inner(self, router, xd, yd, hidden)
+        y.copy_(yd)
+        assert _exchanges(self) == before + 1
+    monkeypatch.setattr(ExpertParallelLayer, "forward", forward)
+    return inner
+
+
+@pytest.mark.parametrize("T", [8, 96])
+def test_single_rank_through_the_exchange_buffer(cuda_device, tmp_path, exchanged, T):
+    test_single_rank_expert_parallel_layer(cuda_device, tmp_path, T, "peer")
+
+
+def test_full_size_mixed_batch_through_the_exchange_buffer(cuda_device, exchanged):
+    test_full_size_mixed_batch_on_one_rank(cuda_device)
+
+
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+def test_exchanged_output_rows_that_are_not_whole_vectors(cuda_device, exchanged, dtype):
+    test_output_rows_that_are_not_whole_vectors(cuda_device, dtype)
+
+
+def test_handles_launch_as_before_once_rows_were_exchanged(cuda_device, exchanged):
+    """The forward that exchanges sets the handles' launches itself, and puts them back."""
+    from shrike_b200.moe import RouterOperands
+    test_handles_launch_as_before_once_a_forward_is_over(cuda_device)
+    cfg, T = _config(), 96
+    layer = _build_layer(cfg, 0, 1, T, 3, "peer")
+    x, router = _problem(T, cfg)
+    xd, y = _rows(cfg, torch.from_numpy(x).cuda(), True)
+    ops = RouterOperands(weights=torch.from_numpy(router).cuda())
+    edges = _edges(lambda: exchanged(layer, ops, xd, y))   # (looked at, never run)
+    assert edges[0] > 0 and edges[1] == 0
+    layer.close()
+
+
+@pytest.mark.parametrize("T", [1, 2, 64, 65, 200])
+def test_which_rows_a_rank_alone_exchanges(cuda_device, T):
+    """Those whose y begins inside x, and one row whose y or hidden is not 16-byte aligned; the same rows either way."""
+    from shrike_b200.moe import RouterOperands
+    cfg = _config()
+    x, router = _problem(T, cfg)
+    _, _, y_ref = _oracle(cfg, x, router, 31)
+    layer = _build_layer(cfg, 0, 1, T, 31, "peer")
+    ops = RouterOperands(weights=torch.from_numpy(router).to(layer.dev))
+    exchanges = 0
+    for across, skip_y, skip_h in ((False, 0, 0), (True, 0, 0), (False, 1, 0), (False, 0, 1)):
+        xd, y = _rows(cfg, torch.from_numpy(x).to(layer.dev), across, skip_y)
+        h = torch.zeros(x.size + 8, device=layer.dev)[skip_h:skip_h + x.size].view(x.shape)
+        h.copy_(torch.from_numpy(x))
+        layer.forward(ops, xd, y, h)
+        layer.status()
+        exchanges += across or (T == 1 and skip_y + skip_h > 0)
+        assert _exchanges(layer) == exchanges
+        got = y.cpu().numpy()
+        assert np.linalg.norm(got - y_ref) / np.linalg.norm(y_ref) <= 1e-3
+        assert np.abs(h.cpu().numpy() - (x + got)).max() <= 1e-5 * np.abs(x).max()
+        assert layer.last_counts() == ([T], T, 0)
+    layer.close()
+
+
+@pytest.mark.parametrize("T,exchanges", [(48, 0), (49, 1), (64, 1)])
+def test_more_than_48_rows_of_odd_groups_exchange(cuda_device, T, exchanges):
+    """An odd number of groups, a home handle of up to 64 rows: per-tile kernels up to 48 rows, beyond them the exchange, whose experts
+    run on the grouped GEMM."""
+    from shrike_b200.moe import RouterOperands
+    cfg = dataclasses.replace(_config(), f=192, shared_f=192)
+    x, router = _problem(T, cfg)
+    _, _, y_ref = _oracle(cfg, x, router, 33)
+    layer = _build_layer(cfg, 0, 1, 64, 33, "peer")
+    xd, y = _rows(cfg, torch.from_numpy(x).to(layer.dev), False)
+    layer.forward(RouterOperands(weights=torch.from_numpy(router).to(layer.dev)), xd, y)
+    layer.status()
+    assert _exchanges(layer) == exchanges
+    assert np.linalg.norm(y.cpu().numpy() - y_ref) / np.linalg.norm(y_ref) <= 1e-3
+    assert layer.last_counts() == ([T], T, 0)
     layer.close()
