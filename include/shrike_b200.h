@@ -370,8 +370,9 @@ int shrike_ep_encode_combine(shrike_moe* moe, void* stream, const void* recv_y, 
  *                      `stream` alone, and that can be captured. It exchanges with itself, and is not capturable, when
  *                      there are no rows, when the routed experts' weight_bits, group_size or meta_dtype are not
  *                      `home`'s, when y overlaps x without beginning where x does, when one row's y or hidden is
- *                      not 16-byte aligned, and for 49 to 64 rows on a `home` of at most 64 whose shape the one-launch
- *                      decode kernels do not take.
+ *                      not 16-byte aligned, and for up to 64 rows of 4-bit experts where the layer call is the slower or the less exact
+ *                      one: behind a clamped SwiGLU in groups of 64, or of a shape that the one-launch decode kernels do not
+ *                      take; 49 to 64 rows of any such shape on a `home` of at most 64 rows.
  *                      A rank whose peer never arrives waits about a second per exchange, then the next
  *                      shrike_ep_status returns SHRIKE_ETIMEDOUT; the rows of that peer are missing from y.
  *   wait_polls         0 = the default limit (about one second); tests pass a small number. */

@@ -1060,14 +1060,23 @@ int shrike_ep_set_wait_polls(shrike_ep* ep, uint32_t wait_polls) {
 // on the host, keeps them where they are and runs on one stream. What that call does not take goes the general way: formats of the
 // routed experts that the home handle does not describe, one row whose y or hidden is not 16-byte aligned, y across x. Through the
 // exchange buffer, in some twenty launches, and as the layer call, calls one after the other, us: 256 experts of 2048 x 512 int4, 4 rows 104 / 34; 32 of
-// 2880 x 2880 int4, 3 rows 152 / 72, 144 rows 248 / 195; 256 of 2304 x 1024 int8, 39 rows 318 / 195, 2064 rows 662 / 613. Nor is it the faster way for more than 48 rows of shapes that end up on
-// the per-tile kernels, on a home handle without prefill operands (32 experts of 2880 x 2880 int4 in groups of 64, 64 rows, picks uniform or by Zipf(1.1): 235 /
-// 343, 229 / 392; 256 of 2048 x 576 int4 228 / 244, 133 / 152; at 48 rows 210 / 203, 131 / 119 the last).
+// 2880 x 2880 int4, 3 rows 152 / 72, 144 rows 248 / 195; 256 of 2304 x 1024 int8, 39 rows 318 / 195, 2064 rows 662 / 613.
+// Nor is it taken where up to 64 rows of nibbles would lose by it. The decode kernels sum (1024 + q) x, or (64 + q) x of every second nibble, and
+// take the offset's share away again: behind a clamped SwiGLU, whose products are of one sign, in groups of 64 or all with 1024 (the
+// per-tile kernels) they are further off than the grouped GEMM that the exchange's experts run on. Error against 64 bits, bf16 scales, GEMM and
+// decode kernels: 32 experts of 2880 x 2880, odd groups of 64, 1 row 7.3e-5 and 1.0e-4 (one launch), 17 rows 6.4e-5 and 1.5e-4 (per tile); 256 of 2048 x 512, groups of
+// 64, 8.5e-5 and 1.3e-4. In groups of 32 it is 6.1e-5 and 7.2e-5, 1.4e-4 and 1.1e-4 with fp16 scales; behind SiLU 2.0e-4 and 2.1e-4; of bytes 4.1e-4 and 2.1e-4. And from
+// 49 rows on the per-tile kernels are the slower ones, us: 32 experts of 2880 x 2880 in groups of 64, 64 rows 235 by the exchange and 367 by
+// the layer call, 256 of 2048 x 576 240 and 258.
 static bool ep_alone(const shrike_ep* ep, uint32_t T, const void* x, const void* y, const void* hidden) {
     const shrike_moe_config &c = ep->home->cfg, &r = ep->routed->cfg;
     if (ep->world != 1 || T == 0 || r.weight_bits != c.weight_bits || r.group_size != c.group_size || r.meta_dtype != c.meta_dtype) return false;
     if (T == 1 && (!aligned_to(y, 16) || !aligned_to(hidden, 16))) return false;
-    if (T > 48 && T <= SHRIKE_MAX_DECODE_TOKENS && !ep->home->ws.xs && !stream_takes_shape(ep->home)) return false;
+    const bool gemm = umma_supported(c) && !ep->routed->force_warp_mma;   // what the exchange's experts run on
+    const bool tiles = !(T == 1 ? ep->home->ws.fused_geom != nullptr : stream_takes_shape(ep->home));
+    if (gemm && c.weight_bits == 4 && T <= SHRIKE_MAX_DECODE_TOKENS && !(tiles && T > 48 && ep->home->ws.xs) &&
+        ((tiles && T > 48) || (c.activation == SHRIKE_ACT_CLAMPED_SWIGLU && (tiles || c.group_size == 64))))
+        return false;
     const uintptr_t x0 = (uintptr_t)x, y0 = (uintptr_t)y, elems = (uintptr_t)T * c.d;
     return x0 == y0 || x0 + elems * act_bytes(c.act_dtype) <= y0 || y0 + elems * act_bytes(c.y_dtype) <= x0;
 }
