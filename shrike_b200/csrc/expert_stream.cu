@@ -630,7 +630,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_stream_kernel(const __grid
     // The warps of a team share a row by whole pieces, or by halves of pieces of eight groups where rows end within a piece: of 12
     // pieces (2880 columns in groups of 32) eight warps have one or two, of 23 halves two or three. 32 experts of 2880 x 2880, 64 rows, us
     // over four layers: 960 by pieces, 848 by halves (970 by pieces with initial values of 16 bytes a lane instead of 8: half of the
-    // loops' cycles are reads of shared memory).
+    // loops' cycles are reads of shared memory). The parts of a row's sum meet in another order, no further off: error against 64 bits 7.2e-5
+    // by pieces, 7.1e-5 by halves, fp32 rows, 2 to 64 of them alike.
     constexpr uint32_t kHalves = GP == 8 && !AL ? 2 : 1;
     extern __shared__ __align__(128) uint8_t dsm_raw[];
     uint8_t* const dsm = dsm_raw + ((1024u - (smem_u32(dsm_raw) & 1023u)) & 1023u);   // the swizzle follows the address
