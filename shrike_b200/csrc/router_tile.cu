@@ -27,6 +27,7 @@ struct TileGeom {
     static constexpr uint32_t kRows = kWarpRows * WR, kTokens = kWarpTokens * WT, kThreads = WR * WT * 32;
     static constexpr uint32_t kWRow = BITS == 0 ? kK * 4 : kK * BITS / 8;      // bytes of a row's stage
     static constexpr uint32_t kXRow = DT == SHRIKE_DTYPE_FP32 ? kK * 4 : kK * 2;
+    static constexpr uint32_t kGates = BITS == 0 && DT != SHRIKE_DTYPE_FP32 ? 4 : 1;   // blocks of the gate row, rows of one stage
     static constexpr uint32_t kW = kRows * kWRow, kBuf = kW + kTokens * kXRow;
     static constexpr uint32_t kSb = BITS ? kRows * (kRouterMaxChunks * 2) * 8 : 0;   // {scale, bias} of the block's rows, fp32
     static constexpr uint32_t kSmem = kBufs * kBuf + kSb;
@@ -117,7 +118,7 @@ __device__ __forceinline__ void store_tile(const RouterArgs& a, float (&v)[TW * 
 
 }  // namespace
 
-// grid (row tiles, and one more for the gate row, token tiles)
+// grid (row tiles, and one or more for the gate row, token tiles)
 template <int BITS, int DT, int RW, int TW, int WR, int WT>
 __global__ void __launch_bounds__(WR * WT * 32, RW * TW == 128 ? 8 / (WR * WT) : 1) router_tile_kernel(const RouterArgs a) {
     using G = TileGeom<BITS, DT, RW, TW, WR, WT>;
@@ -130,12 +131,16 @@ __global__ void __launch_bounds__(WR * WT * 32, RW * TW == 128 ? 8 / (WR * WT) :
     const uint32_t e0 = blockIdx.x * G::kRows, t0 = blockIdx.y * G::kTokens;
     if (e0 >= a.ne) {
         // The shared expert's scalar gate: a warp per token at a time, the gate row in registers. (As a kernel of its own it took
-        // 9 us of 4096 rows; only where rows are short and a warp has eight was that the faster way: 512 rows of 256 columns, 256 experts,
-        // the whole router 9.1 us, so 10.9. Two rows beside each other here: 9.7, and up to 14 % more at other sizes.)
+        // 9 us of 4096 rows.)
         const uint32_t chunks = a.d / 4;
         float4 wr[kRouterMaxChunks];
         load_row_f32<kRouterMaxChunks, true>(a.gate_row, chunks, lane, wr);
-        for (uint32_t tk = t0 + warp; tk < min(a.T, t0 + G::kTokens); tk += WR * WT) {
+        uint32_t first = t0, share = G::kTokens;
+        if (G::kGates > 1 && a.d <= kK) {
+            share /= G::kGates;
+            first += (blockIdx.x - (a.ne + G::kRows - 1) / G::kRows) * share;
+        }
+        for (uint32_t tk = first + warp; tk < min(a.T, first + share); tk += WR * WT) {
             const void* xrow = (const uint8_t*)a.hidden + (size_t)tk * a.stride * kXB;
             const float acc = butterfly_sum(lane_dot_f32<kRouterMaxChunks, true>(wr, chunks, lane, xrow, DT, nullptr));
             if (lane == 0) a.gate_out[tk] = sigmoid_det(acc);
@@ -295,7 +300,12 @@ cudaError_t launch_tile(const shrike_moe* m, cudaStream_t st, const RouterArgs& 
     auto k = router_tile_kernel<BITS, DT, RW, TW, WR, WT>;
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::kSmem);
     if (e != cudaSuccess) return e;
-    return launch_after(m, st, k, dim3((a.ne + G::kRows - 1) / G::kRows + (a.gate_row ? 1u : 0u), (a.T + G::kTokens - 1) / G::kTokens), G::kThreads,
+    // Blocks of the gate row for a token tile: of rows of one stage a call waits for the block whose warps have eight tokens each (256
+    // experts of 256 columns, 512 rows: 10.7 us, with four blocks 8.8; 64 rows 5.9, 4.9; 4096 rows 31.9, 29.8). Longer rows, and those whose
+    // tiles take longer, do not wait for it, and four cost them up to a fifth (int8 rows of 256 columns, fp32 activations, 512 rows 10.2, 12.2;
+    // 2048 columns, bf16, 20.5, 22.5).
+    const uint32_t gates = !a.gate_row ? 0u : a.d <= kK ? G::kGates : 1u;
+    return launch_after(m, st, k, dim3((a.ne + G::kRows - 1) / G::kRows + gates, (a.T + G::kTokens - 1) / G::kTokens), G::kThreads,
                         G::kSmem, a);
 }
 
